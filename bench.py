@@ -475,6 +475,7 @@ def run_gb300(args, rank, world):
                     "pair_kernel_ms_avg": k_ms / max(k_n, 1), "pair_kernel_launches": k_n,
                     "path": path}
 
+        ctx64.set_fp64_pair_list(False)  # this leg sweeps the cells
         fp64 = fp64_run(ctx64, "B1: FP64 cell-stencil pair sweep (27 cells per bead), "
                         "Lanczos(24) every step, err1 check every term, one RHS, no graphs",
                         args.fp64_steps)

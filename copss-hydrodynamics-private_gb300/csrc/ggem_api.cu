@@ -138,6 +138,49 @@ int upload_stencil(ggem_ctx *c) {
                    cudaMemcpyHostToDevice);
     if (e) return cuda_fail(c, e, "stencil upload");
   }
+  if (c->prm.nb_mode == GGEM_NB_REFERENCE) {
+    // the stencil with its own element as runs (dy, dz, first dx, last dx):
+    // the particles of a run of elements along x are consecutive slots
+    std::vector<int4> st = c->stencil;
+    st.push_back(make_int4(0, 0, 0, 0));
+    std::sort(st.begin(), st.end(), [](const int4 &a, const int4 &b) {
+      return a.z != b.z ? a.z < b.z : (a.y != b.y ? a.y < b.y : a.x < b.x);
+    });
+    std::vector<int4> runs;
+    for (const int4 &o : st) {
+      if (!runs.empty() && runs.back().x == o.y && runs.back().y == o.z &&
+          runs.back().w + 1 == o.x)
+        runs.back().w = o.x;
+      else
+        runs.push_back(make_int4(o.y, o.z, o.x, o.x));
+    }
+    if ((e = c->d_runs.ensure(runs.size())) ||
+        (e = cudaMemcpy(c->d_runs.p, runs.data(), sizeof(int4) * runs.size(),
+                        cudaMemcpyHostToDevice)))
+      return cuda_fail(c, e, "stencil runs");
+    c->n_runs = (int)runs.size();
+  }
+  if (c->prm.precision == GGEM_FP64) {
+    // the largest r^2 of a listed pair: rc^2, or the far corners of the
+    // stencil's elements
+    double s_max = c->rc2;
+    for (const int4 &o : c->stencil) {
+      if (c->prm.nb_mode != GGEM_NB_REFERENCE) break;
+      const int v[3] = {std::abs(o.x), std::abs(o.y), std::abs(o.z)};
+      double s = 0.0;
+      for (int d = 0; d < 3; ++d) s += (v[d] + 1.0) * (v[d] + 1.0) * c->grid.h[d] * c->grid.h[d];
+      s_max = std::max(s_max, s);
+    }
+    if (c->prm.nb_mode == GGEM_NB_REFERENCE)  // (a stencil of the own element alone)
+      for (int d = 0; d < 3; ++d) s_max += c->grid.h[d] * c->grid.h[d];
+    std::vector<double4_32a> rec;
+    fit_tensor_f64(c->cst, s_max * (1.0 + 1e-9), rec, &c->t64);
+    if ((e = c->tab64.ensure(rec.size())) ||
+        (e = cudaMemcpy(c->tab64.p, rec.data(), sizeof(double4_32a) * rec.size(),
+                        cudaMemcpyHostToDevice)))
+      return cuda_fail(c, e, "FP64 tensor");
+    c->t64.rec = c->tab64.p;
+  }
   // FP32 cell shift per entry code (cut-off mode only: codes < kMaxCode)
   std::vector<float4> sh(kMaxCode, make_float4(0.f, 0.f, 0.f, 0.f));
   if (c->prm.nb_mode == GGEM_NB_CUTOFF) {
@@ -399,6 +442,7 @@ static int set_particles_common(ggem_ctx *ctx, int64_t n, const double *xyz, boo
   ctx->cells_built = false;
   ctx->list_built = false;
   ctx->list_unchecked = false;  // the pending statistics describe the old positions
+  ctx->f64_skip = false;
   return GGEM_OK;
 }
 
@@ -428,7 +472,14 @@ extern "C" int ggem_build_cells(ggem_ctx *ctx) {
   // checks then share the list's single host readback
   const bool cutoff = ctx->prm.nb_mode == GGEM_NB_CUTOFF;
   const bool fp32 = ctx->prm.precision == GGEM_FP32;
-  const bool with_list = cutoff && (fp32 || ctx->f64_list);
+  if (!fp32 && ctx->f64_list < 0) {
+    // the FP64 path's own list, from the second configuration on that the
+    // operator is applied to (contexts that only spread never pay for it)
+    ctx->f64_skip = false;
+    if (int rc = build_cells(ctx, ctx->f64_wanted)) return rc;
+    return ctx->f64_wanted ? ensure_f64_list(ctx, true) : GGEM_OK;
+  }
+  const bool with_list = cutoff && (fp32 || ctx->f64_list > 0);
   if (int rc = build_cells(ctx, with_list)) return rc;
   if (with_list) {
     if (int rc = build_pair_list(ctx)) return rc;
@@ -441,7 +492,7 @@ static int require_built(ggem_ctx *ctx) {
   if (int rc = settle_list(ctx)) return rc;
   if (!ctx->cells_built)
     return fail(ctx, GGEM_ERR_BAD_ARG, "call ggem_build_cells after setting particles");
-  if ((ctx->prm.precision == GGEM_FP32 || ctx->f64_list) && !ctx->list_built)
+  if ((ctx->prm.precision == GGEM_FP32 || ctx->f64_list > 0) && !ctx->list_built)
     return fail(ctx, GGEM_ERR_BAD_ARG, "pair list not built");
   return GGEM_OK;
 }

@@ -562,6 +562,111 @@ __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
   }
 }
 
+// Element lists (reference mode) as pair-list rows: one warp per target slot,
+// one lane per run of stencil elements along x.  The particles of a run are
+// one or (across a periodic face) two ranges of consecutive slots, every one
+// of them a neighbour (the list has no distance test), so a lane's count is
+// two subtractions, a warp scan places the runs and each lane writes its own.
+// ~110 runs instead of ~1000 elements per target at the h <= 1.414 mesh rule,
+// and once per configuration instead of once per operator application.
+constexpr int kRunWarps = 8;
+
+__global__ void __launch_bounds__(32 * kRunWarps) k_run_list(
+    int64_t n, Grid g, const int4 *__restrict__ runs, int nruns,
+    const int32_t *__restrict__ start, const float4 *__restrict__ pos32, int W,
+    int32_t *__restrict__ count, uint32_t *__restrict__ list,
+    unsigned long long *__restrict__ stat, int *__restrict__ err) {
+  __shared__ int s_tot[kRunWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t s = blockIdx.x * (int64_t)kRunWarps + warp;
+  int total = 0;
+  if (s < n) {
+    const int32_t cid = __float_as_int(pos32[s].w);
+    const int cx = cid % g.nc[0], cy = (cid / g.nc[0]) % g.nc[1], cz = cid / (g.nc[0] * g.nc[1]);
+    uint32_t *row = list + s * (int64_t)W;
+    for (int r0 = 0; r0 < nruns; r0 += 32) {
+      const int r = r0 + lane;
+      int32_t b0 = 0, e0 = 0, b1 = 0, e1 = 0;
+      bool own = false;
+      if (r < nruns) {
+        const int4 o = runs[r];
+        own = o.x == 0 && o.y == 0;
+        int y = cy + o.x, z = cz + o.y;
+        bool ok = true;
+        if (y < 0 || y >= g.nc[1]) {
+          if (g.periodic[1]) y += y < 0 ? g.nc[1] : -g.nc[1];
+          else ok = false;
+        }
+        if (z < 0 || z >= g.nc[2]) {
+          if (g.periodic[2]) z += z < 0 ? g.nc[2] : -g.nc[2];
+          else ok = false;
+        }
+        if (ok) {
+          const int nx = g.nc[0];
+          const int32_t *st = start + (int64_t)nx * (y + (int64_t)g.nc[1] * z);
+          int a = cx + o.z, b = cx + o.w;
+          if (!g.periodic[0]) {
+            a = max(a, 0);
+            b = min(b, nx - 1);
+            if (a <= b) {
+              b0 = st[a];
+              e0 = st[b + 1];
+            }
+          } else {
+            // offsets lie in (-nx, nx) and a run has at most nx elements
+            if (b < 0) a += nx, b += nx;
+            else if (a >= nx) a -= nx, b -= nx;
+            const int lo = max(a, 0), hi = min(b, nx - 1);
+            b0 = st[lo];
+            e0 = st[hi + 1];
+            if (a < 0) {
+              b1 = st[a + nx];
+              e1 = st[nx];
+            } else if (b >= nx) {
+              b1 = st[0];
+              e1 = st[b - nx + 1];
+            }
+          }
+        }
+      }
+      // the own run holds the target itself, which is no neighbour
+      const int cnt = (e0 - b0) + (e1 - b1) - (own ? 1 : 0);
+      int incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      int at = total + incl - cnt;
+      for (int32_t t = b0; t < e0; ++t)
+        if (t != s) {
+          if (at < W) row[at] = (uint32_t)t << kCodeBits;
+          ++at;
+        }
+      for (int32_t t = b1; t < e1; ++t)
+        if (t != s) {
+          if (at < W) row[at] = (uint32_t)t << kCodeBits;
+          ++at;
+        }
+      total += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) count[s] = min(total, W);  // the full length goes to stat
+  }
+  if (lane == 0) s_tot[warp] = total;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long sum = 0;
+    int longest = 0;
+    for (int w = 0; w < kRunWarps; ++w) {
+      sum += (unsigned long long)s_tot[w];
+      longest = max(longest, s_tot[w]);
+    }
+    atomicAdd(&stat[0], sum);
+    atomicMax(&stat[1], (unsigned long long)longest);
+    if (longest > W) atomicOr(err, kErrListCapacity);
+  }
+}
+
 }  // namespace
 
 int device_exclusive_scan_i32(ggem_ctx *c, const int32_t *in, int32_t *out, int64_t n) {
@@ -649,6 +754,12 @@ int cell_flag_error(ggem_ctx *c, int flags) {
 }
 
 void launch_pair_list(ggem_ctx *c, int nst, int W, cudaStream_t st) {
+  if (c->prm.nb_mode == GGEM_NB_REFERENCE) {
+    k_run_list<<<(unsigned)((c->n + kRunWarps - 1) / kRunWarps), 32 * kRunWarps, 0, st>>>(
+        c->n, c->grid, c->d_runs.p, c->n_runs, c->cell_start.p, c->pos32.p, W, c->nb_cnt.p,
+        c->nb_list.p, c->nb_stat.p, c->err.p);
+    return;
+  }
   k_pair_list_warp<<<(unsigned)c->grid.ncell, 32, 0, st>>>(
       c->grid, c->d_stencil.p, nst, c->d_shift.p, c->cell_start.p, c->pos32.p, c->pos64.p,
       c->rc2_lo, c->rc2_hi, c->rc2, W, c->nb_cnt.p, c->nb_list.p, c->nb_stat.p, c->err.p,
@@ -665,8 +776,8 @@ int build_pair_list(ggem_ctx *c) {
     // first build: twice the mean row length of a uniform suspension plus slack
     const Grid &g = c->grid;
     const double vol = g.L[0] * g.L[1] * g.L[2];
-    const double mean = vol > 0 ? (double)n / vol * 4.18879020478639 * c->rc2 * std::sqrt(c->rc2)
-                                : 0.0;
+    const double r = c->prm.nb_mode == GGEM_NB_REFERENCE ? c->search_radius_e : std::sqrt(c->rc2);
+    const double mean = vol > 0 ? (double)n / vol * 4.18879020478639 * r * r * r : 0.0;
     c->nb_w = (int)std::min<double>(((int64_t)(2.0 * mean) + 16 + 7) / 8 * 8, 1 << 20);
   }
   if (n == 0) {
@@ -676,7 +787,8 @@ int build_pair_list(ggem_ctx *c) {
     return GGEM_OK;
   }
   const int nst = (int)c->stencil.size();
-  if (nst > kMaxStencil) return fail(c, GGEM_ERR_BAD_ARG, "stencil too large for the list builder");
+  if (nst > kMaxStencil && c->prm.nb_mode != GGEM_NB_REFERENCE)
+    return fail(c, GGEM_ERR_BAD_ARG, "stencil too large for the list builder");
   if (c->defer_checks && c->list_checked_once) {
     // keep the width of the previous build; a longer row is stored clipped
     // (counts never exceed W) and found when the statistics are read
@@ -706,6 +818,13 @@ int build_pair_list(ggem_ctx *c) {
   c->list_stat_zero = false;
   for (int attempt = 0; attempt < 2; ++attempt) {
     const int W = c->nb_w;
+    // a list that only saves time leaves most of the memory to the caller
+    if (c->f64_list_is_own() && (size_t)n * W > c->nb_list.count) {
+      size_t avail = 0, all = 0;
+      if ((e = cudaMemGetInfo(&avail, &all))) return cuda_fail(c, e, "pair list");
+      if ((size_t)n * W * sizeof(uint32_t) > avail / 4)
+        return fail(c, GGEM_ERR_OOM, "pair list larger than a quarter of the free memory");
+    }
     if ((e = c->nb_list.ensure((size_t)n * W))) return cuda_fail(c, e, "pair list");
     if ((e = cudaMemsetAsync(c->nb_stat.p, 0, 2 * sizeof(unsigned long long), st)))
       return cuda_fail(c, e, "memset");
@@ -735,6 +854,46 @@ int build_pair_list(ggem_ctx *c) {
     if ((e = cudaMemsetAsync(c->err.p, 0, sizeof(int), st))) return cuda_fail(c, e, "memset");
   }
   return fail(c, GGEM_ERR_CELL_OVERFLOW, "pair list rows exceeded their width twice");
+}
+
+bool stream_capturing(const ggem_ctx *c) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+int ensure_f64_list(ggem_ctx *c, bool flags_pending) {
+  if (c->prm.precision != GGEM_FP64 || c->f64_list >= 0 || c->list_built || c->f64_skip ||
+      c->n == 0)
+    return GGEM_OK;
+  cudaError_t e;
+  if (!flags_pending) {
+    // a list build waits for the device, which a capture cannot
+    if (stream_capturing(c)) return GGEM_OK;
+    // (the error word may hold bits of a point sum that have been reported)
+    if ((e = cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream)))
+      return cuda_fail(c, e, "memset");
+  }
+  c->f64_wanted = true;
+  const bool defer = c->defer_checks;
+  c->defer_checks = false;
+  const int rc = build_pair_list(c);
+  c->defer_checks = defer;
+  if (rc != GGEM_ERR_OOM && rc != GGEM_ERR_CELL_OVERFLOW) return rc;
+  // no room for this configuration's list: sweep its cells
+  c->f64_skip = true;
+  c->list_built = false;
+  c->nb_w = 0;
+  if (flags_pending) {
+    int flags = 0;
+    if (int frc = read_error_flags(c, &flags)) return frc;
+    if (int frc = cell_flag_error(c, flags)) return frc;
+  }
+  c->cells_built = true;
+  return GGEM_OK;
 }
 
 int enqueue_list_check(ggem_ctx *c) {

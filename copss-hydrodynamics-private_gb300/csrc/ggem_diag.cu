@@ -149,7 +149,7 @@ extern "C" int ggem_get_pair_count(const ggem_ctx *ctx, int64_t *count) {
   if (!ctx || !count) return GGEM_ERR_BAD_ARG;
   // reading pending statistics of a deferred build updates only cached state
   if (int rc = settle_list(const_cast<ggem_ctx *>(ctx))) return rc;
-  if (!ctx->list_built) return GGEM_ERR_BAD_ARG;
+  if (!ctx->list_built || ctx->f64_list_is_own()) return GGEM_ERR_BAD_ARG;
   *count = ctx->n_pairs;
   return GGEM_OK;
 }
@@ -157,7 +157,7 @@ extern "C" int ggem_get_pair_count(const ggem_ctx *ctx, int64_t *count) {
 extern "C" int ggem_get_pair_storage(const ggem_ctx *ctx, int *row_width, int *tensors_stored) {
   if (!ctx || !row_width || !tensors_stored) return GGEM_ERR_BAD_ARG;
   if (int rc = settle_list(const_cast<ggem_ctx *>(ctx))) return rc;
-  if (!ctx->list_built) return GGEM_ERR_BAD_ARG;
+  if (!ctx->list_built || ctx->f64_list_is_own()) return GGEM_ERR_BAD_ARG;
   *row_width = ctx->nb_w;
   *tensors_stored = ctx->pretensor_ok ? 1 : 0;
   return GGEM_OK;
@@ -167,7 +167,7 @@ extern "C" int ggem_set_fp64_pair_list(ggem_ctx *ctx, int enable) {
   if (!ctx) return GGEM_ERR_BAD_ARG;
   if (ctx->prm.precision != GGEM_FP64 || ctx->prm.nb_mode != GGEM_NB_CUTOFF)
     return ggem::fail(ctx, GGEM_ERR_BAD_ARG, "the FP64 pair list needs a GGEM_FP64 cutoff context");
-  ctx->f64_list = enable != 0;
+  ctx->f64_list = enable ? 1 : 0;
   ctx->cells_built = false;  // the next ggem_build_cells builds (or drops) the list
   ctx->list_built = false;
   return GGEM_OK;

@@ -52,6 +52,20 @@ struct DevConsts {
   double ksi, two_ksi_sqrt_pi, coeff_2, r_eps;
 };
 
+// The local tensor G = A(s) I + B(s) x x^T, s = r^2, in FP64 as piecewise
+// quintics: [0, s0) is one piece, above it every octave of s has
+// 2^kTab64Sub equal pieces, so a piece is found from the top bits of s and
+// the expansion variable is s minus the piece's midpoint (one FP64
+// subtraction).  Record: (A0, B0, A1, B1), (A2, B2, A3, B3), (A4, B4, A5, B5).
+struct Tensor64 {
+  const double4_32a *rec;
+  int base;    // (high word of s >> (20 - kTab64Sub)) - base = piece
+  int last;    // last piece (larger s is clamped: outside every list)
+  double mid0; // midpoint of the first piece
+};
+constexpr int kTab64Sub = 7;
+constexpr int kTab64Deg = 5;
+
 // uniform cell grid over the box (cells == elements in reference mode)
 struct Grid {
   double lo[3], L[3], h[3];
@@ -124,10 +138,21 @@ struct ggem_ctx {
   ggem::DevBuf<float4> pos32;
   ggem::DevBuf<int> err;
 
-  // FP32 pair list (built for GGEM_FP64 contexts too when f64_list is set:
-  // the FP64 pair kernel then walks the exact list instead of sweeping cells)
+  // FP32 pair list (built for GGEM_FP64 contexts too: the FP64 pair kernel
+  // then walks the exact list instead of sweeping cells).  f64_list: 1 = with
+  // every cell build, 0 = never, -1 (default) = by the first operator
+  // application after a cell build, and with the cell build itself once the
+  // context has applied its operator (f64_wanted); f64_skip: the current
+  // configuration's list does not fit (the cells are swept).
   bool list_built = false;
-  bool f64_list = false;
+  int f64_list = -1;
+  bool f64_wanted = false, f64_skip = false;
+  // the list is the FP64 path's own (default mode), not one the caller asked for
+  bool f64_list_is_own() const { return prm.precision == GGEM_FP64 && f64_list != 1; }
+  ggem::DevBuf<int4> d_runs;  // reference mode: the stencil's runs along x
+  int n_runs = 0;
+  ggem::DevBuf<double4_32a> tab64;
+  ggem::Tensor64 t64{};
   // symmetric pair sums (ggem_set_symmetric_pairs): the list build also
   // writes the half list (each unordered pair once, in the row of its smaller
   // slot, same row width) and single-RHS FP32 matvecs evaluate each tensor
@@ -291,6 +316,10 @@ int fit_tensor_table(const ggem_constants &c, double s_max, int nt, std::vector<
                      double *max_err);
 int fit_tensor_poly(const ggem_constants &c, double s_max, float *a, float *b, float *x0,
                     float *x1, float *e_coef, double *max_err);
+// the FP64 piecewise tensor for s in [0, s_max] (records of three double4_32a
+// per piece); base, last and mid0 of *t are set, rec is the caller's
+void fit_tensor_f64(const ggem_constants &c, double s_max, std::vector<double4_32a> &rec,
+                    Tensor64 *t);
 bool tensor_b_nonnegative(const ggem_constants &c, double s_max);
 void tridiag_extremes(int k, const double *a, const double *b, double *lmin, double *lmax);
 void cheb_coeffs_host(int N, double da, double db, int method, double *coef);
@@ -302,6 +331,12 @@ void cheb_coeffs_host_many(int N, int K, const double *da, const double *db, int
 int build_cells(ggem_ctx *c, bool defer_flags = false);
 int cell_flag_error(ggem_ctx *c, int flags);
 int build_pair_list(ggem_ctx *c);
+// GGEM_FP64 contexts in the default list mode: build the list of the current
+// cells if there is none yet.  Returns GGEM_OK without a list where it does
+// not fit or the stream is being captured (the caller sweeps the cells).
+// flags_pending: the cell build's error word has not been read yet.
+int ensure_f64_list(ggem_ctx *c, bool flags_pending = false);
+bool stream_capturing(const ggem_ctx *c);
 // deferred builds: copy the list statistics and the error word to the host
 // mirror (asynchronous), then, after the stream has synchronised, evaluate
 // them; *rebuilt is set when the rows had overflowed and the list (and the

@@ -6,8 +6,9 @@
 // self term of PMSystemStokes::compute_point_velocity (pm_system_stokes.C:446-455).
 //
 // Two arithmetic paths:
-//  * FP64 ("plain"): one thread per target slot sweeps the neighbour cells of
-//    the stencil, minimum image and cut-off in FP64, erf/exp per pair.
+//  * FP64: groups of lanes walk the target's row of the pair list, minimum
+//    image and tensor (piecewise quintics in r^2) in FP64; without a list one
+//    thread per target slot sweeps the neighbour cells of the stencil.
 //  * FP32: groups of kGroup lanes share one target and walk its cached CSR
 //    pair list (consecutive entries, so the gathered sources of a group sit
 //    in the same cells).  The displacement is formed from cell-relative
@@ -21,6 +22,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 
 #include "ggem_ff.cuh"
 #include "ggem_internal.cuh"
@@ -44,25 +47,6 @@ __device__ __forceinline__ void min_image(const Grid &g, double d[3]) {
   }
 }
 
-// green_tensor_local_regularized applied to f: G f = k[(c1+c2) f + (c1-c2)(x.f/r^2) x]
-__device__ __forceinline__ void green_apply64(const DevConsts &K, const double x[3], double r,
-                                              const double f[3], double out[3]) {
-  if (r < K.r_eps) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) out[a] = K.coeff_2 * f[a];
-    return;
-  }
-  const double r2 = r * r;
-  const double kr = K.ksi * r, kr2 = kr * kr;
-  const double ar = K.alpha * r, ar2 = ar * ar;
-  const double c1 = (erf(kr) - erf(ar)) / r;
-  const double c2 = K.two_ksi_sqrt_pi * exp(-kr2) - K.two_alpha_sqrt_pi * exp(-ar2);
-  const double xf = (x[0] * f[0] + x[1] * f[1] + x[2] * f[2]) / r2;
-  const double p = (c1 + c2) * K.one_eight_pi_mu, m = (c1 - c2) * xf * K.one_eight_pi_mu;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) out[a] = p * f[a] + m * x[a];
-}
-
 __device__ __forceinline__ void self_term(const DevConsts &K, int self_mode, const double f[3],
                                           double u[3]) {
   if (self_mode == GGEM_SELF_BEAD) {
@@ -74,18 +58,77 @@ __device__ __forceinline__ void self_term(const DevConsts &K, int self_mode, con
   }
 }
 
+// minimum image of one axis (pm_periodic_boundary.C:350-374: d <= -L/2 adds
+// L, d > L/2 subtracts it) with the comparisons on the bit patterns: an FP64
+// comparison costs as much of the FP64 pipe as an addition, an integer one
+// nothing of it.  half: the bits of L/2, or of infinity on an open axis;
+// wrapped positions keep |d| < L, so one shift suffices.
+struct MinImage {
+  long long half[3], L[3];
+};
+
+__device__ __forceinline__ double min_image_bits(double d, long long half, long long L) {
+  const long long b = __double_as_longlong(d);
+  const long long sign = b & (long long)0x8000000000000000ull;
+  const long long mag = b ^ sign;
+  const bool out = mag + (sign ? 1 : 0) > half;
+  // +L for a negative d, -L for a positive one, +0 inside
+  const long long w = out ? (L | (sign ^ (long long)0x8000000000000000ull)) : 0ll;
+  return d + __longlong_as_double(w);
+}
+
+// one 256-bit read-only load
+__device__ __forceinline__ double4_32a ld_f64x4(const double4_32a *p) {
+  double4_32a v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+      : "l"(p));
+  return v;
+}
+
+// The FP64 tensor of a pair (Tensor64): ten fused multiply-adds and one
+// subtraction on the FP64 pipe, against ~230 instructions for a square root,
+// two divisions, two erf and two exp.  eps2: the bits of r_eps^2, below
+// which the tensor is coeff_2 I (ggem_stokes.C:304-357).
+__device__ __forceinline__ void tensor64(const Tensor64 &T, double s, long long eps2,
+                                         double coeff_2, double &A, double &B) {
+  const int hi = __double2hiint(s);
+  const int idx = min(max((hi >> (20 - kTab64Sub)) - T.base, 0), T.last);
+  const double4_32a *r = T.rec + 3 * idx;
+  const double4_32a r2 = ld_f64x4(r + 2), r1 = ld_f64x4(r + 1), r0 = ld_f64x4(r);
+  constexpr int low = (1 << (20 - kTab64Sub)) - 1;
+  const double mid = __hiloint2double((hi & ~low) | ((low + 1) >> 1), 0);
+  const double t = s - (idx == 0 ? T.mid0 : mid);
+  A = fma(r2.z, t, r2.x);
+  B = fma(r2.w, t, r2.y);
+  A = fma(A, t, r1.z);
+  B = fma(B, t, r1.w);
+  A = fma(A, t, r1.x);
+  B = fma(B, t, r1.y);
+  A = fma(A, t, r0.z);
+  B = fma(B, t, r0.w);
+  A = fma(A, t, r0.x);
+  B = fma(B, t, r0.y);
+  const bool close = __double_as_longlong(s) < eps2;
+  A = close ? coeff_2 : A;
+  B = close ? 0.0 : B;
+}
+
 // FP64 plain sweep.  own_first: reference mode (own cell, then the element
 // stencil that excludes (0,0,0), no cut-off); otherwise the cut-off stencil.
+// Runs where there is no pair list (ggem_set_fp64_pair_list(0), no room for
+// one, or a first application under stream capture).
 template <int NR>
-__global__ void __launch_bounds__(128) k_matvec_f64(int64_t n, Grid g, DevConsts K,
+__global__ void __launch_bounds__(128) k_matvec_f64(int64_t n, Grid g, DevConsts K, Tensor64 T,
                                                     const int4 *__restrict__ stencil, int nst,
                                                     int own_first, int use_cutoff, double rc2,
+                                                    long long eps2,
                                                     const int32_t *__restrict__ start,
                                                     const double4_32a *__restrict__ pos64,
                                                     const float4 *__restrict__ pos32,
                                                     const double *__restrict__ f,
                                                     double *__restrict__ u, int self_mode,
-                                                    int nrhs_total, int r0) {
+                                                    int r0) {
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   const double4_32a pi = pos64[s];
@@ -119,16 +162,16 @@ __global__ void __launch_bounds__(128) k_matvec_f64(int64_t n, Grid g, DevConsts
                                      __dmul_rn(x[2], x[2]));
         if (!(r2c < rc2)) continue;
       }
-      const double r = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+      double A, B;
+      tensor64(T, fma(x[2], x[2], fma(x[1], x[1], x[0] * x[0])), eps2, K.coeff_2, A, B);
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
         const double *fj = f + (int64_t)(r0 + q) * vstride + 3 * (int64_t)t;
-        const double fv[3] = {fj[0], fj[1], fj[2]};
-        double g3[3];
-        green_apply64(K, x, r, fv, g3);
-        acc[q][0] += g3[0];
-        acc[q][1] += g3[1];
-        acc[q][2] += g3[2];
+        const double f0 = fj[0], f1 = fj[1], f2 = fj[2];
+        const double xf = B * fma(x[2], f2, fma(x[1], f1, x[0] * f0));
+        acc[q][0] = fma(A, f0, fma(xf, x[0], acc[q][0]));
+        acc[q][1] = fma(A, f1, fma(xf, x[1], acc[q][1]));
+        acc[q][2] = fma(A, f2, fma(xf, x[2], acc[q][2]));
       }
     }
   }
@@ -142,68 +185,65 @@ __global__ void __launch_bounds__(128) k_matvec_f64(int64_t n, Grid g, DevConsts
     ui[1] = acc[q][1];
     ui[2] = acc[q][2];
   }
-  (void)nrhs_total;
 }
 
-// FP64 pair sum over the exact pair list: only the in-cutoff pairs (the
-// list is the oracle's), the oracle's arithmetic per pair (minimum image of
-// the wrapped FP64 positions, pm_periodic_boundary.C:350-374, and
-// green_tensor_local_regularized with erf and exp in FP64,
-// ggem_stokes.C:304-357); the tensor's two coefficients are formed once per
-// pair and applied to NR right-hand sides.  kGroup lanes per target take
-// every kGroup-th entry of its row and add their sums by shuffles.
-template <int NR>
-__global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, Grid g, DevConsts K,
+// FP64 pair sum over the pair list (cut-off lists and element lists alike):
+// minimum image of the wrapped FP64 positions (pm_periodic_boundary.C:350-374)
+// and green_tensor_local_regularized (ggem_stokes.C:304-357) as its piecewise
+// quintic; the tensor's two coefficients are formed once per pair and applied
+// to NR right-hand sides.  G lanes per target take every G-th entry of its
+// row and add their sums by shuffles.
+//
+// Bound by the FP64 pipe (two lanes per SM and clock): 30 FP64 instructions
+// per pair and right-hand side pass (6 displacement, 3 r^2, 11 tensor, 10
+// product), which is 0.32 ms at N = 200k, phi = 0.1 (6.74 M pairs).
+// Measured there: 0.50 ms (the rest is lanes idle at the ends of rows of
+// uneven length), against 2.85 ms with erf and exp per pair and 15.0 ms for
+// the cell sweep.  The tensors themselves are closer to the exact ones than
+// the formula's: 1.2e-16 of u from their rounding against 3.8e-16 (N = 400,
+// 30-digit reference), since the closed form cancels.
+template <int NR, int G>
+__global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, MinImage mi, DevConsts K,
+                                                       Tensor64 T, long long eps2,
                                                        const int32_t *__restrict__ cnt, int W,
                                                        const uint32_t *__restrict__ list,
                                                        const double4_32a *__restrict__ pos64,
                                                        const double *__restrict__ f,
                                                        double *__restrict__ u, int self_mode,
                                                        int r0) {
-  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
-  const int sub = (int)(threadIdx.x % kGroup);
+  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  const int sub = (int)(threadIdx.x % G);
   const bool act = gid < n;
   const int64_t s = act ? gid : n - 1;
-  const double4_32a pi = pos64[s];
+  const double4_32a pi = ld_f64x4(pos64 + s);
   const int64_t vstride = 3 * n;
   double acc[NR][3];
 #pragma unroll
   for (int q = 0; q < NR; ++q) acc[q][0] = acc[q][1] = acc[q][2] = 0.0;
   const int m = act ? cnt[s] : 0;
   const uint32_t *row = list + s * (int64_t)W;
-  for (int k = sub; k < m; k += kGroup) {
-    const int64_t t = (int64_t)(__ldg(row + k) >> kCodeBits);
-    const double4_32a pj = pos64[t];
-    double x[3] = {pj.x - pi.x, pj.y - pi.y, pj.z - pi.z};
-    min_image(g, x);
-    const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-    const double r = sqrt(r2);
-    if (r < K.r_eps) {
-#pragma unroll
-      for (int q = 0; q < NR; ++q) {
-        const double *fj = f + (int64_t)(r0 + q) * vstride + 3 * t;
-        acc[q][0] += K.coeff_2 * fj[0];
-        acc[q][1] += K.coeff_2 * fj[1];
-        acc[q][2] += K.coeff_2 * fj[2];
-      }
-      continue;
-    }
-    const double kr = K.ksi * r, ar = K.alpha * r;
-    const double c1 = (erf(kr) - erf(ar)) / r;
-    const double c2 = K.two_ksi_sqrt_pi * exp(-kr * kr) - K.two_alpha_sqrt_pi * exp(-ar * ar);
-    const double p = (c1 + c2) * K.one_eight_pi_mu, mc = (c1 - c2) * K.one_eight_pi_mu / r2;
+  uint32_t nxt = sub < m ? __ldg(row + sub) : 0u;
+  for (int k = sub; k < m; k += G) {
+    const int64_t t = (int64_t)(nxt >> kCodeBits);
+    if (k + G < m) nxt = __ldg(row + k + G);
+    const double4_32a pj = ld_f64x4(pos64 + t);
+    const double x = min_image_bits(pj.x - pi.x, mi.half[0], mi.L[0]);
+    const double y = min_image_bits(pj.y - pi.y, mi.half[1], mi.L[1]);
+    const double z = min_image_bits(pj.z - pi.z, mi.half[2], mi.L[2]);
+    double A, B;
+    tensor64(T, fma(z, z, fma(y, y, x * x)), eps2, K.coeff_2, A, B);
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
       const double *fj = f + (int64_t)(r0 + q) * vstride + 3 * t;
-      const double f0 = fj[0], f1 = fj[1], f2 = fj[2];
-      const double xf = (x[0] * f0 + x[1] * f1 + x[2] * f2) * mc;
-      acc[q][0] += p * f0 + xf * x[0];
-      acc[q][1] += p * f1 + xf * x[1];
-      acc[q][2] += p * f2 + xf * x[2];
+      const double f0 = __ldg(fj), f1 = __ldg(fj + 1), f2 = __ldg(fj + 2);
+      const double xf = B * fma(z, f2, fma(y, f1, x * f0));
+      acc[q][0] = fma(A, f0, fma(xf, x, acc[q][0]));
+      acc[q][1] = fma(A, f1, fma(xf, y, acc[q][1]));
+      acc[q][2] = fma(A, f2, fma(xf, z, acc[q][2]));
     }
   }
 #pragma unroll
-  for (int o = 1; o < kGroup; o <<= 1)
+  for (int o = 1; o < G; o <<= 1)
 #pragma unroll
     for (int q = 0; q < NR; ++q)
 #pragma unroll
@@ -1336,25 +1376,53 @@ __global__ void k_from_slots(int64_t n, int nrhs, const int32_t *__restrict__ ra
   dst[2] = src[2];
 }
 
+MinImage min_image_of(const Grid &g) {
+  MinImage m;
+  for (int d = 0; d < 3; ++d) {
+    const double half = g.periodic[d] ? g.L[d] / 2.0 : INFINITY;
+    std::memcpy(&m.half[d], &half, 8);
+    std::memcpy(&m.L[d], &g.L[d], 8);
+  }
+  return m;
+}
+
+template <int NR, int G>
+void launch_list_f64(ggem_ctx *c, const double *f, double *u, int self_mode, int r0,
+                     long long eps2) {
+  const int64_t threads = c->n * G;
+  k_pair_list_f64<NR, G><<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(
+      c->n, min_image_of(c->grid), c->dc, c->t64, eps2, c->nb_cnt.p, c->nb_w, c->nb_list.p,
+      c->pos64.p, f, u, self_mode, r0);
+}
+
 template <int NR>
 int launch_f64(ggem_ctx *c, const double *f, double *u, int self_mode, int r0) {
-  if (c->f64_list && c->list_built) {
-    const int64_t threads = c->n * kGroup;
-    kt_start(c, kKPairF64);
-    k_pair_list_f64<NR><<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(
-        c->n, c->grid, c->dc, c->nb_cnt.p, c->nb_w, c->nb_list.p, c->pos64.p, f, u, self_mode,
-        r0);
+  long long eps2;
+  const double e2 = c->dc.r_eps * c->dc.r_eps;
+  std::memcpy(&eps2, &e2, 8);
+  kt_start(c, kKPairF64);
+  // (a caller's graph outlives this configuration: it holds the sweep, whose
+  // buffers depend on the particle count alone, not a list of this width)
+  if (c->list_built && !(c->f64_list_is_own() && stream_capturing(c))) {
+    // lanes per target: four fill the FP64 pipe from ~80k targets on (fewer
+    // lanes would idle in rows of ~35 entries of uneven length); smaller
+    // counts need more lanes to cover the latency of a row walk.  us per
+    // application with 4 / 8 / 16 / 32 lanes, phi = 0.1: N = 1000 (phi 0.05)
+    // 21 / 15 / 13 / 11, 4000 33 / 21 / 23 / 29, 12000 58 / 48 / 46 / 63,
+    // 60000 173 / 171 / 199 / 269, 200000 499 / 528 / 637 / 866
+    if (c->n >= 80000) launch_list_f64<NR, 4>(c, f, u, self_mode, r0, eps2);
+    else if (c->n >= 2500) launch_list_f64<NR, 8>(c, f, u, self_mode, r0, eps2);
+    else launch_list_f64<NR, 32>(c, f, u, self_mode, r0, eps2);
     kt_stop(c, kKPairF64);
     return check_launch(c, "matvec f64 list");
   }
   const int T = 128;
   const unsigned bn = (unsigned)((c->n + T - 1) / T);
   const bool ref = c->prm.nb_mode == GGEM_NB_REFERENCE;
-  kt_start(c, kKPairF64);
-  k_matvec_f64<NR><<<bn, T, 0, c->stream>>>(c->n, c->grid, c->dc, c->d_stencil.p,
+  k_matvec_f64<NR><<<bn, T, 0, c->stream>>>(c->n, c->grid, c->dc, c->t64, c->d_stencil.p,
                                              (int)c->stencil.size(), ref ? 1 : 0, ref ? 0 : 1,
-                                             c->rc2, c->cell_start.p, c->pos64.p, c->pos32.p, f,
-                                             u, self_mode, 0, r0);
+                                             c->rc2, eps2, c->cell_start.p, c->pos64.p,
+                                             c->pos32.p, f, u, self_mode, r0);
   kt_stop(c, kKPairF64);
   return check_launch(c, "matvec f64");
 }
@@ -1822,6 +1890,7 @@ double self_coefficient(const ggem_ctx *c, int self_mode) {
 int matvec_slots(ggem_ctx *c, int nrhs, const double *f, double *u, int self_mode) {
   if (c->n == 0) return GGEM_OK;
   if (c->prm.precision == GGEM_FP64) {
+    if (int rc = ensure_f64_list(c)) return rc;
     int r0 = 0;
     while (r0 < nrhs) {
       const int left = nrhs - r0;

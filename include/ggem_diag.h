@@ -42,10 +42,12 @@ int ggem_get_pair_storage(const ggem_ctx *ctx, int *row_width, int *tensors_stor
 /* allow (1, the default when B(s) >= 0 on [0, rc^2]) or forbid (0) stored
  * pair tensors; takes effect at the next ggem_build_cells */
 int ggem_set_pair_tensors(ggem_ctx *ctx, int enable);
-/* GGEM_FP64 cutoff contexts: 1 = build the exact pair list with the cells
- * and walk it in the FP64 pair kernel (only in-cutoff pairs, the
- * reference's FP64 arithmetic per pair); 0 (default) = sweep the 27 cells
- * around every bead.  Takes effect at the next ggem_build_cells. */
+/* GGEM_FP64 cutoff contexts: 1 = build the exact pair list with every
+ * ggem_build_cells (only in-cutoff pairs are visited); 0 = sweep the 27
+ * cells around every bead.  Takes effect at the next ggem_build_cells.
+ * Without this call the context builds the list itself for the
+ * configurations that the operator is applied to, where it takes at most a
+ * quarter of the free device memory. */
 int ggem_set_fp64_pair_list(ggem_ctx *ctx, int enable);
 /* GGEM_FP32 cutoff contexts: 1 = single-RHS matvecs with tensors evaluated
  * per pair use the symmetry G_ij = G_ji: the list build also writes the
