@@ -249,7 +249,8 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   uint32_t *mq = queue + warp * kSpQueue;
   float4 *mb = batch + warp * 32;
   const unsigned lt_mask = (1u << lane) - 1u;
-  for (int c0 = 0; c0 < total; c0 += CAP) {
+  // (a brick without particles in reach makes one empty pass: its sums are 0)
+  for (int c0 = 0; c0 == 0 || c0 < total; c0 += CAP) {
     const int cn = min(CAP, total - c0);
     // stage particles [c0, c0 + cn): segment by binary search
     for (int k = threadIdx.x; k < cn; k += kSpThreads) {

@@ -118,3 +118,27 @@ def test_spread_wide_stencil_compact_bitmap():
     rng = np.random.default_rng(6)
     L = 12 * 0.55
     _check((0, 0, 0), (L,) * 3, (12, 12, 12), (0, 0, 0), rng.uniform(0, L, (60, 3)), 5)
+
+
+@pytest.mark.parametrize("prec", [G.FP64, G.FP32])
+def test_spread_writes_zeros_where_no_particle_reaches(prec):
+    """one bead in the corner of a wide mesh: the points out of its reach get
+    0, whatever the output held before"""
+    import torch
+    nm, h = 40, 1.4
+    L = nm * h
+    q, nq = gauss_points((0, 0, 0), (L,) * 3, (nm,) * 3)
+    with G.Context(alpha=ALPHA, box_hi=(L,) * 3, periodic=(0, 0, 0), nb_mode=G.NB_REFERENCE,
+                   n_mesh=(nm,) * 3, search_radius_e=0.5 * h + 8.0 + 1e-3,
+                   precision=G.FP64) as ctx:
+        ctx.set_particles(np.array([[0.7, 0.7, 0.7]]))
+        ctx.build_cells()
+        ctx.set_quadrature(q, nq)
+        f = torch.ones(3, dtype=torch.float64, device="cuda")
+        rho = torch.full((len(q), 3), float("nan"), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.spread_elements_dev(f.data_ptr(), rho.data_ptr(), prec)
+        ctx.synchronize()
+        rho = rho.cpu().numpy()
+    assert np.all(rho[np.abs(q).max(axis=1) > 0.7 + 8.7 + 2 * h] == 0.0)
+    assert np.all(np.isfinite(rho)) and rho.max() > 0.0
