@@ -213,6 +213,15 @@ struct ggem_ctx {
   ggem::DevBuf<float4> q_rel;
   ggem::DevBuf<uint32_t> sp_bits;
   ggem::DevBuf<unsigned long long> sp_pairs;
+  // the points as a tensor grid (q_grid): points per element and axis, the
+  // axis coordinates, the point of each (row, index along x); the spread's
+  // per-particle axis factors
+  bool q_grid = false;
+  int q_p[3] = {0, 0, 0};
+  signed char q_map[32] = {0};
+  ggem::DevBuf<double> q_ax[3];
+  ggem::DevBuf<int> q_flag;
+  ggem::DevBuf<double2> sp_fac;
 
   // scan scratch (one per recursion level)
   std::vector<ggem::DevBuf<int64_t> *> scan_scratch;

@@ -27,7 +27,7 @@
 //
 // Two arithmetic paths over the same lists:
 //  * FP64: the oracle's arithmetic (minimum-image point_vector in FP64,
-//    exp in FP64);
+//    exp in FP64), factorised per axis where the points form a tensor grid;
 //  * FP32: positions relative to the element centres (|x| <= h/2), the
 //    element offset as an exact FP32 shift, e^{-alpha^2 s} on the
 //    special-function unit with the exponent split into hi + lo parts,
@@ -502,6 +502,361 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   }
 }
 
+// ---- separable FP64 spread -------------------------------------------------
+// On a mesh whose quadrature points form a tensor grid (every point's x
+// depends on its element column and an index alone, likewise y and z;
+// checked bit for bit when the points are set), the Gaussian factorises:
+// with h_d = alpha^2 d^2 and g_d = e^{-h_d} per axis,
+//   g_alpha = alpha^3 pi^{-3/2} g_x g_y g_z (2.5 - h_x - h_y - h_z).
+// k_axis_factors forms (g, h) of every particle at every axis coordinate of
+// its stencil window once (~80 exponentials per particle instead of one per
+// pair); k_spread_sep combines them: for a row of PX points along x,
+// F = (g_y g_z) f, w = (2.5 - h_y) - h_z and, per point, v = w g_x - g_x h_x
+// and three fused multiply-adds, i.e. 5 + 4 PX FP64 instructions per row and
+// member (6.5 per pair at 2 x 2 x 2 points) against ~50 with the minimum
+// image, r^2 and exp per pair.  GB300's FP64 pipe (two lanes per SM and
+// clock) bounds both; the products of three factors carry the rounding that
+// alpha^2 r^2 carried before.
+//
+// A brick of B^3 elements stages the particles that any of its elements
+// lists, each with its factors at the brick's B p coordinates per axis and
+// its force.  A lane owns one row of one element (E = 32 / R elements per
+// warp, R rows each) and walks the set bits of the element's member mask:
+// neighbouring elements list nearly the same particles, so the lanes stay
+// level without a reduction at the end.
+struct SepGeo {
+  int p[3];       // points per element and axis
+  int R, E;       // rows per element, elements per warp
+  int aoff[3];    // offset of an axis inside a particle's factors
+  int nfac;       // factors per particle (double2 each)
+  int stride;     // staged double2 per particle: B (px + py + pz) + 2
+  int cap, nw;    // staged particles per pass (a multiple of 32), mask words
+  signed char qmap[32];  // point index of (row, a)
+};
+
+// window[slot][axis][offset - lo][a] = (g, g h) on x, (g, 2.5 - h) on y,
+// (alpha^3 pi^{-3/2} g, h) on z; the offset is the particle's element minus
+// the point's, zero where that element lies outside an open axis
+__global__ void __launch_bounds__(256) k_axis_factors(
+    int64_t n, SpreadGeo sg, SepGeo sp, DevConsts K, const double *__restrict__ ax0,
+    const double *__restrict__ ax1, const double *__restrict__ ax2,
+    const float4 *__restrict__ pos32, const double4_32a *__restrict__ pos64,
+    double2 *__restrict__ fac) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= n * sp.nfac) return;
+  const int64_t s = t / sp.nfac;
+  const int r = (int)(t - s * sp.nfac);
+  const int d = r >= sp.aoff[2] ? 2 : (r >= sp.aoff[1] ? 1 : 0);
+  const int k = r - sp.aoff[d];
+  const int off = sg.lo[d] + k / sp.p[d], a = k % sp.p[d];
+  const int cid = __float_as_int(pos32[s].w);
+  const int nc0 = sg.g.nc[0], nc1 = sg.g.nc[1], nc = sg.g.nc[d];
+  int e = (d == 0 ? cid % nc0 : (d == 1 ? (cid / nc0) % nc1 : cid / (nc0 * nc1))) - off;
+  double2 v = make_double2(0.0, 0.0);
+  if (sg.g.periodic[d]) e = wrap_cell(e, nc);
+  if (e >= 0 && e < nc) {
+    const double4_32a P = pos64[s];
+    const double q = (d == 0 ? ax0 : (d == 1 ? ax1 : ax2))[e * sp.p[d] + a];
+    double x = (d == 0 ? P.x : (d == 1 ? P.y : P.z)) - q;
+    if (sg.g.periodic[d]) {  // minimum image (pm_periodic_boundary.C:350-374)
+      const double xs = sg.g.L[d];
+      if (x <= -xs / 2.0) x += xs;
+      if (x > xs / 2.0) x -= xs;
+    }
+    // h as a double and its remainder: e^{-h} would carry h times the
+    // rounding of h, and three factors make one Gaussian
+    const double x2 = x * x, h = K.alpha2 * x2;
+    const double lo = fma(K.alpha2, fma(x, x, -x2), fma(K.alpha2, x2, -h));
+    const double g0 = exp(-h), g = fma(-lo, g0, g0);
+    v = d == 0 ? make_double2(g, g * h)
+               : (d == 1 ? make_double2(g, 2.5 - h) : make_double2(K.alpha3_pi_23 * g, h));
+  }
+  fac[t] = v;
+}
+
+template <int PX, bool ANYFULL>
+__global__ void __launch_bounds__(kSpThreads, 2) k_spread_sep(
+    SpreadGeo sg, SepGeo sp, const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
+    const double *__restrict__ f_slot, const double2 *__restrict__ fac,
+    const uint32_t *__restrict__ bits, double *__restrict__ rho,
+    unsigned long long *__restrict__ pairs) {
+  extern __shared__ __align__(16) unsigned char sp_smem[];
+  double2 *stage = reinterpret_cast<double2 *>(sp_smem);  // [cap][stride]
+  uint32_t *mask = reinterpret_cast<uint32_t *>(stage + (size_t)sp.cap * sp.stride);  // [B^3][nw]
+  int2 *item = reinterpret_cast<int2 *>(mask + 64 * sp.nw);  // [cap] (slot, frame coordinates)
+  int32_t *seg_begin = reinterpret_cast<int32_t *>(item + sp.cap);
+  int32_t *seg_pre = seg_begin + kSpMaxSeg + 1;
+  uint32_t *s_bits = reinterpret_cast<uint32_t *>(seg_pre + kSpMaxSeg + 1);
+  __shared__ int wsum[kSpWarps];
+  __shared__ int s_next;
+  for (int k = threadIdx.x; k < sg.nwords; k += kSpThreads) s_bits[k] = bits[k];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int B = sg.B;
+  int bid = blockIdx.x;
+  const int bx = bid % sg.nb[0];
+  bid /= sg.nb[0];
+  const int e0[3] = {bx * B, (bid % sg.nb[1]) * B, (bid / sg.nb[1]) * B};
+  const int e1[3] = {min(e0[0] + B, sg.g.nc[0]), min(e0[1] + B, sg.g.nc[1]),
+                     min(e0[2] + B, sg.g.nc[2])};
+  Frame fr[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    fr[d] = brick_frame(sg, d, e0[d], e1[d]);
+    if (!ANYFULL) fr[d].full = 0;
+  }
+  // slot ranges of the dilated brick's rows along x (as in k_spread_brick)
+  const int nx = sg.g.nc[0];
+  const int xa = fr[0].F, xz = fr[0].F + fr[0].E - 1;
+  const int xaw = sg.g.periodic[0] ? wrap_cell(xa, nx) : xa;
+  const int nseg_x = (!fr[0].full && sg.g.periodic[0] && (xa < 0 || xz >= nx)) ? 2 : 1;
+  const int nseg = fr[1].E * fr[2].E * nseg_x;  // <= kSpMaxSeg (checked on the host)
+  int total = 0;
+  for (int s0 = 0; s0 < nseg; s0 += kSpThreads) {
+    const int s = s0 + threadIdx.x;
+    int b = 0, cnt = 0;
+    if (s < nseg) {
+      const int row = s / nseg_x, k = s - row * nseg_x;
+      int cy = fr[1].F + row % fr[1].E, cz = fr[2].F + row / fr[1].E;
+      if (sg.g.periodic[1]) cy = wrap_cell(cy, sg.g.nc[1]);
+      if (sg.g.periodic[2]) cz = wrap_cell(cz, sg.g.nc[2]);
+      int x0 = fr[0].full ? 0 : xaw, x1 = x0 + fr[0].E - 1;
+      if (nseg_x == 2) {
+        if (k == 0) x1 = nx - 1;
+        else x0 = 0, x1 = wrap_cell(xz, nx);
+      }
+      const int64_t rowc = (int64_t)nx * (cy + (int64_t)sg.g.nc[1] * cz);
+      b = start[rowc + x0];
+      cnt = start[rowc + x1 + 1] - b;
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int before = total;
+    for (int w = 0; w < kSpWarps; ++w) {
+      if (w < warp) before += wsum[w];
+      total += wsum[w];
+    }
+    if (s < nseg) {
+      seg_begin[s] = b;
+      seg_pre[s] = before + incl - cnt;
+    }
+    __syncthreads();
+  }
+  const int ebx = e1[0] - e0[0], eby = e1[1] - e0[1], ebz = e1[2] - e0[2];
+  const int nel = ebx * eby * ebz;
+  const int u0[3] = {fr[0].full ? e0[0] : e0[0] - fr[0].F, fr[1].full ? e0[1] : e0[1] - fr[1].F,
+                     fr[2].full ? e0[2] : e0[2] - fr[2].F};
+  // is a particle (frame coordinates u) listed by the element at frame
+  // coordinates (x, y, z)?
+  auto lists = [&](uint32_t u, int x, int y, int z) -> bool {
+    if (sg.pad) {
+      const int idx = (int)u - ((x + sg.lo[0] - B + 1) + 32 * (y + sg.lo[1] - B + 1) +
+                                1024 * (z + sg.lo[2] - B + 1));
+      return (s_bits[idx >> 5] >> (idx & 31)) & 1u;
+    }
+    const int ix = axis_offset(sg, 0, (int)(u & 31u), x, ANYFULL && fr[0].full) - sg.lo[0];
+    const int iy = axis_offset(sg, 1, (int)((u >> 5) & 31u), y, ANYFULL && fr[1].full) - sg.lo[1];
+    const int iz = axis_offset(sg, 2, (int)(u >> 10), z, ANYFULL && fr[2].full) - sg.lo[2];
+    if ((unsigned)ix >= (unsigned)sg.dim[0] || (unsigned)iy >= (unsigned)sg.dim[1] ||
+        (unsigned)iz >= (unsigned)sg.dim[2])
+      return false;
+    const int idx = (iz * sg.dim[1] + iy) * sg.dim[0] + ix;
+    return (s_bits[idx >> 5] >> (idx & 31)) & 1u;
+  };
+  unsigned long long my_pairs = 0;
+  bool first = true;
+  int c0 = 0;
+  do {
+    // the next particles that some element of the brick lists, in order, up
+    // to cap of them; s_next: the candidate where the next pass resumes
+    int kept = 0;
+    while (c0 < total && kept < sp.cap) {
+      const int v = c0 + threadIdx.x;
+      bool in = v < total;
+      int2 it = make_int2(0, 0);
+      if (in) {
+        int lo = 0, hi = nseg - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (seg_pre[mid] <= v) lo = mid;
+          else hi = mid - 1;
+        }
+        const int slot = seg_begin[lo] + (v - seg_pre[lo]);
+        const int row = lo / nseg_x, kk = lo - row * nseg_x;
+        const int cx = __float_as_int(pos32[slot].w) % nx;
+        int ux = cx;
+        if (!fr[0].full) ux = cx - xaw + (kk == 1 ? nx : 0);
+        it = make_int2(slot, ux | ((row % fr[1].E) << 5) | ((row / fr[1].E) << 10));
+        in = false;
+        for (int z = 0; z < ebz && !in; ++z)
+          for (int y = 0; y < eby && !in; ++y)
+            for (int x = 0; x < ebx && !in; ++x)
+              in = lists((uint32_t)it.y, u0[0] + x, u0[1] + y, u0[2] + z);
+      }
+      const unsigned bal = __ballot_sync(0xffffffffu, in);
+      if (lane == 0) wsum[warp] = __popc(bal);
+      if (threadIdx.x == 0) s_next = min(c0 + kSpThreads, total);
+      __syncthreads();
+      int at = kept, found = kept;
+      for (int w = 0; w < kSpWarps; ++w) {
+        if (w < warp) at += wsum[w];
+        found += wsum[w];
+      }
+      at += __popc(bal & lt_mask);
+      if (in && at < sp.cap) item[at] = it;
+      if (in && at == sp.cap) s_next = v;  // the first one without room
+      __syncthreads();
+      kept = min(found, sp.cap);
+      c0 = s_next;
+      __syncthreads();
+    }
+    // stage the kept particles: one warp per particle, one lane per factor
+    for (int r = lane; r < sp.stride; r += 32) {
+      const int nfx = B * sp.p[0], nfy = nfx + B * sp.p[1], nfz = nfy + B * sp.p[2];
+      const int d = r >= nfz ? 3 : (r >= nfy ? 2 : (r >= nfx ? 1 : 0));
+      const int k = r - (d == 3 ? nfz : (d == 2 ? nfy : (d == 1 ? nfx : 0)));
+      const int pd = d < 3 ? sp.p[d] : 1;
+      const int a = k % pd, ue = d < 3 ? u0[d] + k / pd : 0;
+      for (int p = warp; p < kept; p += kSpWarps) {
+        const int2 it = item[p];
+        double2 v = make_double2(0.0, 0.0);
+        if (d == 3) {
+          const double *fp = f_slot + 3 * (int64_t)it.x;
+          v = k == 0 ? make_double2(fp[0], fp[1]) : make_double2(fp[2], 0.0);
+        } else {
+          const int i =
+              axis_offset(sg, d, (it.y >> (5 * d)) & 31, ue, ANYFULL && fr[d].full) - sg.lo[d];
+          if ((unsigned)i < (unsigned)sg.dim[d])
+            v = fac[(int64_t)it.x * sp.nfac + sp.aoff[d] + i * pd + a];
+        }
+        stage[p * sp.stride + r] = v;
+      }
+    }
+    __syncthreads();
+    const int nw = (kept + 31) >> 5;
+    for (int g = warp; g * sp.E < nel; g += kSpWarps) {
+      const int el0 = g * sp.E, ne = min(sp.E, nel - el0);
+      for (int q = 0; q < ne; ++q) {
+        const int le = el0 + q;
+        const int x = u0[0] + le % ebx, y = u0[1] + (le / ebx) % eby, z = u0[2] + le / (ebx * eby);
+        for (int w = 0; w < nw; ++w) {
+          const int k = 32 * w + lane;
+          const unsigned m = __ballot_sync(
+              0xffffffffu, k < kept && lists((uint32_t)item[min(k, kept - 1)].y, x, y, z));
+          if (lane == 0) mask[le * sp.nw + w] = m;
+          my_pairs += (unsigned long long)__popc(m);
+        }
+      }
+      __syncwarp();
+      const int q = lane / sp.R, row = lane - q * sp.R;
+      const bool act = q < ne;
+      const int le = el0 + (act ? q : 0);
+      const int lx = le % ebx, ly = (le / ebx) % eby, lz = le / (ebx * eby);
+      const int b = row % sp.p[1], c = row / sp.p[1];
+      const double2 *X = stage + lx * PX;
+      const double2 *Y = stage + B * PX + ly * sp.p[1] + b;
+      const double2 *Z = stage + B * (PX + sp.p[1]) + lz * sp.p[2] + c;
+      const double2 *Fp = stage + sp.stride - 2;
+      const uint32_t *mrow = mask + le * sp.nw;
+      // kAcc sums per point, members in turn: one sum over ~70 members
+      // rounds three times as much as the lanes of k_spread_brick did
+      constexpr int kAcc = PX == 1 ? 8 : (PX == 2 ? 6 : 3);
+      double acc[kAcc][PX][3];
+#pragma unroll
+      for (int u = 0; u < kAcc; ++u)
+#pragma unroll
+        for (int a = 0; a < PX; ++a) acc[u][a][0] = acc[u][a][1] = acc[u][a][2] = 0.0;
+      int w = 0;
+      uint32_t m = act && nw > 0 ? mrow[0] : 0u;
+      const int wend = act ? nw : 0;
+      bool more = true;
+      while (more) {
+#pragma unroll
+        for (int u = 0; u < kAcc; ++u) {
+          while (m == 0u && w + 1 < wend) m = mrow[++w];
+          const bool has = m != 0u;
+          more = __any_sync(0xffffffffu, has);
+          if (!more) break;
+          if (has) {
+            const int o = (32 * w + __ffs(m) - 1) * sp.stride;
+            m &= m - 1u;
+            const double2 gy = Y[o], gz = Z[o], f01 = Fp[o], f2 = Fp[o + 1];
+            const double gyz = gy.x * gz.x, wv = gy.y - gz.y;
+            const double F0 = gyz * f01.x, F1 = gyz * f01.y, F2 = gyz * f2.x;
+#pragma unroll
+            for (int a = 0; a < PX; ++a) {
+              const double2 gx = X[o + a];
+              const double v = fma(wv, gx.x, -gx.y);
+              acc[u][a][0] = fma(v, F0, acc[u][a][0]);
+              acc[u][a][1] = fma(v, F1, acc[u][a][1]);
+              acc[u][a][2] = fma(v, F2, acc[u][a][2]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 1; u < kAcc; ++u)
+#pragma unroll
+        for (int a = 0; a < PX; ++a)
+#pragma unroll
+          for (int d = 0; d < 3; ++d) acc[0][a][d] += acc[u][a][d];
+      if (act) {
+        const int64_t e = (e0[0] + lx) + (int64_t)nx * ((e0[1] + ly) +
+                                                        (int64_t)sg.g.nc[1] * (e0[2] + lz));
+#pragma unroll
+        for (int a = 0; a < PX; ++a) {
+          double *dst = rho + 3 * (e * sg.nq + sp.qmap[row * PX + a]);
+#pragma unroll
+          for (int d = 0; d < 3; ++d) dst[d] = first ? acc[0][a][d] : dst[d] + acc[0][a][d];
+        }
+      }
+      __syncwarp();  // the warp's masks are rebuilt
+    }
+    first = false;
+    __syncthreads();  // the staged particles are replaced
+  } while (c0 < total);
+  if (pairs && lane == 0 && my_pairs)
+    atomicAdd(pairs, my_pairs * (unsigned long long)sg.nq);
+}
+
+// axis tables of a tensor grid from the elements along each axis:
+// ax[e p + a] = coordinate d of point rep[a] of the axis's element e
+struct AxisMap {
+  signed char rep[3][32];  // a point with index a on the axis
+  signed char idx[3][32];  // the axis index of each point
+};
+
+__global__ void k_axis_table(int d, int nc, int64_t stride, int nq, int p, AxisMap m,
+                             const double *__restrict__ q, double *__restrict__ ax) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nc * p) return;
+  const int64_t e = t / p;
+  ax[t] = q[3 * (e * stride * nq + m.rep[d][t - (int)e * p]) + d];
+}
+
+// flag[0] |= 1 where a point is not bit for bit the grid's
+__global__ void k_check_grid(int64_t nqt, int nq, Grid g, int px, int py, int pz, AxisMap m,
+                             const double *__restrict__ q, const double *__restrict__ ax0,
+                             const double *__restrict__ ax1, const double *__restrict__ ax2,
+                             int *__restrict__ flag) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= nqt) return;
+  const int64_t e = t / nq;
+  const int k = (int)(t - e * nq);
+  const int ex = (int)(e % g.nc[0]), ey = (int)((e / g.nc[0]) % g.nc[1]),
+            ez = (int)(e / ((int64_t)g.nc[0] * g.nc[1]));
+  const bool same = q[3 * t] == ax0[ex * px + m.idx[0][k]] &&
+                    q[3 * t + 1] == ax1[ey * py + m.idx[1][k]] &&
+                    q[3 * t + 2] == ax2[ez * pz + m.idx[2][k]];
+  if (!same) atomicOr(flag, 1);
+}
+
 // quadrature points relative to their element centre (FP64 difference,
 // rounded once to FP32); w = 0
 __global__ void k_qp_rel(int64_t nqt, int nq, Grid g, const double *__restrict__ q,
@@ -611,6 +966,71 @@ int spread_geometry(ggem_ctx *c, SpreadGeo *sg) {
   return GGEM_OK;
 }
 
+// the separable FP64 spread; *done = false where the points are no tensor
+// grid that it takes, or its factors do not fit (the caller sums per pair)
+int spread_separable(ggem_ctx *c, const SpreadGeo &sg, bool any_full, const double *d_f_slot,
+                     double *d_rho, unsigned long long *d_pairs, bool *done) {
+  *done = false;
+  if (!c->q_grid) return GGEM_OK;
+  SepGeo sp;
+  std::memset(&sp, 0, sizeof(sp));
+  int at = 0;
+  sp.stride = 2;
+  for (int d = 0; d < 3; ++d) {
+    sp.p[d] = c->q_p[d];
+    sp.aoff[d] = at;
+    at += sp.p[d] * sg.dim[d];
+    sp.stride += sg.B * sp.p[d];
+  }
+  sp.nfac = at;
+  sp.R = sp.p[1] * sp.p[2];
+  sp.E = 32 / sp.R;
+  std::memcpy(sp.qmap, c->q_map, sizeof(sp.qmap));
+  // 80 KB of staged particles: with the tables, two blocks per SM
+  sp.cap = (int)std::min<size_t>(256, 80 * 1024 / (sp.stride * sizeof(double2))) / 32 * 32;
+  if (sp.cap < 32) return GGEM_OK;
+  sp.nw = sp.cap / 32;
+  cudaError_t e;
+  const size_t nf = (size_t)c->n * sp.nfac;
+  if (nf > c->sp_fac.count) {
+    size_t avail = 0, all = 0;
+    if ((e = cudaMemGetInfo(&avail, &all))) return cuda_fail(c, e, "spread factors");
+    if (nf * sizeof(double2) > avail / 4) return GGEM_OK;
+  }
+  if ((e = c->sp_fac.ensure(nf))) {
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "spread factors");
+    cudaGetLastError();
+    return GGEM_OK;
+  }
+  if (nf) {
+    k_axis_factors<<<(unsigned)((nf + 255) / 256), 256, 0, c->stream>>>(
+        c->n, sg, sp, c->dc, c->q_ax[0].p, c->q_ax[1].p, c->q_ax[2].p, c->pos32.p, c->pos64.p,
+        c->sp_fac.p);
+    if (int rc = check_launch(c, "spread factors")) return rc;
+  }
+  const size_t smem = (size_t)sp.cap * sp.stride * sizeof(double2) +
+                      64 * sp.nw * sizeof(uint32_t) + sp.cap * sizeof(int2) +
+                      2 * (kSpMaxSeg + 1) * sizeof(int32_t) + sg.nwords * sizeof(uint32_t);
+  const unsigned nblk = (unsigned)((int64_t)sg.nb[0] * sg.nb[1] * sg.nb[2]);
+  auto launch = [&](auto kernel) -> int {
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem)))
+      return cuda_fail(c, e, "spread attributes");
+    kernel<<<nblk, kSpThreads, smem, c->stream>>>(sg, sp, c->cell_start.p, c->pos32.p, d_f_slot,
+                                                  c->sp_fac.p, c->sp_bits.p, d_rho, d_pairs);
+    return GGEM_OK;
+  };
+  int rc;
+  switch (sp.p[0]) {
+    case 1: rc = any_full ? launch(k_spread_sep<1, true>) : launch(k_spread_sep<1, false>); break;
+    case 2: rc = any_full ? launch(k_spread_sep<2, true>) : launch(k_spread_sep<2, false>); break;
+    default: rc = any_full ? launch(k_spread_sep<3, true>) : launch(k_spread_sep<3, false>);
+  }
+  if (rc) return rc;
+  *done = true;
+  return check_launch(c, "spread bricks (separable)");
+}
+
 int spread_elements(ggem_ctx *c, int precision, const double *d_f_slot, double *d_rho,
                     unsigned long long *d_pairs) {
   SpreadGeo sg;
@@ -622,6 +1042,11 @@ int spread_elements(ggem_ctx *c, int precision, const double *d_f_slot, double *
   bool any_full = false;
   for (int d = 0; d < 3; ++d)
     any_full = any_full || (sg.g.periodic[d] && sg.B + sg.hi[d] - sg.lo[d] >= sg.g.nc[d]);
+  if (precision == GGEM_FP64) {
+    bool done = false;
+    if (int rc = spread_separable(c, sg, any_full, d_f_slot, d_rho, d_pairs, &done)) return rc;
+    if (done) return GGEM_OK;
+  }
   auto launch = [&](auto kernel) -> int {
     // (the attribute is per device; setting it costs microseconds)
     if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -655,6 +1080,60 @@ int quadrature_common(ggem_ctx *c, int nq) {
   if ((e = c->q_xyz.ensure(3 * nqt)) || (e = c->q_rel.ensure(nqt)))
     return cuda_fail(c, e, "quadrature buffers");
   c->q_per_elem = 0;
+  c->q_grid = false;
+  return GGEM_OK;
+}
+
+// do the points form a tensor grid of at most 3 points per element along x?
+// The first element gives the indices (a point's coordinate among the
+// distinct ones of its axis), the elements along each axis the coordinates;
+// then every point of the mesh is compared.
+int quadrature_grid(ggem_ctx *c, int nq) {
+  const Grid &g = c->grid;
+  double q0[96];
+  cudaError_t e = cudaMemcpyAsync(q0, c->q_xyz.p, sizeof(double) * 3 * nq, cudaMemcpyDeviceToHost,
+                                  c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e) return cuda_fail(c, e, "quadrature");
+  AxisMap m;
+  int p[3];
+  for (int d = 0; d < 3; ++d) {
+    p[d] = 0;
+    for (int k = 0; k < nq; ++k) {
+      int a = 0;
+      while (a < p[d] && q0[3 * m.rep[d][a] + d] != q0[3 * k + d]) ++a;
+      if (a == p[d]) m.rep[d][p[d]++] = (signed char)k;
+      m.idx[d][k] = (signed char)a;
+    }
+  }
+  if (p[0] > 3 || p[0] * p[1] * p[2] != nq) return GGEM_OK;
+  for (int k = 0; k < nq; ++k) c->q_map[k] = -1;
+  for (int k = 0; k < nq; ++k)
+    c->q_map[(m.idx[2][k] * p[1] + m.idx[1][k]) * p[0] + m.idx[0][k]] = (signed char)k;
+  for (int k = 0; k < nq; ++k)
+    if (c->q_map[k] < 0) return GGEM_OK;  // a point twice, another missing
+  int64_t stride = 1;
+  for (int d = 0; d < 3; ++d) {
+    if ((e = c->q_ax[d].ensure((size_t)g.nc[d] * p[d]))) return cuda_fail(c, e, "quadrature axes");
+    k_axis_table<<<(g.nc[d] * p[d] + 255) / 256, 256, 0, c->stream>>>(
+        d, g.nc[d], stride, nq, p[d], m, c->q_xyz.p, c->q_ax[d].p);
+    if (int rc = check_launch(c, "quadrature axes")) return rc;
+    stride *= g.nc[d];
+    c->q_p[d] = p[d];
+  }
+  if ((e = c->q_flag.ensure(1)) ||
+      (e = cudaMemsetAsync(c->q_flag.p, 0, sizeof(int), c->stream)))
+    return cuda_fail(c, e, "quadrature flag");
+  const int64_t nqt = g.ncell * nq;
+  k_check_grid<<<(unsigned)((nqt + 255) / 256), 256, 0, c->stream>>>(
+      nqt, nq, g, p[0], p[1], p[2], m, c->q_xyz.p, c->q_ax[0].p, c->q_ax[1].p, c->q_ax[2].p,
+      c->q_flag.p);
+  if (int rc = check_launch(c, "quadrature grid")) return rc;
+  int flag = 1;
+  e = cudaMemcpyAsync(&flag, c->q_flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e) return cuda_fail(c, e, "quadrature");
+  c->q_grid = flag == 0;
   return GGEM_OK;
 }
 
@@ -663,8 +1142,7 @@ int quadrature_finish(ggem_ctx *c, int nq) {
   k_qp_rel<<<(unsigned)((nqt + 255) / 256), 256, 0, c->stream>>>(nqt, nq, c->grid, c->q_xyz.p,
                                                                  c->q_rel.p);
   if (int rc = check_launch(c, "quadrature")) return rc;
-  cudaError_t e = cudaStreamSynchronize(c->stream);
-  if (e) return cuda_fail(c, e, "quadrature");
+  if (int rc = quadrature_grid(c, nq)) return rc;  // waits for the device
   c->q_per_elem = nq;
   return GGEM_OK;
 }

@@ -142,3 +142,59 @@ def test_spread_writes_zeros_where_no_particle_reaches(prec):
         rho = rho.cpu().numpy()
     assert np.all(rho[np.abs(q).max(axis=1) > 0.7 + 8.7 + 2 * h] == 0.0)
     assert np.all(np.isfinite(rho)) and rho.max() > 0.0
+
+
+def _grid_points(lo, L, nm, p, order):
+    """p[0] x p[1] x p[2] points per element; order: which axis index runs
+    fastest first"""
+    h = np.asarray(L, float) / np.asarray(nm)
+    g = [0.5 + 0.4 * np.linspace(-1.0, 1.0, k) if k > 1 else np.array([0.37]) for k in p]
+    loc = []
+    for idx in np.ndindex(*[p[d] for d in order[::-1]]):
+        i = dict(zip(order[::-1], idx))
+        loc.append([g[d][i[d]] for d in range(3)])
+    ez, ey, ex = np.meshgrid(np.arange(nm[2]), np.arange(nm[1]), np.arange(nm[0]), indexing="ij")
+    base = np.stack([ex.ravel(), ey.ravel(), ez.ravel()], axis=1)
+    q = (base[:, None, :] + np.array(loc)[None, :, :]) * h + np.asarray(lo, float)
+    return q.reshape(-1, 3), len(loc)
+
+
+@pytest.mark.parametrize("p,order,nm,periodic,jitter", [
+    ((2, 2, 2), (0, 1, 2), (21, 18, 17), (1, 1, 1), 0.0),   # frames inside the axes
+    ((2, 2, 2), (2, 1, 0), (13, 6, 21), (1, 1, 0), 0.0),    # an axis shorter than the stencil
+    ((3, 3, 3), (0, 1, 2), (18, 10, 5), (0, 1, 0), 0.0),    # three of 32 lanes idle
+    ((1, 1, 1), (0, 1, 2), (19, 21, 3), (1, 0, 1), 0.0),    # 32 elements per warp
+    ((3, 1, 2), (1, 2, 0), (7, 19, 18), (1, 1, 1), 0.0),    # uneven rule, partial bricks
+    ((1, 16, 2), (1, 0, 2), (9, 5, 6), (0, 0, 0), 0.0),     # 32 points in 32 rows
+    ((32, 1, 1), (0, 1, 2), (5, 4, 6), (0, 0, 0), 0.0),     # summed per pair: 32 along x
+    ((2, 2, 2), (0, 1, 2), (17, 18, 19), (1, 1, 1), 1e-13),  # summed per pair: no grid
+])
+def test_spread_tensor_grid_matches_oracle(p, order, nm, periodic, jitter):
+    """the separable sum of a tensor grid of points (and where the points are
+    not one, the sum per pair) against the oracle; several bricks hold more
+    members than one pass stages"""
+    lo = np.array([-2.0, 3.0, 0.5])
+    L = np.asarray(nm) * np.array([1.41, 1.3, 1.37])
+    rng = np.random.default_rng(sum(p) + nm[0])
+    n = 500
+    xyz = lo + rng.uniform(0, 1, (n, 3)) * L
+    xyz[:260] = lo + 0.3 * L * rng.uniform(0, 1, (260, 3)) + 0.2 * L  # a crowded corner
+    q, nq = _grid_points(lo, L, nm, p, order)
+    q = q + jitter * rng.standard_normal(q.shape)
+    f = rng.standard_normal((n, 3))
+    sre = 0.5 * 1.41 + 8.0 + 1e-3
+    box, mesh = O.make_box(lo, lo + L, periodic), O.make_mesh(*nm, sre)
+    enb, _ = O.elem_lists(box, mesh, xyz)
+    qe = np.repeat(np.arange(int(np.prod(nm))), nq).astype(np.int32)
+    want = O.spread_qp(O.constants(alpha=ALPHA), box, enb, xyz, f, q, qe)
+    with G.Context(alpha=ALPHA, box_lo=tuple(lo), box_hi=tuple(lo + L), periodic=periodic,
+                   nb_mode=G.NB_REFERENCE, n_mesh=nm, search_radius_e=sre,
+                   precision=G.FP64) as ctx:
+        ctx.set_particles(xyz)
+        ctx.build_cells()
+        ctx.set_quadrature(q, nq)
+        got = ctx.spread_elements(f, G.FP64)
+        assert np.array_equal(got, ctx.spread_elements(f, G.FP64))
+    # ~60 terms per point, each within a few ulp of e^{-alpha^2 r^2} at
+    # alpha^2 r^2 <= 25: 25 * 2^-52 per term, well below 1e-13 of the norm
+    assert rel(got, want) <= 1e-13
