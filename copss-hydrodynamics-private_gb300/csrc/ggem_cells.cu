@@ -29,11 +29,11 @@ __device__ __forceinline__ int wrap_index(int k, int n) {
 
 // cell coordinate along one axis, as the oracle and the reference's element
 // search would compute it: floor((x - lo) / h), periodic axes wrapped first
-__global__ void k_assign(int64_t n, const double *__restrict__ xyz, Grid g,
-                         int32_t *__restrict__ cell_of, int32_t *__restrict__ count,
-                         double4_32a *__restrict__ wrapped, int *__restrict__ err) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ void assign_one(int64_t i, const double *__restrict__ xyz,
+                                           const Grid &g, int32_t *__restrict__ cell_of,
+                                           int32_t *__restrict__ count,
+                                           double4_32a *__restrict__ wrapped,
+                                           int *__restrict__ err) {
   double p[3];
   int c[3];
   bool bad = false, nonfinite = false;
@@ -90,6 +90,13 @@ __global__ void k_assign(int64_t n, const double *__restrict__ xyz, Grid g,
   cell_of[i] = id;
   atomicAdd(&count[id], 1);
   wrapped[i] = make_double4_32a(p[0], p[1], p[2], 0.0);
+}
+
+__global__ void k_assign(int64_t n, const double *__restrict__ xyz, Grid g,
+                         int32_t *__restrict__ cell_of, int32_t *__restrict__ count,
+                         double4_32a *__restrict__ wrapped, int *__restrict__ err) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) assign_one(i, xyz, g, cell_of, count, wrapped, err);
 }
 
 // ---- exclusive scan (warp shuffles, 1024-element blocks) ----------------
@@ -290,13 +297,13 @@ __global__ void k_sort_cells(int64_t ncell, const int32_t *__restrict__ start,
   }
 }
 
-__global__ void k_gather_sorted(int64_t n, Grid g, const int32_t *__restrict__ order,
-                                const int32_t *__restrict__ cell_of,
-                                const double4_32a *__restrict__ wrapped,
-                                int32_t *__restrict__ rank, double4_32a *__restrict__ pos64,
-                                float4 *__restrict__ pos32) {
-  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s >= n) return;
+__device__ __forceinline__ void gather_one(int64_t s, const Grid &g,
+                                           const int32_t *__restrict__ order,
+                                           const int32_t *__restrict__ cell_of,
+                                           const double4_32a *__restrict__ wrapped,
+                                           int32_t *__restrict__ rank,
+                                           double4_32a *__restrict__ pos64,
+                                           float4 *__restrict__ pos32) {
   const int32_t i = order[s];
   rank[i] = (int32_t)s;
   const double4_32a p = wrapped[i];
@@ -309,6 +316,15 @@ __global__ void k_gather_sorted(int64_t n, Grid g, const int32_t *__restrict__ o
   const double ry = p.y - (g.lo[1] + (cy + 0.5) * g.h[1]);
   const double rz = p.z - (g.lo[2] + (cz + 0.5) * g.h[2]);
   pos32[s] = make_float4((float)rx, (float)ry, (float)rz, __int_as_float(cid));
+}
+
+__global__ void k_gather_sorted(int64_t n, Grid g, const int32_t *__restrict__ order,
+                                const int32_t *__restrict__ cell_of,
+                                const double4_32a *__restrict__ wrapped,
+                                int32_t *__restrict__ rank, double4_32a *__restrict__ pos64,
+                                float4 *__restrict__ pos32) {
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (s < n) gather_one(s, g, order, cell_of, wrapped, rank, pos64, pos32);
 }
 
 // neighbour cell of cell coordinate (cx,cy,cz) shifted by o; -1 if outside a
@@ -375,9 +391,9 @@ __device__ __forceinline__ float box_r2(float qx, float qy, float qz, float3 lo,
   return fmaf(bz, bz, fmaf(by, by, bx * bx));
 }
 
-__global__ void __launch_bounds__(32, 32) k_pair_list_warp(
-    Grid g, const int4 *__restrict__ stencil, int nst, const float4 *__restrict__ shift,
-    const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
+__device__ __forceinline__ void pair_list_cell(
+    int64_t C, const Grid &g, const int4 *__restrict__ stencil, int nst,
+    const float4 *__restrict__ shift, const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
     const double4_32a *__restrict__ pos64, float rc2_lo, float rc2_hi, double rc2, int W,
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err,
@@ -390,7 +406,6 @@ __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
   __shared__ int s_mark[32];           // stencil cell starting at each lane of a chunk
   const int lane = threadIdx.x;
   s_mark[lane] = -1;
-  const int64_t C = blockIdx.x;
   const int32_t tb = start[C], te = start[C + 1];
   if (te <= tb) return;
   const int cx = (int)(C % g.nc[0]), cy = (int)((C / g.nc[0]) % g.nc[1]),
@@ -560,6 +575,132 @@ __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
     atomicMax(&stat[1], (unsigned long long)cell_max);
     if (cell_max > W) atomicOr(err, kErrListCapacity);
   }
+}
+
+__global__ void __launch_bounds__(32, 32) k_pair_list_warp(
+    Grid g, const int4 *__restrict__ stencil, int nst, const float4 *__restrict__ shift,
+    const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
+    const double4_32a *__restrict__ pos64, float rc2_lo, float rc2_hi, double rc2, int W,
+    int32_t *__restrict__ count, uint32_t *__restrict__ list,
+    unsigned long long *__restrict__ stat, int *__restrict__ err,
+    int32_t *__restrict__ count_h, uint32_t *__restrict__ list_h) {
+  pair_list_cell(blockIdx.x, g, stencil, nst, shift, start, pos32, pos64, rc2_lo, rc2_hi, rc2, W,
+                 count, list, stat, err, count_h, list_h);
+}
+
+// ---- many suspensions at once ----------------------------------------------
+// The same build over the concatenated cells and slots of K suspensions
+// (BatchGeo: each one's grid, stencil and first cell and slot), so that an
+// ensemble's configuration takes one launch per phase instead of one per
+// phase and suspension: the launches and host waits of 64 separate builds
+// were ~7 ms, their kernels a few microseconds each.
+__global__ void k_batch_susp(int64_t ntot, int K, const int64_t *__restrict__ off,
+                             int32_t *__restrict__ susp) {
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (s >= ntot) return;
+  int lo = 0, hi = K - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= s) lo = mid;
+    else hi = mid - 1;
+  }
+  susp[s] = lo;
+}
+
+__global__ void k_batch_assign(int64_t ntot, const double *__restrict__ xyz,
+                               const BatchGeo *__restrict__ geo, const int32_t *__restrict__ susp,
+                               int32_t *__restrict__ cell_of, int32_t *__restrict__ count,
+                               double4_32a *__restrict__ wrapped, int *__restrict__ err) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= ntot) return;
+  const BatchGeo &b = geo[susp[i]];
+  assign_one(i, xyz, b.g, cell_of, count + b.cell0, wrapped, err);
+}
+
+// one block per suspension: its cells' counts (zeroed as they are read)
+// scanned from its first slot on
+__global__ void __launch_bounds__(1024) k_batch_scan(int K, const BatchGeo *__restrict__ geo,
+                                                     const int64_t *__restrict__ off,
+                                                     int32_t *__restrict__ count,
+                                                     int32_t *__restrict__ start,
+                                                     unsigned long long *__restrict__ stat) {
+  __shared__ int32_t warp_tot[2][32];
+  const int b = blockIdx.x;
+  if (b == 0 && threadIdx.x < 2) stat[threadIdx.x] = 0ull;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t c0 = geo[b].cell0, n = geo[b].g.ncell;
+  int32_t carry = (int32_t)off[b];
+  int buf = 0;
+  for (int64_t t0 = 0; t0 < n; t0 += 4096, buf ^= 1) {
+    int32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t i = t0 + 4 * threadIdx.x + j;
+      v[j] = i < n ? count[c0 + i] : 0;
+      if (i < n) count[c0 + i] = 0;
+    }
+    const int32_t tsum = (v[0] + v[1]) + (v[2] + v[3]);
+    int32_t x = tsum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    int32_t *wt = warp_tot[buf];  // alternate buffers: one barrier per tile
+    if (lane == 31) wt[warp] = x;
+    __syncthreads();
+    int32_t w = wt[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    const int32_t before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+    const int32_t total = __shfl_sync(0xffffffffu, w, 31);
+    int32_t run = carry + (warp ? before : 0) + x - tsum;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t i = t0 + 4 * threadIdx.x + j;
+      if (i < n) start[c0 + i] = run;
+      run += v[j];
+    }
+    carry += total;
+  }
+  if (b == K - 1 && threadIdx.x == 0) start[c0 + n] = carry;
+}
+
+__global__ void k_batch_scatter(int64_t ntot, const BatchGeo *__restrict__ geo,
+                                const int32_t *__restrict__ susp,
+                                const int32_t *__restrict__ cell_of,
+                                const int32_t *__restrict__ start, int32_t *__restrict__ fill,
+                                int32_t *__restrict__ order) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= ntot) return;
+  const int64_t cid = geo[susp[i]].cell0 + cell_of[i];
+  order[start[cid] + atomicAdd(&fill[cid], 1)] = (int32_t)i;
+}
+
+__global__ void k_batch_gather(int64_t ntot, const BatchGeo *__restrict__ geo,
+                               const int32_t *__restrict__ susp,
+                               const int32_t *__restrict__ order,
+                               const int32_t *__restrict__ cell_of,
+                               const double4_32a *__restrict__ wrapped,
+                               int32_t *__restrict__ rank, double4_32a *__restrict__ pos64,
+                               float4 *__restrict__ pos32) {
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (s >= ntot) return;
+  gather_one(s, geo[susp[s]].g, order, cell_of, wrapped, rank, pos64, pos32);
+}
+
+__global__ void __launch_bounds__(32, 32) k_batch_list(
+    const BatchGeo *__restrict__ geo, const int32_t *__restrict__ cell_susp,
+    const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
+    const double4_32a *__restrict__ pos64, float rc2_lo, float rc2_hi, double rc2, int W,
+    int32_t *__restrict__ count, uint32_t *__restrict__ list,
+    unsigned long long *__restrict__ stat, int *__restrict__ err) {
+  const BatchGeo &b = geo[cell_susp[blockIdx.x]];
+  pair_list_cell((int64_t)blockIdx.x - b.cell0, b.g, b.stencil, b.nst, b.shift, start + b.cell0,
+                 pos32, pos64, rc2_lo, rc2_hi, rc2, W, count, list, stat, err, nullptr, nullptr);
 }
 
 // Element lists (reference mode) as pair-list rows: one warp per target slot,
@@ -894,6 +1035,29 @@ int ensure_f64_list(ggem_ctx *c, bool flags_pending) {
   }
   c->cells_built = true;
   return GGEM_OK;
+}
+
+void batch_susp(const BatchBuild &b, const int64_t *off, int32_t *susp, cudaStream_t st) {
+  k_batch_susp<<<(unsigned)((b.ntot + 255) / 256), 256, 0, st>>>(b.ntot, b.K, off, susp);
+}
+
+void batch_cells(const BatchBuild &b, const double *xyz, const int64_t *off, cudaStream_t st) {
+  const unsigned bn = (unsigned)((b.ntot + 255) / 256);
+  k_batch_assign<<<bn, 256, 0, st>>>(b.ntot, xyz, b.geo, b.susp, b.cell_of, b.cell_count,
+                                     b.wrapped, b.err);
+  k_batch_scan<<<b.K, 1024, 0, st>>>(b.K, b.geo, off, b.cell_count, b.cell_start, b.stat);
+  k_batch_scatter<<<bn, 256, 0, st>>>(b.ntot, b.geo, b.susp, b.cell_of, b.cell_start, b.cell_fill,
+                                      b.order);
+  k_sort_cells<<<(unsigned)((b.ncell + 255) / 256), 256, 0, st>>>(b.ncell, b.cell_start, b.order,
+                                                                   b.cell_fill);
+  k_batch_gather<<<bn, 256, 0, st>>>(b.ntot, b.geo, b.susp, b.order, b.cell_of, b.wrapped, b.rank,
+                                     b.pos64, b.pos32);
+}
+
+void batch_list(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st) {
+  k_batch_list<<<(unsigned)b.ncell, 32, 0, st>>>(b.geo, b.cell_susp, b.cell_start, b.pos32, b.pos64,
+                                                 like->rc2_lo, like->rc2_hi, like->rc2, b.W, b.cnt,
+                                                 b.list, b.stat, b.err);
 }
 
 int enqueue_list_check(ggem_ctx *c) {

@@ -1,12 +1,12 @@
 // ggem_ensemble.cu -- K independent suspensions as one block-diagonal
 // operator (include/ggem_ensemble.h).
 //
-// Each suspension is an ordinary FP32 context (its own box, cell list, pair
-// list and stored pair tensors t = (A, sqrt(B) x)).  The ensemble
-// concatenates the rows of all K lists into one fixed-width list over a
-// global slot space (source slots offset by the suspension's first slot),
-// so that the pair kernel needs neither positions nor a cell grid: one launch
-// applies M to every suspension.  Vectors inside the ensemble are
+// The suspensions' cells and slots are concatenated, and one batched build
+// (one launch per phase) fills one fixed-width pair list over the global
+// slot space with the stored pair tensors t = (A, sqrt(B) x), entry for
+// entry those of K separate FP32 contexts, so that the pair kernel needs
+// neither positions nor a cell grid: one launch applies M to every
+// suspension.  Vectors inside the ensemble are
 // [slot][8][3] float64 (right-hand sides padded to 8); the pair kernel maps
 // 8 lanes to one target slot, one lane per right-hand side, so that the
 // 8 forces of a source (FP32, [slot][8] float4) are one 128-byte load.
@@ -34,39 +34,6 @@ namespace ens {
 
 constexpr int kR = GGEM_ENSEMBLE_MAX_RHS;  // right-hand-side lanes per slot
 constexpr int kE = 3 * kR;                 // doubles per slot in a vector
-
-struct SubView {
-  const int32_t *cnt;
-  const uint32_t *list;
-  const float4 *ten;
-  const int32_t *order;
-  const int32_t *rank;
-  int64_t n, off;
-  int W;
-};
-
-// the K lists into the global list: rows re-strided to Wg, source slots
-// offset, suspension id, slot <-> ensemble-index maps
-__global__ void k_ens_gather(const SubView *__restrict__ views, int Wg,
-                             int32_t *__restrict__ cnt_g, uint32_t *__restrict__ list_g,
-                             float4 *__restrict__ ten_g, int32_t *__restrict__ susp,
-                             int32_t *__restrict__ order_g, int32_t *__restrict__ rank_g) {
-  const SubView v = views[blockIdx.y];
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < v.n;
-       s += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t gs = v.off + s;
-    const int c = v.cnt[s];
-    cnt_g[gs] = c;
-    susp[gs] = (int32_t)blockIdx.y;
-    order_g[gs] = (int32_t)(v.off + v.order[s]);
-    rank_g[v.off + s] = (int32_t)(v.off + v.rank[s]);  // s as the caller index here
-    for (int m = 0; m < c; ++m) {
-      const uint32_t en = v.list[s * v.W + m];
-      list_g[gs * Wg + m] = (uint32_t)(((int64_t)(en >> kCodeBits) + v.off) << kCodeBits);
-      ten_g[gs * Wg + m] = v.ten[s * v.W + m];
-    }
-  }
-}
 
 // [bead][nrhs][3] (ensemble order) <-> [slot][8][3] (zero padded)
 __global__ void k_ens_to_slots(int64_t ntot, int nrhs, const int32_t *__restrict__ order_g,
@@ -572,7 +539,19 @@ struct ggem_ensemble {
   DevBuf<int32_t> chunk_off;
   DevBuf<double> chunk_part;
   int nchunk = 0;
-  DevBuf<SubView> views;
+  // the batched build (one launch per phase for all suspensions): the
+  // suspensions' grids and cells, their concatenated cell and slot arrays,
+  // a copy of the positions for the suspensions' own contexts, which are
+  // built only for the calls that work on one of them (sub_built)
+  DevBuf<BatchGeo> geo;
+  DevBuf<int32_t> cell_susp, cell_of, cell_count, cell_fill, cell_start;
+  DevBuf<double4_32a> wrapped, pos64;
+  DevBuf<float4> pos32;
+  DevBuf<double> xyz;
+  DevBuf<unsigned long long> stat;  // [0] entries, [1] longest row, [2] error word
+  int64_t ncell = 0;
+  bool counters_zero = false;
+  std::vector<uint8_t> sub_built;
   // Chebyshev state: vectors [slot][8][3] and FP32 forces [slot][8]
   DevBuf<double> v[6];
   DevBuf<float4> f4[3];
@@ -710,7 +689,7 @@ extern "C" int ggem_ensemble_create(const ggem_params *base, int k, const double
   cudaError_t c;
   if ((c = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) ||
       (c = cudaMallocHost((void **)&e->h_red, sizeof(double) * 4 * kR * (size_t)k)) ||
-      (c = e->d_off.ensure(k + 1)) || (c = e->views.ensure(k)) || (c = e->red.ensure(4 * kR * (size_t)k)) ||
+      (c = e->d_off.ensure(k + 1)) || (c = e->red.ensure(4 * kR * (size_t)k)) ||
       (c = e->active.ensure(kR * (size_t)k)) || (c = e->da.ensure(k)) || (c = e->db.ensure(k)) ||
       (c = e->two_da.ensure(k)) || (c = e->c1x.ensure(k))) {
     cudaGetLastError();
@@ -734,6 +713,28 @@ extern "C" int ggem_ensemble_create(const ggem_params *base, int k, const double
       ggem_ensemble_destroy(e);
       return GGEM_ERR_BAD_ARG;  // the ensemble operator needs stored pair tensors (B >= 0)
     }
+  }
+  // the grids belong to the boxes; first cells of the concatenation
+  std::vector<BatchGeo> geo(k);
+  std::vector<int32_t> cell_susp;
+  for (int b = 0; b < k; ++b) {
+    const ggem_ctx *s = e->sub[b];
+    geo[b] = BatchGeo{s->grid, s->d_stencil.p, s->d_shift.p, (int)s->stencil.size(), e->ncell};
+    e->ncell += s->grid.ncell;
+    cell_susp.resize((size_t)e->ncell, b);
+  }
+  if (e->ncell > 0x7fffffff) {  // (a grid of one block per cell)
+    ggem_ensemble_destroy(e);
+    return GGEM_ERR_BAD_ARG;
+  }
+  if ((c = e->geo.ensure(k)) || (c = e->cell_susp.ensure(cell_susp.size())) ||
+      (c = e->stat.ensure(3)) ||
+      (c = cudaMemcpy(e->geo.p, geo.data(), sizeof(BatchGeo) * k, cudaMemcpyHostToDevice)) ||
+      (c = cudaMemcpy(e->cell_susp.p, cell_susp.data(), sizeof(int32_t) * cell_susp.size(),
+                      cudaMemcpyHostToDevice))) {
+    cudaGetLastError();
+    ggem_ensemble_destroy(e);
+    return c == cudaErrorMemoryAllocation ? GGEM_ERR_OOM : GGEM_ERR_CUDA;
   }
   e->self_c = self_coefficient(e->sub[0], e->base.point_type == GGEM_LAGRANGIAN_POINT
                                               ? GGEM_SELF_LAGRANGIAN
@@ -760,54 +761,32 @@ extern "C" const char *ggem_ensemble_last_error(const ggem_ensemble *e) {
   return e ? e->err.c_str() : "null ensemble";
 }
 
-extern "C" int ggem_ensemble_set_particles_dev(ggem_ensemble *e, const int64_t *n,
-                                               const double *d_xyz) {
-  if (!e || !n || !d_xyz) return GGEM_ERR_BAD_ARG;
-  EnsGuard g(e->device);
-  e->built = false;
-  e->n.assign(n, n + e->K);
-  e->off.assign(e->K + 1, 0);
-  for (int b = 0; b < e->K; ++b) {
-    if (n[b] < 1) return efail(e, GGEM_ERR_BAD_ARG, "every suspension needs beads");
-    e->off[b + 1] = e->off[b] + n[b];
-  }
-  e->ntot = e->off[e->K];
-  if (e->ntot >= ((int64_t)1 << (32 - kCodeBits)))
-    return efail(e, GGEM_ERR_BAD_ARG, "ensemble larger than the pair-entry slot space");
-  // every suspension: cells, list, stored tensors (on its own stream)
-  e->W = 0;
-  e->pairs = 0;
-  std::vector<SubView> views(e->K);
-  for (int b = 0; b < e->K; ++b) {
-    ggem_ctx *c = e->sub[b];
-    if (int rc = ggem_set_particles_dev(c, n[b], d_xyz + 3 * e->off[b]))
-      return efail(e, rc, "suspension " + std::to_string(b) + ": " + c->last_error);
-    if (int rc = ggem_build_cells(c))
-      return efail(e, rc, "suspension " + std::to_string(b) + ": " + c->last_error);
-    if (!c->pretensor_ok)
-      return efail(e, GGEM_ERR_OOM, "suspension " + std::to_string(b) + ": no pair tensors");
-    e->W = std::max(e->W, c->nb_w);
-    e->pairs += c->n_pairs;
-    views[b] = SubView{c->nb_cnt.p, c->nb_list.p, c->pair_ten.p, c->order.p, c->rank.p,
-                       n[b], e->off[b], c->nb_w};
-  }
-  for (ggem_ctx *c : e->sub) cudaStreamSynchronize(c->stream);
+namespace {
+
+// suspension b as an ordinary context (cells, list, stored tensors on its
+// own stream) for the calls that work on one suspension
+int ensure_sub(ggem_ensemble *e, int b) {
+  if (e->sub_built[b]) return GGEM_OK;
+  ggem_ctx *c = e->sub[b];
+  int rc = ggem_set_particles_dev(c, e->n[b], e->xyz.p + 3 * e->off[b]);
+  if (!rc) rc = ggem_build_cells(c);
+  if (rc) return efail(e, rc, "suspension " + std::to_string(b) + ": " + c->last_error);
+  e->sub_built[b] = 1;
+  return GGEM_OK;
+}
+
+// tables that depend on the bead counts alone: first slots, the suspension
+// of every slot, the dot chunks (each within one suspension)
+int ensemble_tables(ggem_ensemble *e, const BatchBuild &b) {
   cudaError_t c;
-  if ((c = e->cnt.ensure(e->ntot)) || (c = e->susp.ensure(e->ntot)) ||
-      (c = e->order_g.ensure(e->ntot)) || (c = e->rank_g.ensure(e->ntot)) ||
-      (c = e->list.ensure((size_t)e->ntot * e->W)) || (c = e->ten.ensure((size_t)e->ntot * e->W)))
-    return ecuda(e, c, "ensemble operator");
-  if ((c = cudaMemcpyAsync(e->views.p, views.data(), sizeof(SubView) * e->K,
-                           cudaMemcpyHostToDevice, e->stream)) ||
-      (c = cudaMemcpyAsync(e->d_off.p, e->off.data(), sizeof(int64_t) * (e->K + 1),
+  if ((c = cudaMemcpyAsync(e->d_off.p, e->off.data(), sizeof(int64_t) * (e->K + 1),
                            cudaMemcpyHostToDevice, e->stream)))
     return ecuda(e, c, "ensemble tables");
-  // the dot chunks (each within one suspension)
   std::vector<int64_t> cs;
   std::vector<int32_t> coff(e->K + 1, 0);
-  for (int b = 0; b < e->K; ++b) {
-    coff[b] = (int32_t)cs.size();
-    for (int64_t s0 = e->off[b]; s0 < e->off[b + 1]; s0 += kDotSlots) cs.push_back(s0);
+  for (int k = 0; k < e->K; ++k) {
+    coff[k] = (int32_t)cs.size();
+    for (int64_t s0 = e->off[k]; s0 < e->off[k + 1]; s0 += kDotSlots) cs.push_back(s0);
   }
   coff[e->K] = (int32_t)cs.size();
   e->nchunk = (int)cs.size();
@@ -819,13 +798,117 @@ extern "C" int ggem_ensemble_set_particles_dev(ggem_ensemble *e, const int64_t *
       (c = cudaMemcpyAsync(e->chunk_off.p, coff.data(), sizeof(int32_t) * coff.size(),
                            cudaMemcpyHostToDevice, e->stream)))
     return ecuda(e, c, "ensemble dot chunks");
-  int64_t nmax = 0;
-  for (int b = 0; b < e->K; ++b) nmax = std::max(nmax, n[b]);
-  dim3 grid(eblocks(nmax, 256), e->K);
-  k_ens_gather<<<grid, 256, 0, e->stream>>>(e->views.p, e->W, e->cnt.p, e->list.p, e->ten.p,
-                                            e->susp.p, e->order_g.p, e->rank_g.p);
-  if (int rc = elaunch(e, "ensemble gather")) return rc;
-  if ((c = cudaStreamSynchronize(e->stream))) return ecuda(e, c, "ensemble gather");
+  batch_susp(b, e->d_off.p, e->susp.p, e->stream);
+  e->tiles_for_ntot = -1;  // the series' tiles follow the bead counts too
+  return elaunch(e, "ensemble tables");
+}
+
+}  // namespace
+
+extern "C" int ggem_ensemble_set_particles_dev(ggem_ensemble *e, const int64_t *n,
+                                               const double *d_xyz) {
+  if (!e || !n || !d_xyz) return GGEM_ERR_BAD_ARG;
+  EnsGuard g(e->device);
+  e->built = false;
+  const std::vector<int64_t> before = std::move(e->n);
+  e->n.assign(n, n + e->K);
+  e->off.assign(e->K + 1, 0);
+  for (int b = 0; b < e->K; ++b) {
+    if (n[b] < 1) {
+      e->n.clear();
+      return efail(e, GGEM_ERR_BAD_ARG, "every suspension needs beads");
+    }
+    e->off[b + 1] = e->off[b] + n[b];
+  }
+  e->ntot = e->off[e->K];
+  if (e->ntot >= ((int64_t)1 << (32 - kCodeBits))) {
+    e->n.clear();
+    return efail(e, GGEM_ERR_BAD_ARG, "ensemble larger than the pair-entry slot space");
+  }
+  const bool same_counts = before == e->n;
+  std::vector<int64_t> counts;
+  counts.swap(e->n);  // stays empty until the tables are in place
+  // rows of twice the densest suspension's mean length, or as wide as needed before
+  for (int b = 0; b < e->K; ++b) {
+    const ggem_ctx *s = e->sub[b];
+    const double vol = s->grid.L[0] * s->grid.L[1] * s->grid.L[2];
+    const double mean = (double)n[b] / vol * 4.18879020478639 * s->rc2 * std::sqrt(s->rc2);
+    e->W = std::max(e->W, (int)std::min<double>(((int64_t)(2.0 * mean) + 16 + 7) / 8 * 8, 1 << 20));
+  }
+  e->sub_built.assign(e->K, 0);
+  cudaError_t c;
+  const size_t nt = (size_t)e->ntot;
+  const int32_t *counters = e->cell_count.p;
+  if ((c = e->cnt.ensure(nt)) || (c = e->susp.ensure(nt)) || (c = e->order_g.ensure(nt)) ||
+      (c = e->rank_g.ensure(nt)) || (c = e->cell_of.ensure(nt)) || (c = e->wrapped.ensure(nt)) ||
+      (c = e->pos64.ensure(nt)) || (c = e->pos32.ensure(nt)) || (c = e->xyz.ensure(3 * nt)) ||
+      (c = e->cell_count.ensure(e->ncell)) || (c = e->cell_fill.ensure(e->ncell)) ||
+      (c = e->cell_start.ensure(e->ncell + 1)))
+    return ecuda(e, c, "ensemble operator");
+  BatchBuild B;
+  B.K = e->K;
+  B.ntot = e->ntot;
+  B.ncell = e->ncell;
+  B.geo = e->geo.p;
+  B.susp = e->susp.p;
+  B.cell_susp = e->cell_susp.p;
+  B.cell_of = e->cell_of.p;
+  B.cell_count = e->cell_count.p;
+  B.cell_fill = e->cell_fill.p;
+  B.cell_start = e->cell_start.p;
+  B.order = e->order_g.p;
+  B.rank = e->rank_g.p;
+  B.cnt = e->cnt.p;
+  B.wrapped = e->wrapped.p;
+  B.pos64 = e->pos64.p;
+  B.pos32 = e->pos32.p;
+  B.stat = e->stat.p;
+  B.err = reinterpret_cast<int *>(e->stat.p + 2);
+  if (!same_counts)
+    if (int rc = ensemble_tables(e, B)) return rc;
+  // (the counters were left at zero by the previous build)
+  if (!e->counters_zero || counters != e->cell_count.p)
+    if ((c = cudaMemsetAsync(e->cell_count.p, 0, sizeof(int32_t) * e->ncell, e->stream)) ||
+        (c = cudaMemsetAsync(e->cell_fill.p, 0, sizeof(int32_t) * e->ncell, e->stream)))
+      return ecuda(e, c, "ensemble counters");
+  e->counters_zero = false;
+  if ((c = cudaMemcpyAsync(e->xyz.p, d_xyz, sizeof(double) * 3 * nt, cudaMemcpyDeviceToDevice,
+                           e->stream)) ||
+      (c = cudaMemsetAsync(e->stat.p, 0, 3 * sizeof(unsigned long long), e->stream)))
+    return ecuda(e, c, "ensemble positions");
+  batch_cells(B, e->xyz.p, e->d_off.p, e->stream);
+  if (int rc = elaunch(e, "ensemble cells")) return rc;
+  unsigned long long h[3] = {0, 0, 0};
+  for (int attempt = 0;; ++attempt) {
+    if ((c = e->list.ensure(nt * e->W)) || (c = e->ten.ensure(nt * e->W)))
+      return ecuda(e, c, "ensemble operator");
+    B.W = e->W;
+    B.list = e->list.p;
+    B.ten = e->ten.p;
+    batch_list(B, e->sub[0], e->stream);
+    batch_tensors(B, e->sub[0], e->stream);
+    if (int rc = elaunch(e, "ensemble lists")) return rc;
+    if ((c = cudaMemcpyAsync(h, e->stat.p, sizeof(h), cudaMemcpyDeviceToHost, e->stream)) ||
+        (c = cudaStreamSynchronize(e->stream)))
+      return ecuda(e, c, "ensemble lists");
+    const int flags = (int)h[2];
+    if (flags & (kErrNonFinite | kErrOutOfDomain)) {
+      e->counters_zero = true;
+      e->n = counts;
+      for (int b = 0; b < e->K; ++b)  // the suspension at fault names itself
+        if (int rc = ensure_sub(e, b)) return rc;
+      return efail(e, GGEM_ERR_BAD_ARG, "non-finite position");
+    }
+    if (!(flags & kErrListCapacity)) break;
+    if (attempt) return efail(e, GGEM_ERR_CELL_OVERFLOW, "pair list rows exceeded their width twice");
+    // rows longer than the width: widen them and fill once more
+    e->W = (int)std::min<unsigned long long>((h[1] + h[1] / 8 + 8 + 7) / 8 * 8, 1u << 24);
+    if ((c = cudaMemsetAsync(e->stat.p, 0, 3 * sizeof(unsigned long long), e->stream)))
+      return ecuda(e, c, "ensemble lists");
+  }
+  e->counters_zero = true;
+  e->pairs = (int64_t)h[0];
+  e->n = counts;
   if (int rc = ensure_vectors(e)) return rc;
   e->built = true;
   return GGEM_OK;
@@ -1434,10 +1517,12 @@ extern "C" int ggem_ensemble_intervals(ggem_ensemble *e, ggem_surrogate *s,
   if (!e->built) return efail(e, GGEM_ERR_BAD_ARG, "set the ensemble's particles first");
   EnsGuard g(e->device);
   std::vector<float> X((size_t)e->K * GGEM_SUR_FEATURES), Y((size_t)e->K * GGEM_SUR_OUTPUTS);
-  for (int b = 0; b < e->K; ++b)
+  for (int b = 0; b < e->K; ++b) {
+    if (int rc = ensure_sub(e, b)) return rc;
     if (int rc = ggem_surrogate_features(e->sub[b], chain_fraction ? chain_fraction[b] : 0.0,
                                          X.data() + (size_t)b * GGEM_SUR_FEATURES))
       return efail(e, rc, e->sub[b]->last_error);
+  }
   // one batched forward pass for all suspensions
   if (int rc = ggem_surrogate_predict(s, X.data(), e->K, Y.data()))
     return efail(e, rc, ggem_surrogate_last_error(s));
@@ -1452,6 +1537,8 @@ extern "C" int ggem_ensemble_lanczos(ggem_ensemble *e, int b, int k, uint64_t se
                                      double *eig_min, double *eig_max) {
   if (!e || b < 0 || b >= e->K) return GGEM_ERR_BAD_ARG;
   if (!e->built) return efail(e, GGEM_ERR_BAD_ARG, "set the ensemble's particles first");
+  EnsGuard g(e->device);
+  if (int rc = ensure_sub(e, b)) return rc;
   if (int rc = ggem_lanczos_bounds(e->sub[b], k, seed, eig_min, eig_max))
     return efail(e, rc, e->sub[b]->last_error);
   return GGEM_OK;

@@ -359,6 +359,35 @@ constexpr int kListStatSlot = 4088;  // h_red[4088 .. 4090]: deferred list stati
 int device_exclusive_scan_i32(ggem_ctx *c, const int32_t *in, int32_t *out, int64_t n);
 int device_exclusive_scan_i64(ggem_ctx *c, const int64_t *in, int64_t *out, int64_t n);
 
+// the same build for K suspensions at once (the ensemble): cells and slots
+// concatenated, cell ids local to their suspension, slots global
+struct BatchGeo {
+  Grid g;
+  const int4 *stencil;
+  const float4 *shift;
+  int nst;
+  int64_t cell0;  // first cell
+};
+struct BatchBuild {
+  int K = 0, W = 0;
+  int64_t ntot = 0, ncell = 0;
+  const BatchGeo *geo = nullptr;     // [K]
+  const int32_t *susp = nullptr;     // [ntot] suspension of every slot and of every bead
+  const int32_t *cell_susp = nullptr;  // [ncell]
+  int32_t *cell_of = nullptr, *cell_count = nullptr, *cell_fill = nullptr, *cell_start = nullptr;
+  int32_t *order = nullptr, *rank = nullptr, *cnt = nullptr;
+  double4_32a *wrapped = nullptr, *pos64 = nullptr;
+  float4 *pos32 = nullptr;
+  uint32_t *list = nullptr;
+  float4 *ten = nullptr;
+  unsigned long long *stat = nullptr;  // [0] entries, [1] longest row
+  int *err = nullptr;
+};
+void batch_susp(const BatchBuild &b, const int64_t *off, int32_t *susp, cudaStream_t st);
+void batch_cells(const BatchBuild &b, const double *xyz, const int64_t *off, cudaStream_t st);
+void batch_list(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st);
+void batch_tensors(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st);
+
 // pair sums (ggem_pair.cu); vectors in slot order, [r][slot][3] doubles
 int matvec_slots(ggem_ctx *c, int nrhs, const double *d_f_slot, double *d_u_slot,
                  int self_mode);

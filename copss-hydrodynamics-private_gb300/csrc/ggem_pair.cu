@@ -785,14 +785,11 @@ __global__ void k_to_slots_rec(int64_t n, const int32_t *__restrict__ order,
 // G f = A f + (x~ . f) x~ with x~ = sqrt(B) x, no position gathers and no
 // polynomial per pair and matvec.
 template <int CD, bool POLY>
-__global__ void __launch_bounds__(256) k_pair_tensor(
-    int64_t n, const float4 *__restrict__ pos32, const int32_t *__restrict__ cnt, int W,
-    const uint32_t *__restrict__ list, PolyAB P, const Rec32 *__restrict__ tab, float inv_ds,
-    float hx, float hy, float hz, float4 *__restrict__ ten) {
-  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
-  const int sub = (int)(threadIdx.x % kGroup);
-  if (gid >= n) return;
-  const int64_t s = gid;
+__device__ __forceinline__ void tensor_row(int64_t s, int sub, const float4 *__restrict__ pos32,
+                                           const int32_t *__restrict__ cnt, int W,
+                                           const uint32_t *__restrict__ list, const PolyAB &P,
+                                           const Rec32 *__restrict__ tab, float inv_ds, float hx,
+                                           float hy, float hz, float4 *__restrict__ ten) {
   const float4 pi = pos32[s];
   const int64_t b = s * (int64_t)W, e = b + cnt[s];
   for (int64_t m = b + sub; m < e; m += 2 * kGroup) {
@@ -814,6 +811,31 @@ __global__ void __launch_bounds__(256) k_pair_tensor(
       __stcs(ten + m + q * kGroup, make_float4(A, w * dx, w * dy, w * dz));
     }
   }
+}
+
+template <int CD, bool POLY>
+__global__ void __launch_bounds__(256) k_pair_tensor(
+    int64_t n, const float4 *__restrict__ pos32, const int32_t *__restrict__ cnt, int W,
+    const uint32_t *__restrict__ list, PolyAB P, const Rec32 *__restrict__ tab, float inv_ds,
+    float hx, float hy, float hz, float4 *__restrict__ ten) {
+  const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
+  if (s < n)
+    tensor_row<CD, POLY>(s, (int)(threadIdx.x % kGroup), pos32, cnt, W, list, P, tab, inv_ds, hx,
+                         hy, hz, ten);
+}
+
+// the tensors of K suspensions' concatenated rows
+template <int CD, bool POLY>
+__global__ void __launch_bounds__(256) k_batch_tensor(
+    int64_t n, const BatchGeo *__restrict__ geo, const int32_t *__restrict__ susp,
+    const float4 *__restrict__ pos32, const int32_t *__restrict__ cnt, int W,
+    const uint32_t *__restrict__ list, PolyAB P, const Rec32 *__restrict__ tab, float inv_ds,
+    float4 *__restrict__ ten) {
+  const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
+  if (s >= n) return;
+  const float *h = geo[susp[s]].g.h32;
+  tensor_row<CD, POLY>(s, (int)(threadIdx.x % kGroup), pos32, cnt, W, list, P, tab, inv_ds, h[0],
+                       h[1], h[2], ten);
 }
 
 // forces of one right-hand side as one float4 per slot (w = 0)
@@ -1878,6 +1900,18 @@ int build_pair_tensors(ggem_ctx *c) {
   if (int rc = check_launch(c, "pair tensors")) return rc;
   c->pretensor_ok = true;
   return GGEM_OK;
+}
+
+void batch_tensors(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st) {
+  const unsigned grid = (unsigned)((b.ntot * kGroup + 255) / 256);
+  const Rec32 *tab = reinterpret_cast<const Rec32 *>(like->tab.p);
+  const bool cd2 = like->prm.cell_div == 2;
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, 256, 0, st>>>(b.ntot, b.geo, b.susp, b.pos32, b.cnt, b.W, b.list, poly_of(like),
+                                 tab, like->tab_inv_ds, b.ten);
+  };
+  if (like->use_poly) cd2 ? launch(k_batch_tensor<2, true>) : launch(k_batch_tensor<1, true>);
+  else cd2 ? launch(k_batch_tensor<2, false>) : launch(k_batch_tensor<1, false>);
 }
 
 double self_coefficient(const ggem_ctx *c, int self_mode) {

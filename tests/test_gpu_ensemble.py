@@ -304,3 +304,59 @@ def test_series_autotuner_and_its_cache(tmp_path):
         assert rel(got, dw.cpu().numpy()) <= 1e-12
     print(f"series autotune: shape {out[0][0]}, {out[0][1]} slots per tile, "
           f"{out[0][2]:.3f} ms per 14-term step; tuning {out[0][3]:.2f} s, cache hit {out[1][3]:.3f} s")
+
+
+@pytest.mark.parametrize("cell_div", [1, 2])
+def test_batched_build_equals_single_suspensions(cell_div):
+    """one batched build of all suspensions gives every one of them the rows
+    (bit for bit: the same operator) that it has alone, over new positions,
+    other counts of the same total, grids from 3^3 cells up and rows that
+    outgrow their width; a bad position names its suspension"""
+    import torch
+    R = 3
+    sets = [_ensemble(4, 11, (500, 9000)), _ensemble(4, 13, (500, 9000))]
+    L = [max(a[1], b[1]) for a, b in zip(*sets)]
+    L[2] = 21.5
+    rng = np.random.default_rng(2)
+    # third configuration: the first one's total in other counts, crowded
+    counts = [len(x) for x, _ in sets[0]]
+    moved = [np.asarray(x) % l for (x, _), l in zip(sets[0], L)]
+    other = [rng.uniform(0.0, min(9.0, l), (n, 3)) for n, l in zip([700, 300, 40], L)]
+    other.append(rng.uniform(0.0, L[3], (sum(counts) - 1040, 3)))
+
+    def u_of(ens, conf):
+        d_x = _device(np.concatenate(conf))
+        d_f = _device(np.concatenate([np.cos(np.arange(x.size * R)).reshape(-1, R, 3)
+                                      for x in conf]))
+        d_u = torch.zeros_like(d_f)
+        torch.cuda.synchronize()
+        ens.set_particles_dev([len(x) for x in conf], d_x.data_ptr())
+        ens.matvec_dev(R, d_f.data_ptr(), d_u.data_ptr(), G.SELF_BEAD)
+        return d_u.cpu().numpy(), ens.sizes()[1]
+
+    confs = [moved, [np.asarray(x) % l for (x, _), l in zip(sets[1], L)], other, moved]
+    with G.Ensemble(L, cell_div=cell_div) as ens:
+        for conf in confs:
+            u, pairs = u_of(ens, conf)
+            off = total = 0
+            for x, l in zip(conf, L):
+                with G.Ensemble([l], cell_div=cell_div) as one:
+                    want, p = u_of(one, [x])
+                assert np.array_equal(u[off:off + len(x)], want)
+                off += len(x)
+                total += p
+            assert pairs == total
+        alone = []
+        for b in range(4):
+            with G.Context(box_hi=(L[b],) * 3, precision=G.FP32, cell_div=cell_div) as ctx:
+                ctx.set_particles(confs[-1][b])
+                ctx.build_cells()
+                alone.append(ctx.lanczos_bounds(12, 7))
+        assert [ens.lanczos(b, 12, 7) for b in range(4)] == alone
+        bad = np.concatenate(moved)
+        bad[sum(counts[:2]) + 5, 1] = np.nan
+        with pytest.raises(G.GGEMError, match="suspension 2") as e:
+            ens.set_particles_dev(counts, _device(bad).data_ptr())
+        assert e.value.code == G.ERR_BAD_ARG
+        u, _ = u_of(ens, moved)
+        assert np.all(np.isfinite(u))
