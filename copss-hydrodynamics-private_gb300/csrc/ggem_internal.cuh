@@ -233,6 +233,7 @@ struct ggem_ctx {
   ggem::DevBuf<float> w_fb2;    // the next term's staging in a fused batched series
   ggem::DevBuf<double> w_red;   // reduction partials
   ggem::DevBuf<double> lz_Q;    // Lanczos basis
+  ggem::DevBuf<unsigned char> lz_state;  // its scalars (ggem_cheb.cu, LanczosState)
   double *h_red = nullptr;      // pinned host mirror of reductions
   cudaEvent_t ev_readback = nullptr;  // recorded behind the reductions' readback
   // host inputs of ggem_brownian_displacement: copied on their own stream
