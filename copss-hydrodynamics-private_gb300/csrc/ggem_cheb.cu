@@ -263,8 +263,6 @@ __global__ void k_axpy_into(int64_t tot, double s, const double *__restrict__ a,
 // fused multiply-adds (two lanes per SM and clock bound them: 15 us per pass
 // over 12 vectors at N = 200k).  N = 200k, k = 24: 5.47 -> 2.83 ms.
 constexpr int kLzThreads = 256;
-constexpr int kLzElems = 8;                        // elements per thread and tile
-constexpr int kLzTile = kLzThreads * kLzElems;
 constexpr int kLzBlocks = 608;                     // four per SM
 constexpr int kLzMax = 512;                        // steps
 
@@ -273,8 +271,14 @@ struct LanczosState {
   unsigned int arrived;  // blocks of the running reduction, zero between kernels
 };
 
+// elements per thread and tile: eight spread the cost of a warp's sums over
+// eight multiply-adds, one and two where eight would leave SMs without a tile
+int lz_elems(int64_t D) {
+  return D >= 8 * kLzThreads * 152 ? 8 : (D >= 2 * kLzThreads * 152 ? 2 : 1);
+}
 int lz_blocks(int64_t D) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((D + kLzTile - 1) / kLzTile, kLzBlocks));
+  const int64_t tile = (int64_t)kLzThreads * lz_elems(D);
+  return (int)std::max<int64_t>(1, std::min<int64_t>((D + tile - 1) / tile, kLzBlocks));
 }
 
 // true in every thread of the last block to arrive; the others' partials
@@ -345,6 +349,7 @@ __device__ __forceinline__ double warp_sum8(double v[8]) {
 }
 
 // w -= alpha_j q_j + beta_{j-1} q_{j-1}; h_i = Q_i . w for i <= j
+template <int kLzElems>
 __global__ void __launch_bounds__(kLzThreads) k_lz_project(int64_t D, int j,
                                                            const double *__restrict__ Q,
                                                            double *__restrict__ w,
@@ -356,6 +361,7 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_project(int64_t D, int j,
   for (int i = threadIdx.x; i < (kLzThreads / 32) * m8; i += kLzThreads) sh[i] = 0.0;
   __syncthreads();
   const double al = S->alpha[j], be = j > 0 ? S->beta[j - 1] : 0.0;
+  constexpr int kLzTile = kLzThreads * kLzElems;
   const double *qj = Q + (int64_t)j * D, *qp = Q + (int64_t)(j > 0 ? j - 1 : 0) * D;
   for (int64_t t0 = blockIdx.x * (int64_t)kLzTile; t0 < D; t0 += (int64_t)gridDim.x * kLzTile) {
     double v[kLzElems];
@@ -402,6 +408,7 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_project(int64_t D, int j,
 
 // w -= sum_{i < m} h_i Q_i; beta_j = |w| and its reciprocal (m = 0: the norm
 // of the start vector)
+template <int kLzElems>
 __global__ void __launch_bounds__(kLzThreads) k_lz_update(int64_t D, int m,
                                                           const double *__restrict__ Q,
                                                           double *__restrict__ w,
@@ -411,6 +418,7 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_update(int64_t D, int m,
   __shared__ double red[32];
   for (int i = threadIdx.x; i < m; i += kLzThreads) sh[i] = S->h[i];
   __syncthreads();
+  constexpr int kLzTile = kLzThreads * kLzElems;
   double acc = 0.0;
   for (int64_t t0 = blockIdx.x * (int64_t)kLzTile; t0 < D; t0 += (int64_t)gridDim.x * kLzTile) {
     double v[kLzElems];
@@ -682,10 +690,13 @@ constexpr int kRestartCheb = 1;
 // spec_dw (optional, caller order): every error check also queues M dw into
 // it before the host waits for the check's readback; when the series ends at
 // a check, *spec_done says that spec_dw already holds M y.
+// out (optional, caller order): a series that runs as one launch writes y
+// (out_y) or, once converged, M y there itself and sets *out_done.
 int cheb_slots_impl(ggem_ctx *c, int nrhs, int N, double eig_min, double eig_max, double tol,
                     int check_every, const double *xi, ggem_cheb_report *rep, bool *dm_is_my,
-                    double *spec_dw, bool *spec_done) {
+                    double *spec_dw, bool *spec_done, double *out, bool out_y, bool *out_done) {
   if (spec_done) *spec_done = false;
+  *out_done = false;
   const int64_t D = 3 * c->n;
   const int sm = brownian_self_mode(c);
   const bool faithful = check_every == 1;
@@ -742,6 +753,37 @@ int cheb_slots_impl(ggem_ctx *c, int nrhs, int N, double eig_min, double eig_max
   const int k_first = (check_every == 0) ? std::max(2, c->cheb_pred_terms > 0 ? c->cheb_pred_terms : 8)
                                          : 0;
   *dm_is_my = false;
+  // the degree the next adaptive call checks first (see the end)
+  auto predict = [&](int first_check) {
+    int worst = 0;
+    bool all = true;
+    for (int r = 0; r < nrhs; ++r) {
+      all = all && rep[r].converged;
+      worst = std::max(worst, rep[r].n_terms);
+    }
+    // The series error shrinks by about rho = (sqrt(k) - 1) / (sqrt(k) + 1)
+    // per degree (k = eig_max / eig_min, the Chebyshev rate for x^(-1/2));
+    // the next call tries one degree less only when the first check passed
+    // with that much room, so a workload converging at a steady degree does
+    // not pay a failing check (an extra matvec and host round trip) every
+    // other call.
+    double e1 = 0.0;
+    for (int r = 0; r < nrhs; ++r) e1 = std::max(e1, rep[r].err1);
+    const double kap = eig_min > 0 ? eig_max / eig_min : 1e30;
+    const double rho = (std::sqrt(kap) - 1.0) / (std::sqrt(kap) + 1.0);
+    const bool lower = worst == first_check && e1 <= 0.8 * rho * tol;
+    if (all) c->cheb_pred_terms = lower ? std::max(2, worst - 1) : worst;
+  };
+  if (nrhs == 1 && out && c->prm.precision == GGEM_FP64) {
+    int first = -1;
+    if (int rc = series_f64(c, N, X.data(), da, db, tol, check_every, k_first, sm, xi, out, out_y,
+                            rep, &first, out_done))
+      return rc;
+    if (*out_done) {
+      if (check_every == 0) predict(first);
+      return GGEM_OK;
+    }
+  }
   // x0 = xi; x1 = M x0; aux2 = x1.x0; x1 = db x0 + da x1   (:1036-1041)
   // dw = c0 x0, dw += c1 x1 (with both norms unless fused)  (:1050-1056)
   bool records_fresh = false;
@@ -1032,34 +1074,16 @@ int cheb_slots_impl(ggem_ctx *c, int nrhs, int N, double eig_min, double eig_max
     x1 = xm;
     xm = t;
   }
-  if (check_every == 0) {
-    int worst = 0;
-    bool all = true;
-    for (int r = 0; r < nrhs; ++r) {
-      all = all && rep[r].converged;
-      worst = std::max(worst, rep[r].n_terms);
-    }
-    // The series error shrinks by about rho = (sqrt(k) - 1) / (sqrt(k) + 1)
-    // per degree (k = eig_max / eig_min, the Chebyshev rate for x^(-1/2));
-    // the next call tries one degree less only when the first check passed
-    // with that much room, so a workload converging at a steady degree does
-    // not pay a failing check (an extra matvec and host round trip) every
-    // other call.
-    double e1 = 0.0;
-    for (int r = 0; r < nrhs; ++r) e1 = std::max(e1, rep[r].err1);
-    const double kap = eig_min > 0 ? eig_max / eig_min : 1e30;
-    const double rho = (std::sqrt(kap) - 1.0) / (std::sqrt(kap) + 1.0);
-    const bool lower = worst == first_check && e1 <= 0.8 * rho * tol;
-    if (all) c->cheb_pred_terms = lower ? std::max(2, worst - 1) : worst;
-  }
+  if (check_every == 0) predict(first_check);
   return GGEM_OK;
 }
 
 int cheb_slots(ggem_ctx *c, int nrhs, int N, double eig_min, double eig_max, double tol,
                int check_every, const double *xi, ggem_cheb_report *rep, bool *dm_is_my,
-               double *spec_dw = nullptr, bool *spec_done = nullptr) {
+               double *out, bool out_y, bool *out_done, double *spec_dw = nullptr,
+               bool *spec_done = nullptr) {
   const int rc = cheb_slots_impl(c, nrhs, N, eig_min, eig_max, tol, check_every, xi, rep,
-                                 dm_is_my, spec_dw, spec_done);
+                                 dm_is_my, spec_dw, spec_done, out, out_y, out_done);
   kt_span_end(c);  // a span left open by an early return or a series ending unchecked
   return rc;
 }
@@ -1096,11 +1120,13 @@ extern "C" int ggem_cheb_inv_sqrt_dev(ggem_ctx *ctx, int nrhs, int N, double eig
   DeviceGuard dg(ctx->device);
   const size_t len = (size_t)ctx->n * 3 * nrhs;
   if (int rc = ensure_cheb_buffers(ctx, len)) return rc;
-  bool dm_is_my = false;
-  int rc = cheb_slots(ctx, nrhs, N, eig_min, eig_max, tol_cheb, check_every, d_xi, rep, &dm_is_my);
+  bool dm_is_my = false, out_done = false;
+  int rc = cheb_slots(ctx, nrhs, N, eig_min, eig_max, tol_cheb, check_every, d_xi, rep, &dm_is_my,
+                      d_xi, true, &out_done);
   if (rc == kRestartCheb)  // the deferred list was rebuilt wider: run the series again
-    rc = cheb_slots(ctx, nrhs, N, eig_min, eig_max, tol_cheb, check_every, d_xi, rep, &dm_is_my);
-  if (rc) return rc;
+    rc = cheb_slots(ctx, nrhs, N, eig_min, eig_max, tol_cheb, check_every, d_xi, rep, &dm_is_my,
+                    d_xi, true, &out_done);
+  if (rc || out_done) return rc;
   return permute_from_slots(ctx, nrhs, ctx->w_y.p, d_xi);
 }
 
@@ -1175,15 +1201,15 @@ extern "C" int ggem_brownian_displacement_dev(ggem_ctx *ctx, int nrhs, int N, do
   DeviceGuard dg(ctx->device);
   const size_t len = (size_t)ctx->n * 3 * nrhs;
   if (int rc = ensure_cheb_buffers(ctx, len)) return rc;
-  bool dm_is_my = false, spec_done = false;
+  bool dm_is_my = false, spec_done = false, out_done = false;
   // d_dw is the caller's output alone (unless it is xi itself), so every
   // check may already queue M dw into it (overwritten if the series goes on)
   double *spec = d_dw != d_xi ? d_dw : nullptr;
   int rc = cheb_slots(ctx, nrhs, N, eig_min, eig_max, tol_cheb, check_every, d_xi, rep, &dm_is_my,
-                      spec, &spec_done);
+                      d_dw, false, &out_done, spec, &spec_done);
   if (rc == kRestartCheb)  // the deferred list was rebuilt wider: run the series again
     rc = cheb_slots(ctx, nrhs, N, eig_min, eig_max, tol_cheb, check_every, d_xi, rep, &dm_is_my,
-                    spec, &spec_done);
+                    d_dw, false, &out_done, spec, &spec_done);
   if (rc) return rc;
   bool all = true;
   for (int r = 0; r < nrhs; ++r) all = all && rep[r].converged;
@@ -1192,7 +1218,7 @@ extern "C" int ggem_brownian_displacement_dev(ggem_ctx *ctx, int nrhs, int N, do
                       "Chebyshev polynomial fails to converge (brownian_system.C:1162-1163)");
   // hi_ewald: dw = M y (copss.C:1686); the last error check already
   // computed M y when it ran on the final y (and queued it into d_dw)
-  if (spec_done) return GGEM_OK;
+  if (spec_done || out_done) return GGEM_OK;
   if (!dm_is_my) {
     if (int rc = matvec_slots(ctx, nrhs, ctx->w_y.p, ctx->w_out.p, brownian_self_mode(ctx)))
       return rc;
@@ -1225,7 +1251,10 @@ extern "C" int ggem_lanczos_bounds(ggem_ctx *ctx, int k, uint64_t seed, double *
   // start vector: N(0,1) from the counter-based generator, normalised
   k_philox_normals<<<(unsigned)(((D + 3) / 4 + 255) / 256), 256, 0, st>>>(D, seed, 0x4C414E43ull, Q);
   if (int rc = check_launch(ctx, "lanczos start")) return rc;
-  k_lz_update<<<G, kLzThreads, 0, st>>>(D, 0, Q, Q, part, S, 0);
+  const int E = lz_elems(D);
+  auto project = E == 8 ? k_lz_project<8> : (E == 2 ? k_lz_project<2> : k_lz_project<1>);
+  auto update = E == 8 ? k_lz_update<8> : (E == 2 ? k_lz_update<2> : k_lz_update<1>);
+  update<<<G, kLzThreads, 0, st>>>(D, 0, Q, Q, part, S, 0);
   if (int rc = check_launch(ctx, "lanczos norm")) return rc;
   k_lz_next<<<grid1(D), 256, 0, st>>>(D, Q, Q, S);
   if (int rc = check_launch(ctx, "lanczos next")) return rc;
@@ -1236,9 +1265,9 @@ extern "C" int ggem_lanczos_bounds(ggem_ctx *ctx, int k, uint64_t seed, double *
     if (int rc = check_launch(ctx, "lanczos alpha")) return rc;
     if (j == k - 1) break;  // (the last beta is not used)
     const size_t sh = sizeof(double) * (kLzThreads / 32) * 8 * ((j + 8) / 8);
-    k_lz_project<<<G, kLzThreads, sh, st>>>(D, j, Q, w, part, S);
+    project<<<G, kLzThreads, sh, st>>>(D, j, Q, w, part, S);
     if (int rc = check_launch(ctx, "lanczos project")) return rc;
-    k_lz_update<<<G, kLzThreads, sizeof(double) * (j + 1), st>>>(D, j + 1, Q, w, part, S, j);
+    update<<<G, kLzThreads, sizeof(double) * (j + 1), st>>>(D, j + 1, Q, w, part, S, j);
     if (int rc = check_launch(ctx, "lanczos update")) return rc;
     k_lz_next<<<grid1(D), 256, 0, st>>>(D, w, Q + (size_t)(j + 1) * D, S);
     if (int rc = check_launch(ctx, "lanczos next")) return rc;

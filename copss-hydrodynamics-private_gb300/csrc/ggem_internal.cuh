@@ -232,6 +232,9 @@ struct ggem_ctx {
   ggem::DevBuf<float> w_fb;     // batched forces [slot][3][64] FP32
   ggem::DevBuf<float> w_fb2;    // the next term's staging in a fused batched series
   ggem::DevBuf<double> w_red;   // reduction partials
+  // the one-launch FP64 series: control block and coefficients; its vectors
+  ggem::DevBuf<double> s64_tab;
+  ggem::DevBuf<double4_32a> s64_vec;
   ggem::DevBuf<double> lz_Q;    // Lanczos basis
   ggem::DevBuf<unsigned char> lz_state;  // its scalars (ggem_cheb.cu, LanczosState)
   double *h_red = nullptr;      // pinned host mirror of reductions
@@ -392,6 +395,9 @@ void batch_tensors(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st);
 // pair sums (ggem_pair.cu); vectors in slot order, [r][slot][3] doubles
 int matvec_slots(ggem_ctx *c, int nrhs, const double *d_f_slot, double *d_u_slot,
                  int self_mode);
+int series_f64(ggem_ctx *c, int N, const double *coef, double da, double db, double tol,
+               int check_every, int k_first, int self_mode, const double *xi, double *out,
+               bool out_y, ggem_cheb_report *rep, int *first_check, bool *done);
 int matvec_f32_staged(ggem_ctx *c, int nrhs, const double *d_f_slot, double *d_u_slot,
                       int self_mode);
 // the batched series' first step (x1 = db x0 + da x1, dw = c0 x0 + c1 x1)

@@ -187,6 +187,48 @@ __global__ void __launch_bounds__(128) k_matvec_f64(int64_t n, Grid g, DevConsts
   }
 }
 
+// the row of one target: G lanes take every G-th entry and add their sums by
+// shuffles (every lane holds the totals).  NC: f is constant during the
+// kernel (read-only loads); otherwise it is read through L2.
+template <int NR, int G, bool NC>
+__device__ __forceinline__ void pair_row_f64(int sub, int m, const uint32_t *__restrict__ row,
+                                             const double4_32a &pi, const MinImage &mi,
+                                             const DevConsts &K, const Tensor64 &T,
+                                             long long eps2,
+                                             const double4_32a *__restrict__ pos64,
+                                             const double *f, int64_t vstride,
+                                             double acc[NR][3]) {
+#pragma unroll
+  for (int q = 0; q < NR; ++q) acc[q][0] = acc[q][1] = acc[q][2] = 0.0;
+  uint32_t nxt = sub < m ? __ldg(row + sub) : 0u;
+  for (int k = sub; k < m; k += G) {
+    const int64_t t = (int64_t)(nxt >> kCodeBits);
+    if (k + G < m) nxt = __ldg(row + k + G);
+    const double4_32a pj = ld_f64x4(pos64 + t);
+    const double x = min_image_bits(pj.x - pi.x, mi.half[0], mi.L[0]);
+    const double y = min_image_bits(pj.y - pi.y, mi.half[1], mi.L[1]);
+    const double z = min_image_bits(pj.z - pi.z, mi.half[2], mi.L[2]);
+    double A, B;
+    tensor64(T, fma(z, z, fma(y, y, x * x)), eps2, K.coeff_2, A, B);
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      const double *fj = f + q * vstride + 3 * t;
+      const double f0 = NC ? __ldg(fj) : __ldcg(fj), f1 = NC ? __ldg(fj + 1) : __ldcg(fj + 1),
+                   f2 = NC ? __ldg(fj + 2) : __ldcg(fj + 2);
+      const double xf = B * fma(z, f2, fma(y, f1, x * f0));
+      acc[q][0] = fma(A, f0, fma(xf, x, acc[q][0]));
+      acc[q][1] = fma(A, f1, fma(xf, y, acc[q][1]));
+      acc[q][2] = fma(A, f2, fma(xf, z, acc[q][2]));
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < G; o <<= 1)
+#pragma unroll
+    for (int q = 0; q < NR; ++q)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) acc[q][a] += __shfl_xor_sync(0xffffffffu, acc[q][a], o);
+}
+
 // FP64 pair sum over the pair list (cut-off lists and element lists alike):
 // minimum image of the wrapped FP64 positions (pm_periodic_boundary.C:350-374)
 // and green_tensor_local_regularized (ggem_stokes.C:304-357) as its piecewise
@@ -218,36 +260,8 @@ __global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, MinImage mi, D
   const double4_32a pi = ld_f64x4(pos64 + s);
   const int64_t vstride = 3 * n;
   double acc[NR][3];
-#pragma unroll
-  for (int q = 0; q < NR; ++q) acc[q][0] = acc[q][1] = acc[q][2] = 0.0;
-  const int m = act ? cnt[s] : 0;
-  const uint32_t *row = list + s * (int64_t)W;
-  uint32_t nxt = sub < m ? __ldg(row + sub) : 0u;
-  for (int k = sub; k < m; k += G) {
-    const int64_t t = (int64_t)(nxt >> kCodeBits);
-    if (k + G < m) nxt = __ldg(row + k + G);
-    const double4_32a pj = ld_f64x4(pos64 + t);
-    const double x = min_image_bits(pj.x - pi.x, mi.half[0], mi.L[0]);
-    const double y = min_image_bits(pj.y - pi.y, mi.half[1], mi.L[1]);
-    const double z = min_image_bits(pj.z - pi.z, mi.half[2], mi.L[2]);
-    double A, B;
-    tensor64(T, fma(z, z, fma(y, y, x * x)), eps2, K.coeff_2, A, B);
-#pragma unroll
-    for (int q = 0; q < NR; ++q) {
-      const double *fj = f + (int64_t)(r0 + q) * vstride + 3 * t;
-      const double f0 = __ldg(fj), f1 = __ldg(fj + 1), f2 = __ldg(fj + 2);
-      const double xf = B * fma(z, f2, fma(y, f1, x * f0));
-      acc[q][0] = fma(A, f0, fma(xf, x, acc[q][0]));
-      acc[q][1] = fma(A, f1, fma(xf, y, acc[q][1]));
-      acc[q][2] = fma(A, f2, fma(xf, z, acc[q][2]));
-    }
-  }
-#pragma unroll
-  for (int o = 1; o < G; o <<= 1)
-#pragma unroll
-    for (int q = 0; q < NR; ++q)
-#pragma unroll
-      for (int a = 0; a < 3; ++a) acc[q][a] += __shfl_xor_sync(0xffffffffu, acc[q][a], o);
+  pair_row_f64<NR, G, true>(sub, act ? cnt[s] : 0, list + s * (int64_t)W, pi, mi, K, T, eps2,
+                            pos64, f + (int64_t)r0 * vstride, vstride, acc);
   if (!act || sub != 0) return;
 #pragma unroll
   for (int q = 0; q < NR; ++q) {
@@ -259,6 +273,376 @@ __global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, MinImage mi, D
     ui[1] = acc[q][1];
     ui[2] = acc[q][2];
   }
+}
+
+// ---- the FP64 Chebyshev series of one right-hand side in one launch --------
+// The loop of brownian_system.C:1036-1155 as one cooperative kernel.  Phase i
+// applies M to x_i and, where the degree-i sum dw_i is to be checked, to dw_i
+// in the same row walk (the tensors are formed once for both): the products
+// give the check of dw_i and, ahead of its decision, x_{i+1} and dw_{i+1}.  A
+// grid barrier ends the phase; its last block adds the estimator partials in
+// a fixed order and decides, so the host neither launches nor waits per term
+// (one product is in vain when the series stops).  Vectors travel as 32-byte
+// records through L2 and rotate, so that a phase writes only buffers that no
+// block reads in it.  G lanes walk a target's row; a reduce-scatter leaves
+// each of the six sums (and its component of the vectors) on one lane.
+//
+// CACHE > 0: the first CACHE entries of every lane keep their tensor (six
+// FP64 values) in registers over all phases, which leaves one gather and 18
+// FP64 instructions per pair and phase instead of a list, a position and a
+// tensor gather and 40.  It takes every target resident in one round.
+//
+// Bound: at small counts the barriers and one L2 gather per phase (~7 us a
+// phase at N = 1000), at large ones the FP64 pipe.  us per series, single
+// launches with host checks -> one launch: N = 1000 (7 terms) 431 -> 119,
+// 6000 698 -> 315, 20k 1779 -> 1291, 200k 10476 -> 9075.
+//
+// Waits are bounded (polls): a block that gives up sets the error word and
+// leaves, and so do the others.
+struct SeriesCtl {
+  unsigned int arrive, release;
+  int stop, err;
+  int n_terms, n_matvecs, converged, first_check;
+  double err1, err2, aux2, n0, n1;  // n0 = |dw_{i-1}|^2, n1 = |x_i|^2 of the sum to be checked
+};
+
+struct SeriesF64 {
+  int64_t n;
+  int W, N, rounds, self_mode, check_every, k_first, out_y;
+  uint32_t polls;
+  double da, db, tol;
+  MinImage mi;
+  DevConsts K;
+  Tensor64 T;
+  long long eps2;
+  const int32_t *cnt, *order;
+  const uint32_t *list;
+  const double4_32a *pos64;
+  const double *coef;         // [N + 1]
+  const double *xi;           // caller order
+  double4_32a *x[3], *d[2];   // x_{i-1}, x_i, x_{i+1}; dw_i, dw_{i+1} (rotating)
+  double *dm;                 // M dw of the last check
+  double *out;                // caller order: y (out_y), or M y once converged
+  double *part;               // [3][blocks] partial sums
+  SeriesCtl *ctl;
+};
+
+__device__ __forceinline__ void ld_vec(const double4_32a *p, double &x, double &y, double &z) {
+  const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
+  x = a.x;
+  y = a.y;
+  z = __ldcg(reinterpret_cast<const double *>(p) + 2);
+}
+
+// the sums of v[0..7] over the G lanes of a target: lane sub returns v[0] =
+// sum of v[index], index = sub / (G / 8) (G = 4: v[0], v[1] of 2 sub, 2 sub + 1)
+template <int G>
+__device__ __forceinline__ void group_sum8(int sub, double v[8]) {
+  constexpr int kSplit = G >= 8 ? 3 : 2;
+  int o = G / 2;
+#pragma unroll
+  for (int l = 0; l < kSplit; ++l, o >>= 1) {
+    const int half = 4 >> l;
+    const bool up = sub & o;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i >= half) break;
+      const double keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+}
+
+template <int CACHE>
+struct PairCache {
+  double g[CACHE > 0 ? CACHE : 1][6];  // xx, xy, xz, yy, yz, zz
+  int t[CACHE > 0 ? CACHE : 1];        // source slot, -1 past the row's end
+};
+
+// v[0..2] += G f(t), v[4..6] += G d(t)
+__device__ __forceinline__ void add_pair(const double g[6], const double4_32a *xv,
+                                         const double4_32a *dv, double v[8]) {
+  if (xv) {
+    double f0, f1, f2;
+    ld_vec(xv, f0, f1, f2);
+    v[0] = fma(g[0], f0, fma(g[1], f1, fma(g[2], f2, v[0])));
+    v[1] = fma(g[1], f0, fma(g[3], f1, fma(g[4], f2, v[1])));
+    v[2] = fma(g[2], f0, fma(g[4], f1, fma(g[5], f2, v[2])));
+  }
+  if (dv) {
+    double f0, f1, f2;
+    ld_vec(dv, f0, f1, f2);
+    v[4] = fma(g[0], f0, fma(g[1], f1, fma(g[2], f2, v[4])));
+    v[5] = fma(g[1], f0, fma(g[3], f1, fma(g[4], f2, v[5])));
+    v[6] = fma(g[2], f0, fma(g[4], f1, fma(g[5], f2, v[6])));
+  }
+}
+
+constexpr int kSeriesThreads = 128;
+
+template <int G, int CACHE>
+__global__ void __launch_bounds__(kSeriesThreads, CACHE ? 3 : 7) k_series_f64(SeriesF64 a) {
+  __shared__ double sh[3][kSeriesThreads / 32];
+  __shared__ int s_last, s_ok;
+  const int sub = threadIdx.x % G;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kT = kSeriesThreads / G;  // targets per block and round
+  constexpr int kSpread = G >= 8 ? G / 8 : 1, kVal = G >= 8 ? 1 : 2;
+  const int64_t n = a.n;
+  const bool faithful = a.check_every == 1;
+  const int64_t first = blockIdx.x * (int64_t)(kT * a.rounds) + threadIdx.x / G;
+  PairCache<CACHE> pc;
+  // the tensor of entry en seen from position pi
+  auto tensor = [&](uint32_t en, const double4_32a &pi, double g[6]) {
+    const double4_32a pj = ld_f64x4(a.pos64 + (en >> kCodeBits));
+    const double x = min_image_bits(pj.x - pi.x, a.mi.half[0], a.mi.L[0]);
+    const double y = min_image_bits(pj.y - pi.y, a.mi.half[1], a.mi.L[1]);
+    const double z = min_image_bits(pj.z - pi.z, a.mi.half[2], a.mi.L[2]);
+    double A, B;
+    tensor64(a.T, fma(z, z, fma(y, y, x * x)), a.eps2, a.K.coeff_2, A, B);
+    const double bx = B * x, by = B * y;
+    g[0] = fma(bx, x, A);
+    g[1] = bx * y;
+    g[2] = bx * z;
+    g[3] = fma(by, y, A);
+    g[4] = by * z;
+    g[5] = fma(B * z, z, A);
+  };
+  if (CACHE) {
+    const int64_t s = min(first, n - 1);
+    const int m = first < n ? __ldg(a.cnt + s) : 0;
+    const double4_32a pi = ld_f64x4(a.pos64 + s);
+#pragma unroll
+    for (int p = 0; p < CACHE; ++p) {
+      const int k = sub + p * G;
+      pc.t[p] = -1;
+      if (k < m) {
+        const uint32_t en = __ldg(a.list + s * (int64_t)a.W + k);
+        pc.t[p] = (int)(en >> kCodeBits);
+        tensor(en, pi, pc.g[p]);
+      }
+    }
+  }
+  // M xv (v[0..2]) and M dv (v[4..6]) pair sums of slot s; null: not wanted
+  auto walk = [&](int64_t s, bool act, const double4_32a *xv, const double4_32a *dv, double v[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = 0.0;
+    const int m = act ? __ldg(a.cnt + s) : 0;
+    if (CACHE) {
+#pragma unroll
+      for (int p = 0; p < CACHE; ++p)
+        if (pc.t[p] >= 0)
+          add_pair(pc.g[p], xv ? xv + pc.t[p] : nullptr, dv ? dv + pc.t[p] : nullptr, v);
+    }
+    if (m > CACHE * G) {
+      const double4_32a pi = ld_f64x4(a.pos64 + s);
+      const uint32_t *row = a.list + s * (int64_t)a.W;
+      for (int k = CACHE * G + sub; k < m; k += G) {
+        const uint32_t en = __ldg(row + k);
+        const int64_t t = (int64_t)(en >> kCodeBits);
+        double g[6];
+        tensor(en, pi, g);
+        add_pair(g, xv ? xv + t : nullptr, dv ? dv + t : nullptr, v);
+      }
+    }
+    group_sum8<G>(sub, v);
+  };
+  auto with_self = [&](double u, double own) {
+    if (a.self_mode == GGEM_SELF_BEAD) return (u - a.K.coeff_1 * own) + own;
+    if (a.self_mode == GGEM_SELF_LAGRANGIAN) return u + a.K.coeff_2 * own;
+    return u;
+  };
+  auto comp = [](const double4_32a *p, int c) {
+    return __ldcg(reinterpret_cast<const double *>(p) + c);
+  };
+  auto put = [](double4_32a *p, int c, double v) { reinterpret_cast<double *>(p)[c] = v; };
+  // f(slot, active) over this block's targets, all lanes together
+  auto targets = [&](auto &&f) {
+    for (int r = 0; r < a.rounds; ++r) {
+      const int64_t s = first + (int64_t)r * kT;
+      f(min(s, n - 1), s < n);
+    }
+  };
+  // f(component, vector (0: x, 1: dw), value) for the sums this lane holds
+  auto mine = [&](bool act, const double v[8], auto &&f) {
+    if (!act || sub % kSpread) return;
+#pragma unroll
+    for (int q = 0; q < kVal; ++q) {
+      const int idx = G >= 8 ? sub / kSpread : 2 * sub + q;
+      if ((idx & 3) < 3) f(idx & 3, idx >> 2, v[q]);
+    }
+  };
+  unsigned gen = 0;
+  // the end of a phase: this block's three partials, then all blocks arrive;
+  // the last one runs work(sum0, sum1, sum2) on its first thread and releases
+  // the others.  False: a wait ran out.
+  auto barrier = [&](double p0, double p1, double p2, auto &&work) -> bool {
+    ++gen;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      p0 += __shfl_xor_sync(0xffffffffu, p0, o);
+      p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+      p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+    }
+    if (lane == 0) {
+      sh[0][warp] = p0;
+      sh[1][warp] = p1;
+      sh[2][warp] = p2;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kSeriesThreads / 32; ++w) t += sh[q][w];
+        __stcg(a.part + (int64_t)q * gridDim.x + blockIdx.x, t);
+      }
+      __threadfence();
+      s_last = atomicAdd(&a.ctl->arrive, 1u) == gen * gridDim.x - 1u;
+      s_ok = 1;
+    }
+    __syncthreads();
+    if (s_last) {
+      __threadfence();
+      if (warp < 3) {  // one warp per partial
+        double t = 0.0;
+        for (unsigned b = lane; b < gridDim.x; b += 32)
+          t += __ldcg(a.part + (int64_t)warp * gridDim.x + b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sh[warp][0] = t;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        work(sh[0][0], sh[1][0], sh[2][0]);
+        __threadfence();
+        atomicExch(&a.ctl->release, gen);
+      }
+    } else if (threadIdx.x == 0) {
+      uint32_t k = 0;
+      while (*(volatile unsigned int *)&a.ctl->release < gen) {
+        if (*(volatile int *)&a.ctl->err || ++k > a.polls) {
+          atomicOr(&a.ctl->err, kErrTimeout);
+          s_ok = 0;
+          break;
+        }
+        __nanosleep(20);
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0;
+  };
+
+  double4_32a *xp = a.x[0], *xc = a.x[1], *xn = a.x[2], *dc = a.d[0], *dn = a.d[1];
+  double v[8];
+  // x_0 = xi
+  targets([&](int64_t s, bool act) {
+    if (act && sub < 3) put(xp + s, sub, a.xi[3 * (int64_t)a.order[s] + sub]);
+  });
+  if (!barrier(0.0, 0.0, 0.0, [](double, double, double) {})) return;
+  // m = M x_0; aux2 = m . x_0; x_1 = db x_0 + da m; dw_1 = c0 x_0 + c1 x_1
+  {
+    double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+    const double c0 = a.coef[0], c1 = a.coef[1];
+    targets([&](int64_t s, bool act) {
+      walk(s, act, xp, nullptr, v);
+      mine(act, v, [&](int c, int vec, double u) {
+        if (vec) return;
+        const double x = comp(xp + s, c);
+        const double m = with_self(u, x);
+        const double w = a.db * x + a.da * m;
+        const double t = c0 * x;
+        put(xc + s, c, w);
+        put(dc + s, c, t + c1 * w);
+        p0 = fma(t, t, p0);
+        p1 = fma(w, w, p1);
+        p2 = fma(m, x, p2);
+      });
+    });
+    const bool ok = barrier(p0, p1, p2, [&](double s0, double s1, double s2) {
+      a.ctl->aux2 = s2;
+      a.ctl->n0 = s0;
+      a.ctl->n1 = s1;
+      a.ctl->n_terms = 1;
+      a.ctl->n_matvecs = 1;
+    });
+    if (!ok) return;
+  }
+  for (int i = 1;; ++i) {
+    const int t = i - 1;  // the loop index whose term formed dw_i
+    const bool chk = faithful || (t > 0 && (t == a.N - 1 || (a.check_every > 1
+                                                                ? t % a.check_every == 0
+                                                                : i >= a.k_first)));
+    const bool term = i < a.N;
+    if (!chk && !term) break;
+    const double cn = term ? a.coef[i + 1] : 0.0, ci = a.coef[i];
+    double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+    targets([&](int64_t s, bool act) {
+      if (chk && term) walk(s, act, xc, dc, v);
+      else walk(s, act, term ? xc : nullptr, term ? nullptr : dc, v);
+      mine(act, v, [&](int c, int vec, double u) {
+        if (vec == 0) {
+          if (!term) return;
+          const double x = comp(xc + s, c), y = comp(dc + s, c);
+          double w = (2. * a.db) * x + (2. * a.da) * with_self(u, x);
+          w -= comp(xp + s, c);
+          put(xn + s, c, w);
+          put(dn + s, c, y + cn * w);
+          p0 = fma(y, y, p0);
+          p1 = fma(w, w, p1);
+        } else if (chk) {
+          const double m = with_self(u, comp(dc + s, c));
+          a.dm[3 * s + c] = m;
+          p2 = fma(m, m, p2);
+        }
+      });
+    });
+    const bool ok = barrier(p0, p1, p2, [&](double s0, double s1, double s2) {
+      SeriesCtl &ctl = *a.ctl;
+      if (chk) {
+        const double aux4 = sqrt(ctl.n0), aux3 = sqrt(ctl.n1) * fabs(ci), aux2 = ctl.aux2;
+        ctl.n_matvecs += 1;
+        if (aux2 != 0.0) ctl.err1 = sqrt(fabs(s2 - aux2) / aux2);
+        if (aux4 != 0.0) ctl.err2 = aux3 / aux4;
+        if (t > 0) {
+          if (ctl.first_check < 0) ctl.first_check = i;
+          if (ctl.err1 <= a.tol) {  // brownian_system.C:1138-1147
+            ctl.converged = 1;
+            ctl.stop = 1;
+          } else if (ctl.err2 <= 1E-9) {  // :1150
+            ctl.stop = 1;
+          }
+        }
+      }
+      if (term && !ctl.stop) {
+        ctl.n_matvecs += 1;
+        ctl.n_terms = i + 1;
+      }
+      ctl.n0 = s0;
+      ctl.n1 = s1;
+    });
+    if (!ok) return;
+    if (!term || *(volatile int *)&a.ctl->stop) break;
+    double4_32a *q = xp;
+    xp = xc;
+    xc = xn;
+    xn = q;
+    q = dc;
+    dc = dn;
+    dn = q;
+  }
+  if (!a.out_y && !*(volatile int *)&a.ctl->converged) return;
+  targets([&](int64_t s, bool act) {
+    mine(act, v, [&](int c, int vec, double) {
+      // (M dw is held by the lanes that formed it, y by those of its update)
+      if (vec != (a.out_y ? 0 : 1)) return;
+      a.out[3 * (int64_t)a.order[s] + c] = a.out_y ? comp(dc + s, c) : a.dm[3 * s + c];
+    });
+  });
 }
 
 __device__ __forceinline__ void kahan_add(float &sum, float &comp, float v) {
@@ -1449,6 +1833,33 @@ int launch_f64(ggem_ctx *c, const double *f, double *u, int self_mode, int r0) {
   return check_launch(c, "matvec f64");
 }
 
+// at most max_rounds targets per group of lanes; *done = false: more, or no
+// cooperative launch
+template <int G, int CACHE>
+int launch_series_f64(ggem_ctx *c, SeriesF64 &a, int max_rounds, bool *done) {
+  int sms = 0, per = 0, coop = 0;
+  cudaError_t e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device)) ||
+      (e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device)) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_series_f64<G, CACHE>,
+                                                          kSeriesThreads, 0)))
+    return cuda_fail(c, e, "series occupancy");
+  if (!coop || per < 1) return GGEM_OK;
+  const int64_t kt = kSeriesThreads / G, most = (int64_t)sms * per;
+  a.rounds = (int)((a.n + most * kt - 1) / (most * kt));
+  if (a.rounds > max_rounds) return GGEM_OK;
+  // the same number of rounds in every block
+  const unsigned grid = (unsigned)((a.n + a.rounds * kt - 1) / (a.rounds * kt));
+  if ((e = c->w_red.ensure((size_t)3 * grid))) return cuda_fail(c, e, "series partials");
+  a.part = c->w_red.p;
+  void *args[] = {&a};
+  if ((e = cudaLaunchCooperativeKernel((const void *)k_series_f64<G, CACHE>, dim3(grid),
+                                       dim3(kSeriesThreads), args, 0, c->stream)))
+    return cuda_fail(c, e, "series launch");
+  *done = true;
+  return check_launch(c, "series f64");
+}
+
 PolyAB poly_of(const ggem_ctx *c) {
   PolyAB P;
   for (int q = 0; q <= kPolyDeg; ++q) P.ab[q] = make_float2(c->poly_a[q], c->poly_b[q]);
@@ -1918,6 +2329,83 @@ double self_coefficient(const ggem_ctx *c, int self_mode) {
   if (self_mode == GGEM_SELF_BEAD) return 1.0 - c->cst.coeff_1;
   if (self_mode == GGEM_SELF_LAGRANGIAN) return c->cst.coeff_2;
   return 0.0;
+}
+
+// The whole FP64 series of one right-hand side (k_series_f64): xi and out in
+// caller order, y left in w_y.  *done = false: not taken (no pair list, the
+// kernel timer or the launch trace wants the single launches, a deferred
+// list build to be checked first, or no cooperative launch).
+int series_f64(ggem_ctx *c, int N, const double *coef, double da, double db, double tol,
+               int check_every, int k_first, int self_mode, const double *xi, double *out,
+               bool out_y, ggem_cheb_report *rep, int *first_check, bool *done) {
+  *done = false;
+  if (c->prm.precision != GGEM_FP64 || c->timing || c->trace || c->n == 0) return GGEM_OK;
+  if (int rc = ensure_f64_list(c)) return rc;
+  if (!c->list_built || c->list_unchecked) return GGEM_OK;
+  cudaError_t e;
+  // control block and coefficients in one upload, through pinned memory
+  // where they fit the context's mirror
+  constexpr int kCtl = (sizeof(SeriesCtl) + 7) / 8;
+  const size_t words = kCtl + N + 1;
+  if ((e = c->s64_tab.ensure(words))) return cuda_fail(c, e, "series tables");
+  std::vector<double> big;
+  double *up = c->h_red + 64;
+  if (words > 3072) {
+    big.resize(words);
+    up = big.data();
+  }
+  SeriesCtl ctl;
+  std::memset(&ctl, 0, sizeof(ctl));
+  ctl.first_check = -1;
+  std::memcpy(up, &ctl, sizeof(ctl));
+  std::memcpy(up + kCtl, coef, sizeof(double) * (N + 1));
+  if ((e = cudaMemcpyAsync(c->s64_tab.p, up, sizeof(double) * words, cudaMemcpyHostToDevice,
+                           c->stream)))
+    return cuda_fail(c, e, "series tables");
+  SeriesF64 a;
+  a.n = c->n;
+  a.W = c->nb_w;
+  a.N = N;
+  a.self_mode = self_mode;
+  a.check_every = check_every;
+  a.k_first = k_first;
+  a.out_y = out_y ? 1 : 0;
+  a.polls = 1u << 26;
+  a.da = da;
+  a.db = db;
+  a.tol = tol;
+  a.mi = min_image_of(c->grid);
+  a.K = c->dc;
+  a.T = c->t64;
+  const double e2 = c->dc.r_eps * c->dc.r_eps;
+  std::memcpy(&a.eps2, &e2, 8);
+  a.cnt = c->nb_cnt.p;
+  a.order = c->order.p;
+  a.list = c->nb_list.p;
+  a.pos64 = c->pos64.p;
+  a.coef = c->s64_tab.p + kCtl;
+  a.xi = xi;
+  if ((e = c->s64_vec.ensure(5 * (size_t)c->n))) return cuda_fail(c, e, "series vectors");
+  for (int q = 0; q < 3; ++q) a.x[q] = c->s64_vec.p + q * c->n;
+  for (int q = 0; q < 2; ++q) a.d[q] = c->s64_vec.p + (3 + q) * c->n;
+  a.dm = c->w_out.p;
+  a.out = out;
+  a.ctl = reinterpret_cast<SeriesCtl *>(c->s64_tab.p);
+  int rc = launch_series_f64<16, 4>(c, a, 1, done);
+  if (!rc && !*done) {
+    if (c->n >= 80000) rc = launch_series_f64<4, 0>(c, a, 1 << 30, done);
+    else rc = launch_series_f64<8, 0>(c, a, 1 << 30, done);
+  }
+  if (rc || !*done) return rc;
+  if ((e = cudaMemcpyAsync(c->h_red, c->s64_tab.p, sizeof(ctl), cudaMemcpyDeviceToHost,
+                           c->stream)) ||
+      (e = cudaStreamSynchronize(c->stream)))
+    return cuda_fail(c, e, "series report");
+  std::memcpy(&ctl, c->h_red, sizeof(ctl));
+  if (ctl.err) return fail(c, GGEM_ERR_TIMEOUT, "a wait of the FP64 series ran out");
+  *rep = ggem_cheb_report{ctl.converged, ctl.n_terms, ctl.n_matvecs, ctl.err1, ctl.err2};
+  *first_check = ctl.first_check;
+  return GGEM_OK;
 }
 
 // u = M f on slot-ordered FP64 vectors [r][n][3]
