@@ -1716,24 +1716,50 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 4) k_pair_b64(
   const int64_t s0 = blockIdx.x * (int64_t)kBatchWarps;
   const int ns = (int)(n - s0 < kBatchWarps ? n - s0 : kBatchWarps);
   constexpr int kRow = 3 * kBatchWarps;
-  for (int k = threadIdx.x; k < nr * kRow; k += blockDim.x) {
-    const int r = k / kRow, q = k - r * kRow;
-    const int t = q / 3, c = q - t * 3;
-    if (t >= ns) continue;
-    const float2 v = s_out[t][r][c];
-    const int64_t idx = ((int64_t)r * n + s0) * 3 + q;
-    double m = f2d_bits(v.x) + f2d_bits(v.y);
-    if (CHEB) {
-      // x_{k+1} = 2da M x_k + (2db x_k - x_{k-1}), dw += c x_{k+1}: four
-      // FP64 operations per element with the add above (FP64 issues at a
-      // small fraction of the FP32 rate on this GPU)
-      const double x = fma(two_da, m, fma(two_db, x1[idx], -x0[idx]));
-      dw[idx] = fma(cf.c[r], x, dw[idx]);
-      m = x;
-      // FP32 staging of x_{k+1}, transposed through shared memory below
-      reinterpret_cast<float *>(&s_out[t][r][c])[0] = d2f_bits(x);
+  if (CHEB) {
+    // x_{k+1} = 2da M x_k + (2db x_k - x_{k-1}), dw += c x_{k+1}: four FP64
+    // operations per element with the add below (FP64 issues at a small
+    // fraction of the FP32 rate on this GPU).  The vectors exceed L2, so
+    // three elements' nine loads are in flight before the first is used (one
+    // element at a time waited out three DRAM latencies per pass: 5.95 ->
+    // 5.46 ms per 14-term step of N = 100k chains)
+    constexpr int kFly = 3;
+    const int total = nr * kRow;
+    for (int k0 = threadIdx.x; k0 < total; k0 += kFly * 32 * kBatchWarps) {
+      double va[kFly], vb[kFly], vd[kFly];
+      int64_t at[kFly];
+#pragma unroll
+      for (int i = 0; i < kFly; ++i) {
+        const int k = k0 + i * 32 * kBatchWarps, r = k / kRow, q = k - r * kRow;
+        at[i] = k < total && q < 3 * ns ? ((int64_t)r * n + s0) * 3 + q : -1;
+        if (at[i] >= 0) {
+          va[i] = x0[at[i]];
+          vb[i] = x1[at[i]];
+          vd[i] = dw[at[i]];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kFly; ++i) {
+        if (at[i] < 0) continue;
+        const int k = k0 + i * 32 * kBatchWarps, r = k / kRow, q = k - r * kRow;
+        const int t = q / 3, c = q - t * 3;
+        const float2 v = s_out[t][r][c];
+        const double m = f2d_bits(v.x) + f2d_bits(v.y);
+        const double x = fma(two_da, m, fma(two_db, vb[i], -va[i]));
+        dw[at[i]] = fma(cf.c[r], x, vd[i]);
+        u[at[i]] = x;
+        // FP32 staging of x_{k+1}, transposed through shared memory below
+        reinterpret_cast<float *>(&s_out[t][r][c])[0] = d2f_bits(x);
+      }
     }
-    u[idx] = m;
+  } else {
+    for (int k = threadIdx.x; k < nr * kRow; k += blockDim.x) {
+      const int r = k / kRow, q = k - r * kRow;
+      const int t = q / 3, c = q - t * 3;
+      if (t >= ns) continue;
+      const float2 v = s_out[t][r][c];
+      u[((int64_t)r * n + s0) * 3 + q] = f2d_bits(v.x) + f2d_bits(v.y);
+    }
   }
   if (CHEB) {
     __syncthreads();
