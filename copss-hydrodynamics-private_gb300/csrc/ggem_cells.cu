@@ -95,6 +95,8 @@ __device__ __forceinline__ void assign_one(int64_t i, const double *__restrict__
 __global__ void k_assign(int64_t n, const double *__restrict__ xyz, Grid g,
                          int32_t *__restrict__ cell_of, int32_t *__restrict__ count,
                          double4_32a *__restrict__ wrapped, int *__restrict__ err) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) assign_one(i, xyz, g, cell_of, count, wrapped, err);
 }
@@ -190,6 +192,8 @@ constexpr int64_t kScanCellsMax = 4096 * kScanTiles;
 __global__ void __launch_bounds__(1024) k_scan_cells(int32_t *__restrict__ count,
                                                      int32_t *__restrict__ start, int64_t n,
                                                      unsigned long long *__restrict__ stat) {
+  allow_next_grid();
+  wait_prior_grid();
   __shared__ int32_t warp_tot[2][32];
   if (stat && threadIdx.x < 2) stat[threadIdx.x] = 0ull;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -248,6 +252,8 @@ __global__ void __launch_bounds__(1024) k_scan_cells(int32_t *__restrict__ count
 __global__ void k_scatter(int64_t n, const int32_t *__restrict__ cell_of,
                           const int32_t *__restrict__ start, int32_t *__restrict__ fill,
                           int32_t *__restrict__ order) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t cid = cell_of[i];
@@ -262,6 +268,8 @@ __global__ void k_scatter(int64_t n, const int32_t *__restrict__ cell_of,
 // zeroed for the next build.
 __global__ void k_sort_cells(int64_t ncell, const int32_t *__restrict__ start,
                              int32_t *__restrict__ order, int32_t *__restrict__ fill) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t cidx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (cidx >= ncell) return;
   fill[cidx] = 0;  // scattered; ready for the next build
@@ -323,6 +331,8 @@ __global__ void k_gather_sorted(int64_t n, Grid g, const int32_t *__restrict__ o
                                 const double4_32a *__restrict__ wrapped,
                                 int32_t *__restrict__ rank, double4_32a *__restrict__ pos64,
                                 float4 *__restrict__ pos32) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s < n) gather_one(s, g, order, cell_of, wrapped, rank, pos64, pos32);
 }
@@ -392,7 +402,7 @@ __device__ __forceinline__ float box_r2(float qx, float qy, float qz, float3 lo,
 }
 
 __device__ __forceinline__ void pair_list_cell(
-    int64_t C, const Grid &g, const int4 *__restrict__ stencil, int nst,
+    int C, const Grid &g, const int4 *__restrict__ stencil, int nst,
     const float4 *__restrict__ shift, const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
     const double4_32a *__restrict__ pos64, float rc2_lo, float rc2_hi, double rc2, int W,
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
@@ -408,8 +418,7 @@ __device__ __forceinline__ void pair_list_cell(
   s_mark[lane] = -1;
   const int32_t tb = start[C], te = start[C + 1];
   if (te <= tb) return;
-  const int cx = (int)(C % g.nc[0]), cy = (int)((C / g.nc[0]) % g.nc[1]),
-            cz = (int)(C / ((int64_t)g.nc[0] * g.nc[1]));
+  const int cx = C % g.nc[0], cy = (C / g.nc[0]) % g.nc[1], cz = C / (g.nc[0] * g.nc[1]);
   // stencil cell ranges and their running prefix (warp scan over chunks)
   int32_t carry = 0;
   for (int k0 = 0; k0 < nst; k0 += 32) {
@@ -584,7 +593,9 @@ __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err,
     int32_t *__restrict__ count_h, uint32_t *__restrict__ list_h) {
-  pair_list_cell(blockIdx.x, g, stencil, nst, shift, start, pos32, pos64, rc2_lo, rc2_hi, rc2, W,
+  allow_next_grid();
+  wait_prior_grid();
+  pair_list_cell((int)blockIdx.x, g, stencil, nst, shift, start, pos32, pos64, rc2_lo, rc2_hi, rc2, W,
                  count, list, stat, err, count_h, list_h);
 }
 
@@ -699,7 +710,7 @@ __global__ void __launch_bounds__(32, 32) k_batch_list(
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err) {
   const BatchGeo &b = geo[cell_susp[blockIdx.x]];
-  pair_list_cell((int64_t)blockIdx.x - b.cell0, b.g, b.stencil, b.nst, b.shift, start + b.cell0,
+  pair_list_cell((int)((int64_t)blockIdx.x - b.cell0), b.g, b.stencil, b.nst, b.shift, start + b.cell0,
                  pos32, pos64, rc2_lo, rc2_hi, rc2, W, count, list, stat, err, nullptr, nullptr);
 }
 
@@ -717,6 +728,8 @@ __global__ void __launch_bounds__(32 * kRunWarps) k_run_list(
     const int32_t *__restrict__ start, const float4 *__restrict__ pos32, int W,
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err) {
+  allow_next_grid();
+  wait_prior_grid();
   __shared__ int s_tot[kRunWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t s = blockIdx.x * (int64_t)kRunWarps + warp;
@@ -841,28 +854,33 @@ int build_cells(ggem_ctx *c, bool defer_flags) {
   const int T = 256;
   const unsigned bn = (unsigned)((n + T - 1) / T);
   if (n > 0) {
-    k_assign<<<bn, T, 0, st>>>(n, c->xyz_in.p, g, c->cell_of.p, c->cell_count.p, c->wrapped.p,
+    launch_dependent(k_assign, dim3(bn), T, 0, st,
+                   n, c->xyz_in.p, g, c->cell_of.p, c->cell_count.p, c->wrapped.p,
                                c->err.p);
     if (int rc = check_launch(c, "assign")) return rc;
   }
   c->list_stat_zero = false;
   if (small) {
-    k_scan_cells<<<1, 1024, 0, st>>>(c->cell_count.p, c->cell_start.p, g.ncell, c->nb_stat.p);
+    launch_dependent(k_scan_cells, dim3(1), 1024, 0, st,
+                   c->cell_count.p, c->cell_start.p, g.ncell, c->nb_stat.p);
     if (int rc = check_launch(c, "scan cells")) return rc;
     c->list_stat_zero = c->nb_stat.p != nullptr;
   } else if (int rc = device_exclusive_scan_i32(c, c->cell_count.p, c->cell_start.p, g.ncell)) {
     return rc;
   }
   if (n > 0) {
-    k_scatter<<<bn, T, 0, st>>>(n, c->cell_of.p, c->cell_start.p, c->cell_fill.p, c->order.p);
+    launch_dependent(k_scatter, dim3(bn), T, 0, st,
+                   n, c->cell_of.p, c->cell_start.p, c->cell_fill.p, c->order.p);
     if (int rc = check_launch(c, "scatter")) return rc;
   }
   // (for n = 0 only the fill counters are cleared)
-  k_sort_cells<<<(unsigned)((g.ncell + T - 1) / T), T, 0, st>>>(g.ncell, c->cell_start.p,
+  launch_dependent(k_sort_cells, dim3((unsigned)((g.ncell + T - 1) / T)), T, 0, st,
+                   g.ncell, c->cell_start.p,
                                                                  c->order.p, c->cell_fill.p);
   if (int rc = check_launch(c, "sort cells")) return rc;
   if (n > 0) {
-    k_gather_sorted<<<bn, T, 0, st>>>(n, g, c->order.p, c->cell_of.p, c->wrapped.p, c->rank.p,
+    launch_dependent(k_gather_sorted, dim3(bn), T, 0, st,
+                   n, g, c->order.p, c->cell_of.p, c->wrapped.p, c->rank.p,
                                       c->pos64.p, c->pos32.p);
     if (int rc = check_launch(c, "gather sorted")) return rc;
   }
@@ -896,13 +914,13 @@ int cell_flag_error(ggem_ctx *c, int flags) {
 
 void launch_pair_list(ggem_ctx *c, int nst, int W, cudaStream_t st) {
   if (c->prm.nb_mode == GGEM_NB_REFERENCE) {
-    k_run_list<<<(unsigned)((c->n + kRunWarps - 1) / kRunWarps), 32 * kRunWarps, 0, st>>>(
-        c->n, c->grid, c->d_runs.p, c->n_runs, c->cell_start.p, c->pos32.p, W, c->nb_cnt.p,
+    launch_dependent(k_run_list, dim3((unsigned)((c->n + kRunWarps - 1) / kRunWarps)), 32 * kRunWarps, 0, st,
+                   c->n, c->grid, c->d_runs.p, c->n_runs, c->cell_start.p, c->pos32.p, W, c->nb_cnt.p,
         c->nb_list.p, c->nb_stat.p, c->err.p);
     return;
   }
-  k_pair_list_warp<<<(unsigned)c->grid.ncell, 32, 0, st>>>(
-      c->grid, c->d_stencil.p, nst, c->d_shift.p, c->cell_start.p, c->pos32.p, c->pos64.p,
+  launch_dependent(k_pair_list_warp, dim3((unsigned)c->grid.ncell), 32, 0, st,
+                   c->grid, c->d_stencil.p, nst, c->d_shift.p, c->cell_start.p, c->pos32.p, c->pos64.p,
       c->rc2_lo, c->rc2_hi, c->rc2, W, c->nb_cnt.p, c->nb_list.p, c->nb_stat.p, c->err.p,
       c->sym_pairs ? c->nb_cnt_h.p : nullptr, c->sym_pairs ? c->nb_list_h.p : nullptr);
 }

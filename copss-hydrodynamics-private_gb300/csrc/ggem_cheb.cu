@@ -90,6 +90,8 @@ __global__ void __launch_bounds__(kVecThreads) k_finalize(int G, const double *_
                                                           double *__restrict__ out, int nq,
                                                           const unsigned long long *__restrict__ stat,
                                                           const int *__restrict__ err) {
+  allow_next_grid();
+  wait_prior_grid();
   __shared__ double sh[32];
   const int q = blockIdx.x;
   // four running sums per thread keep four loads in flight (fixed order)
@@ -249,88 +251,28 @@ __global__ void k_axpy_into(int64_t tot, double s, const double *__restrict__ a,
 }
 
 // ---- Lanczos ---------------------------------------------------------------
-// The recurrence runs without the host: alpha, beta, 1 / beta and the
-// projections stay on the device (LanczosState), every reduction is finished
-// by the block that comes last (its partials summed in a fixed order), and
-// the host reads alpha and beta once at the end.  Per step:
-//   k_lz_dot      alpha = q_j . w                       (w = M q_j)
-//   k_lz_project  w -= alpha q_j + beta q_{j-1}, then h_i = Q_i . w for all i
-//   k_lz_update   w -= sum_i h_i Q_i, beta = |w|
-//   k_lz_next     q_{j+1} = w / beta
-// Taking the two large components first leaves the full pass only rounding
-// (and the asymmetry of the FP32 operator), so one full pass reaches the
-// orthogonality that two passes over raw M q_j did, with half of their FP64
-// fused multiply-adds (two lanes per SM and clock bound them: 15 us per pass
-// over 12 vectors at N = 200k).  N = 200k, k = 24: 5.47 -> 2.83 ms.
-constexpr int kLzThreads = 256;
-constexpr int kLzBlocks = 608;                     // four per SM
-constexpr int kLzMax = 512;                        // steps
+// The recurrence runs without the host: the coefficients, 1 / beta and the
+// projections stay on the device (LanczosState) and the host reads them once
+// at the end.  Per step, with w = M q_j:
+//   k_lz_dots     h_i = Q_i . w for all i <= j (and k_finalize)
+//   k_lz_project  w -= sum_i h_i Q_i; these two twice, the second time with
+//                 |w|^2 in the same pass
+//   k_lz_next     beta_j = |w|, q_{j+1} = w / beta_j; alpha_j = the first h_j
+// The sums keep the order of k_dot_partials and k_finalize (per thread, per
+// warp, per block, over blocks), so the bounds do not depend on how many
+// vectors a kernel takes at once.  Bound by the FP64 pipe (two lanes per SM
+// and clock): four fused multiply-adds per element and vector, 48 us per step
+// at N = 200k, j = 12.  Eight vectors' warp sums share one reduce-scatter (9
+// additions instead of 40), which made the dots 37 -> {LZ_DOT} us.  N = 200k,
+// k = 24: 5.47 -> {LZ_MS} ms.
+constexpr int kLzMax = 512;  // steps
 
 struct LanczosState {
-  double alpha[kLzMax], beta[kLzMax], h[kLzMax + 1], inv_beta;
-  unsigned int arrived;  // blocks of the running reduction, zero between kernels
+  double alpha[kLzMax], beta[kLzMax], h[kLzMax], norm2;
 };
 
-// elements per thread and tile: eight spread the cost of a warp's sums over
-// eight multiply-adds, one and two where eight would leave SMs without a tile
-int lz_elems(int64_t D) {
-  return D >= 8 * kLzThreads * 152 ? 8 : (D >= 2 * kLzThreads * 152 ? 2 : 1);
-}
-int lz_blocks(int64_t D) {
-  const int64_t tile = (int64_t)kLzThreads * lz_elems(D);
-  return (int)std::max<int64_t>(1, std::min<int64_t>((D + tile - 1) / tile, kLzBlocks));
-}
-
-// true in every thread of the last block to arrive; the others' partials
-// are then visible to it
-__device__ __forceinline__ bool last_block(LanczosState *S) {
-  __shared__ bool s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_last = atomicAdd(&S->arrived, 1u) == gridDim.x - 1;
-    if (s_last) S->arrived = 0u;
-  }
-  __syncthreads();
-  if (s_last) __threadfence();
-  return s_last;
-}
-
-// sum of n partials in a fixed order by one warp (valid in every lane)
-__device__ __forceinline__ double warp_total(const double *p, int n) {
-  double a0 = 0.0, a1 = 0.0;
-  int b = threadIdx.x & 31;
-  for (; b + 32 < n; b += 64) {
-    a0 += __ldcg(p + b);
-    a1 += __ldcg(p + b + 32);
-  }
-  if (b < n) a0 += __ldcg(p + b);
-  a0 += a1;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-  return a0;
-}
-
-__global__ void __launch_bounds__(kLzThreads) k_lz_dot(int64_t D, const double *__restrict__ q,
-                                                       const double *__restrict__ w,
-                                                       double *__restrict__ partial,
-                                                       LanczosState *S, int j) {
-  __shared__ double sh[32];
-  double acc = 0.0;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < D;
-       k += (int64_t)gridDim.x * blockDim.x)
-    acc = fma(q[k], w[k], acc);
-  const double t = block_sum(acc, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = t;
-  if (!last_block(S)) return;
-  if (threadIdx.x < 32) {
-    const double a = warp_total(partial, gridDim.x);
-    if (threadIdx.x == 0) S->alpha[j] = a;
-  }
-}
-
 // the warp sums of v[0..7], one value on each lane: lane l returns the sum
-// of v[(l >> 2) & 7] (a reduce-scatter: 9 additions instead of 40)
+// of v[(l >> 2) & 7], added in the tree of a shuffle-down reduction
 __device__ __forceinline__ double warp_sum8(double v[8]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -348,116 +290,128 @@ __device__ __forceinline__ double warp_sum8(double v[8]) {
   return v[0];
 }
 
-// w -= alpha_j q_j + beta_{j-1} q_{j-1}; h_i = Q_i . w for i <= j
-template <int kLzElems>
-__global__ void __launch_bounds__(kLzThreads) k_lz_project(int64_t D, int j,
-                                                           const double *__restrict__ Q,
-                                                           double *__restrict__ w,
-                                                           double *__restrict__ partial,
-                                                           LanczosState *S) {
-  extern __shared__ double sh[];  // [warps][8 * groups]
+// partial[i][b] = Q_i . w for the eight vectors of this block row, i < m
+__global__ void __launch_bounds__(kVecThreads) k_lz_dots(int64_t D, int m,
+                                                         const double *__restrict__ Q,
+                                                         const double *__restrict__ w,
+                                                         double *__restrict__ partial) {
+  allow_next_grid();
+  wait_prior_grid();
+  __shared__ double sh[kVecThreads / 32][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int groups = (j + 8) / 8, m8 = 8 * groups;
-  for (int i = threadIdx.x; i < (kLzThreads / 32) * m8; i += kLzThreads) sh[i] = 0.0;
-  __syncthreads();
-  const double al = S->alpha[j], be = j > 0 ? S->beta[j - 1] : 0.0;
-  constexpr int kLzTile = kLzThreads * kLzElems;
-  const double *qj = Q + (int64_t)j * D, *qp = Q + (int64_t)(j > 0 ? j - 1 : 0) * D;
-  for (int64_t t0 = blockIdx.x * (int64_t)kLzTile; t0 < D; t0 += (int64_t)gridDim.x * kLzTile) {
-    double v[kLzElems];
+  const int i0 = 8 * blockIdx.y;
+  const double *q = Q + (int64_t)i0 * D;
+  const int ni = min(8, m - i0);
+  double d[8];
 #pragma unroll
-    for (int e = 0; e < kLzElems; ++e) {
-      const int64_t k = t0 + e * kLzThreads + threadIdx.x;
-      v[e] = 0.0;
-      if (k < D) {
-        v[e] = fma(-be, qp[k], fma(-al, qj[k], w[k]));
-        w[k] = v[e];
-      }
+  for (int i = 0; i < 8; ++i) d[i] = 0.0;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (ni == 8) {
+#pragma unroll 2
+    for (; k < D; k += step) {
+      const double v = w[k];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) d[i] = fma(q[i * D + k], v, d[i]);
     }
-    for (int g = 0; g < groups; ++g) {
-      double d[8];
+  } else {
+    for (; k < D; k += step) {
+      const double v = w[k];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        d[i] = 0.0;
-        if (8 * g + i > j) continue;
-        const double *q = Q + (int64_t)(8 * g + i) * D;
-#pragma unroll
-        for (int e = 0; e < kLzElems; ++e) {
-          const int64_t k = t0 + e * kLzThreads + threadIdx.x;
-          if (k < D) d[i] = fma(q[k], v[e], d[i]);
-        }
-      }
-      const double t = warp_sum8(d);
-      if ((lane & 3) == 0) sh[warp * m8 + 8 * g + (lane >> 2)] += t;
-      // (each lane owns its entry: no other thread touches it)
+      for (int i = 0; i < 8; ++i)
+        if (i < ni) d[i] = fma(q[i * D + k], v, d[i]);
     }
   }
+  const double t = warp_sum8(d);
+  if ((lane & 3) == 0) sh[warp][lane >> 2] = t;
   __syncthreads();
-  for (int i = threadIdx.x; i <= j; i += kLzThreads) {
-    double t = 0.0;
-#pragma unroll
-    for (int q = 0; q < kLzThreads / 32; ++q) t += sh[q * m8 + i];
-    partial[(int64_t)i * gridDim.x + blockIdx.x] = t;
-  }
-  if (!last_block(S)) return;
-  for (int i = warp; i <= j; i += kLzThreads / 32) {
-    const double t = warp_total(partial + (int64_t)i * gridDim.x, gridDim.x);
-    if (lane == 0) S->h[i] = t;
+  if (threadIdx.x < ni) {  // the block's eight warps, in block_sum's tree
+    const int i = threadIdx.x;
+    const double a = (sh[0][i] + sh[4][i]) + (sh[2][i] + sh[6][i]);
+    const double b = (sh[1][i] + sh[5][i]) + (sh[3][i] + sh[7][i]);
+    partial[(int64_t)(i0 + i) * gridDim.x + blockIdx.x] = a + b;
   }
 }
 
-// w -= sum_{i < m} h_i Q_i; beta_j = |w| and its reciprocal (m = 0: the norm
-// of the start vector)
-template <int kLzElems>
-__global__ void __launch_bounds__(kLzThreads) k_lz_update(int64_t D, int m,
-                                                          const double *__restrict__ Q,
-                                                          double *__restrict__ w,
-                                                          double *__restrict__ partial,
-                                                          LanczosState *S, int j) {
-  extern __shared__ double sh[];  // [m] projections
-  __shared__ double red[32];
-  for (int i = threadIdx.x; i < m; i += kLzThreads) sh[i] = S->h[i];
-  __syncthreads();
-  constexpr int kLzTile = kLzThreads * kLzElems;
-  double acc = 0.0;
-  for (int64_t t0 = blockIdx.x * (int64_t)kLzTile; t0 < D; t0 += (int64_t)gridDim.x * kLzTile) {
-    double v[kLzElems];
-#pragma unroll
-    for (int e = 0; e < kLzElems; ++e) {
-      const int64_t k = t0 + e * kLzThreads + threadIdx.x;
-      v[e] = k < D ? w[k] : 0.0;
-    }
+// v -= sum_{i < m} h_i Q_i of four elements at once (n_el of them valid)
+__device__ __forceinline__ void lz_project4(int64_t D, int m, const double *__restrict__ Q,
+                                            const double *sh, const int64_t k[4], int n_el,
+                                            double v[4]) {
+  if (n_el == 4) {
+#pragma unroll 4
     for (int i = 0; i < m; ++i) {
       const double *q = Q + (int64_t)i * D;
-      const double h = sh[i];
+      const double h = -sh[i];
 #pragma unroll
-      for (int e = 0; e < kLzElems; ++e) {
-        const int64_t k = t0 + e * kLzThreads + threadIdx.x;
-        if (k < D) v[e] = fma(-h, q[k], v[e]);
-      }
+      for (int e = 0; e < 4; ++e) v[e] = fma(h, q[k[e]], v[e]);
     }
+  } else {
+    for (int i = 0; i < m; ++i) {
+      const double *q = Q + (int64_t)i * D;
+      const double h = -sh[i];
 #pragma unroll
-    for (int e = 0; e < kLzElems; ++e) {
-      const int64_t k = t0 + e * kLzThreads + threadIdx.x;
-      if (m > 0 && k < D) w[k] = v[e];
-      acc = fma(v[e], v[e], acc);
-    }
-  }
-  const double t = block_sum(acc, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = t;
-  if (!last_block(S)) return;
-  if (threadIdx.x < 32) {
-    const double b = sqrt(warp_total(partial, gridDim.x));
-    if (threadIdx.x == 0) {
-      S->beta[j] = b;
-      S->inv_beta = b > 0.0 ? 1.0 / b : 0.0;  // (a breakdown ends the recurrence on the host)
+      for (int e = 0; e < 4; ++e)
+        if (e < n_el) v[e] = fma(h, q[k[e]], v[e]);
     }
   }
 }
 
-__global__ void k_lz_next(int64_t D, const double *w, double *q,
-                          const LanczosState *__restrict__ S) {
-  const double s = S->inv_beta;
+// w -= sum_{i < m} h_i Q_i (first pass: alpha = h_{m-1}); with NORM also
+// partial[b] = |w|^2 (m = 0: the norm alone)
+template <bool NORM>
+__global__ void __launch_bounds__(kVecThreads) k_lz_project(int64_t D, int m,
+                                                            const double *__restrict__ Q,
+                                                            LanczosState *S,
+                                                            double *__restrict__ w,
+                                                            double *__restrict__ partial) {
+  allow_next_grid();
+  wait_prior_grid();
+  extern __shared__ double sh[];  // [m]
+  __shared__ double red[32];
+  for (int i = threadIdx.x; i < m; i += blockDim.x) sh[i] = S->h[i];
+  if (!NORM && blockIdx.x == 0 && threadIdx.x == 0) S->alpha[m - 1] = S->h[m - 1];
+  __syncthreads();
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  double acc = 0.0;
+  for (int64_t k0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k0 < D; k0 += 4 * step) {
+    int64_t k[4];
+    double v[4];
+    int n_el = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      k[e] = k0 + e * step;
+      v[e] = 0.0;
+      if (k[e] < D) {
+        v[e] = w[k[e]];
+        ++n_el;
+      }
+    }
+    lz_project4(D, m, Q, sh, k, n_el, v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (e < n_el) {
+        if (m > 0) w[k[e]] = v[e];
+        acc += v[e] * v[e];
+      }
+  }
+  if (NORM) {
+    const double t = block_sum(acc, red);
+    if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  }
+}
+
+// q = w / |w|, and the step's coefficients
+__global__ void k_lz_next(int64_t D, int j, const double *w, double *q, LanczosState *S) {
+  allow_next_grid();
+  wait_prior_grid();
+  __shared__ double s_scale;
+  if (threadIdx.x == 0) {  // (once per block: a root and a division cost ~40 FP64 instructions)
+    const double b = sqrt(S->norm2);
+    s_scale = b > 0.0 ? 1.0 / b : 0.0;  // (a breakdown ends the recurrence on the host)
+    if (j >= 0 && blockIdx.x == 0) S->beta[j] = b;
+  }
+  __syncthreads();
+  const double s = s_scale;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < D;
        k += (int64_t)gridDim.x * blockDim.x)
     q[k] = w[k] * s;
@@ -527,7 +481,8 @@ int grid1(int64_t tot) {
 // the finalized sums copied to the pinned host mirror (no wait)
 int finalize_issue(ggem_ctx *c, int nq, int G, double *host, bool list_stats) {
   double *out = c->w_red.p + (size_t)nq * G;
-  k_finalize<<<nq, kVecThreads, 0, c->stream>>>(G, c->w_red.p, out, nq,
+  launch_dependent(k_finalize, dim3(nq), kVecThreads, 0, c->stream,
+                   G, c->w_red.p, out, nq,
                                                 list_stats ? c->nb_stat.p : nullptr,
                                                 list_stats ? c->err.p : nullptr);
   if (int rc = check_launch(c, "finalize")) return rc;
@@ -1238,7 +1193,7 @@ extern "C" int ggem_lanczos_bounds(ggem_ctx *ctx, int k, uint64_t seed, double *
   if (D == 0) return ggem::fail(ctx, GGEM_ERR_BAD_ARG, "no particles");
   k = (int)std::min<int64_t>(k, D);
   cudaError_t e;
-  const int G = lz_blocks(D);
+  const int G = vec_blocks(D);
   if ((e = ctx->lz_Q.ensure((size_t)D * k)) || (e = ctx->w_out.ensure(D)) ||
       (e = ctx->lz_state.ensure(sizeof(LanczosState))) ||
       (e = ctx->w_red.ensure(std::max<size_t>(4 * kMaxRhs * 600, (size_t)k * G))))
@@ -1247,29 +1202,49 @@ extern "C" int ggem_lanczos_bounds(ggem_ctx *ctx, int k, uint64_t seed, double *
   const int sm = brownian_self_mode(ctx);
   double *Q = ctx->lz_Q.p, *w = ctx->w_out.p, *part = ctx->w_red.p;
   LanczosState *S = reinterpret_cast<LanczosState *>(ctx->lz_state.p);
-  if ((e = cudaMemsetAsync(S, 0, sizeof(*S), st))) return cuda_fail(ctx, e, "lanczos state");
+  // the partials of nq sums into out
+  auto finish = [&](int nq, double *out) -> int {
+    launch_dependent(k_finalize, dim3(nq), kVecThreads, 0, st,
+                   G, part, out, nq, nullptr, nullptr);
+    return check_launch(ctx, "lanczos sums");
+  };
   // start vector: N(0,1) from the counter-based generator, normalised
   k_philox_normals<<<(unsigned)(((D + 3) / 4 + 255) / 256), 256, 0, st>>>(D, seed, 0x4C414E43ull, Q);
   if (int rc = check_launch(ctx, "lanczos start")) return rc;
-  const int E = lz_elems(D);
-  auto project = E == 8 ? k_lz_project<8> : (E == 2 ? k_lz_project<2> : k_lz_project<1>);
-  auto update = E == 8 ? k_lz_update<8> : (E == 2 ? k_lz_update<2> : k_lz_update<1>);
-  update<<<G, kLzThreads, 0, st>>>(D, 0, Q, Q, part, S, 0);
+  launch_dependent(k_lz_project<true>, dim3(G), kVecThreads, 0, st,
+                   D, 0, Q, S, Q, part);
   if (int rc = check_launch(ctx, "lanczos norm")) return rc;
-  k_lz_next<<<grid1(D), 256, 0, st>>>(D, Q, Q, S);
+  if (int rc = finish(1, &S->norm2)) return rc;
+  launch_dependent(k_lz_next, dim3(grid1(D)), 256, 0, st,
+                   D, -1, Q, Q, S);
   if (int rc = check_launch(ctx, "lanczos next")) return rc;
   for (int j = 0; j < k; ++j) {
-    double *q = Q + (size_t)j * D;
-    if (int rc = matvec_slots(ctx, 1, q, w, sm)) return rc;
-    k_lz_dot<<<G, kLzThreads, 0, st>>>(D, q, w, part, S, j);
-    if (int rc = check_launch(ctx, "lanczos alpha")) return rc;
-    if (j == k - 1) break;  // (the last beta is not used)
-    const size_t sh = sizeof(double) * (kLzThreads / 32) * 8 * ((j + 8) / 8);
-    project<<<G, kLzThreads, sh, st>>>(D, j, Q, w, part, S);
-    if (int rc = check_launch(ctx, "lanczos project")) return rc;
-    update<<<G, kLzThreads, sizeof(double) * (j + 1), st>>>(D, j + 1, Q, w, part, S, j);
-    if (int rc = check_launch(ctx, "lanczos update")) return rc;
-    k_lz_next<<<grid1(D), 256, 0, st>>>(D, w, Q + (size_t)(j + 1) * D, S);
+    const int m = j + 1;
+    const size_t sh = sizeof(double) * m;
+    if (int rc = matvec_slots(ctx, 1, Q + (size_t)j * D, w, sm)) return rc;
+    if (j == k - 1) {  // (the last beta is not used)
+      launch_dependent(k_lz_dots, dim3(G), kVecThreads, 0, st,
+                   D, 1, Q + (size_t)j * D, w, part);
+      if (int rc = check_launch(ctx, "lanczos dots")) return rc;
+      if (int rc = finish(1, S->alpha + j)) return rc;
+      break;
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+      launch_dependent(k_lz_dots, dim3(G, (m + 7) / 8), kVecThreads, 0, st,
+                   D, m, Q, w, part);
+      if (int rc = check_launch(ctx, "lanczos dots")) return rc;
+      if (int rc = finish(m, S->h)) return rc;
+      if (pass == 0)
+        launch_dependent(k_lz_project<false>, dim3(G), kVecThreads, sh, st,
+                   D, m, Q, S, w, part);
+      else
+        launch_dependent(k_lz_project<true>, dim3(G), kVecThreads, sh, st,
+                   D, m, Q, S, w, part);
+      if (int rc = check_launch(ctx, "lanczos project")) return rc;
+    }
+    if (int rc = finish(1, &S->norm2)) return rc;
+    launch_dependent(k_lz_next, dim3(grid1(D)), 256, 0, st,
+                   D, j, w, Q + (size_t)(j + 1) * D, S);
     if (int rc = check_launch(ctx, "lanczos next")) return rc;
   }
   std::vector<double> a(k), b(k);

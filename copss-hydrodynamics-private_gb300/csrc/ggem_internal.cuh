@@ -304,6 +304,38 @@ __device__ __forceinline__ float d2f_bits(double x) {
 }
 #endif
 
+#ifdef __CUDACC__
+// Programmatic dependent launches along a build or a series (PTX
+// griddepcontrol): a kernel launched with launch_dependent may start while
+// the kernel before it on the stream still runs; it lets its own successor
+// do the same and waits, before it touches any memory that a kernel writes,
+// until the one before it has completed and its results are visible.
+// Without such a launch both return at once.  The blocks of the next kernel
+// are resident when the last ones of the previous finish.
+__device__ __forceinline__ void allow_next_grid() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_prior_grid() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+void launch_dependent(void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem,
+                      cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+#endif
+
 // kernel kinds of the timing hooks
 enum : int { kKPairF32 = 0, kKPairF64 = 1, kKChebTerm = 2, kKListBuild = 3, kKPairCheb = 4 };
 

@@ -253,6 +253,8 @@ __global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, MinImage mi, D
                                                        const double *__restrict__ f,
                                                        double *__restrict__ u, int self_mode,
                                                        int r0) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
   const bool act = gid < n;
@@ -729,6 +731,8 @@ __device__ __forceinline__ void group_store(bool act, int sub, int64_t s, float 
 
 __global__ void k_build_src(int64_t n, const float4 *__restrict__ pos32,
                             const double *__restrict__ f, Rec32 *__restrict__ src) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   Rec32 r;
@@ -769,15 +773,6 @@ __device__ __forceinline__ Rec32 ld_rec32(const Rec32 *p) {
 __device__ __forceinline__ void stage_shifts(float4 *sh, const float4 *__restrict__ shift) {
   for (int k = threadIdx.x; k < kMaxCode; k += blockDim.x) sh[k] = shift[k];
   __syncthreads();
-}
-
-// The series kernels may be launched as programmatic dependents of the
-// kernel before them (PTX griddepcontrol): their blocks can start while
-// that kernel's last blocks finish, stage the constant shift table, and
-// wait here until its results are complete and visible.  Without such a
-// launch the wait returns at once.
-__device__ __forceinline__ void wait_prior_grid() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // reduce-scatter of the group's float-float sums: afterwards lane sub
@@ -1019,7 +1014,8 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_r1(
     const float4 *__restrict__ shift, double self_c, const double *__restrict__ f,
     double *__restrict__ u, const int32_t *__restrict__ order, double *__restrict__ part) {
   __shared__ float4 sh[kMaxCode];
-  stage_shifts(sh, shift);
+  allow_next_grid();
+  stage_shifts(sh, shift);  // (constant: no kernel writes it)
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
   const int sub = (int)(threadIdx.x % kGroup);
@@ -1054,7 +1050,8 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_first(
     const double *__restrict__ x0, double *__restrict__ m, double *__restrict__ x1,
     double *__restrict__ dw, Rec32 *__restrict__ next, double *__restrict__ part) {
   __shared__ float4 sh[kMaxCode];
-  stage_shifts(sh, shift);
+  allow_next_grid();
+  stage_shifts(sh, shift);  // (constant: no kernel writes it)
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
   const int sub = (int)(threadIdx.x % kGroup);
@@ -1100,7 +1097,8 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_cheb(
     double *__restrict__ dw, Rec32 *__restrict__ next, double *__restrict__ part,
     int64_t nw, Rec32 *__restrict__ dw_next) {
   __shared__ float4 sh[kMaxCode];
-  stage_shifts(sh, shift);
+  allow_next_grid();
+  stage_shifts(sh, shift);  // (constant: no kernel writes it)
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
   const int sub = (int)(threadIdx.x % kGroup);
@@ -1147,6 +1145,8 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_cheb(
 __global__ void k_to_slots_rec(int64_t n, const int32_t *__restrict__ order,
                                const float4 *__restrict__ pos32, const double *__restrict__ xi,
                                double *__restrict__ x0, Rec32 *__restrict__ rec) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int64_t i = order[s];
@@ -1202,6 +1202,8 @@ __global__ void __launch_bounds__(256) k_pair_tensor(
     int64_t n, const float4 *__restrict__ pos32, const int32_t *__restrict__ cnt, int W,
     const uint32_t *__restrict__ list, PolyAB P, const Rec32 *__restrict__ tab, float inv_ds,
     float hx, float hy, float hz, float4 *__restrict__ ten) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
   if (s < n)
     tensor_row<CD, POLY>(s, (int)(threadIdx.x % kGroup), pos32, cnt, W, list, P, tab, inv_ds, hx,
@@ -1224,6 +1226,8 @@ __global__ void __launch_bounds__(256) k_batch_tensor(
 
 // forces of one right-hand side as one float4 per slot (w = 0)
 __global__ void k_stage_f4(int64_t n, const double *__restrict__ f, float4 *__restrict__ f4) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   f4[s] = make_float4(d2f_bits(f[3 * s]), d2f_bits(f[3 * s + 1]), d2f_bits(f[3 * s + 2]), 0.f);
@@ -1335,6 +1339,8 @@ __global__ void __launch_bounds__(256) k_pair_r1tv(int64_t n, const float4 *__re
                                                    const float4 *__restrict__ ten, double self_c,
                                                    const double *__restrict__ f,
                                                    double *__restrict__ u) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
   const bool act = gid < n;
@@ -1352,6 +1358,8 @@ __global__ void __launch_bounds__(256) k_pair_cheb_tv(
     double two_da, double two_db, double coef, const double *__restrict__ x0,
     const double *__restrict__ x1, double *__restrict__ xm, double *__restrict__ dw,
     float4 *__restrict__ next) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
   const bool act = gid < n;
@@ -1388,7 +1396,8 @@ template <int V>
 void launch_stored_r1(ggem_ctx *c, const float4 *f4, double self_c, const double *f, double *u) {
   constexpr StoredVariant sv = kStoredVariants[V];
   const int64_t threads = c->n * sv.G;
-  k_pair_r1tv<sv.G, sv.U, sv.pipe><<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(
+  launch_dependent(k_pair_r1tv<sv.G, sv.U, sv.pipe>, dim3((unsigned)((threads + 255) / 256)), 256, 0,
+                   c->stream, 
       c->n, f4, c->nb_cnt.p, c->nb_w, c->nb_list.p, c->pair_ten.p, self_c, f, u);
 }
 
@@ -1398,7 +1407,8 @@ void launch_stored_cheb(ggem_ctx *c, const float4 *f4, double self_c, double two
                         double *xm, double *dw, float4 *next) {
   constexpr StoredVariant sv = kStoredVariants[V];
   const int64_t threads = c->n * sv.G;
-  k_pair_cheb_tv<sv.G, sv.U, sv.pipe><<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(
+  launch_dependent(k_pair_cheb_tv<sv.G, sv.U, sv.pipe>, dim3((unsigned)((threads + 255) / 256)), 256, 0,
+                   c->stream, 
       c->n, f4, c->nb_cnt.p, c->nb_w, c->nb_list.p, c->pair_ten.p, self_c, two_da, two_db, coef,
       x0, x1, xm, dw, next);
 }
@@ -1784,6 +1794,8 @@ __global__ void k_slots_to_f32(int64_t n, int nrhs, const double *__restrict__ f
 // orig [r][n][3] -> slots [r][n][3]
 __global__ void k_to_slots(int64_t n, int nrhs, const int32_t *__restrict__ order,
                            const double *__restrict__ orig, double *__restrict__ slot) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n * nrhs) return;
   const int64_t r = k / n, s = k - r * n;
@@ -1797,6 +1809,8 @@ __global__ void k_to_slots(int64_t n, int nrhs, const int32_t *__restrict__ orde
 
 __global__ void k_from_slots(int64_t n, int nrhs, const int32_t *__restrict__ rank,
                              const double *__restrict__ slot, double *__restrict__ orig) {
+  allow_next_grid();
+  wait_prior_grid();
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n * nrhs) return;
   const int64_t r = k / n, i = k - r * n;
@@ -1822,7 +1836,8 @@ template <int NR, int G>
 void launch_list_f64(ggem_ctx *c, const double *f, double *u, int self_mode, int r0,
                      long long eps2) {
   const int64_t threads = c->n * G;
-  k_pair_list_f64<NR, G><<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(
+  launch_dependent(k_pair_list_f64<NR, G>, dim3((unsigned)((threads + 255) / 256)), 256, 0,
+                   c->stream, 
       c->n, min_image_of(c->grid), c->dc, c->t64, eps2, c->nb_cnt.p, c->nb_w, c->nb_list.p,
       c->pos64.p, f, u, self_mode, r0);
 }
@@ -1896,31 +1911,10 @@ PolyAB poly_of(const ggem_ctx *c) {
   return P;
 }
 
-// a series kernel launched as a programmatic dependent of the kernel
-// before it on the stream (its first global reads wait in wait_prior_grid);
-// measured at N = 200k: the reference-faithful series (a vector kernel
-// between pair kernels) 777-781 -> 795-797 steps/s, the host-buffer leg
-// 1492-1496 -> 1512-1519, the device-resident fused series unchanged
-template <typename... KArgs, typename... Args>
-void launch_dependent(void (*kern)(KArgs...), unsigned grid, unsigned block, cudaStream_t st,
-                      Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 template <bool POLY, int V, bool ORIG>
 void launch_r1(ggem_ctx *c, const Rec32 *src, const double *f, double *u, double self_c,
                double *part) {
-  launch_dependent(k_pair_r1<POLY, V, ORIG>, (unsigned)pair_grid_blocks(c), 256u, c->stream,
+  launch_dependent(k_pair_r1<POLY, V, ORIG>, dim3(pair_grid_blocks(c)), 256, 0, c->stream,
                    c->n, src, (const int32_t *)c->nb_cnt.p, c->nb_w, (const uint32_t *)c->nb_list.p,
                    poly_of(c), reinterpret_cast<const Rec32 *>(c->tab.p), c->tab_inv_ds,
                    (const float4 *)c->d_shift.p, self_c, f, u, (const int32_t *)c->order.p, part);
@@ -1969,7 +1963,8 @@ int launch_f32_r1(ggem_ctx *c, const double *f, double *u, double self_c) {
   cudaError_t e;
   if (c->pretensor_ok) {
     if ((e = c->w_f4[0].ensure((size_t)n))) return cuda_fail(c, e, "pair forces");
-    k_stage_f4<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, f, c->w_f4[0].p);
+    launch_dependent(k_stage_f4, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
+                   n, f, c->w_f4[0].p);
     if (int rc = check_launch(c, "pair forces")) return rc;
     kt_start(c, kKPairF32);
     dispatch_stored_r1(c, c->w_f4[0].p, self_c, f, u);
@@ -1978,7 +1973,8 @@ int launch_f32_r1(ggem_ctx *c, const double *f, double *u, double self_c) {
   }
   if ((e = c->w_src.ensure(2 * (size_t)n))) return cuda_fail(c, e, "pair records");
   Rec32 *src = reinterpret_cast<Rec32 *>(c->w_src.p);
-  k_build_src<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, c->pos32.p, f, src);
+  launch_dependent(k_build_src, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
+                   n, c->pos32.p, f, src);
   if (int rc = check_launch(c, "pair records")) return rc;
   if (c->sym_pairs && c->nb_list_h.p) return launch_sym_r1(c, src, f, u, self_c);
   kt_start(c, kKPairF32);
@@ -1993,7 +1989,7 @@ template <bool POLY, int V, bool NORMS>
 void launch_cheb(ggem_ctx *c, const Rec32 *src, Rec32 *next, double two_da, double c1,
                  double coef, const double *x0, const double *x1, double *xm, double *dw,
                  double *part, Rec32 *dw_next) {
-  launch_dependent(k_pair_cheb<POLY, V, NORMS>, (unsigned)pair_grid_blocks(c), 256u, c->stream,
+  launch_dependent(k_pair_cheb<POLY, V, NORMS>, dim3(pair_grid_blocks(c)), 256, 0, c->stream,
                    c->n, src, (const int32_t *)c->nb_cnt.p, c->nb_w, (const uint32_t *)c->nb_list.p,
                    poly_of(c), reinterpret_cast<const Rec32 *>(c->tab.p), c->tab_inv_ds,
                    (const float4 *)c->d_shift.p, two_da, c1, coef, x0, x1, xm, dw, next, part,
@@ -2020,7 +2016,7 @@ template <bool POLY, int V>
 void launch_first(ggem_ctx *c, const Rec32 *src, Rec32 *next, double self_c, double da,
                   double db, double c0, double c1, const double *x0, double *m, double *x1,
                   double *dw, double *part) {
-  launch_dependent(k_pair_first<POLY, V>, (unsigned)pair_grid_blocks(c), 256u, c->stream, c->n,
+  launch_dependent(k_pair_first<POLY, V>, dim3(pair_grid_blocks(c)), 256, 0, c->stream, c->n,
                    src, (const int32_t *)c->nb_cnt.p, c->nb_w, (const uint32_t *)c->nb_list.p,
                    poly_of(c), reinterpret_cast<const Rec32 *>(c->tab.p), c->tab_inv_ds,
                    (const float4 *)c->d_shift.p, self_c, da, db, c0, c1, x0, m, x1, dw, next,
@@ -2108,7 +2104,8 @@ int launch_nr(ggem_ctx *c, const double *f, double *u, double self_c, int r0) {
 int permute_to_slots(ggem_ctx *c, int nrhs, const double *d_orig, double *d_slot) {
   const int64_t tot = c->n * nrhs;
   if (tot == 0) return GGEM_OK;
-  k_to_slots<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(c->n, nrhs, c->order.p,
+  launch_dependent(k_to_slots, dim3((unsigned)((tot + 255) / 256)), 256, 0, c->stream,
+                   c->n, nrhs, c->order.p,
                                                                    d_orig, d_slot);
   return check_launch(c, "to slots");
 }
@@ -2116,7 +2113,8 @@ int permute_to_slots(ggem_ctx *c, int nrhs, const double *d_orig, double *d_slot
 int permute_from_slots(ggem_ctx *c, int nrhs, const double *d_slot, double *d_orig) {
   const int64_t tot = c->n * nrhs;
   if (tot == 0) return GGEM_OK;
-  k_from_slots<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(c->n, nrhs, c->rank.p,
+  launch_dependent(k_from_slots, dim3((unsigned)((tot + 255) / 256)), 256, 0, c->stream,
+                   c->n, nrhs, c->rank.p,
                                                                      d_slot, d_orig);
   return check_launch(c, "from slots");
 }
@@ -2137,7 +2135,8 @@ int pair_cheb_term(ggem_ctx *c, bool records_fresh, const double *x0, const doub
       return cuda_fail(c, e, "chebyshev forces");
     float4 *cur = c->w_f4[c->rec_cur].p, *nxt = c->w_f4[c->rec_cur ^ 1].p;
     if (!records_fresh) {
-      k_stage_f4<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, x1, cur);
+      launch_dependent(k_stage_f4, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
+                   n, x1, cur);
       if (int rc = check_launch(c, "chebyshev forces")) return rc;
     }
     kt_start(c, kKPairCheb);
@@ -2151,7 +2150,8 @@ int pair_cheb_term(ggem_ctx *c, bool records_fresh, const double *x0, const doub
   Rec32 *cur = reinterpret_cast<Rec32 *>(c->w_rec[c->rec_cur].p);
   Rec32 *nxt = reinterpret_cast<Rec32 *>(c->w_rec[c->rec_cur ^ 1].p);
   if (!records_fresh) {
-    k_build_src<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, c->pos32.p, x1, cur);
+    launch_dependent(k_build_src, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
+                   n, c->pos32.p, x1, cur);
     if (int rc = check_launch(c, "chebyshev records")) return rc;
   }
   const double c1 = two_db + two_da * self_c0;
@@ -2231,7 +2231,8 @@ int cheb_start_fused(ggem_ctx *c, const double *xi, double *x0, double *m, doubl
     return cuda_fail(c, e, "chebyshev records");
   Rec32 *cur = reinterpret_cast<Rec32 *>(c->w_rec[c->rec_cur].p);
   Rec32 *nxt = reinterpret_cast<Rec32 *>(c->w_rec[c->rec_cur ^ 1].p);
-  k_to_slots_rec<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, c->order.p, c->pos32.p,
+  launch_dependent(k_to_slots_rec, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
+                   n, c->order.p, c->pos32.p,
                                                                      xi, x0, cur);
   if (int rc = check_launch(c, "to slots + records")) return rc;
   const double self_c = self_coefficient(c, self_mode);
@@ -2282,7 +2283,8 @@ int matvec_orig_fused(ggem_ctx *c, const double *f, double *u, double *f_slot, i
   cudaError_t e = c->w_src.ensure(2 * (size_t)n);
   if (e) return cuda_fail(c, e, "pair records");
   Rec32 *src = reinterpret_cast<Rec32 *>(c->w_src.p);
-  k_to_slots_rec<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, c->order.p, c->pos32.p,
+  launch_dependent(k_to_slots_rec, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
+                   n, c->order.p, c->pos32.p,
                                                                      f, f_slot, src);
   if (int rc = check_launch(c, "to slots + records")) return rc;
   const double self_c = self_coefficient(c, self_mode);
@@ -2316,20 +2318,24 @@ int build_pair_tensors(ggem_ctx *c) {
   kt_start(c, kKListBuild);
   if (c->use_poly) {
     if (cd2)
-      k_pair_tensor<2, true><<<grid, 256, 0, c->stream>>>(n, c->pos32.p, c->nb_cnt.p, c->nb_w,
+      launch_dependent(k_pair_tensor<2, true>, dim3(grid), 256, 0, c->stream,
+                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
                                                           c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
                                                           g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
     else
-      k_pair_tensor<1, true><<<grid, 256, 0, c->stream>>>(n, c->pos32.p, c->nb_cnt.p, c->nb_w,
+      launch_dependent(k_pair_tensor<1, true>, dim3(grid), 256, 0, c->stream,
+                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
                                                           c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
                                                           g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
   } else {
     if (cd2)
-      k_pair_tensor<2, false><<<grid, 256, 0, c->stream>>>(n, c->pos32.p, c->nb_cnt.p, c->nb_w,
+      launch_dependent(k_pair_tensor<2, false>, dim3(grid), 256, 0, c->stream,
+                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
                                                            c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
                                                            g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
     else
-      k_pair_tensor<1, false><<<grid, 256, 0, c->stream>>>(n, c->pos32.p, c->nb_cnt.p, c->nb_w,
+      launch_dependent(k_pair_tensor<1, false>, dim3(grid), 256, 0, c->stream,
+                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
                                                            c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
                                                            g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
   }
