@@ -95,7 +95,6 @@ __device__ __forceinline__ void assign_one(int64_t i, const double *__restrict__
 __global__ void k_assign(int64_t n, const double *__restrict__ xyz, Grid g,
                          int32_t *__restrict__ cell_of, int32_t *__restrict__ count,
                          double4_32a *__restrict__ wrapped, int *__restrict__ err) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) assign_one(i, xyz, g, cell_of, count, wrapped, err);
@@ -192,7 +191,6 @@ constexpr int64_t kScanCellsMax = 4096 * kScanTiles;
 __global__ void __launch_bounds__(1024) k_scan_cells(int32_t *__restrict__ count,
                                                      int32_t *__restrict__ start, int64_t n,
                                                      unsigned long long *__restrict__ stat) {
-  allow_next_grid();
   wait_prior_grid();
   __shared__ int32_t warp_tot[2][32];
   if (stat && threadIdx.x < 2) stat[threadIdx.x] = 0ull;
@@ -252,7 +250,6 @@ __global__ void __launch_bounds__(1024) k_scan_cells(int32_t *__restrict__ count
 __global__ void k_scatter(int64_t n, const int32_t *__restrict__ cell_of,
                           const int32_t *__restrict__ start, int32_t *__restrict__ fill,
                           int32_t *__restrict__ order) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -268,7 +265,6 @@ __global__ void k_scatter(int64_t n, const int32_t *__restrict__ cell_of,
 // zeroed for the next build.
 __global__ void k_sort_cells(int64_t ncell, const int32_t *__restrict__ start,
                              int32_t *__restrict__ order, int32_t *__restrict__ fill) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t cidx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (cidx >= ncell) return;
@@ -331,7 +327,6 @@ __global__ void k_gather_sorted(int64_t n, Grid g, const int32_t *__restrict__ o
                                 const double4_32a *__restrict__ wrapped,
                                 int32_t *__restrict__ rank, double4_32a *__restrict__ pos64,
                                 float4 *__restrict__ pos32) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s < n) gather_one(s, g, order, cell_of, wrapped, rank, pos64, pos32);
@@ -593,7 +588,6 @@ __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err,
     int32_t *__restrict__ count_h, uint32_t *__restrict__ list_h) {
-  allow_next_grid();
   wait_prior_grid();
   pair_list_cell((int)blockIdx.x, g, stencil, nst, shift, start, pos32, pos64, rc2_lo, rc2_hi, rc2, W,
                  count, list, stat, err, count_h, list_h);
@@ -728,7 +722,6 @@ __global__ void __launch_bounds__(32 * kRunWarps) k_run_list(
     const int32_t *__restrict__ start, const float4 *__restrict__ pos32, int W,
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err) {
-  allow_next_grid();
   wait_prior_grid();
   __shared__ int s_tot[kRunWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

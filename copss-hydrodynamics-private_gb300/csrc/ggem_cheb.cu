@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(kVecThreads) k_finalize(int G, const double *_
                                                           double *__restrict__ out, int nq,
                                                           const unsigned long long *__restrict__ stat,
                                                           const int *__restrict__ err) {
-  allow_next_grid();
   wait_prior_grid();
   __shared__ double sh[32];
   const int q = blockIdx.x;
@@ -263,8 +262,8 @@ __global__ void k_axpy_into(int64_t tot, double s, const double *__restrict__ a,
 // vectors a kernel takes at once.  Bound by the FP64 pipe (two lanes per SM
 // and clock): four fused multiply-adds per element and vector, 48 us per step
 // at N = 200k, j = 12.  Eight vectors' warp sums share one reduce-scatter (9
-// additions instead of 40), which made the dots 37 -> {LZ_DOT} us.  N = 200k,
-// k = 24: 5.47 -> {LZ_MS} ms.
+// additions instead of 40), which made the dots 37 -> 27 us.  N = 200k,
+// k = 24: 5.47 -> 3.44 ms.
 constexpr int kLzMax = 512;  // steps
 
 struct LanczosState {
@@ -295,7 +294,6 @@ __global__ void __launch_bounds__(kVecThreads) k_lz_dots(int64_t D, int m,
                                                          const double *__restrict__ Q,
                                                          const double *__restrict__ w,
                                                          double *__restrict__ partial) {
-  allow_next_grid();
   wait_prior_grid();
   __shared__ double sh[kVecThreads / 32][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -364,7 +362,6 @@ __global__ void __launch_bounds__(kVecThreads) k_lz_project(int64_t D, int m,
                                                             LanczosState *S,
                                                             double *__restrict__ w,
                                                             double *__restrict__ partial) {
-  allow_next_grid();
   wait_prior_grid();
   extern __shared__ double sh[];  // [m]
   __shared__ double red[32];
@@ -402,7 +399,6 @@ __global__ void __launch_bounds__(kVecThreads) k_lz_project(int64_t D, int m,
 
 // q = w / |w|, and the step's coefficients
 __global__ void k_lz_next(int64_t D, int j, const double *w, double *q, LanczosState *S) {
-  allow_next_grid();
   wait_prior_grid();
   __shared__ double s_scale;
   if (threadIdx.x == 0) {  // (once per block: a root and a division cost ~40 FP64 instructions)

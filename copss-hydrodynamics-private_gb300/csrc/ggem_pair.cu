@@ -253,7 +253,6 @@ __global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, MinImage mi, D
                                                        const double *__restrict__ f,
                                                        double *__restrict__ u, int self_mode,
                                                        int r0) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
@@ -731,7 +730,6 @@ __device__ __forceinline__ void group_store(bool act, int sub, int64_t s, float 
 
 __global__ void k_build_src(int64_t n, const float4 *__restrict__ pos32,
                             const double *__restrict__ f, Rec32 *__restrict__ src) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
@@ -1014,7 +1012,6 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_r1(
     const float4 *__restrict__ shift, double self_c, const double *__restrict__ f,
     double *__restrict__ u, const int32_t *__restrict__ order, double *__restrict__ part) {
   __shared__ float4 sh[kMaxCode];
-  allow_next_grid();
   stage_shifts(sh, shift);  // (constant: no kernel writes it)
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
@@ -1050,7 +1047,6 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_first(
     const double *__restrict__ x0, double *__restrict__ m, double *__restrict__ x1,
     double *__restrict__ dw, Rec32 *__restrict__ next, double *__restrict__ part) {
   __shared__ float4 sh[kMaxCode];
-  allow_next_grid();
   stage_shifts(sh, shift);  // (constant: no kernel writes it)
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
@@ -1097,7 +1093,6 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_cheb(
     double *__restrict__ dw, Rec32 *__restrict__ next, double *__restrict__ part,
     int64_t nw, Rec32 *__restrict__ dw_next) {
   __shared__ float4 sh[kMaxCode];
-  allow_next_grid();
   stage_shifts(sh, shift);  // (constant: no kernel writes it)
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
@@ -1145,7 +1140,6 @@ __global__ void __launch_bounds__(256, kComputedMinBlocks[V]) k_pair_cheb(
 __global__ void k_to_slots_rec(int64_t n, const int32_t *__restrict__ order,
                                const float4 *__restrict__ pos32, const double *__restrict__ xi,
                                double *__restrict__ x0, Rec32 *__restrict__ rec) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
@@ -1202,7 +1196,6 @@ __global__ void __launch_bounds__(256) k_pair_tensor(
     int64_t n, const float4 *__restrict__ pos32, const int32_t *__restrict__ cnt, int W,
     const uint32_t *__restrict__ list, PolyAB P, const Rec32 *__restrict__ tab, float inv_ds,
     float hx, float hy, float hz, float4 *__restrict__ ten) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
   if (s < n)
@@ -1226,7 +1219,6 @@ __global__ void __launch_bounds__(256) k_batch_tensor(
 
 // forces of one right-hand side as one float4 per slot (w = 0)
 __global__ void k_stage_f4(int64_t n, const double *__restrict__ f, float4 *__restrict__ f4) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
@@ -1339,7 +1331,6 @@ __global__ void __launch_bounds__(256) k_pair_r1tv(int64_t n, const float4 *__re
                                                    const float4 *__restrict__ ten, double self_c,
                                                    const double *__restrict__ f,
                                                    double *__restrict__ u) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
@@ -1358,7 +1349,6 @@ __global__ void __launch_bounds__(256) k_pair_cheb_tv(
     double two_da, double two_db, double coef, const double *__restrict__ x0,
     const double *__restrict__ x1, double *__restrict__ xm, double *__restrict__ dw,
     float4 *__restrict__ next) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
@@ -1794,7 +1784,6 @@ __global__ void k_slots_to_f32(int64_t n, int nrhs, const double *__restrict__ f
 // orig [r][n][3] -> slots [r][n][3]
 __global__ void k_to_slots(int64_t n, int nrhs, const int32_t *__restrict__ order,
                            const double *__restrict__ orig, double *__restrict__ slot) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n * nrhs) return;
@@ -1809,7 +1798,6 @@ __global__ void k_to_slots(int64_t n, int nrhs, const int32_t *__restrict__ orde
 
 __global__ void k_from_slots(int64_t n, int nrhs, const int32_t *__restrict__ rank,
                              const double *__restrict__ slot, double *__restrict__ orig) {
-  allow_next_grid();
   wait_prior_grid();
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n * nrhs) return;
