@@ -8,12 +8,13 @@
 // predicts the interval from configuration features, the FP64 Chebyshev
 // error check judges every prediction, and Lanczos stays the fallback.
 //
-// Every matrix product (forward, both backward products) is one tcgen05
-// kernel: BF16 operands staged in shared memory in the K-major core-matrix
-// layout, one thread issues 128 x N x 16 MMAs accumulating FP32 in TMEM,
-// completion arrives on an mbarrier (bounded wait), and four warps read the
-// 128 TMEM lanes back.  Bias, SiLU, the loss gradient, the bias gradients
-// and Adam are small fused elementwise kernels.  Master weights stay FP32;
+// The products are tcgen05: BF16 operands staged in shared memory in the
+// K-major core-matrix layout, one thread issues 128 x N x 16 MMAs
+// accumulating FP32 in TMEM, completion arrives on an mbarrier (bounded
+// wait) and the warps read their TMEM lanes back.  Inference and the forward
+// and backward pass of training each chain their products in one kernel with
+// bias, SiLU and the loss gradient in the epilogues; the weight gradients of
+// all layers are a second launch, Adam small ones.  Master weights stay FP32;
 // the products use BF16 copies (K-major W^T for the forward product, W for
 // the input-gradient product).
 //
@@ -353,119 +354,385 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(
 // ---- elementwise pieces ---------------------------------------------------
 __device__ __forceinline__ float sigmoidf(float z) { return sigmoid_sfu(z); }
 
-// standardised, zero-padded inputs: X [B x 48] and X^T [48 x B] (BF16);
-// rows >= n (batch padding) are zero
-__global__ void k_stage_inputs(const float *__restrict__ x, const int32_t *__restrict__ idx,
-                               int n, int B, const float *__restrict__ mean,
-                               const float *__restrict__ inv_std, bf16 *__restrict__ X,
-                               bf16 *__restrict__ Xt) {
+// standardised, zero-padded inputs X [B x 48] (BF16); rows >= n (batch
+// padding) are zero
+__global__ void k_stage_inputs(const float *__restrict__ x, int n, int B,
+                               const float *__restrict__ mean,
+                               const float *__restrict__ inv_std, bf16 *__restrict__ X) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= B * kInPad) return;
   const int r = k / kInPad, c = k - r * kInPad;
   float v = 0.f;
-  if (r < n && c < kIn) {
-    const int src = idx ? idx[r] : r;
-    v = (x[(int64_t)src * kIn + c] - mean[c]) * inv_std[c];
-  }
-  const bf16 b = __float2bfloat16_rn(v);
-  X[k] = b;
-  Xt[(int64_t)c * B + r] = b;
+  if (r < n && c < kIn) v = (x[(int64_t)r * kIn + c] - mean[c]) * inv_std[c];
+  X[k] = __float2bfloat16_rn(v);
 }
 
-// Z += bias; hidden layers: H = silu(Z) as BF16 [B x 128] and H^T, Z kept
-// for the backward pass; output layer: Y[:, 0:2] = Z + b (FP32)
-__global__ void k_bias_act(float *__restrict__ Z, const float *__restrict__ bias, int B,
-                           int hidden, bf16 *__restrict__ H, bf16 *__restrict__ Ht,
-                           float *__restrict__ Y) {
+// hidden layers: H = silu(Z + b) as BF16 [B x 128]; output layer:
+// Y[:, 0:2] = Z + b (FP32)
+__global__ void k_bias_act(const float *__restrict__ Z, const float *__restrict__ bias, int B,
+                           int hidden, bf16 *__restrict__ H, float *__restrict__ Y) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= B * kHid) return;
   const int r = k / kHid, c = k - r * kHid;
   const float z = Z[k] + bias[c];
-  Z[k] = z;
   if (hidden) {
-    const bf16 h = __float2bfloat16_rn(silu_f(z));
-    H[k] = h;
-    Ht[(int64_t)c * B + r] = h;
+    H[k] = __float2bfloat16_rn(silu_f(z));
   } else if (c < kOut) {
     Y[(int64_t)r * kOut + c] = z;
   }
 }
 
-// dL/dY for L = mean_r sum_c (Y - T)^2 over the n valid rows, as the output
-// layer's dZ (FP32 for the bias gradient, BF16 and its transpose for the
-// products); partial sums of the loss per block
-__global__ void k_loss_grad(const float *__restrict__ Y, const float *__restrict__ T,
-                            const int32_t *__restrict__ idx, int n, int B,
-                            float *__restrict__ dZf, bf16 *__restrict__ dZ,
-                            bf16 *__restrict__ dZt, float *__restrict__ loss_part) {
-  __shared__ float sh[256];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.f;
-  if (k < B * kHid) {
-    const int r = k / kHid, c = k - r * kHid;
-    float g = 0.f;
-    if (r < n && c < kOut) {
-      const int src = idx ? idx[r] : r;
-      const float e = Y[(int64_t)r * kOut + c] - T[(int64_t)src * kOut + c];
-      l = e * e;
-      g = 2.f * e / (float)n;
+// ---- one training pass: forward and backward --------------------------------
+// A minibatch is 128-row tiles whose rows never mix until the weight
+// gradients, so one CTA of 32 warps takes a tile through all four forward
+// products, the loss gradient and the three input-gradient products: the
+// weights of both directions (182 KB) arrive in shared memory by
+// asynchronous copies in the order of their use, the activations (then the
+// dZ) live in one shared tile, and the hidden layers' pre-activations stay in
+// TMEM (3 x 128 of its 512 columns) until the backward epilogue reads them
+// again.  Only what the weight gradients contract leaves the CTA: H^T and
+// dZ^T (BF16), and dZ^T in FP32 for the biases.  k_train_grads then forms all
+// weight gradients (one CTA per 16 input columns of a layer), bias gradients
+// and the loss in one launch.  The products, their K order and the
+// elementwise arithmetic are those of one kernel per product and per
+// elementwise pass, 23 launches of 30-49 us (128 threads that staged a tile
+// 16 bytes at a time) and 3-4 us; latency of the dependent products bounds
+// both.  2000 predictions and one 256-row gradient 486 -> 154 us, copies included.
+constexpr size_t kTrW0 = kMlpActBytes;
+constexpr size_t kTrW1 = kTrW0 + (size_t)kHid * kInPad * 2;
+constexpr size_t kTrW2 = kTrW1 + (size_t)kHid * kHid * 2;
+constexpr size_t kTrW3 = kTrW2 + (size_t)kHid * kHid * 2;
+constexpr size_t kTrV3 = kTrW3 + (size_t)kOutN * kHid * 2;  // W of the output layer, 16 columns
+constexpr size_t kTrV2 = kTrV3 + (size_t)kHid * kOutN * 2;
+constexpr size_t kTrV1 = kTrV2 + (size_t)kHid * kHid * 2;
+constexpr size_t kTrBias = kTrV1 + (size_t)kHid * kHid * 2;
+constexpr size_t kTrSmem = kTrBias + (size_t)(kLayers - 1) * kHid * 4;
+
+struct TrainPass {
+  const float *x, *t;         // raw features [.][35], standardised targets [.][2]
+  const int32_t *idx;         // row of the batch -> row of x and t (or null)
+  int n, ld;                  // valid rows, leading dimension of the transposed arrays
+  const float *mean, *inv_std;
+  const bf16 *wt[kLayers], *w[kLayers];
+  const float *params;
+  bf16 *Xt, *Ht[3];           // [48][ld], [128][ld]
+  bf16 *dZt[kLayers];         // [128][ld]; the output layer's rows >= 2 stay zero
+  float *dZft[kLayers];       // [128][ld]; output layer: rows 0, 1
+  float *loss_part;           // one per two rows
+  uint32_t polls;
+  int *err;
+};
+
+__global__ void __launch_bounds__(kMlpThreads) k_train_pass(TrainPass a) {
+  extern __shared__ __align__(1024) uint8_t mlp_smem[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t tslot;
+  uint8_t *sA = mlp_smem;
+  float *s_bias = reinterpret_cast<float *>(mlp_smem + kTrBias);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, cb = warp >> 2;
+  const int row = quarter * 32 + lane;  // this thread's row = its TMEM lane
+  const int row_g = blockIdx.x * kRowBlock + row;
+  const int c0 = cb * kMlpCols;         // its columns c0 .. c0 + 15
+  const bool valid = row_g < a.n;
+  const int src = valid ? (a.idx ? a.idx[row_g] : row_g) : 0;
+  if (warp == 0) tc::tmem_alloc(&tslot, 512u);
+  if (tid == 0) {
+    tc::mbar_init(&bar, 1);
+    tc::mbar_fence_init();
+  }
+  // weights in the order of their use, one copy group per product
+  stage_wt(mlp_smem + kTrW0, a.wt[0], kHid, kInPad);
+  stage_f32(s_bias, a.params + bias_off_d(0), kHid / 4);
+  cp_async_commit();
+  stage_wt(mlp_smem + kTrW1, a.wt[1], kHid, kHid);
+  stage_f32(s_bias + kHid, a.params + bias_off_d(1), kHid / 4);
+  cp_async_commit();
+  stage_wt(mlp_smem + kTrW2, a.wt[2], kHid, kHid);
+  stage_f32(s_bias + 2 * kHid, a.params + bias_off_d(2), kHid / 4);
+  cp_async_commit();
+  stage_wt(mlp_smem + kTrW3, a.wt[3], kOutN, kHid);
+  // the first 16 columns of W [in x out]: the output layer's dZ is zero past 2
+  for (int c = tid; c < kHid * 2; c += blockDim.x)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     tc::smem_u32(mlp_smem + kTrV3 + tile_off(c >> 1, c & 1, 2))),
+                 "l"(a.w[3] + (c >> 1) * kHid + (c & 1) * 8)
+                 : "memory");
+  cp_async_commit();
+  stage_wt(mlp_smem + kTrV2, a.w[2], kHid, kHid);
+  cp_async_commit();
+  stage_wt(mlp_smem + kTrV1, a.w[1], kHid, kHid);
+  cp_async_commit();
+  // meanwhile the standardised input rows (48 BF16, zero padded)
+  if (warp < 4) {
+#pragma unroll
+    for (int kb = 0; kb < kInPad / 8; ++kb) {
+      __align__(16) bf16 h[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int c = kb * 8 + i;
+        const float v =
+            (valid && c < kIn) ? (a.x[(int64_t)src * kIn + c] - a.mean[c]) * a.inv_std[c] : 0.f;
+        h[i] = __float2bfloat16_rn(v);
+        a.Xt[(int64_t)c * a.ld + row_g] = h[i];
+      }
+      *reinterpret_cast<uint4 *>(sA + tile_off(row, kb, kInPad / 8)) =
+          *reinterpret_cast<const uint4 *>(h);
     }
-    dZf[k] = g;
-    const bf16 b = __float2bfloat16_rn(g);
-    dZ[k] = b;
-    dZt[(int64_t)c * B + r] = b;
   }
-  sh[threadIdx.x] = l;
+  cp_async_wait_upto<5>();  // layer 0's weights and bias
+  tc::fence_proxy_async_smem();
+  tc::fence_before_sync();
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  tc::fence_after_sync();
+  const uint32_t tmem = tslot;
+  const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+  constexpr uint32_t kWork = 3 * kHid;  // TMEM columns of the output and backward products
+  bool ok = true;
+  uint32_t phase = 0;
+  // one product of the A tile into TMEM column d; every thread waits for it
+  auto product = [&](size_t b_off, int K, int N, uint32_t d) {
+    if (tid == 0) {
+      const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(mlp_smem + b_off);
+      const uint32_t idesc = tc::idesc_bf16_f32(kRowBlock, N);
+      for (int q = 0; q < K / 16; ++q) {
+        const uint64_t ad = tc::smem_desc(a0 + q * 256, 128, (uint32_t)(K / 8) * 128);
+        const uint64_t bd = tc::smem_desc(b0 + q * 256, 128, (uint32_t)(K / 8) * 128);
+        tc::mma_bf16(tmem + d, ad, bd, idesc, q > 0 ? 1u : 0u);
+      }
+      tc::mma_commit(&bar);
+    }
+    const bool done = tc::mbar_wait_bounded(&bar, phase, a.polls);
+    phase ^= 1u;
+    ok = __syncthreads_and(done) != 0;
+    if (ok) tc::fence_after_sync();
+    return ok;
+  };
+  // the tile and the next product's weights are in place for the tensor core
+  auto ready = [&]() {
+    tc::fence_proxy_async_smem();
+    tc::fence_before_sync();
     __syncthreads();
+    tc::fence_after_sync();
+  };
+  // forward, hidden layers: H = silu(Z + b) into the tile and H^T
+  auto hidden = [&](int l, size_t b_off, int K) {
+    if (!product(b_off, K, kHid, (uint32_t)(l * kHid))) return;
+    const float *bias = s_bias + l * kHid + c0;
+    float v[16];
+    tc::tmem_ld16(lane_base + (uint32_t)(l * kHid + c0), v);
+#pragma unroll
+    for (int h8 = 0; h8 < kMlpCols / 8; ++h8) {
+      __align__(16) bf16 h[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        h[i] = __float2bfloat16_rn(silu_f(v[8 * h8 + i] + bias[8 * h8 + i]));
+        a.Ht[l][(int64_t)(c0 + 8 * h8 + i) * a.ld + row_g] = h[i];
+      }
+      *reinterpret_cast<uint4 *>(sA + tile_off(row, (c0 >> 3) + h8, kHid / 8)) =
+          *reinterpret_cast<const uint4 *>(h);
+    }
+  };
+  // backward: dZ of hidden layer l = (dZ of the next layer) W * silu'(Z),
+  // into the tile where another product follows
+  auto back = [&](int l, size_t b_off, int K, bool tile) {
+    if (!product(b_off, K, kHid, kWork)) return;
+    const float *bias = s_bias + l * kHid + c0;
+    float d[16], v[16];
+    tc::tmem_ld16(lane_base + kWork + (uint32_t)c0, d);
+    tc::tmem_ld16(lane_base + (uint32_t)(l * kHid + c0), v);
+#pragma unroll
+    for (int h8 = 0; h8 < kMlpCols / 8; ++h8) {
+      __align__(16) bf16 h[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float z = v[8 * h8 + i] + bias[8 * h8 + i], sg = sigmoid_sfu(z);
+        const float g = d[8 * h8 + i] * sg * (1.f + z * (1.f - sg));
+        const int64_t at = (int64_t)(c0 + 8 * h8 + i) * a.ld + row_g;
+        h[i] = __float2bfloat16_rn(g);
+        a.dZft[l][at] = g;
+        a.dZt[l][at] = h[i];
+      }
+      if (tile)
+        *reinterpret_cast<uint4 *>(sA + tile_off(row, (c0 >> 3) + h8, kHid / 8)) =
+            *reinterpret_cast<const uint4 *>(h);
+    }
+  };
+  do {
+    hidden(0, kTrW0, kInPad);
+    if (!ok) break;
+    cp_async_wait_upto<4>();
+    ready();
+    hidden(1, kTrW1, kHid);
+    if (!ok) break;
+    cp_async_wait_upto<3>();
+    ready();
+    hidden(2, kTrW2, kHid);
+    if (!ok) break;
+    cp_async_wait_upto<2>();
+    ready();
+    // the two outputs, their loss and dZ = 2 (y - t) / n
+    if (!product(kTrW3, kHid, kOutN, kWork)) break;
+    if (warp < 4) {
+      float v[8];
+      tc::tmem_ld8(lane_base + kWork, v);
+      const float *bias = a.params + bias_off_d(kLayers - 1);
+      float g[kOut], l[kOut];
+#pragma unroll
+      for (int c = 0; c < kOut; ++c) {
+        g[c] = l[c] = 0.f;
+        if (valid) {
+          const float e = v[c] + bias[c] - a.t[(int64_t)src * kOut + c];
+          l[c] = e * e;
+          g[c] = 2.f * e / (float)a.n;
+        }
+      }
+      // (the sum of two rows, column by column first)
+      const float p0 = l[0] + __shfl_down_sync(0xffffffffu, l[0], 1);
+      const float p1 = l[1] + __shfl_down_sync(0xffffffffu, l[1], 1);
+      if (!(lane & 1)) a.loss_part[row_g >> 1] = p0 + p1;
+      __align__(16) bf16 h[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) h[c] = __float2bfloat16_rn(c < kOut ? g[c & 1] : 0.f);
+#pragma unroll
+      for (int c = 0; c < kOut; ++c) {
+        a.dZft[3][(int64_t)c * a.ld + row_g] = g[c];
+        a.dZt[3][(int64_t)c * a.ld + row_g] = h[c];
+      }
+      *reinterpret_cast<uint4 *>(sA + tile_off(row, 0, 2)) = *reinterpret_cast<const uint4 *>(h);
+      *reinterpret_cast<uint4 *>(sA + tile_off(row, 1, 2)) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    ready();
+    back(2, kTrV3, kOutN, true);
+    if (!ok) break;
+    cp_async_wait_upto<1>();
+    ready();
+    back(1, kTrV2, kHid, true);
+    if (!ok) break;
+    cp_async_wait_upto<0>();
+    ready();
+    back(0, kTrV1, kHid, false);
+  } while (false);
+  if (!ok) {
+    if (tid == 0) atomicOr(a.err, kErrTimeout);
+    // the product still in flight completes before TMEM is freed
+    tc::mbar_wait_bounded(&bar, phase ^ 1u, kMaxPolls);
   }
-  if (threadIdx.x == 0) loss_part[blockIdx.x] = sh[0];
+  cp_async_wait_upto<0>();  // no copy outlives the block (the timeout path)
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 512u);
+  }
 }
 
-// dZ = dH * silu'(Z)
-__global__ void k_act_back(const float *__restrict__ dH, const float *__restrict__ Z, int B,
-                           float *__restrict__ dZf, bf16 *__restrict__ dZ,
-                           bf16 *__restrict__ dZt) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= B * kHid) return;
-  const int r = k / kHid, c = k - r * kHid;
-  const float z = Z[k], s = sigmoidf(z);
-  const float g = dH[k] * s * (1.f + z * (1.f - s));
-  dZf[k] = g;
-  const bf16 b = __float2bfloat16_rn(g);
-  dZ[k] = b;
-  dZt[(int64_t)c * B + r] = b;
+// All gradients of a pass.  Blocks 0 .. 26: dW^T [128 x 16] = dZ^T [128 x B]
+// (prev^T)^T of 16 input columns of a layer (3 of layer 0, 8 of the others);
+// then one warp per bias (the tree of 128 running sums); the last block adds
+// the loss partials to *loss.
+constexpr int kGradN = 16, kGradChunk = 256;
+constexpr int kGradTiles = kInPad / kGradN + 3 * (kHid / kGradN);
+constexpr int kGradBias = kLayers * kHid / 4;
+constexpr size_t kGradSmem = (size_t)(kRowBlock + kGradN) * kGradChunk * 2;
+
+__device__ __forceinline__ float sum128(float (&q)[4]) {
+  float v = (q[0] + q[2]) + (q[1] + q[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// db[c] = sum_r dZ[r][c], fixed order per column
-__global__ void k_colsum(const float *__restrict__ dZf, int B, float *__restrict__ db) {
-  __shared__ float sh[128];
-  const int c = blockIdx.x;
-  float acc = 0.f;
-  for (int r = threadIdx.x; r < B; r += blockDim.x) acc += dZf[(int64_t)r * kHid + c];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
+__global__ void __launch_bounds__(128) k_train_grads(TrainPass a, int B, float *__restrict__ g,
+                                                     float *__restrict__ loss) {
+  extern __shared__ __align__(1024) uint8_t gr_smem[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t tslot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int bid = blockIdx.x;
+  if (bid >= kGradTiles) {
+    const bool is_loss = bid == kGradTiles + kGradBias;
+    const int col = (bid - kGradTiles) * 4 + warp, l = col / kHid, c = col - l * kHid;
+    if (is_loss && (warp || !loss)) return;
+    const float *v = is_loss ? a.loss_part : a.dZft[l] + (int64_t)c * a.ld;
+    const int m = is_loss ? B / 2 : (l == kLayers - 1 && c >= kOut ? 0 : B);
+    float q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[i] = 0.f;
+      for (int r = lane + 32 * i; r < m; r += 128) q[i] += v[r];
+    }
+    const float t = sum128(q);
+    if (lane == 0) {
+      if (is_loss) loss[0] += t;
+      else g[bias_off_d(l) + c] = t;
+    }
+    return;
   }
-  if (threadIdx.x == 0) db[c] = sh[0];
-}
-
-// acc[0] += sum of count partials, fixed order (one block)
-__global__ void k_sum_parts(const float *__restrict__ parts, int count, float *__restrict__ acc) {
-  __shared__ float sh[128];
-  float a = 0.f;
-  for (int i = threadIdx.x; i < count; i += blockDim.x) a += parts[i];
-  sh[threadIdx.x] = a;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
+  const int l = bid < kInPad / kGradN ? 0 : 1 + (bid - kInPad / kGradN) / (kHid / kGradN);
+  const int n0 = kGradN * (l == 0 ? bid : (bid - kInPad / kGradN) % (kHid / kGradN));
+  const int in_dim = l == 0 ? kInPad : kHid;
+  const bf16 *A = a.dZt[l], *Bt = (l == 0 ? a.Xt : a.Ht[l - 1]) + (int64_t)n0 * a.ld;
+  uint8_t *sA = gr_smem, *sB = gr_smem + (size_t)kRowBlock * kGradChunk * 2;
+  if (warp == 0) tc::tmem_alloc(&tslot, 32u);
+  if (tid == 0) {
+    tc::mbar_init(&bar, 1);
+    tc::mbar_fence_init();
   }
-  if (threadIdx.x == 0) acc[0] += sh[0];
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tslot;
+  const uint32_t idesc = tc::idesc_bf16_f32(kRowBlock, kGradN);
+  uint32_t phase = 0;
+  bool ok = true;
+  for (int k0 = 0; k0 < B && ok; k0 += kGradChunk) {
+    const int kp = min(kGradChunk, B - k0) >> 3;  // 16-byte pieces per row
+    for (int c = tid; c < (kRowBlock + kGradN) * kp; c += blockDim.x) {
+      const int r = c / kp, kb = c - r * kp;
+      const bool in_a = r < kRowBlock;
+      const int rr = in_a ? r : r - kRowBlock;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       tc::smem_u32((in_a ? sA : sB) + tile_off(rr, kb, kp))),
+                   "l"((in_a ? A : Bt) + (int64_t)rr * a.ld + k0 + kb * 8)
+                   : "memory");
+    }
+    cp_async_wait();
+    tc::fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tc::fence_after_sync();
+      const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB);
+      for (int q = 0; q < kp / 2; ++q) {
+        const uint64_t ad = tc::smem_desc(a0 + q * 256, 128, (uint32_t)kp * 128);
+        const uint64_t bd = tc::smem_desc(b0 + q * 256, 128, (uint32_t)kp * 128);
+        tc::mma_bf16(tmem, ad, bd, idesc, (k0 > 0 || q > 0) ? 1u : 0u);
+      }
+      tc::mma_commit(&bar);
+    }
+    const bool done = tc::mbar_wait_bounded(&bar, phase, a.polls);
+    phase ^= 1u;
+    ok = __syncthreads_and(done) != 0;
+  }
+  if (!ok) {
+    if (tid == 0) atomicOr(a.err, kErrTimeout);
+    tc::mbar_wait_bounded(&bar, phase ^ 1u, kMaxPolls);
+  } else {
+    tc::fence_after_sync();
+    float v[16];
+    tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16), v);
+    const int wo = l == 0 ? 0 : kHid * kInPad + kHid + (l - 1) * (kHid * kHid + kHid);
+    float4 *dst = reinterpret_cast<float4 *>(g + wo + (warp * 32 + lane) * in_dim + n0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 32u);
+  }
 }
 
 // Adam (Kingma & Ba) on the FP32 master parameters; weights [out x in] also
@@ -571,8 +838,11 @@ struct ggem_surrogate {
   float norm[GGEM_SUR_NORM] = {0};
   DevBuf<float> d_mean, d_inv_std;
   int cap = 0;                            // batch capacity (rows)
-  DevBuf<bf16> X, Xt, H[3], Ht[3], dZ, dZt;
-  DevBuf<float> Z[kLayers], Y, dZf, dH, loss_part, loss_acc;
+  DevBuf<bf16> X, H[3];                   // the layer-by-layer predictions
+  DevBuf<float> Z, Y;
+  int tcap = 0;                           // a training pass's rows (leading dimension)
+  DevBuf<bf16> tXt, tHt[3], tdZt[kLayers];
+  DevBuf<float> tdZft[kLayers], loss_part, loss_acc;
   DevBuf<float> xin, yin;
   DevBuf<int32_t> idx;
   DevBuf<int> flag;
@@ -612,17 +882,33 @@ int ensure_cap(ggem_surrogate *s, int B) {
   if (B <= s->cap) return GGEM_OK;
   cudaError_t e = cudaSuccess;
   const size_t b = (size_t)B;
-  if ((e = s->X.ensure(b * kInPad)) || (e = s->Xt.ensure(b * kInPad)) ||
-      (e = s->dZ.ensure(b * kHid)) || (e = s->dZt.ensure(b * kHid)) ||
-      (e = s->Y.ensure(b * kOut)) || (e = s->dZf.ensure(b * kHid)) ||
-      (e = s->dH.ensure(b * kHid)) || (e = s->loss_part.ensure(b * kHid / 256 + 1)))
+  if ((e = s->X.ensure(b * kInPad)) ||
+      (e = s->Z.ensure(b * kHid)) || (e = s->Y.ensure(b * kOut)))
     return scuda(s, e, "surrogate activations");
-  for (int l = 0; l < kLayers; ++l)
-    if ((e = s->Z[l].ensure(b * kHid))) return scuda(s, e, "surrogate activations");
   for (int l = 0; l < 3; ++l)
-    if ((e = s->H[l].ensure(b * kHid)) || (e = s->Ht[l].ensure(b * kHid)))
-      return scuda(s, e, "surrogate activations");
+    if ((e = s->H[l].ensure(b * kHid))) return scuda(s, e, "surrogate activations");
   s->cap = B;
+  return GGEM_OK;
+}
+
+// the arrays of a training pass over up to B rows (their leading dimension
+// stays the capacity, so the output layer's rows 2 .. 127 of dZ^T stay zero)
+int ensure_train(ggem_surrogate *s, int B) {
+  if (B <= s->tcap) return GGEM_OK;
+  s->tcap = 0;
+  cudaError_t e = cudaSuccess;
+  const size_t b = (size_t)B;
+  if ((e = s->tXt.ensure(b * kInPad)) || (e = s->loss_part.ensure(b / 2)))
+    return scuda(s, e, "training pass");
+  for (int l = 0; l < 3; ++l)
+    if ((e = s->tHt[l].ensure(b * kHid))) return scuda(s, e, "training pass");
+  for (int l = 0; l < kLayers; ++l)
+    if ((e = s->tdZt[l].ensure(b * kHid)) ||
+        (e = s->tdZft[l].ensure(b * (l < kLayers - 1 ? kHid : kOut))))
+      return scuda(s, e, "training pass");
+  if ((e = cudaMemsetAsync(s->tdZt[kLayers - 1].p, 0, sizeof(bf16) * b * kHid, s->stream)))
+    return scuda(s, e, "training pass");
+  s->tcap = B;
   return GGEM_OK;
 }
 
@@ -650,17 +936,15 @@ int forward_fused(ggem_surrogate *s, const float *d_x, int64_t n, float *d_y) {
 
 unsigned blocks(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-// the staged batch X, Xt (B rows) through the four layers into s->Y
+// the staged batch X (B rows) through the four layers into s->Y
 int forward(ggem_surrogate *s, int B) {
   const bf16 *in = s->X.p;
   int in_dim = kInPad;
   for (int l = 0; l < kLayers; ++l) {
-    if (int rc = gemm(s, in, in_dim, s->wt[l].p, in_dim, s->Z[l].p, kHid, B, kHid, in_dim))
-      return rc;
+    if (int rc = gemm(s, in, in_dim, s->wt[l].p, in_dim, s->Z.p, kHid, B, kHid, in_dim)) return rc;
     const bool hidden = l < kLayers - 1;
     k_bias_act<<<blocks((int64_t)B * kHid), 256, 0, s->stream>>>(
-        s->Z[l].p, s->p.p + bias_off(l), B, hidden ? 1 : 0, hidden ? s->H[l].p : nullptr,
-        hidden ? s->Ht[l].p : nullptr, s->Y.p);
+        s->Z.p, s->p.p + bias_off(l), B, hidden ? 1 : 0, hidden ? s->H[l].p : nullptr, s->Y.p);
     if (int rc = slaunch(s, "bias/activation")) return rc;
     if (hidden) {
       in = s->H[l].p;
@@ -670,34 +954,40 @@ int forward(ggem_surrogate *s, int B) {
   return GGEM_OK;
 }
 
-// gradient of the loss over n valid rows of the staged batch into s->g
-int backward(ggem_surrogate *s, int B, int n, const int32_t *d_idx, const float *d_T,
-             float *d_loss) {
-  const unsigned nb = blocks((int64_t)B * kHid);
-  k_loss_grad<<<nb, 256, 0, s->stream>>>(s->Y.p, d_T, d_idx, n, B, s->dZf.p, s->dZ.p, s->dZt.p,
-                                         s->loss_part.p);
-  if (int rc = slaunch(s, "loss gradient")) return rc;
-  if (d_loss) {
-    k_sum_parts<<<1, 128, 0, s->stream>>>(s->loss_part.p, (int)nb, d_loss);
-    if (int rc = slaunch(s, "loss sum")) return rc;
+// forward and backward pass over n rows (through d_idx when given) into s->g;
+// the summed squared error is added to *d_loss
+int train_pass(ggem_surrogate *s, const float *d_x, const float *d_t, const int32_t *d_idx, int n,
+               int B, float *d_loss) {
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute(k_train_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kTrSmem)) ||
+      (e = cudaFuncSetAttribute(k_train_grads, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kGradSmem)))
+    return scuda(s, e, "network attributes");
+  TrainPass a;
+  a.x = d_x;
+  a.t = d_t;
+  a.idx = d_idx;
+  a.n = n;
+  a.ld = s->tcap;
+  a.mean = s->d_mean.p;
+  a.inv_std = s->d_inv_std.p;
+  a.params = s->p.p;
+  a.Xt = s->tXt.p;
+  for (int l = 0; l < kLayers; ++l) {
+    a.wt[l] = s->wt[l].p;
+    a.w[l] = s->w[l].p;
+    a.dZt[l] = s->tdZt[l].p;
+    a.dZft[l] = s->tdZft[l].p;
+    if (l < 3) a.Ht[l] = s->tHt[l].p;
   }
-  for (int l = kLayers - 1; l >= 0; --l) {
-    const int in_dim = kInDim[l];
-    const bf16 *prevT = l > 0 ? s->Ht[l - 1].p : s->Xt.p;
-    // dW^T [128 x in] = dZ^T [128 x B] * prev [B x in]
-    if (int rc = gemm(s, s->dZt.p, B, prevT, B, s->g.p + kWOff[l], in_dim, kHid, in_dim, B))
-      return rc;
-    k_colsum<<<kHid, 128, 0, s->stream>>>(s->dZf.p, B, s->g.p + bias_off(l));
-    if (int rc = slaunch(s, "bias gradient")) return rc;
-    if (l == 0) break;
-    // dH [B x in] = dZ [B x 128] * W [in x 128]^T
-    if (int rc = gemm(s, s->dZ.p, kHid, s->w[l].p, kHid, s->dH.p, kHid, B, in_dim, kHid))
-      return rc;
-    k_act_back<<<nb, 256, 0, s->stream>>>(s->dH.p, s->Z[l - 1].p, B, s->dZf.p, s->dZ.p,
-                                          s->dZt.p);
-    if (int rc = slaunch(s, "activation gradient")) return rc;
-  }
-  return GGEM_OK;
+  a.loss_part = s->loss_part.p;
+  a.polls = s->polls;
+  a.err = s->flag.p;
+  k_train_pass<<<B / kRowBlock, kMlpThreads, kTrSmem, s->stream>>>(a);
+  if (int rc = slaunch(s, "training pass")) return rc;
+  k_train_grads<<<kGradTiles + kGradBias + 1, 128, kGradSmem, s->stream>>>(a, B, s->g.p, d_loss);
+  return slaunch(s, "gradients");
 }
 
 }  // namespace
@@ -730,6 +1020,8 @@ int upload_norm(ggem_surrogate *s) {
   return GGEM_OK;
 }
 
+// waits for the stream (and so for the copies issued before) and evaluates
+// the error word
 int check_flag(ggem_surrogate *s) {
   int f = 0;
   cudaError_t e;
@@ -740,10 +1032,10 @@ int check_flag(ggem_surrogate *s) {
   return GGEM_OK;
 }
 
-// stage rows [0, n) of device features x (through idx when given) as batch B
-int stage(ggem_surrogate *s, const float *d_x, const int32_t *d_idx, int n, int B) {
-  k_stage_inputs<<<blocks((int64_t)B * kInPad), 256, 0, s->stream>>>(
-      d_x, d_idx, n, B, s->d_mean.p, s->d_inv_std.p, s->X.p, s->Xt.p);
+// stage rows [0, n) of device features x as batch B
+int stage(ggem_surrogate *s, const float *d_x, int n, int B) {
+  k_stage_inputs<<<blocks((int64_t)B * kInPad), 256, 0, s->stream>>>(d_x, n, B, s->d_mean.p,
+                                                                     s->d_inv_std.p, s->X.p);
   return slaunch(s, "stage inputs");
 }
 
@@ -805,38 +1097,9 @@ extern "C" void ggem_surrogate_destroy(ggem_surrogate *s) {
   {
     SurDeviceGuard dg(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    s->p.release();
-    s->m.release();
-    s->v.release();
-    s->g.release();
-    for (int l = 0; l < kLayers; ++l) {
-      s->wt[l].release();
-      s->w[l].release();
-      s->Z[l].release();
-    }
-    for (int l = 0; l < 3; ++l) {
-      s->H[l].release();
-      s->Ht[l].release();
-    }
-    s->X.release();
-    s->Xt.release();
-    s->dZ.release();
-    s->dZt.release();
-    s->Y.release();
-    s->dZf.release();
-    s->dH.release();
-    s->loss_part.release();
-    s->loss_acc.release();
-    s->xin.release();
-    s->yin.release();
-    s->idx.release();
-    s->flag.release();
-    s->yout.release();
-    s->d_mean.release();
-    s->d_inv_std.release();
     if (s->stream) cudaStreamDestroy(s->stream);
+    delete s;  // (its buffers, on their device)
   }
-  delete s;
 }
 
 extern "C" const char *ggem_surrogate_last_error(const ggem_surrogate *s) {
@@ -884,9 +1147,11 @@ extern "C" int ggem_surrogate_get_params(ggem_surrogate *s, float *params) {
 
 namespace {
 
-// standardised targets (n x 2) and raw features (n x 35) on the device
-int upload_data(ggem_surrogate *s, const float *X, const float *Y, int64_t n) {
-  std::vector<float> t(Y ? (size_t)n * kOut : 0);
+// standardised targets t (n x 2, kept by the caller until the stream has
+// synchronised) and raw features (n x 35) on the device
+int upload_data(ggem_surrogate *s, const float *X, const float *Y, int64_t n,
+                std::vector<float> &t) {
+  t.resize(Y ? (size_t)n * kOut : 0);
   for (int64_t r = 0; r < (Y ? n : 0); ++r)
     for (int c = 0; c < kOut; ++c) {
       const float sd = s->norm[2 * kIn + kOut + c];
@@ -902,7 +1167,6 @@ int upload_data(ggem_surrogate *s, const float *X, const float *Y, int64_t n) {
   if (Y && (e = cudaMemcpyAsync(s->yin.p, t.data(), sizeof(float) * n * kOut,
                                 cudaMemcpyHostToDevice, s->stream)))
     return scuda(s, e, "surrogate data");
-  if ((e = cudaStreamSynchronize(s->stream))) return scuda(s, e, "surrogate data");
   return GGEM_OK;
 }
 
@@ -932,8 +1196,9 @@ extern "C" int ggem_surrogate_train(ggem_surrogate *s, const float *X, const flo
     return s ? sfail(s, GGEM_ERR_BAD_ARG, "train: bad arguments (batch a multiple of 128)")
              : GGEM_ERR_BAD_ARG;
   SurDeviceGuard dg(s->device);
-  if (int rc = ensure_cap(s, batch)) return rc;
-  if (int rc = upload_data(s, X, Y, n)) return rc;
+  if (int rc = ensure_train(s, batch)) return rc;
+  std::vector<float> targets;
+  if (int rc = upload_data(s, X, Y, n, targets)) return rc;
   cudaError_t e;
   if ((e = s->idx.ensure((size_t)n)) || (e = s->loss_acc.ensure((size_t)epochs)))
     return scuda(s, e, "train buffers");
@@ -956,9 +1221,7 @@ extern "C" int ggem_surrogate_train(ggem_surrogate *s, const float *X, const flo
       const int nb = (int)std::min<int64_t>(batch, n - b0);
       const int B = round_rows(nb);
       const int32_t *ib = s->idx.p + b0;
-      if (int rc = stage(s, s->xin.p, ib, nb, B)) return rc;
-      if (int rc = forward(s, B)) return rc;
-      if (int rc = backward(s, B, nb, ib, s->yin.p, s->loss_acc.p + ep)) return rc;
+      if (int rc = train_pass(s, s->xin.p, s->yin.p, ib, nb, B, s->loss_acc.p + ep)) return rc;
       // cosine decay to lr / 20
       const float f = (float)(0.05 + 0.95 * 0.5 * (1.0 + std::cos(kPiS * step / total)));
       if (int rc = adam_step(s, lr * f)) return rc;
@@ -980,7 +1243,8 @@ extern "C" int ggem_surrogate_train(ggem_surrogate *s, const float *X, const flo
 extern "C" int ggem_surrogate_predict(ggem_surrogate *s, const float *X, int64_t n, float *Y) {
   if (!s || !X || !Y || n <= 0 || n > (int64_t)1 << 30) return GGEM_ERR_BAD_ARG;
   SurDeviceGuard dg(s->device);
-  if (int rc = upload_data(s, X, nullptr, n)) return rc;
+  std::vector<float> none;
+  if (int rc = upload_data(s, X, nullptr, n, none)) return rc;
   cudaError_t e;
   if ((e = s->yout.ensure((size_t)n * kOut)) ||
       (e = cudaMemsetAsync(s->flag.p, 0, sizeof(int), s->stream)))
@@ -989,8 +1253,7 @@ extern "C" int ggem_surrogate_predict(ggem_surrogate *s, const float *X, int64_t
   if (int rc = forward_fused(s, s->xin.p, n, s->yout.p)) return rc;
   std::vector<float> out((size_t)n * kOut);
   if ((e = cudaMemcpyAsync(out.data(), s->yout.p, sizeof(float) * n * kOut,
-                           cudaMemcpyDeviceToHost, s->stream)) ||
-      (e = cudaStreamSynchronize(s->stream)))
+                           cudaMemcpyDeviceToHost, s->stream)))
     return scuda(s, e, "predict readback");
   if (int rc = check_flag(s)) return rc;
   for (int64_t r = 0; r < n; ++r)
@@ -1005,14 +1268,15 @@ extern "C" int ggem_surrogate_predict_layers(ggem_surrogate *s, const float *X, 
   SurDeviceGuard dg(s->device);
   const int cap = std::max(s->cap, std::min(round_rows(n), 4096));
   if (int rc = ensure_cap(s, cap)) return rc;
-  if (int rc = upload_data(s, X, nullptr, n)) return rc;
+  std::vector<float> none;
+  if (int rc = upload_data(s, X, nullptr, n, none)) return rc;
   cudaError_t e;
   if ((e = cudaMemsetAsync(s->flag.p, 0, sizeof(int), s->stream))) return scuda(s, e, "predict");
   std::vector<float> out((size_t)cap * kOut);
   for (int64_t r0 = 0; r0 < n; r0 += cap) {
     const int nb = (int)std::min<int64_t>(cap, n - r0);
     const int B = round_rows(nb);
-    if (int rc = stage(s, s->xin.p + r0 * kIn, nullptr, nb, B)) return rc;
+    if (int rc = stage(s, s->xin.p + r0 * kIn, nb, B)) return rc;
     if (int rc = forward(s, B)) return rc;
     if ((e = cudaMemcpyAsync(out.data(), s->Y.p, sizeof(float) * nb * kOut,
                              cudaMemcpyDeviceToHost, s->stream)) ||
@@ -1063,23 +1327,22 @@ extern "C" int ggem_surrogate_gradient(ggem_surrogate *s, const float *X, const 
   if (!s || !X || !Y || n <= 0 || n > 4096 || !grad) return GGEM_ERR_BAD_ARG;
   SurDeviceGuard dg(s->device);
   const int B = round_rows(n);
-  if (int rc = ensure_cap(s, B)) return rc;
-  if (int rc = upload_data(s, X, Y, n)) return rc;
+  if (int rc = ensure_train(s, B)) return rc;
+  std::vector<float> targets;
+  if (int rc = upload_data(s, X, Y, n, targets)) return rc;
   cudaError_t e;
   if ((e = cudaMemsetAsync(s->flag.p, 0, sizeof(int), s->stream)) ||
       (e = cudaMemsetAsync(s->loss_acc.p, 0, sizeof(float), s->stream)))
     return scuda(s, e, "gradient");
-  if (int rc = stage(s, s->xin.p, nullptr, (int)n, B)) return rc;
-  if (int rc = forward(s, B)) return rc;
-  if (int rc = backward(s, B, (int)n, nullptr, s->yin.p, s->loss_acc.p)) return rc;
+  if (int rc = train_pass(s, s->xin.p, s->yin.p, nullptr, (int)n, B, s->loss_acc.p)) return rc;
   float l = 0.f;
   if ((e = cudaMemcpyAsync(grad, s->g.p, sizeof(float) * GGEM_SUR_PARAMS, cudaMemcpyDeviceToHost,
                            s->stream)) ||
-      (e = cudaMemcpyAsync(&l, s->loss_acc.p, sizeof(float), cudaMemcpyDeviceToHost, s->stream)) ||
-      (e = cudaStreamSynchronize(s->stream)))
+      (e = cudaMemcpyAsync(&l, s->loss_acc.p, sizeof(float), cudaMemcpyDeviceToHost, s->stream)))
     return scuda(s, e, "gradient readback");
+  const int rc = check_flag(s);
   if (loss) *loss = l / (float)n;
-  return check_flag(s);
+  return rc;
 }
 
 extern "C" int ggem_surrogate_features(ggem_ctx *ctx, double chain_fraction, float *features) {
