@@ -55,9 +55,10 @@ constexpr int kSpMaxExt = 32;    // dilated brick extent per axis (5-bit coordin
 constexpr size_t kSpRecBytes = 16384;
 constexpr int kSpMaxWords = 1024;  // stencil bitmap words (32768 element offsets)
 constexpr int kSpQueue = 64;      // queued members per warp (< 32 left + 32 new)
-constexpr size_t kSpShared = kSpRecBytes + kSpWarps * (32 * sizeof(float4) + kSpQueue * sizeof(uint32_t)) +
-                             2 * (kSpMaxSeg + 1) * sizeof(int32_t) +
-                             kSpMaxWords * sizeof(uint32_t);
+constexpr int kSpReachWords = 1024;  // union bitmap of a brick's elements
+constexpr size_t kSpShared =
+    kSpRecBytes + kSpWarps * (32 * sizeof(float4) + kSpQueue * sizeof(uint32_t)) +
+    2 * (kSpMaxSeg + 1) * sizeof(int32_t) + (kSpMaxWords + kSpReachWords) * sizeof(uint32_t);
 
 struct SpreadGeo {
   Grid g;
@@ -163,6 +164,9 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   for (int k = threadIdx.x; k < 3 * kSpMaxExt; k += kSpThreads)
     s_shift[k / kSpMaxExt][k % kSpMaxExt] = sg.shift[k / kSpMaxExt][k % kSpMaxExt];
   for (int k = threadIdx.x; k < sg.nwords; k += kSpThreads) s_bits[k] = bits[k];
+  uint32_t *s_reach = s_bits + kSpMaxWords;
+  if (F32 && PAD)
+    for (int k = threadIdx.x; k < kSpReachWords; k += kSpThreads) s_reach[k] = bits[sg.nwords + k];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int B = sg.B;
@@ -249,40 +253,79 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   uint32_t *mq = queue + warp * kSpQueue;
   float4 *mb = batch + warp * 32;
   const unsigned lt_mask = (1u << lane) - 1u;
+  // with the padded bitmap, a particle at frame coordinates u is listed by
+  // some element of the brick when the union bitmap holds u (shifted where
+  // an open face clips the frame)
+  int clip = 0;
+  if (PAD)
+    clip = (fr[0].F - (e0[0] + sg.lo[0])) + 32 * (fr[1].F - (e0[1] + sg.lo[1])) +
+           1024 * (fr[2].F - (e0[2] + sg.lo[2]));
+  __shared__ int s_kept[kSpWarps];
   // (a brick without particles in reach makes one empty pass: its sums are 0)
   for (int c0 = 0; c0 == 0 || c0 < total; c0 += CAP) {
-    const int cn = min(CAP, total - c0);
-    // stage particles [c0, c0 + cn): segment by binary search
-    for (int k = threadIdx.x; k < cn; k += kSpThreads) {
+    const int cw = min(CAP, total - c0);
+    // stage particles [c0, c0 + cw), in order; the FP32 kernel drops those
+    // that no element of the brick lists (about half of the dilated box), so
+    // that every element's membership pass is as much shorter: 144^3 elements
+    // x 8 points, N = 200k 4.22 -> 3.90 ms
+    int cn = 0;
+    for (int k0 = 0; k0 < cw; k0 += kSpThreads) {
+      const int k = k0 + threadIdx.x;
       const int v = c0 + k;
-      int lo = 0, hi = nseg - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (seg_pre[mid] <= v) lo = mid;
-        else hi = mid - 1;
+      bool keep = k < cw;
+      int slot = 0;
+      uint32_t u = 0;
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (keep) {  // segment by binary search
+        int lo = 0, hi = nseg - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (seg_pre[mid] <= v) lo = mid;
+          else hi = mid - 1;
+        }
+        slot = seg_begin[lo] + (v - seg_pre[lo]);
+        const int row = lo / nseg_x, kk = lo - row * nseg_x;
+        const int uy = row % fr[1].E, uz = row / fr[1].E;
+        p = pos32[slot];
+        const int cid = __float_as_int(p.w);
+        const int cx = cid % sg.g.nc[0];
+        int ux;
+        if (fr[0].full) ux = cx;
+        else if (!sg.g.periodic[0]) ux = cx - fr[0].F;
+        else if (nseg_x == 1) ux = cx - wrap_cell(xa, sg.g.nc[0]);
+        else ux = kk == 0 ? cx - wrap_cell(xa, sg.g.nc[0]) : cx + (sg.g.nc[0] - wrap_cell(xa, sg.g.nc[0]));
+        u = (uint32_t)ux | ((uint32_t)uy << 5) | ((uint32_t)uz << 10);
+        if (F32 && PAD) {
+          const int idx = (int)u + clip;
+          keep = (s_reach[idx >> 5] >> (idx & 31)) & 1u;
+        }
       }
-      const int slot = seg_begin[lo] + (v - seg_pre[lo]);
-      const int row = lo / nseg_x, kk = lo - row * nseg_x;
-      const int uy = row % fr[1].E, uz = row / fr[1].E;
-      const float4 p = pos32[slot];
-      const int cid = __float_as_int(p.w);
-      const int cx = cid % sg.g.nc[0];
-      int ux;
-      if (fr[0].full) ux = cx;
-      else if (!sg.g.periodic[0]) ux = cx - fr[0].F;
-      else if (nseg_x == 1) ux = cx - wrap_cell(xa, sg.g.nc[0]);
-      else ux = kk == 0 ? cx - wrap_cell(xa, sg.g.nc[0]) : cx + (sg.g.nc[0] - wrap_cell(xa, sg.g.nc[0]));
-      const uint32_t u = (uint32_t)ux | ((uint32_t)uy << 5) | ((uint32_t)uz << 10);
-      const double *fp = f_slot + 3 * (int64_t)slot;
-      if (F32) {
-        rec32[k] = make_float4(p.x, p.y, p.z, __uint_as_float(u));
-        rec32[kSpCap32 + k] = make_float4(d2f_bits(fp[0]), d2f_bits(fp[1]), d2f_bits(fp[2]), 0.f);
-      } else {
-        const double4_32a q = pos64[slot];
-        rec64[2 * k] = make_double4_32a(q.x, q.y, q.z, __longlong_as_double((long long)u));
-        rec64[2 * k + 1] = make_double4_32a(fp[0], fp[1], fp[2], 0.0);
+      int at = k;
+      if (F32 && PAD) {  // position among the kept ones
+        const unsigned bal = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) s_kept[warp] = __popc(bal);
+        __syncthreads();
+        at = cn + __popc(bal & lt_mask);
+        for (int w = 0; w < kSpWarps; ++w) {
+          if (w < warp) at += s_kept[w];
+          cn += s_kept[w];
+        }
+        __syncthreads();
+      }
+      if (keep) {
+        const double *fp = f_slot + 3 * (int64_t)slot;
+        if (F32) {
+          rec32[at] = make_float4(p.x, p.y, p.z, __uint_as_float(u));
+          rec32[kSpCap32 + at] =
+              make_float4(d2f_bits(fp[0]), d2f_bits(fp[1]), d2f_bits(fp[2]), 0.f);
+        } else {
+          const double4_32a q = pos64[slot];
+          rec64[2 * at] = make_double4_32a(q.x, q.y, q.z, __longlong_as_double((long long)u));
+          rec64[2 * at + 1] = make_double4_32a(fp[0], fp[1], fp[2], 0.0);
+        }
       }
     }
+    if (!(F32 && PAD)) cn = cw;
     __syncthreads();
     for (int le = warp; le < nel; le += kSpWarps) {
       const int lx = le % ebx, ly = (le / ebx) % eby, lz = le / (ebx * eby);
@@ -948,6 +991,19 @@ int spread_geometry(ggem_ctx *c, SpreadGeo *sg) {
   };
   set(0, 0, 0);  // the element's own particles come first in its list
   for (const int4 &o : c->stencil) set(o.x, o.y, o.z);
+  if (sg->pad) {
+    // the particles that some element of a brick lists: bit u is the union of
+    // the stencil bits u + (jx, jy, jz), 0 <= j < B (the elements of a brick
+    // read the bitmap at u + B - 1 - l); one word per (y, z), x in its bits
+    std::vector<uint32_t> x(kSpReachWords, 0u), y(kSpReachWords, 0u), z(kSpReachWords, 0u);
+    for (int k = 0; k < sg->nwords; ++k)
+      for (int j = 0; j < B; ++j) x[k] |= bits[k] >> j;
+    for (int k = 0; k < kSpReachWords; ++k)
+      for (int j = 0; j < B && (k & 31) + j < 32; ++j) y[k] |= x[k + j];
+    for (int k = 0; k < kSpReachWords; ++k)
+      for (int j = 0; j < B && k + 32 * j < kSpReachWords; ++j) z[k] |= y[k + 32 * j];
+    bits.insert(bits.end(), z.begin(), z.end());
+  }
   cudaError_t e = c->sp_bits.ensure(bits.size());
   if (e) return cuda_fail(c, e, "spread stencil");
   if ((e = cudaMemcpyAsync(c->sp_bits.p, bits.data(), sizeof(uint32_t) * bits.size(),
