@@ -367,22 +367,36 @@ __device__ __forceinline__ bool exact_within(const Grid &g, double4_32a a, doubl
 // Warp-per-cell pair list, one pass into fixed-width rows.  The candidates
 // of a target cell are the concatenation of its stencil cells (stencil
 // order, slot order inside a cell).  For each chunk of up to 32 targets the
-// lanes first take 32 consecutive candidates at a time with coalesced loads
-// and keep those within reach of the chunk's bounding box; the kept ones
-// queue in shared memory, in candidate order, and every 32 of them are
-// tested against the chunk's targets, which are broadcast one at a time from
-// shared memory; a ballot prefix places each accepted candidate.  Entries
+// lanes, one stencil cell each, write the candidates' entries to shared
+// memory in that order; 64 of them at a time are then loaded, and those
+// within reach of the chunk's bounding box queue in shared memory, still in
+// order.  A full queue is tested against the chunk's targets, four at a time
+// (list_targets); a ballot prefix places each accepted candidate.  Entries
 // therefore come out in exactly the per-target order of a sequential sweep.
 // Row s holds entries [s*W, s*W + cnt[s]); a row longer than W is counted
 // but not stored: the kernel records the longest row and sets
 // kErrListCapacity, and the host rebuilds with a wider W.
+//
+// The instruction issue bounds it (58 M warp instructions at N = 200k, phi =
+// 0.1, 78% of the issue slots, DRAM 1%), so the work is in instructions per
+// test.  One target at a time with its count in a lane took 83.5 M and 92 us;
+// four targets' coordinates, row pointers and counts held in registers over
+// a whole queue, two targets per packed instruction, 82 us; the stencil
+// lanes writing the entries, instead of a marked scan that looks up each
+// candidate's cell, 73 us; two loads in flight per lane 68 us; the box by
+// warp-wide reductions 67 us (N = 400k: 167 -> 121 us).  Eight targets at a
+// time spilled (75 us), a queue of 128 went over the targets too often (86 us
+// where 256 took 82), three or four loads in flight 69 us.
 // One warp per block, one block per cell: cells hold different numbers of
-// targets, and a block of several cell-warps held its resources until its
-// longest cell was done (N = 200k, phi = 0.1: 92 us against 101 us with 8
-// warps per block, and against 97 us with 8-warp blocks claiming cells from
-// a counter).
+// targets, and a block of several cell-warps holds its resources until its
+// longest cell is done; with the cell no longer block-uniform its row
+// addresses also leave the uniform registers (two warps per block: 90 us).
+// Resident blocks that stride over the cells balance worse (91 to 102 us
+// where the former kernel took 92).
 constexpr int kMaxStencil = 128;  // stencil cells per target cell
-constexpr int kListQueue = 64;    // queued candidates per warp (< 32 left + 32 new)
+constexpr int kListIndex = 256;   // candidates per round: their entries in order
+constexpr int kListLoads = 2;     // candidates in flight per lane
+constexpr int kListQueue = 160 + 32 * kListLoads;  // kept candidates: tested once past 160
 
 // FP32 distance of a candidate from the targets' box, formed like the pair
 // test's r2 below (the same subtractions, squares and fused adds, each
@@ -396,6 +410,108 @@ __device__ __forceinline__ float box_r2(float qx, float qy, float qz, float3 lo,
   return fmaf(bz, bz, fmaf(by, by, bx * bx));
 }
 
+// a warp's minimum and maximum (NaN ignored, as fminf and fmaxf do)
+__device__ __forceinline__ float warp_min(float x) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// A queue of candidates against GT of the chunk's ntc targets, i0 and on (slot
+// t0 + i0 and on; past the last target s_pi is far from everything).  The
+// targets and their rows stay in registers over all batches of 32, two
+// targets per packed instruction (each half rounds as the scalar form does).
+template <int GT, bool HALF>
+__device__ __forceinline__ void list_targets(int i0, int ntc, int32_t t0, int queued, bool last,
+                                             const float4 *s_q, const float4 *s_pi, const Grid &g,
+                                             const double4_32a *__restrict__ pos64, float rc2_lo,
+                                             float rc2_hi, double rc2, int W,
+                                             uint32_t *__restrict__ list,
+                                             uint32_t *__restrict__ list_h, int32_t &own_cnt,
+                                             int32_t &own_cnt_h) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  float2 px[GT / 2], py[GT / 2], pz[GT / 2];
+  int32_t at[GT], at_h[GT];
+  uint32_t *row[GT];
+#pragma unroll
+  for (int q = 0; q < GT; q += 2) {
+    const float4 a = s_pi[i0 + q], b = s_pi[i0 + q + 1];
+    px[q / 2] = make_float2(-a.x, -b.x);
+    py[q / 2] = make_float2(-a.y, -b.y);
+    pz[q / 2] = make_float2(-a.z, -b.z);
+  }
+#pragma unroll
+  for (int q = 0; q < GT; ++q) {
+    at[q] = __shfl_sync(0xffffffffu, own_cnt, i0 + q);
+    at_h[q] = HALF ? __shfl_sync(0xffffffffu, own_cnt_h, i0 + q) : 0;
+    row[q] = list + (int64_t)(t0 + i0 + q) * W;
+  }
+  // a partial batch only after the last candidates
+  const int stop = last ? queued : queued & ~31;
+  for (int b = 0; b < stop; b += 32) {
+    // lanes past the queue carry a far point: r2 overflows, never accepted
+    const float4 c = b + lane < queued ? s_q[b + lane] : make_float4(1e30f, 1e30f, 1e30f, 0.f);
+    const uint32_t en = __float_as_uint(c.w);
+    const int32_t tj = (int32_t)(en >> kCodeBits);
+    const float2 cx = make_float2(c.x, c.x), cy = make_float2(c.y, c.y), cz = make_float2(c.z, c.z);
+    bool in[GT];
+    bool band = false;
+#pragma unroll
+    for (int q = 0; q < GT; q += 2) {
+      const float2 dx = __fadd2_rn(cx, px[q / 2]), dy = __fadd2_rn(cy, py[q / 2]),
+                   dz = __fadd2_rn(cz, pz[q / 2]);
+      const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+      // accepted below rc2_lo, rejected above rc2_hi; in between (FP32
+      // rounding of |r| = rc) the exact FP64 test decides, behind a
+      // warp-uniform branch so that the common case carries none of it
+      in[q] = tj != t0 + i0 + q && !(r2.x > rc2_hi);
+      in[q + 1] = tj != t0 + i0 + q + 1 && !(r2.y > rc2_hi);
+      band |= in[q] && !(r2.x < rc2_lo);
+      band |= in[q + 1] && !(r2.y < rc2_lo);
+    }
+    if (__any_sync(0xffffffffu, band)) {
+#pragma unroll
+      for (int q = 0; q < GT; ++q) {
+        const float4 pi = s_pi[i0 + q];
+        const float dx = c.x - pi.x, dy = c.y - pi.y, dz = c.z - pi.z;
+        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        if (in[q] && !(r2 < rc2_lo))
+          in[q] = i0 + q < ntc && exact_within(g, pos64[t0 + i0 + q], pos64[tj], rc2);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < GT; ++q) {
+      const unsigned bal = __ballot_sync(0xffffffffu, in[q]);
+      const int32_t k = at[q] + __popc(bal & lt_mask);
+      if (in[q] && k < W) row[q][k] = en;
+      at[q] += __popc(bal);
+      if (HALF) {
+        // the half list: each unordered pair once, in the row of its
+        // smaller slot (the full list is symmetric, its predicate exact)
+        const bool in_h = in[q] && tj > t0 + i0 + q;
+        const unsigned bal_h = __ballot_sync(0xffffffffu, in_h);
+        const int32_t kh = at_h[q] + __popc(bal_h & lt_mask);
+        if (in_h && kh < W) list_h[(int64_t)(t0 + i0 + q) * W + kh] = en;
+        at_h[q] += __popc(bal_h);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < GT; ++q) {
+    if (lane == i0 + q) {
+      own_cnt = at[q];
+      if (HALF) own_cnt_h = at_h[q];
+    }
+  }
+}
+
+template <bool HALF>
 __device__ __forceinline__ void pair_list_cell(
     int C, const Grid &g, const int4 *__restrict__ stencil, int nst,
     const float4 *__restrict__ shift, const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
@@ -403,47 +519,13 @@ __device__ __forceinline__ void pair_list_cell(
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err,
     int32_t *__restrict__ count_h, uint32_t *__restrict__ list_h) {
-  __shared__ int32_t s_base[kMaxStencil];
-  __shared__ int32_t s_pre[kMaxStencil + 1];
-  __shared__ int32_t s_code[kMaxStencil];
-  __shared__ float4 s_pi[32];          // the targets of the current chunk
-  __shared__ float4 s_q[kListQueue];   // kept candidates: frame position, entry
-  __shared__ int s_mark[32];           // stencil cell starting at each lane of a chunk
+  __shared__ float4 s_pi[32];             // the targets of the current chunk
+  __shared__ float4 s_q[kListQueue];      // kept candidates: frame position, entry
+  __shared__ uint32_t s_idx[kListIndex];  // entries of the current round's candidates
   const int lane = threadIdx.x;
-  s_mark[lane] = -1;
   const int32_t tb = start[C], te = start[C + 1];
   if (te <= tb) return;
   const int cx = C % g.nc[0], cy = (C / g.nc[0]) % g.nc[1], cz = C / (g.nc[0] * g.nc[1]);
-  // stencil cell ranges and their running prefix (warp scan over chunks)
-  int32_t carry = 0;
-  for (int k0 = 0; k0 < nst; k0 += 32) {
-    const int k = k0 + lane;
-    int32_t cnt = 0, base = 0, code = 0;
-    if (k < nst) {
-      const int4 o = stencil[k];
-      const int32_t nc = shifted_cell(g, cx, cy, cz, o);
-      code = o.w;
-      if (nc >= 0) {
-        base = start[nc];
-        cnt = start[nc + 1] - base;
-      }
-    }
-    int32_t incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (k < nst) {
-      s_base[k] = base;
-      s_code[k] = code;
-      s_pre[k] = carry + incl - cnt;
-    }
-    carry += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  if (lane == 0) s_pre[nst] = carry;
-  __syncwarp();
-  const int32_t V = carry;
   const unsigned lt_mask = (1u << lane) - 1u;
   unsigned long long cell_total = 0;
   int32_t cell_max = 0;
@@ -452,128 +534,103 @@ __device__ __forceinline__ void pair_list_cell(
     const int32_t own = t0 + lane;
     const bool own_ok = lane < ntc;
     __syncwarp();  // the previous chunk's targets are no longer read
-    const float4 mine = own_ok ? pos32[own] : make_float4(0.f, 0.f, 0.f, 0.f);
+    // slots past the chunk's targets are as far from every candidate as the
+    // padding candidates are on the other side: r2 overflows
+    const float4 mine = own_ok ? pos32[own] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
     s_pi[lane] = mine;
     // the chunk's bounding box (FP32 min / max of the targets' own values)
     float3 blo = own_ok ? make_float3(mine.x, mine.y, mine.z)
                         : make_float3(INFINITY, INFINITY, INFINITY);
     float3 bhi = own_ok ? make_float3(mine.x, mine.y, mine.z)
                         : make_float3(-INFINITY, -INFINITY, -INFINITY);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      blo.x = fminf(blo.x, __shfl_xor_sync(0xffffffffu, blo.x, o));
-      blo.y = fminf(blo.y, __shfl_xor_sync(0xffffffffu, blo.y, o));
-      blo.z = fminf(blo.z, __shfl_xor_sync(0xffffffffu, blo.z, o));
-      bhi.x = fmaxf(bhi.x, __shfl_xor_sync(0xffffffffu, bhi.x, o));
-      bhi.y = fmaxf(bhi.y, __shfl_xor_sync(0xffffffffu, bhi.y, o));
-      bhi.z = fmaxf(bhi.z, __shfl_xor_sync(0xffffffffu, bhi.z, o));
-    }
+    blo = make_float3(warp_min(blo.x), warp_min(blo.y), warp_min(blo.z));
+    bhi = make_float3(warp_max(bhi.x), warp_max(bhi.y), warp_max(bhi.z));
     __syncwarp();
     int32_t own_cnt = 0, own_cnt_h = 0;
     int queued = 0;  // warp-uniform
-    int kcur = -1;   // warp-uniform: the stencil cell of candidate v0 - 1
-    for (int32_t v0 = 0; v0 < V; v0 += 32) {
-      const int32_t v = v0 + lane;
-      const bool valid = v < V;
-      // stencil cell of candidate v, the last k with s_pre[k] <= v: the
-      // cells after kcur that start inside this chunk mark their first lane
-      // (the largest k wins, skipping empty cells), and a max-scan over the
-      // lanes carries each cell forward
-      for (int kk = kcur + 1;; kk += 32) {
-        const int k = kk + lane;
-        const int p = k < nst ? s_pre[k] - v0 : 32;
-        if (p < 32) atomicMax(&s_mark[p], k);
-        if (__shfl_sync(0xffffffffu, p, 31) >= 32) break;
+    for (int k0 = 0; k0 < nst; k0 += 32) {
+      // one stencil cell per lane: its slots and where they go in the order
+      const int k = k0 + lane;
+      int32_t cnt = 0, base = 0;
+      uint32_t code = 0;
+      if (k < nst) {
+        const int4 o = stencil[k];
+        const int32_t nc = shifted_cell(g, cx, cy, cz, o);
+        code = (uint32_t)o.w;
+        if (nc >= 0) {
+          base = start[nc];
+          cnt = start[nc + 1] - base;
+        }
       }
-      __syncwarp();
-      int lo = max(s_mark[lane], kcur);
-      s_mark[lane] = -1;  // ready for the next chunk
-      __syncwarp();
+      int32_t incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, lo, o);
-        if (lane >= o) lo = max(lo, y);
+        const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
-      kcur = __shfl_sync(0xffffffffu, lo, 31);
-      const int32_t t = valid ? s_base[lo] + (v - s_pre[lo]) : 0;
-      const int code = s_code[lo];
-      const float4 sh = shift[code];
-      const float4 pj = valid ? pos32[t] : make_float4(0.f, 0.f, 0.f, 0.f);
-      // the candidate in the target cell's frame (the shift added once per
-      // candidate; the filter's band absorbs the different rounding)
-      const float qx = pj.x + sh.x, qy = pj.y + sh.y, qz = pj.z + sh.z;
-      const bool keep = valid && !(box_r2(qx, qy, qz, blo, bhi) > rc2_hi);
-      const unsigned kb = __ballot_sync(0xffffffffu, keep);
-      if (keep)
-        s_q[queued + __popc(kb & lt_mask)] =
-            make_float4(qx, qy, qz, __uint_as_float(((uint32_t)t << kCodeBits) | (uint32_t)code));
-      queued += __popc(kb);
-      const bool last = v0 + 32 >= V;
-      // test the queue 32 at a time (a partial batch only after the last
-      // candidates); at most two batches per pass
-      while (queued >= 32 || (last && queued > 0)) {
+      const int32_t V = __shfl_sync(0xffffffffu, incl, 31);
+      const int32_t first = incl - cnt;
+      for (int32_t r0 = 0; r0 == 0 || r0 < V; r0 += kListIndex) {
+        const int32_t Vr = min(V - r0, kListIndex);
+        __syncwarp();  // the previous round's candidates are read
+        for (int32_t v = max(first, r0); v < min(incl, r0 + kListIndex); ++v)
+          s_idx[v - r0] = ((uint32_t)(base + v - first) << kCodeBits) | code;
         __syncwarp();
-        const int m = min(queued, 32);
-        // lanes past the batch carry a far point: r2 overflows, never accepted
-        const float4 c = lane < m ? s_q[lane] : make_float4(1e30f, 1e30f, 1e30f, 0.f);
-        const uint32_t en = __float_as_uint(c.w);
-        const int32_t tj = (int32_t)(en >> kCodeBits);
-        for (int i = 0; i < ntc; ++i) {
-          const float4 pi = s_pi[i];  // one broadcast read
-          const int32_t ti = t0 + i;
-          const float dx = c.x - pi.x;
-          const float dy = c.y - pi.y;
-          const float dz = c.z - pi.z;
-          const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-          // accepted below rc2_lo, rejected above rc2_hi; in between (FP32
-          // rounding of |r| = rc) the exact FP64 test decides, behind a
-          // warp-uniform branch so that the common case carries none of it
-          bool in = tj != ti && !(r2 > rc2_hi);
-          const bool band = in && !(r2 < rc2_lo);
-          if (__any_sync(0xffffffffu, band)) {
-            if (band) in = exact_within(g, pos64[ti], pos64[tj], rc2);
+        for (int32_t v0 = 0; v0 == 0 || v0 < Vr; v0 += 32 * kListLoads) {
+          uint32_t en[kListLoads];
+          float4 sh[kListLoads], pj[kListLoads];
+#pragma unroll
+          for (int h = 0; h < kListLoads; ++h) {
+            const int32_t v = v0 + 32 * h + lane;
+            en[h] = v < Vr ? s_idx[v] : 0u;
+            sh[h] = shift[en[h] & ((1u << kCodeBits) - 1u)];
+            pj[h] = v < Vr ? pos32[en[h] >> kCodeBits] : make_float4(0.f, 0.f, 0.f, 0.f);
           }
-          const unsigned bal = __ballot_sync(0xffffffffu, in);
-          const int32_t at = __shfl_sync(0xffffffffu, own_cnt, i);
-          if (in) {
-            const int32_t k = at + __popc(bal & lt_mask);
-            if (k < W) list[(int64_t)ti * W + k] = en;
+#pragma unroll
+          for (int h = 0; h < kListLoads; ++h) {
+            // the candidate in the target cell's frame (the shift added once
+            // per candidate; the filter's band absorbs the different rounding)
+            const float qx = pj[h].x + sh[h].x, qy = pj[h].y + sh[h].y, qz = pj[h].z + sh[h].z;
+            const bool keep =
+                v0 + 32 * h + lane < Vr && !(box_r2(qx, qy, qz, blo, bhi) > rc2_hi);
+            const unsigned kb = __ballot_sync(0xffffffffu, keep);
+            if (keep)
+              s_q[queued + __popc(kb & lt_mask)] = make_float4(qx, qy, qz, __uint_as_float(en[h]));
+            queued += __popc(kb);
           }
-          if (lane == i) own_cnt += __popc(bal);
-          if (list_h) {
-            // the half list: each unordered pair once, in the row of its
-            // smaller slot (the full list is symmetric, its predicate exact)
-            const bool in_h = in && tj > ti;
-            const unsigned bal_h = __ballot_sync(0xffffffffu, in_h);
-            const int32_t at_h = __shfl_sync(0xffffffffu, own_cnt_h, i);
-            if (in_h) {
-              const int32_t k = at_h + __popc(bal_h & lt_mask);
-              if (k < W) list_h[(int64_t)ti * W + k] = en;
+          const bool last =
+              k0 + 32 >= nst && r0 + kListIndex >= V && v0 + 32 * kListLoads >= Vr;
+          if (queued <= kListQueue - 32 * kListLoads && !last) continue;
+          // the queue against every target: whole batches, the rest moves to
+          // its front, or all of it after the last candidates
+          __syncwarp();
+          for (int i = 0; i < ntc;) {
+            if (ntc - i > 2) {
+              list_targets<4, HALF>(i, ntc, t0, queued, last, s_q, s_pi, g, pos64, rc2_lo, rc2_hi,
+                                    rc2, W, list, list_h, own_cnt, own_cnt_h);
+              i += 4;
+            } else {
+              list_targets<2, HALF>(i, ntc, t0, queued, last, s_q, s_pi, g, pos64, rc2_lo, rc2_hi,
+                                    rc2, W, list, list_h, own_cnt, own_cnt_h);
+              i += 2;
             }
-            if (lane == i) own_cnt_h += __popc(bal_h);
           }
+          const int done = queued & ~31;
+          queued -= done;
+          const float4 r = lane < queued ? s_q[done + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+          __syncwarp();
+          if (lane < queued) s_q[lane] = r;
         }
-        // move the rest of the queue to its front
-        const int rest = queued - m;
-        const float4 r = lane < rest ? s_q[32 + lane] : c;
-        __syncwarp();
-        if (lane < rest) s_q[lane] = r;
-        queued = rest;
       }
     }
     if (own_ok) {
-      if (count_h) count_h[own] = min(own_cnt_h, W);
+      if (HALF) count_h[own] = min(own_cnt_h, W);
       count[own] = min(own_cnt, W);  // the stored entries; the full length goes to stat
-      cell_total += (unsigned long long)own_cnt;
-      cell_max = max(cell_max, own_cnt);
     }
+    cell_total += __reduce_add_sync(0xffffffffu, (unsigned)own_cnt);
+    cell_max = max(cell_max, __reduce_max_sync(0xffffffffu, own_cnt));
   }
-  // one atomic per warp (per cell) for the list statistics
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cell_total += __shfl_xor_sync(0xffffffffu, cell_total, o);
-    cell_max = max(cell_max, __shfl_xor_sync(0xffffffffu, cell_max, o));
-  }
+  // one pair of atomics per cell for the list statistics
   if (lane == 0) {
     atomicAdd(&stat[0], cell_total);
     atomicMax(&stat[1], (unsigned long long)cell_max);
@@ -581,6 +638,7 @@ __device__ __forceinline__ void pair_list_cell(
   }
 }
 
+template <bool HALF>
 __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
     Grid g, const int4 *__restrict__ stencil, int nst, const float4 *__restrict__ shift,
     const int32_t *__restrict__ start, const float4 *__restrict__ pos32,
@@ -589,7 +647,7 @@ __global__ void __launch_bounds__(32, 32) k_pair_list_warp(
     unsigned long long *__restrict__ stat, int *__restrict__ err,
     int32_t *__restrict__ count_h, uint32_t *__restrict__ list_h) {
   wait_prior_grid();
-  pair_list_cell((int)blockIdx.x, g, stencil, nst, shift, start, pos32, pos64, rc2_lo, rc2_hi, rc2, W,
+  pair_list_cell<HALF>((int)blockIdx.x, g, stencil, nst, shift, start, pos32, pos64, rc2_lo, rc2_hi, rc2, W,
                  count, list, stat, err, count_h, list_h);
 }
 
@@ -704,7 +762,7 @@ __global__ void __launch_bounds__(32, 32) k_batch_list(
     int32_t *__restrict__ count, uint32_t *__restrict__ list,
     unsigned long long *__restrict__ stat, int *__restrict__ err) {
   const BatchGeo &b = geo[cell_susp[blockIdx.x]];
-  pair_list_cell((int)((int64_t)blockIdx.x - b.cell0), b.g, b.stencil, b.nst, b.shift, start + b.cell0,
+  pair_list_cell<false>((int)((int64_t)blockIdx.x - b.cell0), b.g, b.stencil, b.nst, b.shift, start + b.cell0,
                  pos32, pos64, rc2_lo, rc2_hi, rc2, W, count, list, stat, err, nullptr, nullptr);
 }
 
@@ -912,10 +970,11 @@ void launch_pair_list(ggem_ctx *c, int nst, int W, cudaStream_t st) {
         c->nb_list.p, c->nb_stat.p, c->err.p);
     return;
   }
-  launch_dependent(k_pair_list_warp, dim3((unsigned)c->grid.ncell), 32, 0, st,
-                   c->grid, c->d_stencil.p, nst, c->d_shift.p, c->cell_start.p, c->pos32.p, c->pos64.p,
-      c->rc2_lo, c->rc2_hi, c->rc2, W, c->nb_cnt.p, c->nb_list.p, c->nb_stat.p, c->err.p,
-      c->sym_pairs ? c->nb_cnt_h.p : nullptr, c->sym_pairs ? c->nb_list_h.p : nullptr);
+  launch_dependent(c->sym_pairs ? k_pair_list_warp<true> : k_pair_list_warp<false>,
+                   dim3((unsigned)c->grid.ncell), 32, 0, st, c->grid, c->d_stencil.p, nst,
+                   c->d_shift.p, c->cell_start.p, c->pos32.p, c->pos64.p, c->rc2_lo, c->rc2_hi, c->rc2,
+                   W, c->nb_cnt.p, c->nb_list.p, c->nb_stat.p, c->err.p,
+                   c->sym_pairs ? c->nb_cnt_h.p : nullptr, c->sym_pairs ? c->nb_list_h.p : nullptr);
 }
 
 int build_pair_list(ggem_ctx *c) {
