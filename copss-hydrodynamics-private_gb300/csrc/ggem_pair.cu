@@ -58,23 +58,37 @@ __device__ __forceinline__ void self_term(const DevConsts &K, int self_mode, con
   }
 }
 
-// minimum image of one axis (pm_periodic_boundary.C:350-374: d <= -L/2 adds
-// L, d > L/2 subtracts it) with the comparisons on the bit patterns: an FP64
-// comparison costs as much of the FP64 pipe as an addition, an integer one
-// nothing of it.  half: the bits of L/2, or of infinity on an open axis;
-// wrapped positions keep |d| < L, so one shift suffices.
+// Minimum image (pm_periodic_boundary.C:350-374: d <= -L/2 adds L, d > L/2
+// subtracts it) with the comparisons on the bit patterns: an FP64 comparison
+// costs as much of the FP64 pipe as an addition, an integer one nothing of
+// it.  half: the bits of L/2, or of infinity on an open axis; wrapped
+// positions keep |d| < L, so one shift suffices.
 struct MinImage {
   long long half[3], L[3];
 };
 
-__device__ __forceinline__ double min_image_bits(double d, long long half, long long L) {
+__device__ __forceinline__ bool past_half(double d, long long half) {
   const long long b = __double_as_longlong(d);
-  const long long sign = b & (long long)0x8000000000000000ull;
-  const long long mag = b ^ sign;
-  const bool out = mag + (sign ? 1 : 0) > half;
-  // +L for a negative d, -L for a positive one, +0 inside
-  const long long w = out ? (L | (sign ^ (long long)0x8000000000000000ull)) : 0ll;
-  return d + __longlong_as_double(w);
+  return (b & 0x7fffffffffffffffll) + (b < 0 ? 1 : 0) > half;
+}
+
+// +L for a negative d, -L for a positive one
+__device__ __forceinline__ double shift_image(double d, long long L) {
+  const long long sign = __double_as_longlong(d) & (long long)0x8000000000000000ull;
+  return d + __longlong_as_double(L | (sign ^ (long long)0x8000000000000000ull));
+}
+
+// The three axes of a pair.  The additions are behind a branch of the warp's
+// active lanes: away from the box faces (81% of the targets at N = 200k, phi
+// = 0.1) no lane takes them, which is 3 of a pair's 33 FP64 instructions.
+__device__ __forceinline__ void min_image3(const MinImage &mi, double &x, double &y, double &z) {
+  const bool ox = past_half(x, mi.half[0]), oy = past_half(y, mi.half[1]),
+             oz = past_half(z, mi.half[2]);
+  if (__any_sync(__activemask(), ox || oy || oz)) {
+    if (ox) x = shift_image(x, mi.L[0]);
+    if (oy) y = shift_image(y, mi.L[1]);
+    if (oz) z = shift_image(z, mi.L[2]);
+  }
 }
 
 // one 256-bit read-only load
@@ -205,9 +219,8 @@ __device__ __forceinline__ void pair_row_f64(int sub, int m, const uint32_t *__r
     const int64_t t = (int64_t)(nxt >> kCodeBits);
     if (k + G < m) nxt = __ldg(row + k + G);
     const double4_32a pj = ld_f64x4(pos64 + t);
-    const double x = min_image_bits(pj.x - pi.x, mi.half[0], mi.L[0]);
-    const double y = min_image_bits(pj.y - pi.y, mi.half[1], mi.L[1]);
-    const double z = min_image_bits(pj.z - pi.z, mi.half[2], mi.L[2]);
+    double x = pj.x - pi.x, y = pj.y - pi.y, z = pj.z - pi.z;
+    min_image3(mi, x, y, z);
     double A, B;
     tensor64(T, fma(z, z, fma(y, y, x * x)), eps2, K.coeff_2, A, B);
 #pragma unroll
@@ -273,11 +286,13 @@ __device__ __forceinline__ int64_t block_target_by_length(int64_t n, const int32
 // to NR right-hand sides.  G lanes per target take every G-th entry of its
 // row and add their sums by shuffles.
 //
-// Bound by the FP64 pipe (two lanes per SM and clock): 30 FP64 instructions
-// per pair and right-hand side pass (6 displacement, 3 r^2, 11 tensor, 10
-// product), which is 0.32 ms at N = 200k, phi = 0.1 (6.74 M pairs).
-// Measured there: 0.45 ms with a block's targets in order of row length (0.50
-// ms in slot order: lanes idle at the ends of uneven rows), against 2.85 ms with erf and exp per pair and 15.0 ms for
+// Bound by the FP64 pipe (two lanes per SM and clock): 27 FP64 instructions
+// per pair and right-hand side pass (3 displacement, 3 r^2, 11 tensor, 10
+// product; 3 more where a warp's pairs cross a box face), which is 0.29 ms at
+// N = 200k, phi = 0.1 (6.74 M pairs).
+// Measured there: 0.42 ms; 0.45 ms with the box-face additions for every
+// pair, 0.50 ms also with the targets in slot order (lanes idle at the ends
+// of uneven rows), 2.85 ms also with erf and exp per pair, and 15.0 ms for
 // the cell sweep.  The tensors themselves are closer to the exact ones than
 // the formula's: 1.2e-16 of u from their rounding against 3.8e-16 (N = 400,
 // 30-digit reference), since the closed form cancels.
@@ -436,9 +451,8 @@ __global__ void __launch_bounds__(kSeriesThreads, CACHE ? 3 : 7) k_series_f64(Se
   // the tensor of entry en seen from position pi
   auto tensor = [&](uint32_t en, const double4_32a &pi, double g[6]) {
     const double4_32a pj = ld_f64x4(a.pos64 + (en >> kCodeBits));
-    const double x = min_image_bits(pj.x - pi.x, a.mi.half[0], a.mi.L[0]);
-    const double y = min_image_bits(pj.y - pi.y, a.mi.half[1], a.mi.L[1]);
-    const double z = min_image_bits(pj.z - pi.z, a.mi.half[2], a.mi.L[2]);
+    double x = pj.x - pi.x, y = pj.y - pi.y, z = pj.z - pi.z;
+    min_image3(a.mi, x, y, z);
     double A, B;
     tensor64(a.T, fma(z, z, fma(y, y, x * x)), a.eps2, a.K.coeff_2, A, B);
     const double bx = B * x, by = B * y;
