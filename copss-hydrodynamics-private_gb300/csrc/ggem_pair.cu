@@ -1538,9 +1538,19 @@ __global__ void __launch_bounds__(256) k_pair_nr(
 // the CTA transposes the float-float results through shared memory so that
 // the FP64 velocities [r][slot][3] (self term added in FP64) are written
 // coalesced.
+//
+// Bound by the L1 data path (78% of its wavefronts), then by latency.  A
+// broadcast of an entry's data takes 128 B per clock like any other load: as
+// (x, x) pairs ready for the packed arithmetic an entry took 11 cycles of it,
+// as single values 6, the pairs being made in registers (14-term step of N =
+// 100k chains, 64 right-hand sides: 5.37 -> 4.97 ms).  The first three
+// sources' forces are requested before the tensors are formed (4.93 ms), and
+// a CTA holds four targets (4.70 ms; 2: 5.64, 5: 4.92, 8: 4.93, 16: 5.24):
+// fewer wait for the longest row of theirs, and a write-out run is still 96
+// bytes.  24 warps per SM instead of 32: 5.5 ms; 40, with spills: 6.9 ms.
 constexpr int kBatchR = 64;      // right-hand sides per pass
 constexpr int kBatchMinRhs = 16; // fewer go through k_pair_nr in chunks of 8
-constexpr int kBatchWarps = 8;   // target slots per CTA
+constexpr int kBatchWarps = 4;   // target slots per CTA
 
 __global__ void __launch_bounds__(256) k_stage_b64(int64_t n, int nr, const double *__restrict__ f,
                                                    float *__restrict__ fb) {
@@ -1623,25 +1633,24 @@ __global__ void __launch_bounds__(256) k_cheb_start_b64(int64_t n, int nr, doubl
   }
 }
 
-// forces of row entry q (clamped to the last one) for the two right-hand
-// sides of this lane: fw = fb + lane, jw = the warp's source slots
-__device__ __forceinline__ void b64_fetch(const float2 *__restrict__ fw, const uint32_t *jw, int q,
-                                          int np, float2 &x, float2 &y, float2 &z) {
-  const float2 *fp = fw + (int64_t)jw[min(q, np - 1)] * (3 * 32);
+// forces of source slot j for the two right-hand sides of this lane
+// (fw = fb + lane)
+__device__ __forceinline__ void b64_fetch(const float2 *__restrict__ fw, uint32_t j, float2 &x,
+                                          float2 &y, float2 &z) {
+  const float2 *fp = fw + (int64_t)j * (3 * 32);
   x = __ldg(fp);
   y = __ldg(fp + 32);
   z = __ldg(fp + 64);
 }
 
 // blk += A f + B (x.f) x for both right-hand sides of the lane (packed)
-__device__ __forceinline__ void b64_accumulate(const float4 &g0, const float4 &g1,
-                                               const float2 &g2, const float2 &fx,
+__device__ __forceinline__ void b64_accumulate(const float4 &g, float B, const float2 &fx,
                                                const float2 &fy, const float2 &fz, float2 &b0,
                                                float2 &b1, float2 &b2) {
-  const float2 dx2 = make_float2(g0.x, g0.y), dy2 = make_float2(g0.z, g0.w);
-  const float2 dz2 = make_float2(g1.x, g1.y), A2 = make_float2(g1.z, g1.w);
+  const float2 dx2 = make_float2(g.x, g.x), dy2 = make_float2(g.y, g.y);
+  const float2 dz2 = make_float2(g.z, g.z), A2 = make_float2(g.w, g.w);
   float2 d = __ffma2_rn(dz2, fz, __ffma2_rn(dy2, fy, __fmul2_rn(dx2, fx)));
-  d = __fmul2_rn(g2, d);
+  d = __fmul2_rn(make_float2(B, B), d);
   b0 = __ffma2_rn(d, dx2, __ffma2_rn(A2, fx, b0));
   b1 = __ffma2_rn(d, dy2, __ffma2_rn(A2, fy, b1));
   b2 = __ffma2_rn(d, dz2, __ffma2_rn(A2, fz, b2));
@@ -1670,19 +1679,20 @@ struct BatchCoef {
 // u is x_{k+1}: u = (2db x1 + 2da M x1) - x0, dw += c_r u, and fb_next
 // receives the FP32 staging of u for the next term.
 template <int CD, bool POLY, bool CHEB>
-__global__ void __launch_bounds__(32 * kBatchWarps, 4) k_pair_b64(
+__global__ void __launch_bounds__(32 * kBatchWarps, 8) k_pair_b64(
     int64_t n, int nr, const float4 *__restrict__ pos32, const float2 *__restrict__ fb,
     const int32_t *__restrict__ cnt, int W, const uint32_t *__restrict__ list, PolyAB P,
     const Rec32 *__restrict__ tab, float inv_ds, float hx, float hy, float hz, float self_hi,
     float self_lo, double *__restrict__ u, double two_da, double two_db, BatchCoef cf,
     const double *__restrict__ x0, const double *__restrict__ x1, double *__restrict__ dw,
     float *__restrict__ fb_next) {
-  // per entry, pre-duplicated for the packed arithmetic:
-  // g0 = (dx, dx, dy, dy), g1 = (dz, dz, A, A), g2 = (B, B), source slot
-  __shared__ float4 s_g0[kBatchWarps][32], s_g1[kBatchWarps][32];
-  __shared__ float2 s_g2[kBatchWarps][32];
+  // per entry: (dx, dy, dz, A), B, source slot
+  __shared__ float4 s_g[kBatchWarps][32];
+  __shared__ float s_b[kBatchWarps][32];
   __shared__ uint32_t s_j[kBatchWarps][32];
-  __shared__ float2 s_out[kBatchWarps][kBatchR][3];  // float-float results
+  // float-float results; the padding puts a right-hand side's consecutive
+  // (target, component) values in consecutive banks
+  __shared__ float2 s_out[kBatchWarps][kBatchR + 1][3];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t s = blockIdx.x * (int64_t)kBatchWarps + w;
   const bool act = s < n;
@@ -1711,9 +1721,17 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 4) k_pair_b64(
     int nb = 0;
     for (int m0 = 0; m0 < e; m0 += 32) {
       const int np = min(32, e - m0);
+      const uint32_t en = lane < np ? __ldg(list + b + m0 + lane) : 0u;
+      const uint32_t j = en >> kCodeBits;
+      // three force slots in flight: each is refilled with the entry three
+      // ahead right after its own entry is used (no register rotation); the
+      // first three are on their way while the tensors are formed
+      const float2 *fw = fb + lane;
+      float2 ax, ay, az, bx, by, bz, cx, cy, cz;
+      b64_fetch(fw, __shfl_sync(0xffffffffu, j, 0), ax, ay, az);
+      b64_fetch(fw, __shfl_sync(0xffffffffu, j, min(1, np - 1)), bx, by, bz);
+      b64_fetch(fw, __shfl_sync(0xffffffffu, j, min(2, np - 1)), cx, cy, cz);
       if (lane < np) {
-        const uint32_t en = __ldg(list + b + m0 + lane);
-        const uint32_t j = en >> kCodeBits;
         const float4 pj = __ldg(pos32 + j);
         float ox, oy, oz;
         decode_shift<CD>(en, hx, hy, hz, ox, oy, oz);
@@ -1721,32 +1739,24 @@ __global__ void __launch_bounds__(32 * kBatchWarps, 4) k_pair_b64(
         const float s2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
         float A, B;
         tensor_ab32<POLY>(s2, P, tab, inv_ds, A, B);
-        s_g0[w][lane] = make_float4(dx, dx, dy, dy);
-        s_g1[w][lane] = make_float4(dz, dz, A, A);
-        s_g2[w][lane] = make_float2(B, B);
+        s_g[w][lane] = make_float4(dx, dy, dz, A);
+        s_b[w][lane] = B;
         s_j[w][lane] = j;
       }
       __syncwarp();
-      // three force slots in flight: each is refilled with the entry three
-      // ahead right after its own entry is used (no register rotation)
-      const float2 *fw = fb + lane;
       const uint32_t *jw = s_j[w];
-      float2 ax, ay, az, bx, by, bz, cx, cy, cz;
-      b64_fetch(fw, jw, 0, np, ax, ay, az);
-      b64_fetch(fw, jw, 1, np, bx, by, bz);
-      b64_fetch(fw, jw, 2, np, cx, cy, cz);
       for (int p = 0; p < np; p += 3) {
-        b64_accumulate(s_g0[w][p], s_g1[w][p], s_g2[w][p], ax, ay, az, blk0, blk1, blk2);
-        b64_fetch(fw, jw, p + 3, np, ax, ay, az);
+        b64_accumulate(s_g[w][p], s_b[w][p], ax, ay, az, blk0, blk1, blk2);
+        b64_fetch(fw, jw[min(p + 3, np - 1)], ax, ay, az);
         if (p + 1 < np) {
-          b64_accumulate(s_g0[w][p + 1], s_g1[w][p + 1], s_g2[w][p + 1], bx, by, bz, blk0, blk1,
+          b64_accumulate(s_g[w][p + 1], s_b[w][p + 1], bx, by, bz, blk0, blk1,
                          blk2);
-          b64_fetch(fw, jw, p + 4, np, bx, by, bz);
+          b64_fetch(fw, jw[min(p + 4, np - 1)], bx, by, bz);
         }
         if (p + 2 < np) {
-          b64_accumulate(s_g0[w][p + 2], s_g1[w][p + 2], s_g2[w][p + 2], cx, cy, cz, blk0, blk1,
+          b64_accumulate(s_g[w][p + 2], s_b[w][p + 2], cx, cy, cz, blk0, blk1,
                          blk2);
-          b64_fetch(fw, jw, p + 5, np, cx, cy, cz);
+          b64_fetch(fw, jw[min(p + 5, np - 1)], cx, cy, cz);
         }
         if (++nb == 3) {  // every 9 entries into the compensated sums
           b64_flush(sum, cmp, blk0, blk1, blk2);
