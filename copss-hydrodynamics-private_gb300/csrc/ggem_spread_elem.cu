@@ -54,10 +54,12 @@ constexpr int kSpMaxSeg = 2048;  // contiguous slot ranges of one dilated brick
 constexpr int kSpMaxExt = 32;    // dilated brick extent per axis (5-bit coordinates)
 constexpr size_t kSpRecBytes = 16384;
 constexpr int kSpMaxWords = 1024;  // stencil bitmap words (32768 element offsets)
-constexpr int kSpQueue = 64;      // queued members per warp (< 32 left + 32 new)
+constexpr int kSpQueue = 96;      // queued members per warp (< 32 left + 64 new)
+constexpr int kSpBatch = 6 * 32;  // floats of a staged batch of 32 members (FP32)
 constexpr int kSpReachWords = 1024;  // union bitmap of a brick's elements
 constexpr size_t kSpShared =
-    kSpRecBytes + kSpWarps * (32 * sizeof(float4) + kSpQueue * sizeof(uint32_t)) +
+    kSpRecBytes + kSpCap32 * sizeof(uint32_t) +
+    kSpWarps * (kSpBatch * sizeof(float) + kSpQueue * sizeof(uint32_t)) +
     2 * (kSpMaxSeg + 1) * sizeof(int32_t) + (kSpMaxWords + kSpReachWords) * sizeof(uint32_t);
 
 struct SpreadGeo {
@@ -136,7 +138,16 @@ __device__ __forceinline__ int axis_offset(const SpreadGeo &sg, int d, int us, i
 }
 
 // ANYFULL: some brick frame spans a whole periodic axis (small meshes);
-// without it the wrapped-offset and minimum-image code is compiled out
+// without it the wrapped-offset and minimum-image code is compiled out.
+//
+// The FP32 form is bound by instruction issue (81%) and shared-memory data
+// (66% of its cycles): 144^3 elements x 8 points, N = 200k took 4.09 G warp
+// instructions and 3.90 ms, now 3.68 G and 3.72 ms.  Two members of a lane
+// share packed arithmetic up to the block sums, their positions and forces
+// staged together (6 words a member instead of a position and a gathered
+// record, 8); a point's four lanes reduce-scatter, so each converts and
+// writes one component; the lanes decode 32 elements at once; two windows of
+// candidates per pass.
 template <bool F32, bool ANYFULL, bool PAD>
 __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
     SpreadGeo sg, DevConsts K, const int32_t *__restrict__ start,
@@ -151,8 +162,11 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   // than 32-byte records would
   float4 *rec32 = reinterpret_cast<float4 *>(sp_smem);        // [2][CAP]
   double4_32a *rec64 = reinterpret_cast<double4_32a *>(sp_smem);  // [CAP][2]
-  float4 *batch = reinterpret_cast<float4 *>(sp_smem + kSpRecBytes);       // [warps][32]
-  uint32_t *queue = reinterpret_cast<uint32_t *>(batch + kSpWarps * 32);  // [warps][kSpQueue]
+  float *batch = reinterpret_cast<float *>(sp_smem + kSpRecBytes);  // [warps][kSpBatch]
+  // FP32: the staged particles' frame coordinates once more, for the
+  // membership pass (a 16-byte stride would take four times the banks)
+  uint32_t *rec_u = reinterpret_cast<uint32_t *>(batch + kSpWarps * kSpBatch);  // [CAP]
+  uint32_t *queue = rec_u + kSpCap32;                                // [warps][kSpQueue]
   int32_t *seg_begin = reinterpret_cast<int32_t *>(queue + kSpWarps * kSpQueue);
   int32_t *seg_pre = seg_begin + kSpMaxSeg + 1;
   uint32_t *s_bits = reinterpret_cast<uint32_t *>(seg_pre + kSpMaxSeg + 1);
@@ -251,7 +265,7 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   // position plus the offset's shift, formed once per member instead of
   // once per point, one member per lane) with the staged index in .w
   uint32_t *mq = queue + warp * kSpQueue;
-  float4 *mb = batch + warp * 32;
+  float *mb = batch + warp * kSpBatch;
   const unsigned lt_mask = (1u << lane) - 1u;
   // with the padded bitmap, a particle at frame coordinates u is listed by
   // some element of the brick when the union bitmap holds u (shifted where
@@ -315,7 +329,8 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
       if (keep) {
         const double *fp = f_slot + 3 * (int64_t)slot;
         if (F32) {
-          rec32[at] = make_float4(p.x, p.y, p.z, __uint_as_float(u));
+          rec32[at] = make_float4(p.x, p.y, p.z, 0.f);
+          rec_u[at] = u;
           rec32[kSpCap32 + at] =
               make_float4(d2f_bits(fp[0]), d2f_bits(fp[1]), d2f_bits(fp[2]), 0.f);
         } else {
@@ -327,18 +342,29 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
     }
     if (!(F32 && PAD)) cn = cw;
     __syncthreads();
-    for (int le = warp; le < nel; le += kSpWarps) {
-      const int lx = le % ebx, ly = (le / ebx) % eby, lz = le / (ebx * eby);
-      const int ex = e0[0] + lx, ey = e0[1] + ly, ez = e0[2] + lz;
-      const int64_t e = ex + (int64_t)sg.g.nc[0] * (ey + (int64_t)sg.g.nc[1] * ez);
-      const int uex = fr[0].full ? ex : ex - fr[0].F;
-      const int uey = fr[1].full ? ey : ey - fr[1].F;
-      const int uez = fr[2].full ? ez : ez - fr[2].F;
-      // with the padded bitmap, the packed frame coordinates u of a staged
-      // particle minus qe index the bitmap directly (each 5-bit field stays
-      // in [0, 32) for every particle of the brick's frame)
-      const int qe = (uex + sg.lo[0] - B + 1) + 32 * (uey + sg.lo[1] - B + 1) +
-                     1024 * (uez + sg.lo[2] - B + 1);
+    // each lane decodes one of the warp's next 32 elements
+    int64_t my_e = 0;
+    int my_u = 0, my_q = 0;
+    for (int it = 0; warp + kSpWarps * it < nel; ++it) {
+      if ((it & 31) == 0) {
+        const int le = min(warp + kSpWarps * (it + lane), nel - 1);
+        const int lx = le % ebx, ly = (le / ebx) % eby, lz = le / (ebx * eby);
+        const int ex = e0[0] + lx, ey = e0[1] + ly, ez = e0[2] + lz;
+        my_e = ex + (int64_t)sg.g.nc[0] * (ey + (int64_t)sg.g.nc[1] * ez);
+        const int ux = fr[0].full ? ex : ex - fr[0].F;
+        const int uy = fr[1].full ? ey : ey - fr[1].F;
+        const int uz = fr[2].full ? ez : ez - fr[2].F;
+        my_u = ux | (uy << 10) | (uz << 20);
+        // with the padded bitmap, the packed frame coordinates u of a staged
+        // particle minus qe index the bitmap directly (each 5-bit field stays
+        // in [0, 32) for every particle of the brick's frame)
+        my_q = (ux + sg.lo[0] - B + 1) + 32 * (uy + sg.lo[1] - B + 1) +
+               1024 * (uz + sg.lo[2] - B + 1);
+      }
+      const int64_t e = __shfl_sync(0xffffffffu, my_e, it & 31);
+      const int ue = __shfl_sync(0xffffffffu, my_u, it & 31);
+      const int uex = ue & 1023, uey = (ue >> 10) & 1023, uez = ue >> 20;
+      const int qe = __shfl_sync(0xffffffffu, my_q, it & 31);
       const bool qok = qi < nq;
       const int64_t qg = e * nq + (qok ? qi : 0);
       float4 qr = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -352,53 +378,67 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
       }
       float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
       float bx_ = 0.f, by_ = 0.f, bz_ = 0.f;
-      int blk = 0;
+      int blk = 0, elem_pairs = 0;
+      // minimum image (pm_periodic_boundary.C:350-374); only an axis whose
+      // frame is the whole box can produce |d| > L/2
+      auto axis32 = [&](int k, float d) {
+        if (ANYFULL && fr[k].full) {
+          if (d <= -0.5f * sg.L32[k]) d += sg.L32[k];
+          if (d > 0.5f * sg.L32[k]) d -= sg.L32[k];
+        }
+        return d;
+      };
       double ax = 0.0, ay = 0.0, az = 0.0;
       // members: staged particles whose element offset is a stencil offset,
       // queued in staging order and summed 32 at a time; lane (qi, sub)
       // takes members sub, sub + lq, ... of each batch, so every lane sees its
       // members in the order of one pass over the whole member list
       int queued = 0;  // warp-uniform
-      for (int k0 = 0; k0 < cn; k0 += 32) {
-        const int k = k0 + lane;
-        bool in = false;
-        uint32_t item = 0;
-        if (k < cn) {
-          const uint32_t u = F32 ? __float_as_uint(rec32[k].w)
-                                 : (uint32_t)__double_as_longlong(rec64[2 * k].w);
-          if (PAD) {
-            const int idx = (int)u - qe;
-            in = (s_bits[idx >> 5] >> (idx & 31)) & 1u;
-            item = (uint32_t)k | ((uint32_t)idx << 10);
-          } else {
-            const int ix =
-                axis_offset(sg, 0, (int)(u & 31u), uex, ANYFULL && fr[0].full) - sg.lo[0];
-            const int iy =
-                axis_offset(sg, 1, (int)((u >> 5) & 31u), uey, ANYFULL && fr[1].full) - sg.lo[1];
-            const int iz =
-                axis_offset(sg, 2, (int)(u >> 10), uez, ANYFULL && fr[2].full) - sg.lo[2];
-            if ((unsigned)ix < (unsigned)sg.dim[0] && (unsigned)iy < (unsigned)sg.dim[1] &&
-                (unsigned)iz < (unsigned)sg.dim[2]) {
-              const int idx = (iz * sg.dim[1] + iy) * sg.dim[0] + ix;
+      for (int k0 = 0; k0 < cn; k0 += 64) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int k = k0 + 32 * h + lane;
+          bool in = false;
+          uint32_t item = 0;
+          if (k < cn) {
+            const uint32_t u = F32 ? rec_u[k] : (uint32_t)__double_as_longlong(rec64[2 * k].w);
+            if (PAD) {
+              const int idx = (int)u - qe;
               in = (s_bits[idx >> 5] >> (idx & 31)) & 1u;
-              item = (uint32_t)k | ((uint32_t)ix << 10) | ((uint32_t)iy << 15) |
-                     ((uint32_t)iz << 20);
+              item = (uint32_t)k | ((uint32_t)idx << 10);
+            } else {
+              const int ix =
+                  axis_offset(sg, 0, (int)(u & 31u), uex, ANYFULL && fr[0].full) - sg.lo[0];
+              const int iy =
+                  axis_offset(sg, 1, (int)((u >> 5) & 31u), uey, ANYFULL && fr[1].full) - sg.lo[1];
+              const int iz =
+                  axis_offset(sg, 2, (int)(u >> 10), uez, ANYFULL && fr[2].full) - sg.lo[2];
+              if ((unsigned)ix < (unsigned)sg.dim[0] && (unsigned)iy < (unsigned)sg.dim[1] &&
+                  (unsigned)iz < (unsigned)sg.dim[2]) {
+                const int idx = (iz * sg.dim[1] + iy) * sg.dim[0] + ix;
+                in = (s_bits[idx >> 5] >> (idx & 31)) & 1u;
+                item = (uint32_t)k | ((uint32_t)ix << 10) | ((uint32_t)iy << 15) |
+                       ((uint32_t)iz << 20);
+              }
             }
           }
+          const unsigned bal = __ballot_sync(0xffffffffu, in);
+          if (in) mq[queued + __popc(bal & lt_mask)] = item;
+          queued += __popc(bal);
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, in);
-        if (in) mq[queued + __popc(bal & lt_mask)] = item;
-        queued += __popc(bal);
-        my_pairs += (unsigned long long)__popc(bal);
-        const bool last = k0 + 32 >= cn;
-        while (queued >= 32 || (last && queued > 0)) {
+        const bool last = k0 + 64 >= cn;
+        int head = 0;  // warp-uniform: members of the queue that are done
+        while (queued - head >= 32 || (last && queued > head)) {
           __syncwarp();
-          const int m = min(queued, 32);
-          if (F32 && lane < m) {
-            const uint32_t en = mq[lane];
-            const int kk = (int)(en & 1023u);
-            float4 v = make_float4(0.f, 0.f, 0.f, __uint_as_float((uint32_t)kk));
-            if (F32) {
+          const int m = min(queued - head, 32);
+          if (F32) {
+            // member j in pair slot (j / 8, j % 4), half (j / 4) % 2: the two
+            // members that a lane takes one after the other at four lanes per
+            // point; past the last member zeros, whose terms are exact zeros
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f), fv = v;
+            if (lane < m) {
+              const uint32_t en = mq[head + lane];
+              const int kk = (int)(en & 1023u);
               int ix, iy, iz;
               if (PAD) {
                 const int idx = (int)(en >> 10);
@@ -410,43 +450,62 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
                 iy = (int)((en >> 15) & 31u);
                 iz = (int)(en >> 20);
               }
-              const float4 a = rec32[kk];
-              v.x = a.x + s_shift[0][ix];
-              v.y = a.y + s_shift[1][iy];
-              v.z = a.z + s_shift[2][iz];
+              v = rec32[kk];
+              fv = rec32[kSpCap32 + kk];
+              v.x += s_shift[0][ix];
+              v.y += s_shift[1][iy];
+              v.z += s_shift[2][iz];
             }
-            mb[lane] = v;
+            float *o = mb + 12 * ((lane >> 3) * 4 + (lane & 3)) + ((lane >> 2) & 1);
+            o[0] = v.x;
+            o[2] = v.y;
+            o[4] = v.z;
+            o[6] = fv.x;
+            o[8] = fv.y;
+            o[10] = fv.z;
           }
           __syncwarp();
           // one (point, member) term of the FP32 sum into the block sums
-          auto term32 = [&](const float4 &mp) {
-            const float4 fb = rec32[kSpCap32 + (int)__float_as_uint(mp.w)];
-            float dx = mp.x - qr.x;
-            float dy = mp.y - qr.y;
-            float dz = mp.z - qr.z;
-            // minimum image (pm_periodic_boundary.C:350-374); only an axis
-            // whose frame is the whole box can produce |d| > L/2
-            if (ANYFULL && fr[0].full) {
-              if (dx <= -0.5f * sg.L32[0]) dx += sg.L32[0];
-              if (dx > 0.5f * sg.L32[0]) dx -= sg.L32[0];
-            }
-            if (ANYFULL && fr[1].full) {
-              if (dy <= -0.5f * sg.L32[1]) dy += sg.L32[1];
-              if (dy > 0.5f * sg.L32[1]) dy -= sg.L32[1];
-            }
-            if (ANYFULL && fr[2].full) {
-              if (dz <= -0.5f * sg.L32[2]) dz += sg.L32[2];
-              if (dz > 0.5f * sg.L32[2]) dz -= sg.L32[2];
-            }
+          auto term32 = [&](int j) {
+            const float *o = mb + 12 * ((j >> 3) * 4 + (j & 3)) + ((j >> 2) & 1);
+            const float dx = axis32(0, o[0] - qr.x);
+            const float dy = axis32(1, o[2] - qr.y);
+            const float dz = axis32(2, o[4] - qr.z);
             const float s2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
             const float p = s2 * sg.e_hi;
             const float r = fmaf(s2, sg.e_lo, fmaf(s2, sg.e_hi, -p));
             const float E0 = ex2_approx(p);
             const float E = fmaf(E0, r * 0.6931471805599453f, E0);
             const float gv = E * fmaf(-sg.c1, s2, sg.c25);
-            bx_ = fmaf(gv, fb.x, bx_);
-            by_ = fmaf(gv, fb.y, by_);
-            bz_ = fmaf(gv, fb.z, bz_);
+            bx_ = fmaf(gv, o[6], bx_);
+            by_ = fmaf(gv, o[8], by_);
+            bz_ = fmaf(gv, o[10], bz_);
+          };
+          // two members of a pair slot, one after the other into the block
+          // sums; what precedes the sums in packed arithmetic (each half
+          // rounds as the scalar form does)
+          auto pair32 = [&](const float4 *o) {
+            const float4 a = o[0], b = o[1], c = o[2];
+            float2 dx = __fadd2_rn(make_float2(a.x, a.y), make_float2(-qr.x, -qr.x));
+            float2 dy = __fadd2_rn(make_float2(a.z, a.w), make_float2(-qr.y, -qr.y));
+            float2 dz = __fadd2_rn(make_float2(b.x, b.y), make_float2(-qr.z, -qr.z));
+            if (ANYFULL) {
+              dx = make_float2(axis32(0, dx.x), axis32(0, dx.y));
+              dy = make_float2(axis32(1, dy.x), axis32(1, dy.y));
+              dz = make_float2(axis32(2, dz.x), axis32(2, dz.y));
+            }
+            const float2 s2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+            const float2 pn = __fmul2_rn(s2, make_float2(-sg.e_hi, -sg.e_hi));
+            const float2 r = __ffma2_rn(s2, make_float2(sg.e_lo, sg.e_lo),
+                                        __ffma2_rn(s2, make_float2(sg.e_hi, sg.e_hi), pn));
+            const float2 E0 = make_float2(ex2_approx(-pn.x), ex2_approx(-pn.y));
+            const float2 E = __ffma2_rn(
+                E0, __fmul2_rn(r, make_float2(0.6931471805599453f, 0.6931471805599453f)), E0);
+            const float2 gv = __fmul2_rn(E, __ffma2_rn(make_float2(-sg.c1, -sg.c1), s2,
+                                                       make_float2(sg.c25, sg.c25)));
+            bx_ = fmaf(gv.y, b.w, fmaf(gv.x, b.z, bx_));
+            by_ = fmaf(gv.y, c.y, fmaf(gv.x, c.x, by_));
+            bz_ = fmaf(gv.y, c.w, fmaf(gv.x, c.z, bz_));
           };
           auto flush32 = [&]() {  // the block sums into the compensated sums
             kahan_acc(sx, cx, bx_);
@@ -455,20 +514,26 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
             bx_ = by_ = bz_ = 0.f;
             blk = 0;
           };
-          if (F32 && lq == 4 && m == 32 && qok) {
-            // a full batch with four lanes per point: eight members per
-            // lane, which is one block of the compensated sums (blk is 0
-            // here: every earlier batch was full)
+          if (F32 && lq == 4) {
+            // four lanes per point: up to eight members per lane, which is one
+            // block of the compensated sums (blk is 0 here: every earlier
+            // batch was full)
+            const float4 *o = reinterpret_cast<const float4 *>(mb) + 3 * sub;
+            if (m == 32) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) term32(mb[sub + 4 * t]);
-            flush32();
+              for (int t = 0; t < 4; ++t) pair32(o + 12 * t);
+              flush32();
+            } else {
+              for (int t = 0; 8 * t < m; ++t) pair32(o + 12 * t);
+              if (m > 28 + sub) flush32();  // the lane had eight
+            }
           } else {
             for (int j = sub; j < m && qok; j += lq) {
               if (F32) {
-                term32(mb[j]);
+                term32(j);
                 if (++blk == 8) flush32();  // every 8 pairs into the compensated sums
               } else {
-                const int kk = (int)(mq[j] & 1023u);
+                const int kk = (int)(mq[head + j] & 1023u);
                 const double4_32a a = rec64[2 * kk], fb = rec64[2 * kk + 1];
                 // point_vector(q, x_j) with the minimum image (pm_periodic_boundary.C:350-374)
                 double x[3] = {a.x - q0, a.y - q1, a.z - q2};
@@ -490,14 +555,18 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
               }
             }
           }
-          // the rest of the queue to its front
-          const int rest = queued - m;
-          const uint32_t rv = lane < rest ? mq[32 + lane] : 0u;
+          head += m;
+        }
+        elem_pairs += head;
+        // the rest of the queue to its front
+        if (head) {
+          queued -= head;
+          const uint32_t rv = lane < queued ? mq[head + lane] : 0u;
           __syncwarp();
-          if (lane < rest) mq[lane] = rv;
-          queued = rest;
+          if (lane < queued) mq[lane] = rv;
         }
       }
+      my_pairs += (unsigned)elem_pairs;
       __syncwarp();
       double out[3];
       if (F32) {
@@ -505,6 +574,28 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
         kahan_acc(sy, cy, by_);
         kahan_acc(sz, cz, bz_);
         float h[3] = {sx, sy, sz}, l[3] = {-cx, -cy, -cz};
+        if (lq == 4) {
+          // reduce-scatter over the point's four lanes, (0 + 1) + (2 + 3):
+          // lane 0 ends with x, 1 and 3 with y, 2 with z
+          const bool odd = sub & 1, high = sub & 2;
+          float kh = odd ? h[1] : h[0], kl = odd ? l[1] : l[0];
+          ff_add(kh, kl, __shfl_xor_sync(0xffffffffu, odd ? h[0] : h[1], 1),
+                 __shfl_xor_sync(0xffffffffu, odd ? l[0] : l[1], 1));
+          ff_add(h[2], l[2], __shfl_xor_sync(0xffffffffu, h[2], 1),
+                 __shfl_xor_sync(0xffffffffu, l[2], 1));
+          const bool z = !odd && high;  // keeps z, sends x; lane 0 the other way, odd lanes y
+          float oh = z ? h[2] : kh, ol = z ? l[2] : kl;
+          ff_add(oh, ol, __shfl_xor_sync(0xffffffffu, odd || z ? kh : h[2], 2),
+                 __shfl_xor_sync(0xffffffffu, odd || z ? kl : l[2], 2));
+          if (qok && sub < 3) {
+            const double v = f2d_bits(oh) + f2d_bits(ol);
+            double *dst = rho + 3 * qg + sub;
+            // a brick staged in several passes adds each pass's sums
+            *dst = c0 == 0 ? v : *dst + v;
+          }
+          __syncwarp();  // the member list is rebuilt for the next element
+          continue;
+        }
         for (int o = 1; o < lq; o <<= 1) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) {

@@ -198,3 +198,25 @@ def test_spread_tensor_grid_matches_oracle(p, order, nm, periodic, jitter):
     # ~60 terms per point, each within a few ulp of e^{-alpha^2 r^2} at
     # alpha^2 r^2 <= 25: 25 * 2^-52 per term, well below 1e-13 of the norm
     assert rel(got, want) <= 1e-13
+
+
+@pytest.mark.parametrize("p", [(1, 1, 1), (3, 1, 1), (5, 1, 1), (2, 2, 2), (3, 3, 3)])
+@pytest.mark.parametrize("members", [1, 3, 4, 28, 29, 31, 32, 33, 63, 64, 65, 97])
+def test_fp32_spread_member_batches(p, members):
+    """members per element around the batches of 32, the four lanes of a
+    point and their blocks of eight, for one to 27 points per element, on
+    the padded bitmap: a cluster that every element in reach lists whole,
+    against the FP64 spread (1e-6 norm-wise, as above)"""
+    nm, h = 24, 1.4
+    L = nm * h
+    rng = np.random.default_rng(members)
+    xyz = 11.2 + rng.uniform(0.1, 1.3, (members, 3))
+    f = rng.standard_normal((members, 3))
+    q, nq = _grid_points((0, 0, 0), (L,) * 3, (nm,) * 3, p, (0, 1, 2))
+    with G.Context(alpha=ALPHA, box_hi=(L,) * 3, nb_mode=G.NB_REFERENCE, n_mesh=(nm,) * 3,
+                   search_radius_e=0.5 * h + 8.0 + 1e-3, precision=G.FP64) as ctx:
+        ctx.set_particles(xyz)
+        ctx.build_cells()
+        ctx.set_quadrature(q, nq)
+        want, got = ctx.spread_elements(f, G.FP64), ctx.spread_elements(f, G.FP32)
+    assert rel(got, want) <= 1e-6
