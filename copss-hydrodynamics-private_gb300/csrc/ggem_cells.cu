@@ -178,37 +178,63 @@ int scan_impl(ggem_ctx *c, const T *in, T *out, int64_t n, int level) {
   return check_launch(c, "scan total");
 }
 
-// the cell list's exclusive scan in one block when the grid is small
-// enough: tiles of 4096 counts (four consecutive counts per thread), all
-// loaded before the first tile is scanned, then one block-wide scan of the
-// threads' sums per tile with a running carry; start[0..ncell].  The counts
-// are zeroed as they are read, ready for the next build's k_assign, and so
-// are the pair-list statistics (stat, when given) that the list build of
-// the same configuration accumulates.
-constexpr int kScanTiles = 8;
-constexpr int64_t kScanCellsMax = 4096 * kScanTiles;
+// barrier of all threads of the cluster (shared memory written before it is
+// visible to the cluster after it)
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// the value of another block's copy of a shared variable
+__device__ __forceinline__ int32_t cluster_read(const int32_t *p, int rank) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t r;
+  int32_t v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(r) : "memory");
+  return v;
+}
+
+// the cell list's exclusive scan in one launch of one cluster of up to eight
+// blocks: each takes a consecutive run of tiles of 4096 counts (four
+// consecutive counts per thread, a running carry over its tiles), tells the
+// others its total through distributed shared memory and adds the totals of
+// the blocks before it; start[0..ncell].  The counts are zeroed as they are
+// read, ready for the next build's k_assign, and so are the pair-list
+// statistics (stat, when given) that the list build of the same
+// configuration accumulates.  Latency-bound: one block takes 15 us for 24389
+// counts, and the scan for any size four launches and two clears.  FP32
+// matvec with its list at N = 400k (48778 cells) 353 -> 335 us, FP32 step at
+// N = 200k 565 -> 557 us.  Beyond 131072 cells the blocks of one cluster
+// would be the bottleneck and device_exclusive_scan_i32 runs.
+constexpr int kScanTiles = 4;    // tiles per block
+constexpr int kScanCluster = 8;  // blocks
+constexpr int64_t kScanCellsMax = 4096 * kScanTiles * kScanCluster;
 
 __global__ void __launch_bounds__(1024) k_scan_cells(int32_t *__restrict__ count,
                                                      int32_t *__restrict__ start, int64_t n,
+                                                     int tiles,
                                                      unsigned long long *__restrict__ stat) {
   wait_prior_grid();
   __shared__ int32_t warp_tot[2][32];
-  if (stat && threadIdx.x < 2) stat[threadIdx.x] = 0ull;
+  __shared__ int32_t s_total, s_before;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int tiles = (int)((n + 4095) / 4096);
-  int32_t v[kScanTiles][4];
+  const int rank = blockIdx.x;  // (one cluster)
+  if (rank == 0 && stat && threadIdx.x < 2) stat[threadIdx.x] = 0ull;
+  const int64_t c0 = (int64_t)rank * tiles * 4096 + 4 * threadIdx.x;
+  int32_t v[kScanTiles][4], run[kScanTiles];
 #pragma unroll
   for (int k = 0; k < kScanTiles; ++k)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int64_t i = (int64_t)k * 4096 + 4 * threadIdx.x + j;
+      const int64_t i = c0 + k * 4096 + j;
       v[k][j] = (k < tiles && i < n) ? count[i] : 0;
     }
 #pragma unroll
   for (int k = 0; k < kScanTiles; ++k)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int64_t i = (int64_t)k * 4096 + 4 * threadIdx.x + j;
+      const int64_t i = c0 + k * 4096 + j;
       if (k < tiles && i < n) count[i] = 0;
     }
   int32_t carry = 0;
@@ -233,18 +259,35 @@ __global__ void __launch_bounds__(1024) k_scan_cells(int32_t *__restrict__ count
       }
       // every warp scans the 32 warp totals itself (no second barrier)
       const int32_t before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
-      const int32_t total = __shfl_sync(0xffffffffu, w, 31);
-      int32_t run = carry + (warp ? before : 0) + x - tsum;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int64_t i = (int64_t)k * 4096 + 4 * threadIdx.x + j;
-        if (i < n) start[i] = run;
-        run += v[k][j];
-      }
-      carry += total;
+      run[k] = carry + (warp ? before : 0) + x - tsum;
+      carry += __shfl_sync(0xffffffffu, w, 31);
     }
   }
-  if (threadIdx.x == 0) start[n] = carry;
+  int32_t base = 0;
+  if (gridDim.x > 1) {
+    if (threadIdx.x == 0) s_total = carry;
+    cluster_barrier();
+    if (warp == 0) {  // lane r reads block r's total
+      int32_t t = lane < rank ? cluster_read(&s_total, lane) : 0;
+      t = __reduce_add_sync(0xffffffffu, t);
+      if (lane == 0) s_before = t;
+    }
+    cluster_barrier();  // no block leaves while its total is read
+    base = s_before;
+  }
+#pragma unroll
+  for (int k = 0; k < kScanTiles; ++k) {
+    if (k < tiles) {
+      int32_t r = base + run[k];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t i = c0 + k * 4096 + j;
+        if (i < n) start[i] = r;
+        r += v[k][j];
+      }
+    }
+  }
+  if (rank == (int)gridDim.x - 1 && threadIdx.x == 0) start[n] = base + carry;
 }
 
 __global__ void k_scatter(int64_t n, const int32_t *__restrict__ cell_of,
@@ -892,9 +935,9 @@ int build_cells(ggem_ctx *c, bool defer_flags) {
     return cuda_fail(c, e, "cell buffers");
   cudaStream_t st = c->stream;
   // the cell counters are left at zero by the previous build (the
-  // single-block scan zeroes the counts, k_sort_cells the fills); they are
+  // one-launch scan zeroes the counts, k_sort_cells the fills); they are
   // cleared here only after a reallocation, an interrupted build or on
-  // grids too large for the single-block scan
+  // grids too large for the one-launch scan
   const bool small = g.ncell <= kScanCellsMax;
   const bool clean = small && c->cell_counters_zero && c->cell_count.p == c->cell_counters_at;
   c->cell_counters_zero = false;
@@ -912,8 +955,13 @@ int build_cells(ggem_ctx *c, bool defer_flags) {
   }
   c->list_stat_zero = false;
   if (small) {
-    launch_dependent(k_scan_cells, dim3(1), 1024, 0, st,
-                   c->cell_count.p, c->cell_start.p, g.ncell, c->nb_stat.p);
+    // blocks: a power of two with a tile each, then more tiles per block
+    const int nt = (int)((g.ncell + 4095) / 4096);
+    int blocks = 1;
+    while (blocks < nt && blocks < kScanCluster) blocks *= 2;
+    launch_dependent_cluster(k_scan_cells, dim3(blocks), 1024, 0, st, (unsigned)blocks,
+                             c->cell_count.p, c->cell_start.p, g.ncell,
+                             (nt + blocks - 1) / blocks, c->nb_stat.p);
     if (int rc = check_launch(c, "scan cells")) return rc;
     c->list_stat_zero = c->nb_stat.p != nullptr;
   } else if (int rc = device_exclusive_scan_i32(c, c->cell_count.p, c->cell_start.p, g.ncell)) {

@@ -317,20 +317,30 @@ __device__ __forceinline__ void wait_prior_grid() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// cluster > 1: in clusters of that many blocks
 template <typename... KArgs, typename... Args>
-void launch_dependent(void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem,
-                      cudaStream_t st, Args... args) {
+void launch_dependent_cluster(void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem,
+                              cudaStream_t st, unsigned cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+void launch_dependent(void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem,
+                      cudaStream_t st, Args... args) {
+  launch_dependent_cluster(kern, grid, block, smem, st, 1u, args...);
 }
 #endif
 

@@ -46,3 +46,25 @@ def test_rows_match_oracle(inner, outer, cell_div):
             # each unordered pair once: the same operator as with the full list (FP32 sums of
             # up to ~970 terms in blocks, 6e-8 each: 1e-5 norm-wise)
             assert np.linalg.norm(u - full) <= 1e-5 * np.linalg.norm(full)
+
+
+@pytest.mark.parametrize("nc", [(3, 3, 3), (16, 16, 16), (17, 16, 16), (24, 24, 24), (32, 32, 32),
+                                (33, 32, 32), (64, 64, 32), (65, 64, 32)])
+def test_cell_offsets_over_scan_blocks(nc):
+    """cell counts around the scan's tiles of 4096, its two to eight blocks
+    and its limit of 131072: lists equal to the oracle's, twice (the first
+    build leaves its counters for the second)"""
+    L = 7.0 * np.asarray(nc) + 1.0
+    rng = np.random.default_rng(int(np.prod(nc)))
+    box = O.make_box([0] * 3, list(L), [1, 1, 1])
+    with G.Context(box_hi=tuple(L), rc=7.0) as ctx:
+        for k in range(2):
+            n = (4000, 2500)[k]
+            # half of the beads in a slab, so that some rows have entries
+            xyz = rng.uniform(0.0, 1.0, (n, 3)) * L
+            xyz[::2, 2] = 0.6 * L[2] + 3.0 * xyz[::2, 2] / L[2]
+            nb = O.neighbors_cutoff(box, xyz, 7.0)
+            ctx.set_particles(xyz)
+            ctx.build_cells()
+            off, ids = ctx.neighbors()
+            assert np.array_equal(off, nb.offsets) and np.array_equal(ids, nb.ids)
