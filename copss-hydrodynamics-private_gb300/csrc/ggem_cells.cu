@@ -1,12 +1,11 @@
-// ggem_cells.cu -- Kernel A: the sorted cell list and the cached FP32 pair
-// list.
+// ggem_cells.cu -- Kernel A: the sorted cell list and the cached pair list.
 //
 // Replaces PointMesh::reinit (point_mesh.C:245-289): the element-point
 // containing list (:573-648) becomes a counting sort of particles by cell,
 // and the per-particle neighbour lists (:652-848) with their stored
-// displacement vectors (:220-241) become either an on-the-fly cell stencil
-// sweep (FP64 path) or fixed-width rows of (source slot, stencil code)
-// entries (FP32 path), built in one pass per configuration.
+// displacement vectors (:220-241) become fixed-width rows of (source slot,
+// stencil code) entries, built in one pass per configuration, in both
+// precisions (an FP64 context without a list sweeps the cell stencil).
 //
 // Bound: HBM.  Algorithmic bytes per particle of the cell build: 24 (read
 // xyz) + 4 (cell id) + 4 (order) + 4 (rank) + 32 (pos64) + 16 (pos32) plus

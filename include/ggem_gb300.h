@@ -62,7 +62,8 @@ extern "C" {
 #define GGEM_NB_CUTOFF 1    /* all pairs with |r| < rc                                        */
 
 /* arithmetic of the pair sum */
-#define GGEM_FP64 0 /* FP64 Green's tensors with erf/exp, plain cell-stencil sweep     */
+#define GGEM_FP64 0 /* FP64 Green's tensors as piecewise quintics of erf/exp forms,
+                       cached pair list or cell-stencil sweep                            */
 #define GGEM_FP32 1 /* FP32 cell-relative coordinates, tabulated tensor, compensated sums,
                        cached pair list                                                  */
 
