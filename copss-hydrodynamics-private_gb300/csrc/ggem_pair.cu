@@ -292,8 +292,8 @@ __device__ __forceinline__ int64_t block_target_by_length(int64_t n, const int32
 // N = 200k, phi = 0.1 (6.74 M pairs).
 // Measured there: 0.42 ms; 0.45 ms with the box-face additions for every
 // pair, 0.50 ms also with the targets in slot order (lanes idle at the ends
-// of uneven rows), 2.85 ms also with erf and exp per pair, and 15.0 ms for
-// the cell sweep.  The tensors themselves are closer to the exact ones than
+// of uneven rows), 2.85 ms also with erf and exp per pair; the cell
+// sweep takes 4.8 ms, 15.0 ms with erf and exp.  The tensors themselves are closer to the exact ones than
 // the formula's: 1.2e-16 of u from their rounding against 3.8e-16 (N = 400,
 // 30-digit reference), since the closed form cancels.
 template <int NR, int G>
