@@ -194,6 +194,8 @@ struct ggem_ctx {
   bool use_pretensor = false;   // B >= 0 holds for these constants
   bool allow_pretensor = true;  // ggem_set_pair_tensors
   bool pretensor_ok = false;
+  bool pretensor_pending = false;  // not formed yet (form_pair_tensors)
+  bool pretensor_eager = false;    // formed with the list (a product was captured)
   int stored_variant = 0;         // shape of the stored-tensor pair kernels (autotuned)
   int computed_variant = 0;       // loop shape of the per-matvec-tensor kernels (autotuned)
   ggem::DevBuf<float4> pair_ten;
@@ -453,6 +455,7 @@ int matvec_slots_prestaged(ggem_ctx *c, int nrhs, const double *d_f_slot, double
                            int self_mode);
 double self_coefficient(const ggem_ctx *c, int self_mode);
 int build_pair_tensors(ggem_ctx *c);
+int form_pair_tensors(ggem_ctx *c);
 int pair_cheb_term(ggem_ctx *c, bool records_fresh, const double *x0, const double *x1,
                    double *xm, double *dw, double two_da, double two_db, double coef,
                    int self_mode, double *norms = nullptr);

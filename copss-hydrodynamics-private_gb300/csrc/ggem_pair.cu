@@ -1208,8 +1208,7 @@ __global__ void k_to_slots_rec(int64_t n, const int32_t *__restrict__ order,
 
 // ---- precomputed pair tensors ---------------------------------------------
 //
-// Once per configuration (after the list build), every listed pair's tensor
-// is stored as t = (A, sqrt(B) x) in the list's row layout, valid when
+// Once per configuration, every listed pair's tensor is stored as t = (A, sqrt(B) x) in the list's row layout, valid when
 // B >= 0 on [0, rc^2] (checked at context creation).  A matvec then streams
 // 20 B per pair (entry + tensor, evict-first) and gathers a 16-byte force:
 // G f = A f + (x~ . f) x~ with x~ = sqrt(B) x, no position gathers and no
@@ -1389,6 +1388,74 @@ __global__ void __launch_bounds__(256) k_pair_r1tv(int64_t n, const float4 *__re
   const bool act = gid < n;
   const int64_t s = act ? gid : n - 1;
   const PairSum r = pair_sum_tv<G, U, PIPE>(s, act, sub, f4, cnt, W, list, ten);
+  group_store(act, sub, s, r.hx, r.lx, r.hy, r.ly, r.hz, r.lz, self_c, f, u);
+}
+
+// The first product over a new list: forms each pair's tensor (the
+// arithmetic of tensor_row), stores it for the products after it and applies
+// it (the lanes, order and sums of k_pair_r1tv with four lanes per target),
+// so that it is written once and not read back: a matvec with its list, N =
+// 400k, 337 -> 307 us (tensors 70 us and product 76 us as two kernels).  Two
+// entries in flight per lane (52 registers); four are slower (310 us).
+template <int CD, bool POLY, int U>
+__global__ void __launch_bounds__(256) k_pair_r1tv_first(
+    int64_t n, const float4 *__restrict__ pos32, const float4 *__restrict__ f4,
+    const int32_t *__restrict__ cnt, int W, const uint32_t *__restrict__ list, PolyAB P,
+    const Rec32 *__restrict__ tab, float inv_ds, float hx, float hy, float hz,
+    float4 *__restrict__ ten, double self_c, const double *__restrict__ f,
+    double *__restrict__ u) {
+  wait_prior_grid();
+  constexpr int FLUSH = 8 / U;  // iterations per Kahan flush
+  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
+  const int sub = (int)(threadIdx.x % kGroup);
+  const bool act = gid < n;
+  const int64_t s = act ? gid : n - 1;
+  const float4 pi = pos32[s];
+  const int64_t b = s * (int64_t)W, e = act ? b + cnt[s] : b;
+  float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+  float2 bxy = make_float2(0.f, 0.f);
+  float bz = 0.f;
+  int blk = 0;
+  for (int64_t m = b + sub; m < e; m += U * kGroup) {
+    uint32_t en[U];
+    float4 pj[U], fj[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) en[q] = m + q * kGroup < e ? __ldg(list + m + q * kGroup) : 0u;
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      pj[q] = __ldg(pos32 + (en[q] >> kCodeBits));
+      fj[q] = __ldg(f4 + (en[q] >> kCodeBits));
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      if (m + q * kGroup >= e) break;
+      float ox, oy, oz;
+      decode_shift<CD>(en[q], hx, hy, hz, ox, oy, oz);
+      const float dx = (pj[q].x - pi.x) + ox, dy = (pj[q].y - pi.y) + oy, dz = (pj[q].z - pi.z) + oz;
+      const float s2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      float A, B;
+      tensor_ab32<POLY>(s2, P, tab, inv_ds, A, B);
+      const float w = sqrtf(fmaxf(B, 0.f));
+      const float4 t = make_float4(A, w * dx, w * dy, w * dz);
+      __stcs(ten + m + q * kGroup, t);
+      tensor_apply(t, fj[q], bxy, bz);
+    }
+    if (++blk == FLUSH) {
+      kahan_add(sx, cx, bxy.x);
+      kahan_add(sy, cy, bxy.y);
+      kahan_add(sz, cz, bz);
+      bxy = make_float2(0.f, 0.f);
+      bz = 0.f;
+      blk = 0;
+    }
+  }
+  kahan_add(sx, cx, bxy.x);
+  kahan_add(sy, cy, bxy.y);
+  kahan_add(sz, cz, bz);
+  PairSum r{sx, -cx, sy, -cy, sz, -cz};
+  group_ff_g<kGroup>(r.hx, r.lx);
+  group_ff_g<kGroup>(r.hy, r.ly);
+  group_ff_g<kGroup>(r.hz, r.lz);
   group_store(act, sub, s, r.hx, r.lx, r.hy, r.ly, r.hz, r.lz, self_c, f, u);
 }
 
@@ -2008,6 +2075,18 @@ int launch_sym_r1(ggem_ctx *c, const Rec32 *src, const double *f, double *u, dou
   return check_launch(c, "pair f32 symmetric finish");
 }
 
+void launch_stored_first(ggem_ctx *c, const float4 *f4, double self_c, const double *f,
+                         double *u) {
+  const Grid &g = c->grid;
+  const bool cd2 = c->prm.cell_div == 2;
+  launch_dependent(
+      c->use_poly ? (cd2 ? k_pair_r1tv_first<2, true, 2> : k_pair_r1tv_first<1, true, 2>)
+                  : (cd2 ? k_pair_r1tv_first<2, false, 2> : k_pair_r1tv_first<1, false, 2>),
+      dim3((unsigned)((c->n * kGroup + 255) / 256)), 256, 0, c->stream, c->n, c->pos32.p, f4,
+      c->nb_cnt.p, c->nb_w, c->nb_list.p, poly_of(c), reinterpret_cast<const Rec32 *>(c->tab.p),
+      c->tab_inv_ds, g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p, self_c, f, u);
+}
+
 int launch_f32_r1(ggem_ctx *c, const double *f, double *u, double self_c) {
   const int64_t n = c->n;
   cudaError_t e;
@@ -2016,8 +2095,18 @@ int launch_f32_r1(ggem_ctx *c, const double *f, double *u, double self_c) {
     launch_dependent(k_stage_f4, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
                    n, f, c->w_f4[0].p);
     if (int rc = check_launch(c, "pair forces")) return rc;
+    const bool capturing = stream_capturing(c);
+    if (capturing) c->pretensor_eager = true;
+    if (kStoredVariants[c->stored_variant].G != kGroup)
+      if (int rc = form_pair_tensors(c)) return rc;
     kt_start(c, kKPairF32);
-    dispatch_stored_r1(c, c->w_f4[0].p, self_c, f, u);
+    if (c->pretensor_pending && kStoredVariants[c->stored_variant].G == kGroup) {
+      launch_stored_first(c, c->w_f4[0].p, self_c, f, u);
+      // (a captured product forms them whenever it is replayed)
+      c->pretensor_pending = capturing;
+    } else {
+      dispatch_stored_r1(c, c->w_f4[0].p, self_c, f, u);
+    }
     kt_stop(c, kKPairF32);
     return check_launch(c, "pair f32 r1 (tensors)");
   }
@@ -2180,6 +2269,7 @@ int pair_cheb_term(ggem_ctx *c, bool records_fresh, const double *x0, const doub
   cudaError_t e;
   const double self_c0 = self_coefficient(c, self_mode);
   if (c->pretensor_ok) {
+    if (int rc = form_pair_tensors(c)) return rc;
     if (norms) return fail(c, GGEM_ERR_BAD_ARG, "fused norms need per-matvec pair tensors");
     if ((e = c->w_f4[0].ensure((size_t)n)) || (e = c->w_f4[1].ensure((size_t)n)))
       return cuda_fail(c, e, "chebyshev forces");
@@ -2345,53 +2435,44 @@ int matvec_orig_fused(ggem_ctx *c, const double *f, double *u, double *f_slot, i
   return check_launch(c, "pair f32 r1");
 }
 
-// the per-pair tensors of the current list (k_pair_tensor)
+// The per-pair tensors of the current list: room for them now, the tensors
+// themselves with the first product that reads them (k_pair_r1tv_first), or
+// by form_pair_tensors where another kernel comes first.  A graph that a
+// caller captured may read the stored tensors when it is replayed, so from
+// the first captured product on they are formed with the list.
 int build_pair_tensors(ggem_ctx *c) {
-  c->pretensor_ok = false;
+  c->pretensor_ok = c->pretensor_pending = false;
   if (!c->use_pretensor || !c->allow_pretensor || !c->list_built) return GGEM_OK;
-  const int64_t n = c->n;
-  if (n == 0) {
-    c->pretensor_ok = true;
-    return GGEM_OK;
+  if (c->n > 0) {
+    cudaError_t e = c->pair_ten.ensure((size_t)c->n * c->nb_w);
+    if (e) {
+      // no room for the tensors: the pair kernels evaluate them on the fly
+      cudaGetLastError();
+      return GGEM_OK;
+    }
   }
-  cudaError_t e = c->pair_ten.ensure((size_t)n * c->nb_w);
-  if (e) {
-    // no room for the tensors: the pair kernels evaluate them on the fly
-    cudaGetLastError();
-    return GGEM_OK;
-  }
+  c->pretensor_ok = true;
+  c->pretensor_pending = c->n > 0;
+  return c->pretensor_eager ? form_pair_tensors(c) : GGEM_OK;
+}
+
+int form_pair_tensors(ggem_ctx *c) {
+  if (!c->pretensor_pending) return GGEM_OK;
   const Grid &g = c->grid;
-  const int64_t threads = n * kGroup;
-  const unsigned grid = (unsigned)((threads + 255) / 256);
+  const unsigned grid = (unsigned)((c->n * kGroup + 255) / 256);
   const bool cd2 = c->prm.cell_div == 2;
   const Rec32 *tab = reinterpret_cast<const Rec32 *>(c->tab.p);
   kt_start(c, kKListBuild);
-  if (c->use_poly) {
-    if (cd2)
-      launch_dependent(k_pair_tensor<2, true>, dim3(grid), 256, 0, c->stream,
-                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
-                                                          c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
-                                                          g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
-    else
-      launch_dependent(k_pair_tensor<1, true>, dim3(grid), 256, 0, c->stream,
-                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
-                                                          c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
-                                                          g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
-  } else {
-    if (cd2)
-      launch_dependent(k_pair_tensor<2, false>, dim3(grid), 256, 0, c->stream,
-                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
-                                                           c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
-                                                           g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
-    else
-      launch_dependent(k_pair_tensor<1, false>, dim3(grid), 256, 0, c->stream,
-                   n, c->pos32.p, c->nb_cnt.p, c->nb_w,
-                                                           c->nb_list.p, poly_of(c), tab, c->tab_inv_ds,
-                                                           g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p);
-  }
+  launch_dependent(c->use_poly ? (cd2 ? k_pair_tensor<2, true> : k_pair_tensor<1, true>)
+                               : (cd2 ? k_pair_tensor<2, false> : k_pair_tensor<1, false>),
+                   dim3(grid), 256, 0, c->stream, c->n, c->pos32.p, c->nb_cnt.p, c->nb_w,
+                   c->nb_list.p, poly_of(c), tab, c->tab_inv_ds, g.h32[0], g.h32[1], g.h32[2],
+                   c->pair_ten.p);
   kt_stop(c, kKListBuild);
   if (int rc = check_launch(c, "pair tensors")) return rc;
-  c->pretensor_ok = true;
+  const bool capturing = stream_capturing(c);
+  if (capturing) c->pretensor_eager = true;
+  c->pretensor_pending = capturing;
   return GGEM_OK;
 }
 
@@ -2655,6 +2736,7 @@ extern "C" int ggem_autotune_pair_storage(ggem_ctx *ctx, int reps, double matvec
     ctx->allow_pretensor = true;
     cudaEventRecord(a, ctx->stream);
     rc = build_pair_tensors(ctx);
+    if (!rc) rc = form_pair_tensors(ctx);
     cudaEventRecord(b, ctx->stream);
     cudaEventSynchronize(b);
     float t_pass = 0.f;

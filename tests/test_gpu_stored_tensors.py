@@ -1,0 +1,73 @@
+"""The first product over a new list forms and stores the pair tensors; the
+products after it read them.  The same arithmetic in the same order: equal
+bit for bit.  Graphs that a caller captured, before or after the first
+product, follow rebuilds."""
+import numpy as np
+import pytest
+
+import ggem_gb300 as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    from ggem_gb300 import build as B
+    B.build()
+
+
+@pytest.mark.parametrize("cell_div", [1, 2])
+@pytest.mark.parametrize("n,L", [(1, 28.0), (2, 28.0), (63, 28.0), (64, 28.0), (65, 28.0),
+                                 (300, 28.0), (900, 21.0), (5000, 60.0)])
+def test_first_product_equals_the_next(n, L, cell_div):
+    rng = np.random.default_rng(n)
+    xyz, f = rng.uniform(0.0, L, (n, 3)), rng.standard_normal((n, 3))
+    with G.Context(box_hi=(L,) * 3, rc=7.0, cell_div=cell_div) as ctx:
+        ctx.set_pair_tensors(True)
+        for _ in range(2):
+            ctx.set_particles(xyz)
+            ctx.build_cells()
+            first = ctx.local_matvec(f, G.SELF_BEAD)
+            assert np.array_equal(ctx.local_matvec(f, G.SELF_BEAD), first)
+            assert n < 2 or np.abs(first).max() > 0.0
+
+
+@pytest.mark.parametrize("captured_first", [True, False])
+def test_captured_product_follows_rebuilds(captured_first):
+    import torch
+    n, L = 800, 30.0
+    rng = np.random.default_rng(4)
+    configs = [rng.uniform(0.0, L, (n, 3)) for _ in range(3)]
+    f = torch.from_numpy(rng.standard_normal((n, 3))).cuda()
+    u = torch.zeros_like(f)
+    want = []
+    with G.Context(box_hi=(L,) * 3, rc=7.0) as ctx:
+        for xyz in configs:
+            ctx.set_particles(xyz)
+            ctx.build_cells()
+            want.append(ctx.local_matvec(f.cpu().numpy(), G.SELF_BEAD))
+    st = torch.cuda.Stream()
+    with G.Context(box_hi=(L,) * 3, rc=7.0) as ctx:
+        ctx.set_stream(st.cuda_stream)
+        torch.cuda.synchronize()
+        for k in (0, 0):  # buffers and row width settle
+            ctx.set_particles(configs[k])
+            ctx.build_cells()
+            ctx.local_matvec_dev(f.data_ptr(), u.data_ptr())
+        if captured_first:
+            ctx.build_cells()
+        ctx.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            ctx.local_matvec_dev(f.data_ptr(), u.data_ptr())
+        for xyz, w in zip(configs, want):
+            ctx.set_particles(xyz)
+            ctx.build_cells()
+            u.zero_()
+            torch.cuda.synchronize()
+            g.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(u.cpu().numpy(), w)
+            ctx.local_matvec_dev(f.data_ptr(), u.data_ptr())
+            ctx.synchronize()
+            assert np.array_equal(u.cpu().numpy(), w)
