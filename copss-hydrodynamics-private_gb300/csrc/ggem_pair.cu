@@ -768,16 +768,18 @@ __device__ __forceinline__ void group_ff(float &hi, float &lo) {
 }
 
 // lanes sub = 0, 1, 2 of a group write component sub of the target:
-// u = (hi + lo) + self_c f with the FP64 force of the target
+// u = (hi + lo) + self_c f with the FP64 force of the target (order: u in the
+// caller's particle order)
 __device__ __forceinline__ void group_store(bool act, int sub, int64_t s, float hx, float lx,
                                             float hy, float ly, float hz, float lz,
                                             double self_c, const double *__restrict__ f,
-                                            double *__restrict__ u) {
+                                            double *__restrict__ u,
+                                            const int32_t *__restrict__ order = nullptr) {
   if (!act || sub >= 3) return;
   const float h = sub == 0 ? hx : (sub == 1 ? hy : hz);
   const float l = sub == 0 ? lx : (sub == 1 ? ly : lz);
   const double v = f2d_bits(h) + f2d_bits(l);
-  u[3 * s + sub] = fma(self_c, f[3 * s + sub], v);
+  u[3 * (order ? (int64_t)order[s] : s) + sub] = fma(self_c, f[3 * s + sub], v);
 }
 
 __global__ void k_build_src(int64_t n, const float4 *__restrict__ pos32,
@@ -1268,6 +1270,21 @@ __global__ void __launch_bounds__(256) k_batch_tensor(
                        h[1], h[2], ten);
 }
 
+// xi (caller order) into slot order and one float4 per slot of it
+__global__ void k_to_slots_f4(int64_t n, const int32_t *__restrict__ order,
+                              const double *__restrict__ xi, double *__restrict__ x0,
+                              float4 *__restrict__ f4) {
+  wait_prior_grid();
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  const int64_t i = order[s];
+  const double a = xi[3 * i], b = xi[3 * i + 1], c = xi[3 * i + 2];
+  x0[3 * s] = a;
+  x0[3 * s + 1] = b;
+  x0[3 * s + 2] = c;
+  f4[s] = make_float4(d2f_bits(a), d2f_bits(b), d2f_bits(c), 0.f);
+}
+
 // forces of one right-hand side as one float4 per slot (w = 0)
 __global__ void k_stage_f4(int64_t n, const double *__restrict__ f, float4 *__restrict__ f4) {
   wait_prior_grid();
@@ -1381,14 +1398,14 @@ __global__ void __launch_bounds__(256) k_pair_r1tv(int64_t n, const float4 *__re
                                                    const uint32_t *__restrict__ list,
                                                    const float4 *__restrict__ ten, double self_c,
                                                    const double *__restrict__ f,
-                                                   double *__restrict__ u) {
+                                                   double *__restrict__ u, const int32_t *__restrict__ order) {
   wait_prior_grid();
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
   const int sub = (int)(threadIdx.x % G);
   const bool act = gid < n;
   const int64_t s = act ? gid : n - 1;
   const PairSum r = pair_sum_tv<G, U, PIPE>(s, act, sub, f4, cnt, W, list, ten);
-  group_store(act, sub, s, r.hx, r.lx, r.hy, r.ly, r.hz, r.lz, self_c, f, u);
+  group_store(act, sub, s, r.hx, r.lx, r.hy, r.ly, r.hz, r.lz, self_c, f, u, order);
 }
 
 // The first product over a new list: forms each pair's tensor (the
@@ -1403,7 +1420,7 @@ __global__ void __launch_bounds__(256) k_pair_r1tv_first(
     const int32_t *__restrict__ cnt, int W, const uint32_t *__restrict__ list, PolyAB P,
     const Rec32 *__restrict__ tab, float inv_ds, float hx, float hy, float hz,
     float4 *__restrict__ ten, double self_c, const double *__restrict__ f,
-    double *__restrict__ u) {
+    double *__restrict__ u, const int32_t *__restrict__ order) {
   wait_prior_grid();
   constexpr int FLUSH = 8 / U;  // iterations per Kahan flush
   const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kGroup;
@@ -1456,7 +1473,7 @@ __global__ void __launch_bounds__(256) k_pair_r1tv_first(
   group_ff_g<kGroup>(r.hx, r.lx);
   group_ff_g<kGroup>(r.hy, r.ly);
   group_ff_g<kGroup>(r.hz, r.lz);
-  group_store(act, sub, s, r.hx, r.lx, r.hy, r.ly, r.hz, r.lz, self_c, f, u);
+  group_store(act, sub, s, r.hx, r.lx, r.hy, r.ly, r.hz, r.lz, self_c, f, u, order);
 }
 
 // one Chebyshev term from stored tensors (cf. k_pair_cheb); f4 holds the
@@ -1502,12 +1519,13 @@ constexpr StoredVariant kStoredVariants[] = {{4, 4, false}, {4, 2, true}, {8, 2,
 constexpr int kNumStoredVariants = 4;
 
 template <int V>
-void launch_stored_r1(ggem_ctx *c, const float4 *f4, double self_c, const double *f, double *u) {
+void launch_stored_r1(ggem_ctx *c, const float4 *f4, double self_c, const double *f, double *u,
+                      const int32_t *order) {
   constexpr StoredVariant sv = kStoredVariants[V];
   const int64_t threads = c->n * sv.G;
   launch_dependent(k_pair_r1tv<sv.G, sv.U, sv.pipe>, dim3((unsigned)((threads + 255) / 256)), 256, 0,
                    c->stream, 
-      c->n, f4, c->nb_cnt.p, c->nb_w, c->nb_list.p, c->pair_ten.p, self_c, f, u);
+      c->n, f4, c->nb_cnt.p, c->nb_w, c->nb_list.p, c->pair_ten.p, self_c, f, u, order);
 }
 
 template <int V>
@@ -1522,12 +1540,13 @@ void launch_stored_cheb(ggem_ctx *c, const float4 *f4, double self_c, double two
       x0, x1, xm, dw, next);
 }
 
-void dispatch_stored_r1(ggem_ctx *c, const float4 *f4, double self_c, const double *f, double *u) {
+void dispatch_stored_r1(ggem_ctx *c, const float4 *f4, double self_c, const double *f, double *u,
+                        const int32_t *order) {
   switch (c->stored_variant) {
-    case 1: launch_stored_r1<1>(c, f4, self_c, f, u); break;
-    case 2: launch_stored_r1<2>(c, f4, self_c, f, u); break;
-    case 3: launch_stored_r1<3>(c, f4, self_c, f, u); break;
-    default: launch_stored_r1<0>(c, f4, self_c, f, u); break;
+    case 1: launch_stored_r1<1>(c, f4, self_c, f, u, order); break;
+    case 2: launch_stored_r1<2>(c, f4, self_c, f, u, order); break;
+    case 3: launch_stored_r1<3>(c, f4, self_c, f, u, order); break;
+    default: launch_stored_r1<0>(c, f4, self_c, f, u, order); break;
   }
 }
 
@@ -2076,7 +2095,7 @@ int launch_sym_r1(ggem_ctx *c, const Rec32 *src, const double *f, double *u, dou
 }
 
 void launch_stored_first(ggem_ctx *c, const float4 *f4, double self_c, const double *f,
-                         double *u) {
+                         double *u, const int32_t *order) {
   const Grid &g = c->grid;
   const bool cd2 = c->prm.cell_div == 2;
   launch_dependent(
@@ -2084,7 +2103,26 @@ void launch_stored_first(ggem_ctx *c, const float4 *f4, double self_c, const dou
                   : (cd2 ? k_pair_r1tv_first<2, false, 2> : k_pair_r1tv_first<1, false, 2>),
       dim3((unsigned)((c->n * kGroup + 255) / 256)), 256, 0, c->stream, c->n, c->pos32.p, f4,
       c->nb_cnt.p, c->nb_w, c->nb_list.p, poly_of(c), reinterpret_cast<const Rec32 *>(c->tab.p),
-      c->tab_inv_ds, g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p, self_c, f, u);
+      c->tab_inv_ds, g.h32[0], g.h32[1], g.h32[2], c->pair_ten.p, self_c, f, u, order);
+}
+
+// u = M f from the stored tensors, the FP32 forces staged in w_f4 (order: u
+// in the caller's particle order)
+int stored_product(ggem_ctx *c, double self_c, const double *f, double *u, const int32_t *order) {
+  const bool capturing = stream_capturing(c);
+  if (capturing) c->pretensor_eager = true;
+  if (kStoredVariants[c->stored_variant].G != kGroup)
+    if (int rc = form_pair_tensors(c)) return rc;
+  kt_start(c, kKPairF32);
+  if (c->pretensor_pending && kStoredVariants[c->stored_variant].G == kGroup) {
+    launch_stored_first(c, c->w_f4[0].p, self_c, f, u, order);
+    // (a captured product forms them whenever it is replayed)
+    c->pretensor_pending = capturing;
+  } else {
+    dispatch_stored_r1(c, c->w_f4[0].p, self_c, f, u, order);
+  }
+  kt_stop(c, kKPairF32);
+  return check_launch(c, "pair f32 r1 (tensors)");
 }
 
 int launch_f32_r1(ggem_ctx *c, const double *f, double *u, double self_c) {
@@ -2095,20 +2133,7 @@ int launch_f32_r1(ggem_ctx *c, const double *f, double *u, double self_c) {
     launch_dependent(k_stage_f4, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream,
                    n, f, c->w_f4[0].p);
     if (int rc = check_launch(c, "pair forces")) return rc;
-    const bool capturing = stream_capturing(c);
-    if (capturing) c->pretensor_eager = true;
-    if (kStoredVariants[c->stored_variant].G != kGroup)
-      if (int rc = form_pair_tensors(c)) return rc;
-    kt_start(c, kKPairF32);
-    if (c->pretensor_pending && kStoredVariants[c->stored_variant].G == kGroup) {
-      launch_stored_first(c, c->w_f4[0].p, self_c, f, u);
-      // (a captured product forms them whenever it is replayed)
-      c->pretensor_pending = capturing;
-    } else {
-      dispatch_stored_r1(c, c->w_f4[0].p, self_c, f, u);
-    }
-    kt_stop(c, kKPairF32);
-    return check_launch(c, "pair f32 r1 (tensors)");
+    return stored_product(c, self_c, f, u, nullptr);
   }
   if ((e = c->w_src.ensure(2 * (size_t)n))) return cuda_fail(c, e, "pair records");
   Rec32 *src = reinterpret_cast<Rec32 *>(c->w_src.p);
@@ -2412,14 +2437,21 @@ int matvec_records(ggem_ctx *c, const float4 *rec, const double *f, double *u, i
 }
 
 // u = M f for one right-hand side with f and u in the caller's particle
-// order (FP32 list, per-matvec tensors): the slot permutation of f is fused
-// with its records (k_to_slots_rec) and the pair kernel writes u in caller
-// order, so a matvec is two launches.  f_slot receives f in slot order (the
-// self term reads it).
+// order (FP32 list): the slot permutation of f is fused with the staging of
+// its FP32 forces (k_to_slots_rec, k_to_slots_f4) and the pair kernel writes
+// u in caller order, so a matvec is two launches.  f_slot receives f in slot
+// order (the self term reads it).  N = 400k with stored tensors, list
+// included: 307 -> 298 us against four launches.
 int matvec_orig_fused(ggem_ctx *c, const double *f, double *u, double *f_slot, int self_mode) {
   const int64_t n = c->n;
   if (n == 0) return GGEM_OK;
-  if (c->pretensor_ok) return fail(c, GGEM_ERR_BAD_ARG, "fused matvec needs per-matvec pair tensors");
+  if (c->pretensor_ok) {
+    if (cudaError_t e = c->w_f4[0].ensure((size_t)n)) return cuda_fail(c, e, "pair forces");
+    launch_dependent(k_to_slots_f4, dim3((unsigned)((n + 255) / 256)), 256, 0, c->stream, n,
+                     c->order.p, f, f_slot, c->w_f4[0].p);
+    if (int rc = check_launch(c, "to slots + forces")) return rc;
+    return stored_product(c, self_coefficient(c, self_mode), f_slot, u, c->order.p);
+  }
   cudaError_t e = c->w_src.ensure(2 * (size_t)n);
   if (e) return cuda_fail(c, e, "pair records");
   Rec32 *src = reinterpret_cast<Rec32 *>(c->w_src.p);
