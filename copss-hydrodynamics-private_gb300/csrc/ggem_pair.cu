@@ -1638,15 +1638,31 @@ constexpr int kBatchR = 64;      // right-hand sides per pass
 constexpr int kBatchMinRhs = 16; // fewer go through k_pair_nr in chunks of 8
 constexpr int kBatchWarps = 4;   // target slots per CTA
 
+// elements whose loads a thread of the batched vector passes has in flight (a
+// divisor of 64 * 96 / 256): one at a time waited out a DRAM latency each.  64
+// right-hand sides of N = 100k, us: staging 59 -> 55, slots + staging 99 -> 83,
+// start 176 -> 167
+constexpr int kStageFly = 4;
+
 __global__ void __launch_bounds__(256) k_stage_b64(int64_t n, int nr, const double *__restrict__ f,
                                                    float *__restrict__ fb) {
   // block: 32 slots x 64 right-hand sides; smem [r][96 + 1]
   __shared__ float t[kBatchR][97];
   const int64_t s0 = blockIdx.x * 32LL;
   const int ns = (int)(n - s0 < 32 ? n - s0 : 32);
-  for (int k = threadIdx.x; k < kBatchR * 96; k += blockDim.x) {
-    const int r = k / 96, q = k - r * 96;
-    t[r][q] = (r < nr && q < 3 * ns) ? d2f_bits(f[((int64_t)r * n + s0) * 3 + q]) : 0.f;
+#pragma unroll 1
+  for (int k0 = threadIdx.x; k0 < kBatchR * 96; k0 += kStageFly * 256) {
+    double v[kStageFly];
+#pragma unroll
+    for (int i = 0; i < kStageFly; ++i) {
+      const int k = k0 + 256 * i, r = k / 96, q = k - r * 96;
+      v[i] = (r < nr && q < 3 * ns) ? f[((int64_t)r * n + s0) * 3 + q] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < kStageFly; ++i) {
+      const int k = k0 + 256 * i, r = k / 96, q = k - r * 96;
+      t[r][q] = d2f_bits(v[i]);
+    }
   }
   __syncthreads();
   float *out = fb + s0 * 3 * kBatchR;
@@ -1666,16 +1682,20 @@ __global__ void __launch_bounds__(256) k_to_slots_b64(int64_t n, int nr,
   __shared__ float t[kBatchR][97];
   const int64_t s0 = blockIdx.x * 32LL;
   const int ns = (int)(n - s0 < 32 ? n - s0 : 32);
-  for (int k = threadIdx.x; k < kBatchR * 96; k += blockDim.x) {
-    const int r = k / 96, q = k - r * 96;
-    float v = 0.f;
-    if (r < nr && q < 3 * ns) {
-      const int sl = q / 3, c = q - 3 * sl;
-      const double x = xi[((int64_t)r * n + order[s0 + sl]) * 3 + c];
-      x0[((int64_t)r * n + s0) * 3 + q] = x;
-      v = d2f_bits(x);
+#pragma unroll 1
+  for (int k0 = threadIdx.x; k0 < kBatchR * 96; k0 += kStageFly * 256) {
+    double v[kStageFly];
+#pragma unroll
+    for (int i = 0; i < kStageFly; ++i) {
+      const int k = k0 + 256 * i, r = k / 96, q = k - r * 96, sl = q / 3, c = q - 3 * sl;
+      v[i] = r < nr && q < 3 * ns ? xi[((int64_t)r * n + order[s0 + sl]) * 3 + c] : 0.0;
     }
-    t[r][q] = v;
+#pragma unroll
+    for (int i = 0; i < kStageFly; ++i) {
+      const int k = k0 + 256 * i, r = k / 96, q = k - r * 96;
+      if (r < nr && q < 3 * ns) x0[((int64_t)r * n + s0) * 3 + q] = v[i];
+      t[r][q] = d2f_bits(v[i]);
+    }
   }
   __syncthreads();
   float *out = fb + s0 * 3 * kBatchR;
@@ -1697,19 +1717,31 @@ __global__ void __launch_bounds__(256) k_cheb_start_b64(int64_t n, int nr, doubl
   __shared__ float t[kBatchR][97];
   const int64_t s0 = blockIdx.x * 32LL;
   const int ns = (int)(n - s0 < 32 ? n - s0 : 32);
-  for (int k = threadIdx.x; k < kBatchR * 96; k += blockDim.x) {
-    const int r = k / 96, q = k - r * 96;
-    float v = 0.f;
-    if (r < nr && q < 3 * ns) {
+#pragma unroll 1
+  for (int k0 = threadIdx.x; k0 < kBatchR * 96; k0 += kStageFly * 256) {
+    double vx[kStageFly], vy[kStageFly];
+#pragma unroll
+    for (int i = 0; i < kStageFly; ++i) {
+      const int k = k0 + 256 * i, r = k / 96, q = k - r * 96;
       const int64_t idx = ((int64_t)r * n + s0) * 3 + q;
-      const double x = x0[idx];
-      const double y = db * x + da * x1[idx];
-      x1[idx] = y;
-      const double c0x = c0 * x;
-      dw[idx] = c0x + c1 * y;
-      v = d2f_bits(y);
+      const bool ok = r < nr && q < 3 * ns;
+      vx[i] = ok ? x0[idx] : 0.0;
+      vy[i] = ok ? x1[idx] : 0.0;
     }
-    t[r][q] = v;
+#pragma unroll
+    for (int i = 0; i < kStageFly; ++i) {
+      const int k = k0 + 256 * i, r = k / 96, q = k - r * 96;
+      const int64_t idx = ((int64_t)r * n + s0) * 3 + q;
+      float v = 0.f;
+      if (r < nr && q < 3 * ns) {
+        const double y = db * vx[i] + da * vy[i];
+        x1[idx] = y;
+        const double c0x = c0 * vx[i];
+        dw[idx] = c0x + c1 * y;
+        v = d2f_bits(y);
+      }
+      t[r][q] = v;
+    }
   }
   __syncthreads();
   float *out = fb + s0 * 3 * kBatchR;
