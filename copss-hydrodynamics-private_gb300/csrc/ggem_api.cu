@@ -173,6 +173,9 @@ int upload_stencil(ggem_ctx *c) {
     }
     if (c->prm.nb_mode == GGEM_NB_REFERENCE)  // (a stencil of the own element alone)
       for (int d = 0; d < 3; ++d) s_max += c->grid.h[d] * c->grid.h[d];
+    // from alpha r = 28 on both coefficients are exactly zero, and so is the
+    // last piece, which larger r read: a cut-off beyond the box adds no pieces
+    s_max = std::min(s_max, 784.0 / c->cst.alpha2);
     std::vector<double4_32a> rec;
     fit_tensor_f64(c->cst, s_max * (1.0 + 1e-9), rec, &c->t64);
     if ((e = c->tab64.ensure(rec.size())) ||
@@ -272,6 +275,14 @@ int validate_and_setup(ggem_ctx *c) {
     c->rc2 = p.rc * p.rc;
     c->rc2_lo = (float)(c->rc2 * (1.0 - 1e-4));
     c->rc2_hi = (float)(c->rc2 * (1.0 + 1e-4));
+    // The list decides by FP32 distances outside the band rc2_lo .. rc2_hi.
+    // A difference of two cell-relative coordinates is off by up to 3.5 * 2^-24
+    // h (two coordinates, the shift and their sum), so r^2 at the cut-off by
+    // 7.2e-7 h / rc of itself: within the band's 1e-4 up to cells of 125
+    // cut-offs (an axis capped at 2048 cells can have longer ones), and with
+    // squares that FP32 holds.  Other FP64 contexts keep the sweep.
+    c->f64_list_exact = p.rc >= 1e-12 && p.rc <= 1e15;
+    for (int d = 0; d < 3; ++d) c->f64_list_exact &= g.h[d] <= 64.0 * p.rc;
     if (p.precision == GGEM_FP32) {
       std::vector<float4> tab;
       const double s_max = c->rc2 * (1.0 + 2e-4);
@@ -476,8 +487,9 @@ extern "C" int ggem_build_cells(ggem_ctx *ctx) {
     // the FP64 path's own list, from the second configuration on that the
     // operator is applied to (contexts that only spread never pay for it)
     ctx->f64_skip = false;
-    if (int rc = build_cells(ctx, ctx->f64_wanted)) return rc;
-    return ctx->f64_wanted ? ensure_f64_list(ctx, true) : GGEM_OK;
+    const bool with_cells = ctx->f64_wanted && ctx->f64_list_exact;
+    if (int rc = build_cells(ctx, with_cells)) return rc;
+    return with_cells ? ensure_f64_list(ctx, true) : GGEM_OK;
   }
   const bool with_list = cutoff && (fp32 || ctx->f64_list > 0);
   if (int rc = build_cells(ctx, with_list)) return rc;

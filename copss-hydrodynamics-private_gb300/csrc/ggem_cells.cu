@@ -1125,7 +1125,7 @@ bool stream_capturing(const ggem_ctx *c) {
 
 int ensure_f64_list(ggem_ctx *c, bool flags_pending) {
   if (c->prm.precision != GGEM_FP64 || c->f64_list >= 0 || c->list_built || c->f64_skip ||
-      c->n == 0)
+      !c->f64_list_exact || c->n == 0)
     return GGEM_OK;
   cudaError_t e;
   if (!flags_pending) {

@@ -147,6 +147,7 @@ struct ggem_ctx {
   bool list_built = false;
   int f64_list = -1;
   bool f64_wanted = false, f64_skip = false;
+  bool f64_list_exact = true;  // the list's FP32 filter is sound in this box (ggem_api.cu)
   // the list is the FP64 path's own (default mode), not one the caller asked for
   bool f64_list_is_own() const { return prm.precision == GGEM_FP64 && f64_list != 1; }
   ggem::DevBuf<int4> d_runs;  // reference mode: the stencil's runs along x
