@@ -1035,7 +1035,8 @@ int build_pair_list(ggem_ctx *c) {
     const Grid &g = c->grid;
     const double vol = g.L[0] * g.L[1] * g.L[2];
     const double r = c->prm.nb_mode == GGEM_NB_REFERENCE ? c->search_radius_e : std::sqrt(c->rc2);
-    const double mean = vol > 0 ? (double)n / vol * 4.18879020478639 * r * r * r : 0.0;
+    double mean = vol > 0 ? (double)n / vol * 4.18879020478639 * r * r * r : 0.0;
+    if (c->f64_list_is_own()) mean = std::min(mean, 0.5 * n);  // (a pair is listed once)
     c->nb_w = (int)std::min<double>(((int64_t)(2.0 * mean) + 16 + 7) / 8 * 8, 1 << 20);
   }
   if (n == 0) {

@@ -67,3 +67,17 @@ def test_cutoffs_outside_the_fp32_range(rc, scale):
     got, want = _both(xyz, f, box_hi=(20.0 * scale,) * 3, periodic=(0, 0, 0), rc=rc)
     assert np.all(np.isfinite(want))
     assert rel(got, want) <= TOL
+
+
+def test_rows_no_wider_than_the_particles():
+    """a cut-off beyond an open box lists every pair: rows of n entries"""
+    import torch
+    n = 300
+    rng = np.random.default_rng(4)
+    xyz, f = rng.uniform(0.0, 20.0, (n, 3)), rng.standard_normal((n, 3))
+    with G.Context(precision=G.FP64, box_hi=(20.0,) * 3, periodic=(0, 0, 0), rc=1e4) as ctx:
+        ctx.set_particles(xyz)
+        ctx.build_cells()
+        free = torch.cuda.mem_get_info()[0]
+        ctx.local_matvec(f, G.SELF_BEAD)
+        assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
