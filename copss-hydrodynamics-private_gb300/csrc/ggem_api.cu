@@ -487,7 +487,7 @@ extern "C" int ggem_build_cells(ggem_ctx *ctx) {
     // the FP64 path's own list, from the second configuration on that the
     // operator is applied to (contexts that only spread never pay for it)
     ctx->f64_skip = false;
-    const bool with_cells = ctx->f64_wanted && ctx->f64_list_exact;
+    const bool with_cells = ctx->f64_wanted && f64_list_fits(ctx);
     if (int rc = build_cells(ctx, with_cells)) return rc;
     return with_cells ? ensure_f64_list(ctx, true) : GGEM_OK;
   }

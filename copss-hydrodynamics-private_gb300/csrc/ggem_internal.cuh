@@ -393,6 +393,7 @@ int build_pair_list(ggem_ctx *c);
 // flags_pending: the cell build's error word has not been read yet.
 int ensure_f64_list(ggem_ctx *c, bool flags_pending = false);
 bool stream_capturing(const ggem_ctx *c);
+bool f64_list_fits(const ggem_ctx *c);
 // deferred builds: copy the list statistics and the error word to the host
 // mirror (asynchronous), then, after the stream has synchronised, evaluate
 // them; *rebuilt is set when the rows had overflowed and the list (and the
