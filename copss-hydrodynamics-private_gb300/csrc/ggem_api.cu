@@ -484,10 +484,11 @@ extern "C" int ggem_build_cells(ggem_ctx *ctx) {
   const bool cutoff = ctx->prm.nb_mode == GGEM_NB_CUTOFF;
   const bool fp32 = ctx->prm.precision == GGEM_FP32;
   if (!fp32 && ctx->f64_list < 0) {
-    // the FP64 path's own list, from the second configuration on that the
-    // operator is applied to (contexts that only spread never pay for it)
+    // the FP64 path's own list, where the operator was applied to the
+    // configuration before this one (contexts that only spread don't pay)
     ctx->f64_skip = false;
     const bool with_cells = ctx->f64_wanted && f64_list_fits(ctx);
+    ctx->f64_wanted = false;
     if (int rc = build_cells(ctx, with_cells)) return rc;
     return with_cells ? ensure_f64_list(ctx, true) : GGEM_OK;
   }

@@ -1147,6 +1147,8 @@ bool f64_list_fits(const ggem_ctx *c) {
 }
 
 int ensure_f64_list(ggem_ctx *c, bool flags_pending) {
+  // (a product asks: the next configuration's list comes with its cells)
+  if (!flags_pending) c->f64_wanted = true;
   if (c->prm.precision != GGEM_FP64 || c->f64_list >= 0 || c->list_built || c->f64_skip ||
       !f64_list_fits(c) || c->n == 0)
     return GGEM_OK;
@@ -1158,7 +1160,6 @@ int ensure_f64_list(ggem_ctx *c, bool flags_pending) {
     if ((e = cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream)))
       return cuda_fail(c, e, "memset");
   }
-  c->f64_wanted = true;
   const bool defer = c->defer_checks;
   c->defer_checks = false;
   const int rc = build_pair_list(c);

@@ -141,9 +141,9 @@ struct ggem_ctx {
   // FP32 pair list (built for GGEM_FP64 contexts too: the FP64 pair kernel
   // then walks the exact list instead of sweeping cells).  f64_list: 1 = with
   // every cell build, 0 = never, -1 (default) = by the first operator
-  // application after a cell build, and with the cell build itself once the
-  // context has applied its operator (f64_wanted); f64_skip: the current
-  // configuration's list does not fit (the cells are swept).
+  // application after a cell build, and with the cell build itself if the
+  // operator was applied since the last one (f64_wanted); f64_skip: the
+  // current configuration's list does not fit (the cells are swept).
   bool list_built = false;
   int f64_list = -1;
   bool f64_wanted = false, f64_skip = false;

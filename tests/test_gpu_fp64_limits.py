@@ -81,3 +81,27 @@ def test_rows_no_wider_than_the_particles():
         free = torch.cuda.mem_get_info()[0]
         ctx.local_matvec(f, G.SELF_BEAD)
         assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
+
+
+def test_only_configurations_with_products_build_the_list():
+    """after one product the builds that no product follows (a context that
+    only spreads from then on) cost what they cost before it"""
+    rng = np.random.default_rng(5)
+    xyz, f = rng.uniform(0.0, 40.0, (500, 3)), rng.standard_normal((500, 3))
+    with G.Context(precision=G.FP64, box_hi=(40.0,) * 3) as ctx:
+        def launches(call):
+            a = ctx.launch_count()
+            call()
+            return ctx.launch_count() - a
+
+        ctx.set_particles(xyz)
+        ctx.build_cells()
+        fresh = launches(ctx.build_cells)
+        ctx.local_matvec(f)
+        ctx.build_cells()  # prepared for the product that usually follows
+        assert launches(ctx.build_cells) == fresh
+        # with a product on every configuration the list comes with the build
+        for _ in range(3):
+            ctx.local_matvec(f)
+            ctx.build_cells()
+            assert launches(lambda: ctx.local_matvec(f)) == 3  # order, product, order
