@@ -265,7 +265,10 @@ __global__ void k_axpy_into(int64_t tot, double s, const double *__restrict__ a,
 // ---- Lanczos ---------------------------------------------------------------
 // The recurrence runs without the host: the coefficients, 1 / beta and the
 // projections stay on the device (LanczosState) and the host reads them once
-// at the end.  Per step, with w = M q_j:
+// at the end; a step's last kernel tells it, through pinned memory, how far
+// the recurrence is and whether it ended there (beta = 0: few distinct
+// eigenvalues, as without pairs in reach), so that the host, at most
+// kLzAhead steps ahead, launches no more of them.  Per step, with w = M q_j:
 //   k_lz_dots     h_i = Q_i . w for all i <= j (and k_finalize)
 //   k_lz_project  w -= sum_i h_i Q_i; these two twice, the second time with
 //                 |w|^2 in the same pass
@@ -276,8 +279,9 @@ __global__ void k_axpy_into(int64_t tot, double s, const double *__restrict__ a,
 // and clock): four fused multiply-adds per element and vector, 48 us per step
 // at N = 200k, j = 12.  Eight vectors' warp sums share one reduce-scatter (9
 // additions instead of 40), which made the dots 37 -> 27 us.  N = 200k,
-// k = 24: 5.47 -> 3.44 ms.
+// k = 24: 5.47 -> 3.33 ms.
 constexpr int kLzMax = 512;  // steps
+constexpr int kLzAhead = 1;  // steps launched beyond the last finished one
 
 struct LanczosState {
   double alpha[kLzMax], beta[kLzMax], h[kLzMax], norm2;
@@ -410,14 +414,19 @@ __global__ void __launch_bounds__(kVecThreads) k_lz_project(int64_t D, int m,
   }
 }
 
-// q = w / |w|, and the step's coefficients
-__global__ void k_lz_next(int64_t D, int j, const double *w, double *q, LanczosState *S) {
+// q = w / |w|, and the step's coefficients; *seen = j + 1, negative where the
+// recurrence ends
+__global__ void k_lz_next(int64_t D, int j, const double *w, double *q, LanczosState *S,
+                          volatile double *seen) {
   wait_prior_grid();
   __shared__ double s_scale;
   if (threadIdx.x == 0) {  // (once per block: a root and a division cost ~40 FP64 instructions)
     const double b = sqrt(S->norm2);
-    s_scale = b > 0.0 ? 1.0 / b : 0.0;  // (a breakdown ends the recurrence on the host)
-    if (j >= 0 && blockIdx.x == 0) S->beta[j] = b;
+    s_scale = b > 0.0 ? 1.0 / b : 0.0;
+    if (j >= 0 && blockIdx.x == 0) {
+      S->beta[j] = b;
+      *seen = b < 1e-14 * fabs(S->alpha[j]) + 1e-300 ? -(j + 1.0) : j + 1.0;
+    }
   }
   __syncthreads();
   const double s = s_scale;
@@ -1224,10 +1233,20 @@ extern "C" int ggem_lanczos_bounds(ggem_ctx *ctx, int k, uint64_t seed, double *
                    D, 0, Q, S, Q, part);
   if (int rc = check_launch(ctx, "lanczos norm")) return rc;
   if (int rc = finish(1, &S->norm2)) return rc;
+  double *h = ctx->h_red;
+  volatile double *seen = h + 2 * kLzMax;
+  *seen = 0.0;
   launch_dependent(k_lz_next, dim3(grid1(D)), 256, 0, st,
-                   D, -1, Q, Q, S);
+                   D, -1, Q, Q, S, seen);
   if (int rc = check_launch(ctx, "lanczos next")) return rc;
+  int issued = k;
   for (int j = 0; j < k; ++j) {
+    while (*seen >= 0.0 && j - *seen > kLzAhead)
+      if (cudaStreamQuery(st) != cudaErrorNotReady) break;
+    if (*seen < 0.0) {
+      issued = j;
+      break;
+    }
     const int m = j + 1;
     const size_t sh = sizeof(double) * m;
     if (int rc = matvec_slots(ctx, 1, Q + (size_t)j * D, w, sm)) return rc;
@@ -1253,18 +1272,17 @@ extern "C" int ggem_lanczos_bounds(ggem_ctx *ctx, int k, uint64_t seed, double *
     }
     if (int rc = finish(1, &S->norm2)) return rc;
     launch_dependent(k_lz_next, dim3(grid1(D)), 256, 0, st,
-                   D, j, w, Q + (size_t)(j + 1) * D, S);
+                   D, j, w, Q + (size_t)(j + 1) * D, S, seen);
     if (int rc = check_launch(ctx, "lanczos next")) return rc;
   }
   std::vector<double> a(k), b(k);
-  double *h = ctx->h_red;
   if ((e = cudaMemcpyAsync(h, S->alpha, sizeof(double) * k, cudaMemcpyDeviceToHost, st)) ||
       (e = cudaMemcpyAsync(h + kLzMax, S->beta, sizeof(double) * k, cudaMemcpyDeviceToHost, st)) ||
       (e = cudaStreamSynchronize(st)))
     return cuda_fail(ctx, e, "lanczos readback");
   // the recurrence ends where beta vanishes: q_{j+1} and what follows it is void
-  int m = k;
-  for (int j = 0; j < k; ++j) {
+  int m = issued;
+  for (int j = 0; j < issued; ++j) {
     a[j] = h[j];
     b[j] = h[kLzMax + j];
     if (j < k - 1 && b[j] < 1e-14 * std::fabs(a[j]) + 1e-300) {
