@@ -148,6 +148,10 @@ __device__ __forceinline__ int axis_offset(const SpreadGeo &sg, int d, int us, i
 // record, 8); a point's four lanes reduce-scatter, so each converts and
 // writes one component; the lanes decode 32 elements at once; two windows of
 // candidates per pass.
+// A lane's two members need not come through shared memory with 16 lanes per
+// point (a shuffle) or 32 (one member).  N = 20k, us with one member
+// at a time -> two: 27 points 923 -> 694, 12 points 632 -> 521, 4 points 433
+// -> 424, 2 points 405 -> 398.
 template <bool F32, bool ANYFULL, bool PAD>
 __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
     SpreadGeo sg, DevConsts K, const int32_t *__restrict__ start,
@@ -258,6 +262,7 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   const int nel = ebx * eby * ebz;
   const int nq = sg.nq, lq = sg.lq;
   const int qi = lane / lq, sub = lane - qi * lq;
+  const int llq = 31 - __clz(lq);
   unsigned long long my_pairs = 0;
   // the warp's member queue: per member its staged index (10 bits) and its
   // element offset (the padded bitmap index, or three 5-bit offsets); each
@@ -266,6 +271,10 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   // once per point, one member per lane) with the staged index in .w
   uint32_t *mq = queue + warp * kSpQueue;
   float *mb = batch + warp * kSpBatch;
+  // FP32, up to eight lanes per point: the two members that a lane takes one
+  // after the other share a pair slot, i.e. member j of a batch (the t-th of
+  // lane j % lq of a point) lies in slot (t / 2, j % lq), half t % 2
+  float *mine = mb + 12 * ((qi >> 1) * lq + sub) + (qi & 1);
   const unsigned lt_mask = (1u << lane) - 1u;
   // with the padded bitmap, a particle at frame coordinates u is listed by
   // some element of the brick when the union bitmap holds u (shifted where
@@ -431,11 +440,10 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
         while (queued - head >= 32 || (last && queued > head)) {
           __syncwarp();
           const int m = min(queued - head, 32);
+          // (FP32: position and force of member `lane`; past the last member
+          // zeros, whose terms are exact zeros)
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f), fv = v;
           if (F32) {
-            // member j in pair slot (j / 8, j % 4), half (j / 4) % 2: the two
-            // members that a lane takes one after the other at four lanes per
-            // point; past the last member zeros, whose terms are exact zeros
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f), fv = v;
             if (lane < m) {
               const uint32_t en = mq[head + lane];
               const int kk = (int)(en & 1023u);
@@ -456,36 +464,35 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
               v.y += s_shift[1][iy];
               v.z += s_shift[2][iz];
             }
-            float *o = mb + 12 * ((lane >> 3) * 4 + (lane & 3)) + ((lane >> 2) & 1);
-            o[0] = v.x;
-            o[2] = v.y;
-            o[4] = v.z;
-            o[6] = fv.x;
-            o[8] = fv.y;
-            o[10] = fv.z;
+            if (lq < 16) {
+              mine[0] = v.x;
+              mine[2] = v.y;
+              mine[4] = v.z;
+              mine[6] = fv.x;
+              mine[8] = fv.y;
+              mine[10] = fv.z;
+            }
           }
           __syncwarp();
-          // one (point, member) term of the FP32 sum into the block sums
-          auto term32 = [&](int j) {
-            const float *o = mb + 12 * ((j >> 3) * 4 + (j & 3)) + ((j >> 2) & 1);
-            const float dx = axis32(0, o[0] - qr.x);
-            const float dy = axis32(1, o[2] - qr.y);
-            const float dz = axis32(2, o[4] - qr.z);
+          // this lane's own member into the block sums
+          auto term32 = [&]() {
+            const float dx = axis32(0, v.x - qr.x);
+            const float dy = axis32(1, v.y - qr.y);
+            const float dz = axis32(2, v.z - qr.z);
             const float s2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
             const float p = s2 * sg.e_hi;
             const float r = fmaf(s2, sg.e_lo, fmaf(s2, sg.e_hi, -p));
             const float E0 = ex2_approx(p);
             const float E = fmaf(E0, r * 0.6931471805599453f, E0);
             const float gv = E * fmaf(-sg.c1, s2, sg.c25);
-            bx_ = fmaf(gv, o[6], bx_);
-            by_ = fmaf(gv, o[8], by_);
-            bz_ = fmaf(gv, o[10], bz_);
+            bx_ = fmaf(gv, fv.x, bx_);
+            by_ = fmaf(gv, fv.y, by_);
+            bz_ = fmaf(gv, fv.z, bz_);
           };
-          // two members of a pair slot, one after the other into the block
-          // sums; what precedes the sums in packed arithmetic (each half
-          // rounds as the scalar form does)
-          auto pair32 = [&](const float4 *o) {
-            const float4 a = o[0], b = o[1], c = o[2];
+          // two members, one after the other into the block sums; what
+          // precedes the sums in packed arithmetic (each half rounds as the
+          // scalar form does)
+          auto pair_terms = [&](const float4 &a, const float4 &b, const float4 &c) {
             float2 dx = __fadd2_rn(make_float2(a.x, a.y), make_float2(-qr.x, -qr.x));
             float2 dy = __fadd2_rn(make_float2(a.z, a.w), make_float2(-qr.y, -qr.y));
             float2 dz = __fadd2_rn(make_float2(b.x, b.y), make_float2(-qr.z, -qr.z));
@@ -507,6 +514,7 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
             by_ = fmaf(gv.y, c.y, fmaf(gv.x, c.x, by_));
             bz_ = fmaf(gv.y, c.w, fmaf(gv.x, c.z, bz_));
           };
+          auto pair32 = [&](const float4 *o) { pair_terms(o[0], o[1], o[2]); };
           auto flush32 = [&]() {  // the block sums into the compensated sums
             kahan_acc(sx, cx, bx_);
             kahan_acc(sy, cy, by_);
@@ -514,45 +522,64 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
             bx_ = by_ = bz_ = 0.f;
             blk = 0;
           };
-          if (F32 && lq == 4) {
-            // four lanes per point: up to eight members per lane, which is one
-            // block of the compensated sums (blk is 0 here: every earlier
-            // batch was full)
+          if (F32) {
+            // this lane's members of the batch, eight of them into the
+            // compensated sums at a time (every earlier batch was full)
             const float4 *o = reinterpret_cast<const float4 *>(mb) + 3 * sub;
-            if (m == 32) {
+            const int cnt = (m - sub + lq - 1) >> llq, step = 3 * lq;
+            if (lq == 4 && m == 32) {
 #pragma unroll
               for (int t = 0; t < 4; ++t) pair32(o + 12 * t);
               flush32();
-            } else {
-              for (int t = 0; 8 * t < m; ++t) pair32(o + 12 * t);
-              if (m > 28 + sub) flush32();  // the lane had eight
+            } else if (lq <= 4) {
+              int t = 0;
+              for (; 2 * t + 8 <= cnt; t += 4, o += 4 * step) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) pair32(o + u * step);
+                flush32();
+              }
+              for (; 2 * t < cnt; ++t, o += step) pair32(o);
+            } else if (lq == 8) {
+              for (int t = 0; 2 * t < cnt; ++t) pair32(o + t * step);
+              blk += cnt;
+              if (blk == 8) flush32();
+            } else if (lq == 16) {  // the lane's own member and that of the lane 16 from it
+              const bool up = lane & 16;
+              auto both = [&](float w) {
+                const float other = __shfl_xor_sync(0xffffffffu, w, 16);
+                return up ? make_float2(other, w) : make_float2(w, other);
+              };
+              const float2 x = both(v.x), y = both(v.y), z = both(v.z);
+              const float2 fx = both(fv.x), fy = both(fv.y), fz = both(fv.z);
+              pair_terms(make_float4(x.x, x.y, y.x, y.y), make_float4(z.x, z.y, fx.x, fx.y),
+                         make_float4(fy.x, fy.y, fz.x, fz.y));
+              blk += cnt;
+              if (blk == 8) flush32();
+            } else if (sub < m) {
+              term32();
+              if (++blk == 8) flush32();
             }
           } else {
             for (int j = sub; j < m && qok; j += lq) {
-              if (F32) {
-                term32(j);
-                if (++blk == 8) flush32();  // every 8 pairs into the compensated sums
-              } else {
-                const int kk = (int)(mq[head + j] & 1023u);
-                const double4_32a a = rec64[2 * kk], fb = rec64[2 * kk + 1];
-                // point_vector(q, x_j) with the minimum image (pm_periodic_boundary.C:350-374)
-                double x[3] = {a.x - q0, a.y - q1, a.z - q2};
+              const int kk = (int)(mq[head + j] & 1023u);
+              const double4_32a a = rec64[2 * kk], fb = rec64[2 * kk + 1];
+              // point_vector(q, x_j) with the minimum image (pm_periodic_boundary.C:350-374)
+              double x[3] = {a.x - q0, a.y - q1, a.z - q2};
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                  if (sg.g.periodic[d]) {
-                    const double xs = sg.g.L[d];
-                    if (x[d] <= -xs / 2.0) x[d] += xs;
-                    if (x[d] > xs / 2.0) x[d] -= xs;
-                  }
+              for (int d = 0; d < 3; ++d) {
+                if (sg.g.periodic[d]) {
+                  const double xs = sg.g.L[d];
+                  if (x[d] <= -xs / 2.0) x[d] += xs;
+                  if (x[d] > xs / 2.0) x[d] -= xs;
                 }
-                // smoothed_force_exp (ggem_stokes.C:117-128)
-                const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-                const double a2r2 = K.alpha2 * r2;
-                const double gv = K.alpha3_pi_23 * exp(-a2r2) * (2.5 - a2r2);
-                ax += gv * fb.x;
-                ay += gv * fb.y;
-                az += gv * fb.z;
               }
+              // smoothed_force_exp (ggem_stokes.C:117-128)
+              const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+              const double a2r2 = K.alpha2 * r2;
+              const double gv = K.alpha3_pi_23 * exp(-a2r2) * (2.5 - a2r2);
+              ax += gv * fb.x;
+              ay += gv * fb.y;
+              az += gv * fb.z;
             }
           }
           head += m;

@@ -220,3 +220,26 @@ def test_fp32_spread_member_batches(p, members):
         ctx.set_quadrature(q, nq)
         want, got = ctx.spread_elements(f, G.FP64), ctx.spread_elements(f, G.FP32)
     assert rel(got, want) <= 1e-6
+
+
+@pytest.mark.parametrize("p", [(2, 1, 1), (3, 3, 1), (4, 2, 2)])
+@pytest.mark.parametrize("members", [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 48, 64, 65, 130])
+@pytest.mark.parametrize("nm", [24, 11])
+def test_fp32_spread_lanes_per_point(p, members, nm):
+    """16 and 2 lanes per point around their pairs of members, blocks of eight
+    and batches, on the padded bitmap and on a mesh that the stencil spans,
+    against the FP64 spread (1e-6 norm-wise, as above)"""
+    h = 1.4
+    L = nm * h
+    rng = np.random.default_rng(members)
+    xyz = 5.6 + rng.uniform(0.1, 1.3, (members, 3))
+    f = rng.standard_normal((members, 3))
+    q, nq = _grid_points((0, 0, 0), (L,) * 3, (nm,) * 3, p, (0, 1, 2))
+    with G.Context(alpha=ALPHA, box_hi=(L,) * 3, nb_mode=G.NB_REFERENCE, n_mesh=(nm,) * 3,
+                   search_radius_e=0.5 * h + 8.0 + 1e-3, precision=G.FP64) as ctx:
+        ctx.set_particles(xyz)
+        ctx.build_cells()
+        ctx.set_quadrature(q, nq)
+        want, got = ctx.spread_elements(f, G.FP64), ctx.spread_elements(f, G.FP32)
+        assert np.array_equal(got, ctx.spread_elements(f, G.FP32))
+    assert rel(got, want) <= 1e-6
