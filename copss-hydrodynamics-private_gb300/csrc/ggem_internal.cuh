@@ -215,6 +215,8 @@ struct ggem_ctx {
   ggem::DevBuf<double> q_xyz;
   ggem::DevBuf<float4> q_rel;
   ggem::DevBuf<uint32_t> sp_bits;
+  std::vector<uint32_t> sp_bits_h;
+  bool sp_bits_up = false;
   ggem::DevBuf<unsigned long long> sp_pairs;
   // the points as a tensor grid (q_grid): points per element and axis, the
   // axis coordinates, the point of each (row, index along x); the spread's

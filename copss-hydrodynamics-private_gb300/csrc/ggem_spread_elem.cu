@@ -1045,6 +1045,41 @@ struct DeviceGuard {
   }
 };
 
+// the stencil bitmap (own element included) and, padded, its union over a brick
+int upload_bitmap(ggem_ctx *c, const SpreadGeo &sg) {
+  const int B = sg.B;
+  std::vector<uint32_t> &bits = c->sp_bits_h;  // (a captured copy reads it when replayed)
+  bits.assign(sg.nwords, 0u);
+  auto set = [&](int x, int y, int z) {
+    const int i = x - sg.lo[0], j = y - sg.lo[1], k = z - sg.lo[2];
+    const int idx = sg.pad ? (i + B - 1) + 32 * (j + B - 1) + 1024 * (k + B - 1)
+                            : (k * sg.dim[1] + j) * sg.dim[0] + i;
+    bits[idx >> 5] |= 1u << (idx & 31);
+  };
+  set(0, 0, 0);  // the element's own particles come first in its list
+  for (const int4 &o : c->stencil) set(o.x, o.y, o.z);
+  if (sg.pad) {
+    // the particles that some element of a brick lists: bit u is the union of
+    // the stencil bits u + (jx, jy, jz), 0 <= j < B (the elements of a brick
+    // read the bitmap at u + B - 1 - l); one word per (y, z), x in its bits
+    std::vector<uint32_t> x(kSpReachWords, 0u), y(kSpReachWords, 0u), z(kSpReachWords, 0u);
+    for (int k = 0; k < sg.nwords; ++k)
+      for (int j = 0; j < B; ++j) x[k] |= bits[k] >> j;
+    for (int k = 0; k < kSpReachWords; ++k)
+      for (int j = 0; j < B && (k & 31) + j < 32; ++j) y[k] |= x[k + j];
+    for (int k = 0; k < kSpReachWords; ++k)
+      for (int j = 0; j < B && k + 32 * j < kSpReachWords; ++j) z[k] |= y[k + 32 * j];
+    bits.insert(bits.end(), z.begin(), z.end());
+  }
+  cudaError_t e = c->sp_bits.ensure(bits.size());
+  if (e) return cuda_fail(c, e, "spread stencil");
+  if ((e = cudaMemcpyAsync(c->sp_bits.p, bits.data(), sizeof(uint32_t) * bits.size(),
+                           cudaMemcpyHostToDevice, c->stream)))
+    return cuda_fail(c, e, "spread stencil");
+  c->sp_bits_up = !stream_capturing(c);
+  return GGEM_OK;
+}
+
 // the stencil bitmap (own element included) and the brick geometry
 int spread_geometry(ggem_ctx *c, SpreadGeo *sg) {
   std::memset(sg, 0, sizeof(*sg));
@@ -1100,33 +1135,9 @@ int spread_geometry(ggem_ctx *c, SpreadGeo *sg) {
   sg->nwords = (nbits + 31) / 32;
   if (sg->nwords > kSpMaxWords)
     return fail(c, GGEM_ERR_BAD_ARG, "element stencil bitmap too large for the brick spread");
-  std::vector<uint32_t> bits(sg->nwords, 0u);
-  auto set = [&](int x, int y, int z) {
-    const int i = x - sg->lo[0], j = y - sg->lo[1], k = z - sg->lo[2];
-    const int idx = sg->pad ? (i + B - 1) + 32 * (j + B - 1) + 1024 * (k + B - 1)
-                            : (k * sg->dim[1] + j) * sg->dim[0] + i;
-    bits[idx >> 5] |= 1u << (idx & 31);
-  };
-  set(0, 0, 0);  // the element's own particles come first in its list
-  for (const int4 &o : c->stencil) set(o.x, o.y, o.z);
-  if (sg->pad) {
-    // the particles that some element of a brick lists: bit u is the union of
-    // the stencil bits u + (jx, jy, jz), 0 <= j < B (the elements of a brick
-    // read the bitmap at u + B - 1 - l); one word per (y, z), x in its bits
-    std::vector<uint32_t> x(kSpReachWords, 0u), y(kSpReachWords, 0u), z(kSpReachWords, 0u);
-    for (int k = 0; k < sg->nwords; ++k)
-      for (int j = 0; j < B; ++j) x[k] |= bits[k] >> j;
-    for (int k = 0; k < kSpReachWords; ++k)
-      for (int j = 0; j < B && (k & 31) + j < 32; ++j) y[k] |= x[k + j];
-    for (int k = 0; k < kSpReachWords; ++k)
-      for (int j = 0; j < B && k + 32 * j < kSpReachWords; ++j) z[k] |= y[k + 32 * j];
-    bits.insert(bits.end(), z.begin(), z.end());
-  }
-  cudaError_t e = c->sp_bits.ensure(bits.size());
-  if (e) return cuda_fail(c, e, "spread stencil");
-  if ((e = cudaMemcpyAsync(c->sp_bits.p, bits.data(), sizeof(uint32_t) * bits.size(),
-                           cudaMemcpyHostToDevice, c->stream)))
-    return cuda_fail(c, e, "spread stencil");
+  // (the stencil belongs to the context: its bitmap goes up once)
+  if (!c->sp_bits_up)
+    if (int rc = upload_bitmap(c, *sg)) return rc;
   // e^{-alpha^2 s} = 2^{s k}, k = -alpha^2 log2(e) split into hi + lo floats
   const double k = -c->cst.alpha2 * 1.4426950408889634;
   sg->e_hi = (float)k;
