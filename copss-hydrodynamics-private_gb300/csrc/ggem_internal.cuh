@@ -219,13 +219,11 @@ struct ggem_ctx {
   bool sp_bits_up = false;
   ggem::DevBuf<unsigned long long> sp_pairs;
   // the points as a tensor grid (q_grid): points per element and axis, the
-  // axis coordinates, the point of each (row, index along x); the spread's
-  // per-particle axis factors
+  // point of each (row, index along x) and one with each axis index; the
+  // spread's per-particle axis factors
   bool q_grid = false;
   int q_p[3] = {0, 0, 0};
-  signed char q_map[32] = {0};
-  ggem::DevBuf<double> q_ax[3];
-  ggem::DevBuf<int> q_flag;
+  signed char q_map[32] = {0}, q_rep[3][32] = {};
   ggem::DevBuf<double2> sp_fac;
 
   // scan scratch (one per recursion level)

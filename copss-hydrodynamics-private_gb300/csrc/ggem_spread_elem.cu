@@ -693,14 +693,14 @@ struct SepGeo {
   int stride;     // staged double2 per particle: B (px + py + pz) + 2
   int cap, nw;    // staged particles per pass (a multiple of 32), mask words
   signed char qmap[32];  // point index of (row, a)
+  signed char rep[3][32];  // a point with each axis index
 };
 
 // window[slot][axis][offset - lo][a] = (g, g h) on x, (g, 2.5 - h) on y,
 // (alpha^3 pi^{-3/2} g, h) on z; the offset is the particle's element minus
 // the point's, zero where that element lies outside an open axis
 __global__ void __launch_bounds__(256) k_axis_factors(
-    int64_t n, SpreadGeo sg, SepGeo sp, DevConsts K, const double *__restrict__ ax0,
-    const double *__restrict__ ax1, const double *__restrict__ ax2,
+    int64_t n, SpreadGeo sg, SepGeo sp, DevConsts K, const double *__restrict__ qp,
     const float4 *__restrict__ pos32, const double4_32a *__restrict__ pos64,
     double2 *__restrict__ fac) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -717,7 +717,8 @@ __global__ void __launch_bounds__(256) k_axis_factors(
   if (sg.g.periodic[d]) e = wrap_cell(e, nc);
   if (e >= 0 && e < nc) {
     const double4_32a P = pos64[s];
-    const double q = (d == 0 ? ax0 : (d == 1 ? ax1 : ax2))[e * sp.p[d] + a];
+    const int64_t el = d == 0 ? e : (d == 1 ? e * (int64_t)nc0 : e * (int64_t)nc0 * nc1);
+    const double q = qp[3 * (el * sg.nq + sp.rep[d][a]) + d];
     double x = (d == 0 ? P.x : (d == 1 ? P.y : P.z)) - q;
     if (sg.g.periodic[d]) {  // minimum image (pm_periodic_boundary.C:350-374)
       const double xs = sg.g.L[d];
@@ -986,52 +987,62 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_sep(
     atomicAdd(pairs, my_pairs * (unsigned long long)sg.nq);
 }
 
-// axis tables of a tensor grid from the elements along each axis:
-// ax[e p + a] = coordinate d of point rep[a] of the axis's element e
+// Do the points form a tensor grid?  The first element gives the indices (a
+// point's coordinate among the distinct ones of its axis, -0 and 0 alike) and
+// a point with each index, whose copies in the elements along the axis give
+// the coordinates; every point of the mesh is compared with those.
 struct AxisMap {
-  signed char rep[3][32];  // a point with index a on the axis
-  signed char idx[3][32];  // the axis index of each point
+  int off;                  // a point differs from the grid
+  int p[3];                 // distinct coordinates per element and axis
+  signed char idx[3][32];   // the axis index of each point
+  signed char rep[3][32];   // a point with each index
 };
 
-__global__ void k_axis_table(int d, int nc, int64_t stride, int nq, int p, AxisMap m,
-                             const double *__restrict__ q, double *__restrict__ ax) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nc * p) return;
-  const int64_t e = t / p;
-  ax[t] = q[3 * (e * stride * nq + m.rep[d][t - (int)e * p]) + d];
-}
-
-// flag[0] |= 1 where a point is not bit for bit the grid's
-__global__ void k_check_grid(int64_t nqt, int nq, Grid g, int px, int py, int pz, AxisMap m,
-                             const double *__restrict__ q, const double *__restrict__ ax0,
-                             const double *__restrict__ ax1, const double *__restrict__ ax2,
-                             int *__restrict__ flag) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nqt) return;
-  const int64_t e = t / nq;
-  const int k = (int)(t - e * nq);
-  const int ex = (int)(e % g.nc[0]), ey = (int)((e / g.nc[0]) % g.nc[1]),
-            ez = (int)(e / ((int64_t)g.nc[0] * g.nc[1]));
-  const bool same = q[3 * t] == ax0[ex * px + m.idx[0][k]] &&
-                    q[3 * t + 1] == ax1[ey * py + m.idx[1][k]] &&
-                    q[3 * t + 2] == ax2[ez * pz + m.idx[2][k]];
-  if (!same) atomicOr(flag, 1);
-}
-
 // quadrature points relative to their element centre (FP64 difference,
-// rounded once to FP32); w = 0
-__global__ void k_qp_rel(int64_t nqt, int nq, Grid g, const double *__restrict__ q,
-                         float4 *__restrict__ rel) {
+// rounded once to FP32; w = 0), and the axis map to the host's pinned copy,
+// which costs a set of points 2 us and no other wait
+__global__ void __launch_bounds__(256) k_qp_rel(int64_t nqt, int nq, Grid g,
+                                                const double *__restrict__ q,
+                                                volatile AxisMap *host, float4 *__restrict__ rel) {
+  __shared__ int s_p[3], s_idx[3][32], s_rep[3][32];
+  if (threadIdx.x < 96) {
+    const int d = threadIdx.x >> 5, k = threadIdx.x & 31;
+    const double v = (k < nq ? q[3 * k + d] : 0.0) + 0.0;  // (-0 becomes 0)
+    const unsigned in = __ballot_sync(0xffffffffu, k < nq);
+    const unsigned same =
+        in & __match_any_sync(0xffffffffu, (unsigned long long)__double_as_longlong(v));
+    const int first = same ? __ffs(same) - 1 : 0;
+    const unsigned firsts = __ballot_sync(0xffffffffu, k < nq && first == k);
+    const int a = __popc(firsts & ((1u << first) - 1u));
+    s_idx[d][k] = a;
+    if (k < nq && first == k) s_rep[d][a] = k;
+    if (k == 0) s_p[d] = __popc(firsts);
+    if (blockIdx.x == 0) {
+      host->idx[d][k] = (signed char)a;
+      if (k < nq && first == k) host->rep[d][a] = (signed char)k;
+      if (k == 0) host->p[d] = __popc(firsts);
+    }
+  }
+  __syncthreads();
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nqt) return;
-  const int64_t e = t / nq;
-  const int ex = (int)(e % g.nc[0]), ey = (int)((e / g.nc[0]) % g.nc[1]),
-            ez = (int)(e / ((int64_t)g.nc[0] * g.nc[1]));
-  const double cx = g.lo[0] + (ex + 0.5) * g.h[0];
-  const double cy = g.lo[1] + (ey + 0.5) * g.h[1];
-  const double cz = g.lo[2] + (ez + 0.5) * g.h[2];
-  rel[t] = make_float4((float)(q[3 * t] - cx), (float)(q[3 * t + 1] - cy),
-                       (float)(q[3 * t + 2] - cz), 0.f);
+  bool off = false;
+  if (t < nqt) {
+    const int64_t e = t / nq;
+    const int k = (int)(t - e * nq);
+    const int nx = g.nc[0];
+    const int64_t nxy = (int64_t)nx * g.nc[1];
+    const int ex = (int)(e % nx), ey = (int)((e / nx) % g.nc[1]), ez = (int)(e / nxy);
+    const double cx = g.lo[0] + (ex + 0.5) * g.h[0];
+    const double cy = g.lo[1] + (ey + 0.5) * g.h[1];
+    const double cz = g.lo[2] + (ez + 0.5) * g.h[2];
+    const double x = q[3 * t], y = q[3 * t + 1], z = q[3 * t + 2];
+    rel[t] = make_float4((float)(x - cx), (float)(y - cy), (float)(z - cz), 0.f);
+    if (s_p[0] * s_p[1] * s_p[2] == nq)  // (the host sees that too)
+      off = x != q[3 * (ex * (int64_t)nq + s_rep[0][s_idx[0][k]])] ||
+            y != q[3 * (ey * (int64_t)nx * nq + s_rep[1][s_idx[1][k]]) + 1] ||
+            z != q[3 * (ez * nxy * nq + s_rep[2][s_idx[2][k]]) + 2];
+  }
+  if (__syncthreads_or(off) && threadIdx.x == 0) host->off = 1;
 }
 
 struct DeviceGuard {
@@ -1171,6 +1182,7 @@ int spread_separable(ggem_ctx *c, const SpreadGeo &sg, bool any_full, const doub
   sp.R = sp.p[1] * sp.p[2];
   sp.E = 32 / sp.R;
   std::memcpy(sp.qmap, c->q_map, sizeof(sp.qmap));
+  std::memcpy(sp.rep, c->q_rep, sizeof(sp.rep));
   // 80 KB of staged particles: with the tables, two blocks per SM
   sp.cap = (int)std::min<size_t>(256, 80 * 1024 / (sp.stride * sizeof(double2))) / 32 * 32;
   if (sp.cap < 32) return GGEM_OK;
@@ -1189,7 +1201,7 @@ int spread_separable(ggem_ctx *c, const SpreadGeo &sg, bool any_full, const doub
   }
   if (nf) {
     k_axis_factors<<<(unsigned)((nf + 255) / 256), 256, 0, c->stream>>>(
-        c->n, sg, sp, c->dc, c->q_ax[0].p, c->q_ax[1].p, c->q_ax[2].p, c->pos32.p, c->pos64.p,
+        c->n, sg, sp, c->dc, c->q_xyz.p, c->pos32.p, c->pos64.p,
         c->sp_fac.p);
     if (int rc = check_launch(c, "spread factors")) return rc;
   }
@@ -1269,66 +1281,25 @@ int quadrature_common(ggem_ctx *c, int nq) {
   return GGEM_OK;
 }
 
-// do the points form a tensor grid of at most 3 points per element along x?
-// The first element gives the indices (a point's coordinate among the
-// distinct ones of its axis), the elements along each axis the coordinates;
-// then every point of the mesh is compared.
-int quadrature_grid(ggem_ctx *c, int nq) {
-  const Grid &g = c->grid;
-  double q0[96];
-  cudaError_t e = cudaMemcpyAsync(q0, c->q_xyz.p, sizeof(double) * 3 * nq, cudaMemcpyDeviceToHost,
-                                  c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e) return cuda_fail(c, e, "quadrature");
-  AxisMap m;
-  int p[3];
-  for (int d = 0; d < 3; ++d) {
-    p[d] = 0;
-    for (int k = 0; k < nq; ++k) {
-      int a = 0;
-      while (a < p[d] && q0[3 * m.rep[d][a] + d] != q0[3 * k + d]) ++a;
-      if (a == p[d]) m.rep[d][p[d]++] = (signed char)k;
-      m.idx[d][k] = (signed char)a;
-    }
-  }
-  if (p[0] > 3 || p[0] * p[1] * p[2] != nq) return GGEM_OK;
-  for (int k = 0; k < nq; ++k) c->q_map[k] = -1;
-  for (int k = 0; k < nq; ++k)
-    c->q_map[(m.idx[2][k] * p[1] + m.idx[1][k]) * p[0] + m.idx[0][k]] = (signed char)k;
-  for (int k = 0; k < nq; ++k)
-    if (c->q_map[k] < 0) return GGEM_OK;  // a point twice, another missing
-  int64_t stride = 1;
-  for (int d = 0; d < 3; ++d) {
-    if ((e = c->q_ax[d].ensure((size_t)g.nc[d] * p[d]))) return cuda_fail(c, e, "quadrature axes");
-    k_axis_table<<<(g.nc[d] * p[d] + 255) / 256, 256, 0, c->stream>>>(
-        d, g.nc[d], stride, nq, p[d], m, c->q_xyz.p, c->q_ax[d].p);
-    if (int rc = check_launch(c, "quadrature axes")) return rc;
-    stride *= g.nc[d];
-    c->q_p[d] = p[d];
-  }
-  if ((e = c->q_flag.ensure(1)) ||
-      (e = cudaMemsetAsync(c->q_flag.p, 0, sizeof(int), c->stream)))
-    return cuda_fail(c, e, "quadrature flag");
-  const int64_t nqt = g.ncell * nq;
-  k_check_grid<<<(unsigned)((nqt + 255) / 256), 256, 0, c->stream>>>(
-      nqt, nq, g, p[0], p[1], p[2], m, c->q_xyz.p, c->q_ax[0].p, c->q_ax[1].p, c->q_ax[2].p,
-      c->q_flag.p);
-  if (int rc = check_launch(c, "quadrature grid")) return rc;
-  int flag = 1;
-  e = cudaMemcpyAsync(&flag, c->q_flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e) return cuda_fail(c, e, "quadrature");
-  c->q_grid = flag == 0;
-  return GGEM_OK;
-}
-
 int quadrature_finish(ggem_ctx *c, int nq) {
   const int64_t nqt = c->grid.ncell * nq;
-  k_qp_rel<<<(unsigned)((nqt + 255) / 256), 256, 0, c->stream>>>(nqt, nq, c->grid, c->q_xyz.p,
+  AxisMap *m = reinterpret_cast<AxisMap *>(c->h_red);
+  m->off = 0;
+  k_qp_rel<<<(unsigned)((nqt + 255) / 256), 256, 0, c->stream>>>(nqt, nq, c->grid, c->q_xyz.p, m,
                                                                  c->q_rel.p);
   if (int rc = check_launch(c, "quadrature")) return rc;
-  if (int rc = quadrature_grid(c, nq)) return rc;  // waits for the device
+  if (cudaError_t e = cudaStreamSynchronize(c->stream)) return cuda_fail(c, e, "quadrature");
   c->q_per_elem = nq;
+  // a tensor grid of at most 3 points per element along x?
+  if (m->off || m->p[0] > 3 || m->p[0] * m->p[1] * m->p[2] != nq) return GGEM_OK;
+  for (int k = 0; k < nq; ++k) c->q_map[k] = -1;
+  for (int k = 0; k < nq; ++k)
+    c->q_map[(m->idx[2][k] * m->p[1] + m->idx[1][k]) * m->p[0] + m->idx[0][k]] = (signed char)k;
+  for (int k = 0; k < nq; ++k)
+    if (c->q_map[k] < 0) return GGEM_OK;  // a point twice, another missing
+  for (int d = 0; d < 3; ++d) c->q_p[d] = m->p[d];
+  std::memcpy(c->q_rep, m->rep, sizeof(c->q_rep));
+  c->q_grid = true;
   return GGEM_OK;
 }
 
