@@ -142,7 +142,8 @@ __device__ __forceinline__ int axis_offset(const SpreadGeo &sg, int d, int us, i
 //
 // The FP32 form is bound by instruction issue (81%) and shared-memory data
 // (66% of its cycles): 144^3 elements x 8 points, N = 200k took 4.09 G warp
-// instructions and 3.90 ms, now 3.68 G and 3.72 ms.  Two members of a lane
+// instructions and 3.90 ms, then 3.68 G and 3.72 ms, and 3.53 ms with the four
+// lanes per point known when compiling (LQ).  Two members of a lane
 // share packed arithmetic up to the block sums, their positions and forces
 // staged together (6 words a member instead of a position and a gathered
 // record, 8); a point's four lanes reduce-scatter, so each converts and
@@ -152,7 +153,8 @@ __device__ __forceinline__ int axis_offset(const SpreadGeo &sg, int d, int us, i
 // point (a shuffle) or 32 (one member).  N = 20k, us with one member
 // at a time -> two: 27 points 923 -> 694, 12 points 632 -> 521, 4 points 433
 // -> 424, 2 points 405 -> 398.
-template <bool F32, bool ANYFULL, bool PAD>
+// LQ: the lanes per point, 4 or, read from sg, any (0)
+template <bool F32, bool ANYFULL, bool PAD, int LQ>
 __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
     SpreadGeo sg, DevConsts K, const int32_t *__restrict__ start,
     const float4 *__restrict__ pos32, const double4_32a *__restrict__ pos64,
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
   // elements of this brick, one warp at a time
   const int ebx = e1[0] - e0[0], eby = e1[1] - e0[1], ebz = e1[2] - e0[2];
   const int nel = ebx * eby * ebz;
-  const int nq = sg.nq, lq = sg.lq;
+  const int nq = sg.nq, lq = LQ ? LQ : sg.lq;
   const int qi = lane / lq, sub = lane - qi * lq;
   const int llq = 31 - __clz(lq);
   unsigned long long my_pairs = 0;
@@ -527,11 +529,16 @@ __global__ void __launch_bounds__(kSpThreads, F32 ? 4 : 1) k_spread_brick(
             // compensated sums at a time (every earlier batch was full)
             const float4 *o = reinterpret_cast<const float4 *>(mb) + 3 * sub;
             const int cnt = (m - sub + lq - 1) >> llq, step = 3 * lq;
-            if (lq == 4 && m == 32) {
+            if (LQ == 4) {
+              if (m == 32) {
 #pragma unroll
-              for (int t = 0; t < 4; ++t) pair32(o + 12 * t);
-              flush32();
-            } else if (lq <= 4) {
+                for (int t = 0; t < 4; ++t) pair32(o + 12 * t);
+                flush32();
+              } else {
+                for (int t = 0; 8 * t < m; ++t) pair32(o + 12 * t);
+                if (cnt == 8) flush32();
+              }
+            } else if (lq < 4) {
               int t = 0;
               for (; 2 * t + 8 <= cnt; t += 4, o += 4 * step) {
 #pragma unroll
@@ -1255,14 +1262,18 @@ int spread_elements(ggem_ctx *c, int precision, const double *d_f_slot, double *
     return GGEM_OK;
   };
   int rc;
-  if (precision == GGEM_FP32)
-    rc = any_full   ? launch(k_spread_brick<true, true, false>)
-         : sg.pad   ? launch(k_spread_brick<true, false, true>)
-                    : launch(k_spread_brick<true, false, false>);
+  if (precision == GGEM_FP64)
+    rc = any_full   ? launch(k_spread_brick<false, true, false, 0>)
+         : sg.pad   ? launch(k_spread_brick<false, false, true, 0>)
+                    : launch(k_spread_brick<false, false, false, 0>);
+  else if (sg.lq == 4)
+    rc = any_full   ? launch(k_spread_brick<true, true, false, 4>)
+         : sg.pad   ? launch(k_spread_brick<true, false, true, 4>)
+                    : launch(k_spread_brick<true, false, false, 4>);
   else
-    rc = any_full   ? launch(k_spread_brick<false, true, false>)
-         : sg.pad   ? launch(k_spread_brick<false, false, true>)
-                    : launch(k_spread_brick<false, false, false>);
+    rc = any_full   ? launch(k_spread_brick<true, true, false, 0>)
+         : sg.pad   ? launch(k_spread_brick<true, false, true, 0>)
+                    : launch(k_spread_brick<true, false, false, 0>);
   if (rc) return rc;
   return check_launch(c, "spread bricks");
 }
