@@ -574,6 +574,7 @@ struct ggem_ensemble {
   DevBuf<double4_32a> wrapped, pos64;
   DevBuf<float4> pos32;
   DevBuf<double> xyz;
+  DevBuf<unsigned long long> hist;  // pair distances (intervals)
   DevBuf<unsigned long long> stat;  // [0] entries, [1] longest row, [2] error word
   int64_t ncell = 0;
   bool counters_zero = false;
@@ -1543,12 +1544,31 @@ extern "C" int ggem_ensemble_intervals(ggem_ensemble *e, ggem_surrogate *s,
   if (!e->built) return efail(e, GGEM_ERR_BAD_ARG, "set the ensemble's particles first");
   EnsGuard g(e->device);
   std::vector<float> X((size_t)e->K * GGEM_SUR_FEATURES), Y((size_t)e->K * GGEM_SUR_OUTPUTS);
-  for (int b = 0; b < e->K; ++b) {
-    if (int rc = ensure_sub(e, b)) return rc;
-    if (int rc = ggem_surrogate_features(e->sub[b], chain_fraction ? chain_fraction[b] : 0.0,
-                                         X.data() + (size_t)b * GGEM_SUR_FEATURES))
-      return efail(e, rc, e->sub[b]->last_error);
-  }
+  // the histograms of all suspensions from their concatenated rows
+  const size_t nh = (size_t)e->K * GGEM_SUR_HIST_BINS;
+  std::vector<unsigned long long> hist(nh);
+  BatchBuild B;
+  B.K = e->K;
+  B.W = e->W;
+  B.geo = e->geo.p;
+  B.pos32 = e->pos32.p;
+  B.cnt = e->cnt.p;
+  B.list = e->list.p;
+  cudaError_t c;
+  if ((c = e->hist.ensure(nh)) ||
+      (c = cudaMemsetAsync(e->hist.p, 0, sizeof(unsigned long long) * nh, e->stream)))
+    return ecuda(e, c, "ensemble histograms");
+  batch_hist(B, e->d_off.p, *std::max_element(e->n.begin(), e->n.end()), e->sub[0], e->hist.p,
+             e->stream);
+  if (int rc = elaunch(e, "ensemble histograms")) return rc;
+  if ((c = cudaMemcpyAsync(hist.data(), e->hist.p, sizeof(unsigned long long) * nh,
+                           cudaMemcpyDeviceToHost, e->stream)) ||
+      (c = cudaStreamSynchronize(e->stream)))
+    return ecuda(e, c, "ensemble histograms");
+  for (int b = 0; b < e->K; ++b)
+    hist_features(e->sub[b], e->n[b], hist.data() + (size_t)b * GGEM_SUR_HIST_BINS,
+                  chain_fraction ? chain_fraction[b] : 0.0,
+                  X.data() + (size_t)b * GGEM_SUR_FEATURES);
   // one batched forward pass for all suspensions
   if (int rc = ggem_surrogate_predict(s, X.data(), e->K, Y.data()))
     return efail(e, rc, ggem_surrogate_last_error(s));

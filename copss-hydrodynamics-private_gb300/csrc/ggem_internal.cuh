@@ -435,6 +435,12 @@ void batch_susp(const BatchBuild &b, const int64_t *off, int32_t *susp, cudaStre
 void batch_cells(const BatchBuild &b, const double *xyz, const int64_t *off, cudaStream_t st);
 void batch_list(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st);
 void batch_tensors(const BatchBuild &b, const ggem_ctx *like, cudaStream_t st);
+// the pair-distance histograms of the K suspensions ([K][GGEM_SUR_HIST_BINS],
+// zeroed by the caller) and the network's features from one (ggem_surrogate.cu)
+void batch_hist(const BatchBuild &b, const int64_t *off, int64_t nmax, const ggem_ctx *like,
+                unsigned long long *hist, cudaStream_t st);
+void hist_features(const ggem_ctx *c, int64_t n, const unsigned long long *hist,
+                   double chain_fraction, float *features);
 
 // pair sums (ggem_pair.cu); vectors in slot order, [r][slot][3] doubles
 int matvec_slots(ggem_ctx *c, int nrhs, const double *d_f_slot, double *d_u_slot,

@@ -775,15 +775,18 @@ __global__ void k_to_bf16_pair(int64_t count, const float *__restrict__ p, int i
 namespace ggem {
 namespace sur {
 
-__global__ void k_pair_hist(int64_t n, const float4 *__restrict__ pos32,
-                            const int32_t *__restrict__ cnt, int W,
-                            const uint32_t *__restrict__ list, const float4 *__restrict__ shift,
-                            float r_lo, float inv_dr, int nb, unsigned long long *__restrict__ hist) {
-  __shared__ unsigned int sh[GGEM_SUR_HIST_BINS];
-  if (threadIdx.x < GGEM_SUR_HIST_BINS) sh[threadIdx.x] = 0u;
+// the pair distances of the rows s0, s0 + step, ... below s1 into hist
+__device__ __forceinline__ void hist_rows(int64_t s0, int64_t s1, int64_t step,
+                                          const float4 *__restrict__ pos32,
+                                          const int32_t *__restrict__ cnt, int W,
+                                          const uint32_t *__restrict__ list,
+                                          const float4 *__restrict__ shift, float r_lo,
+                                          float inv_dr, unsigned long long *__restrict__ hist) {
+  constexpr int nb = GGEM_SUR_HIST_BINS;
+  __shared__ unsigned int sh[nb];
+  if (threadIdx.x < nb) sh[threadIdx.x] = 0u;
   __syncthreads();
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n;
-       s += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t s = s0; s < s1; s += step) {
     const float4 pi = pos32[s];
     const int e = cnt[s];
     for (int m = 0; m < e; ++m) {
@@ -797,7 +800,57 @@ __global__ void k_pair_hist(int64_t n, const float4 *__restrict__ pos32,
     }
   }
   __syncthreads();
-  if (threadIdx.x < nb && sh[threadIdx.x]) atomicAdd(&hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
+  if (threadIdx.x < nb && sh[threadIdx.x])
+    atomicAdd(&hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
+}
+
+__global__ void k_pair_hist(int64_t n, const float4 *__restrict__ pos32,
+                            const int32_t *__restrict__ cnt, int W,
+                            const uint32_t *__restrict__ list, const float4 *__restrict__ shift,
+                            float r_lo, float inv_dr, unsigned long long *__restrict__ hist) {
+  hist_rows(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, n, (int64_t)gridDim.x * blockDim.x,
+            pos32, cnt, W, list, shift, r_lo, inv_dr, hist);
+}
+
+// blockIdx.y = suspension of an ensemble's concatenated rows
+__global__ void k_batch_hist(const BatchGeo *__restrict__ geo, const int64_t *__restrict__ off,
+                             const float4 *__restrict__ pos32, const int32_t *__restrict__ cnt,
+                             int W, const uint32_t *__restrict__ list, float r_lo, float inv_dr,
+                             unsigned long long *__restrict__ hist) {
+  const int b = blockIdx.y;
+  hist_rows(off[b] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x, off[b + 1],
+            (int64_t)gridDim.x * blockDim.x, pos32, cnt, W, list, geo[b].shift, r_lo, inv_dr,
+            hist + (int64_t)b * GGEM_SUR_HIST_BINS);
+}
+
+// bins of the distances from contact to the cut-off
+struct HistBins {
+  double lo, hi;
+  float inv_dr() const { return (float)(GGEM_SUR_HIST_BINS / (hi - lo)); }
+};
+
+HistBins hist_bins(const ggem_ctx *c) {
+  const double a = c->prm.br0 > 0 ? c->prm.br0 : 1.0;
+  return HistBins{2.0 * a, std::sqrt(c->rc2)};
+}
+
+// the network's inputs for n beads in the box of c
+void features_of(const ggem_ctx *c, int64_t n, const unsigned long long *hist,
+                 double chain_fraction, float *features) {
+  const double a = c->prm.br0 > 0 ? c->prm.br0 : 1.0;
+  const HistBins h = hist_bins(c);
+  const Grid &g = c->grid;
+  const double vol = g.L[0] * g.L[1] * g.L[2];
+  const double rho = vol > 0 ? (double)n / vol : 0.0;
+  features[0] = (float)(n * 4.0 / 3.0 * kPiS * a * a * a / (vol > 0 ? vol : 1.0));
+  features[1] = (float)std::log((double)std::max<int64_t>(n, 1));
+  const double dr = (h.hi - h.lo) / GGEM_SUR_HIST_BINS;
+  for (int b = 0; b < GGEM_SUR_HIST_BINS; ++b) {
+    const double r0 = h.lo + b * dr, r1 = r0 + dr;
+    const double ideal = n * rho * 4.0 / 3.0 * kPiS * (r1 * r1 * r1 - r0 * r0 * r0);
+    features[2 + b] = (float)(ideal > 0 ? hist[b] / ideal : 0.0);
+  }
+  features[2 + GGEM_SUR_HIST_BINS] = (float)chain_fraction;
 }
 
 constexpr int kWOff[kLayers] = {0, 128 * 48 + 128, 128 * 48 + 128 + 128 * 128 + 128,
@@ -1351,10 +1404,6 @@ extern "C" int ggem_surrogate_features(ggem_ctx *ctx, double chain_fraction, flo
   if (ctx->prm.precision != GGEM_FP32 || !ctx->list_built)
     return fail(ctx, GGEM_ERR_BAD_ARG, "features need the FP32 pair list (build cells first)");
   SurDeviceGuard dg(ctx->device);
-  const double a = ctx->prm.br0 > 0 ? ctx->prm.br0 : 1.0;
-  const double r_lo = 2.0 * a, r_hi = std::sqrt(ctx->rc2);
-  const Grid &g = ctx->grid;
-  const double vol = g.L[0] * g.L[1] * g.L[2];
   const int64_t n = ctx->n;
   std::vector<unsigned long long> hist(GGEM_SUR_HIST_BINS, 0ull);
   if (n > 0) {
@@ -1364,28 +1413,34 @@ extern "C" int ggem_surrogate_features(ggem_ctx *ctx, double chain_fraction, flo
         (e = cudaMemsetAsync(d_hist.p, 0, sizeof(unsigned long long) * GGEM_SUR_HIST_BINS,
                              ctx->stream)))
       return cuda_fail(ctx, e, "histogram");
-    const float inv_dr = (float)(GGEM_SUR_HIST_BINS / (r_hi - r_lo));
+    const HistBins h = hist_bins(ctx);
     const unsigned nblk = (unsigned)std::min<int64_t>((n + 255) / 256, 4096);
     k_pair_hist<<<nblk, 256, 0, ctx->stream>>>(n, ctx->pos32.p, ctx->nb_cnt.p, ctx->nb_w,
-                                               ctx->nb_list.p, ctx->d_shift.p, (float)r_lo,
-                                               inv_dr, GGEM_SUR_HIST_BINS, d_hist.p);
+                                               ctx->nb_list.p, ctx->d_shift.p, (float)h.lo,
+                                               h.inv_dr(), d_hist.p);
     if (int rc = check_launch(ctx, "histogram")) return rc;
     if ((e = cudaMemcpyAsync(hist.data(), d_hist.p, sizeof(unsigned long long) * GGEM_SUR_HIST_BINS,
                              cudaMemcpyDeviceToHost, ctx->stream)) ||
         (e = cudaStreamSynchronize(ctx->stream)))
       return cuda_fail(ctx, e, "histogram");
   }
-  const double rho = vol > 0 ? (double)n / vol : 0.0;
-  features[0] = (float)(n * 4.0 / 3.0 * kPiS * a * a * a / (vol > 0 ? vol : 1.0));
-  features[1] = (float)std::log((double)std::max<int64_t>(n, 1));
-  const double dr = (r_hi - r_lo) / GGEM_SUR_HIST_BINS;
-  for (int b = 0; b < GGEM_SUR_HIST_BINS; ++b) {
-    const double r0 = r_lo + b * dr, r1 = r0 + dr;
-    const double ideal = n * rho * 4.0 / 3.0 * kPiS * (r1 * r1 * r1 - r0 * r0 * r0);
-    features[2 + b] = (float)(ideal > 0 ? hist[b] / ideal : 0.0);
-  }
-  features[2 + GGEM_SUR_HIST_BINS] = (float)chain_fraction;
+  features_of(ctx, n, hist.data(), chain_fraction, features);
   return GGEM_OK;
+}
+
+// the histograms of an ensemble's suspensions (most beads in one: nmax) and
+// the features from one of them
+void ggem::batch_hist(const BatchBuild &b, const int64_t *off, int64_t nmax, const ggem_ctx *like,
+                      unsigned long long *hist, cudaStream_t st) {
+  const HistBins h = hist_bins(like);
+  const unsigned nblk = (unsigned)std::min<int64_t>((nmax + 255) / 256, 4096);
+  k_batch_hist<<<dim3(nblk, b.K), 256, 0, st>>>(b.geo, off, b.pos32, b.cnt, b.W, b.list,
+                                                (float)h.lo, h.inv_dr(), hist);
+}
+
+void ggem::hist_features(const ggem_ctx *c, int64_t n, const unsigned long long *hist,
+                         double chain_fraction, float *features) {
+  features_of(c, n, hist, chain_fraction, features);
 }
 
 extern "C" int ggem_surrogate_interval(ggem_ctx *ctx, ggem_surrogate *s, double chain_fraction,

@@ -360,3 +360,31 @@ def test_batched_build_equals_single_suspensions(cell_div):
         assert e.value.code == G.ERR_BAD_ARG
         u, _ = u_of(ens, moved)
         assert np.all(np.isfinite(u))
+
+
+@pytest.mark.parametrize("k", [1, 7])
+def test_ensemble_intervals_need_no_second_build(k):
+    """the intervals of an ensemble are those of its suspensions alone (the
+    same pair counts and network), from the lists that it has: no device
+    memory for a second set"""
+    import torch
+    sur = G.Surrogate(seed=3)
+    sus = _ensemble(k, 21, n_range=(8000, 20000))
+    n = np.array([len(x) for x, _ in sus])
+    frac = np.linspace(0.0, 1.0, k)
+    with G.Ensemble([L for _, L in sus]) as ens:
+        d_xyz = _device(np.concatenate([x for x, _ in sus]))
+        ens.set_particles_dev(n, d_xyz.data_ptr())
+        sur.predict(np.ones((k, G.SUR_FEATURES), np.float32))  # (the network's own buffers)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        lo, hi = ens.intervals(sur, frac, 0.1, 0.2)
+        assert free - torch.cuda.mem_get_info()[0] <= 4 << 20
+        assert ens.lanczos(0, 8, 1)[0] > 0  # (a context is still made where one is needed)
+    for b, (xyz, L) in enumerate(sus):
+        with G.Context(box_hi=(L,) * 3) as ctx:
+            ctx.set_particles(xyz)
+            ctx.build_cells()
+            want = ctx.surrogate_interval(sur, frac[b], 0.1, 0.2)
+        assert (lo[b], hi[b]) == want
+    sur.close()
