@@ -131,35 +131,37 @@ int build_reference_stencil(ggem_ctx *c) {
 }
 
 int upload_stencil(ggem_ctx *c) {
-  cudaError_t e = c->d_stencil.ensure(std::max<size_t>(1, c->stencil.size()));
+  std::vector<int4> up = c->stencil;
+  if (c->prm.nb_mode == GGEM_NB_REFERENCE) {
+    // behind it the stencil with its own element as runs (dy, dz, first dx,
+    // last dx): the particles of a run of elements along x are consecutive
+    // slots.  (build_reference_stencil goes along x, then y, then z)
+    auto add = [&](const int4 &o) {
+      if (c->n_runs > 0 && up.back().x == o.y && up.back().y == o.z && up.back().w + 1 == o.x) {
+        up.back().w = o.x;
+      } else {
+        up.push_back(make_int4(o.y, o.z, o.x, o.x));
+        ++c->n_runs;
+      }
+    };
+    c->n_runs = 0;
+    bool own = false;
+    for (const int4 &o : c->stencil) {
+      if (!own && (o.z > 0 || (o.z == 0 && (o.y > 0 || (o.y == 0 && o.x > 0))))) {
+        add(make_int4(0, 0, 0, 0));
+        own = true;
+      }
+      add(o);
+    }
+    if (!own) add(make_int4(0, 0, 0, 0));
+  }
+  cudaError_t e = c->d_stencil.ensure(std::max<size_t>(1, up.size()));
   if (e) return cuda_fail(c, e, "stencil");
-  if (!c->stencil.empty()) {
-    e = cudaMemcpy(c->d_stencil.p, c->stencil.data(), sizeof(int4) * c->stencil.size(),
-                   cudaMemcpyHostToDevice);
+  if (!up.empty()) {
+    e = cudaMemcpy(c->d_stencil.p, up.data(), sizeof(int4) * up.size(), cudaMemcpyHostToDevice);
     if (e) return cuda_fail(c, e, "stencil upload");
   }
-  if (c->prm.nb_mode == GGEM_NB_REFERENCE) {
-    // the stencil with its own element as runs (dy, dz, first dx, last dx):
-    // the particles of a run of elements along x are consecutive slots
-    std::vector<int4> st = c->stencil;
-    st.push_back(make_int4(0, 0, 0, 0));
-    std::sort(st.begin(), st.end(), [](const int4 &a, const int4 &b) {
-      return a.z != b.z ? a.z < b.z : (a.y != b.y ? a.y < b.y : a.x < b.x);
-    });
-    std::vector<int4> runs;
-    for (const int4 &o : st) {
-      if (!runs.empty() && runs.back().x == o.y && runs.back().y == o.z &&
-          runs.back().w + 1 == o.x)
-        runs.back().w = o.x;
-      else
-        runs.push_back(make_int4(o.y, o.z, o.x, o.x));
-    }
-    if ((e = c->d_runs.ensure(runs.size())) ||
-        (e = cudaMemcpy(c->d_runs.p, runs.data(), sizeof(int4) * runs.size(),
-                        cudaMemcpyHostToDevice)))
-      return cuda_fail(c, e, "stencil runs");
-    c->n_runs = (int)runs.size();
-  }
+  c->d_runs = c->d_stencil.p + c->stencil.size();
   if (c->prm.precision == GGEM_FP64) {
     // the largest r^2 of a listed pair: rc^2, or the far corners of the
     // stencil's elements
@@ -176,13 +178,7 @@ int upload_stencil(ggem_ctx *c) {
     // from alpha r = 28 on both coefficients are exactly zero, and so is the
     // last piece, which larger r read: a cut-off beyond the box adds no pieces
     s_max = std::min(s_max, 784.0 / c->cst.alpha2);
-    std::vector<double4_32a> rec;
-    fit_tensor_f64(c->cst, s_max * (1.0 + 1e-9), rec, &c->t64);
-    if ((e = c->tab64.ensure(rec.size())) ||
-        (e = cudaMemcpy(c->tab64.p, rec.data(), sizeof(double4_32a) * rec.size(),
-                        cudaMemcpyHostToDevice)))
-      return cuda_fail(c, e, "FP64 tensor");
-    c->t64.rec = c->tab64.p;
+    if (int rc = fit_tensor64(c, s_max * (1.0 + 1e-9))) return rc;
   }
   // FP32 cell shift per entry code (cut-off mode only: codes < kMaxCode)
   std::vector<float4> sh(kMaxCode, make_float4(0.f, 0.f, 0.f, 0.f));
@@ -395,7 +391,8 @@ extern "C" int ggem_create(const ggem_params *p, ggem_ctx **out) {
   int rc = validate_and_setup(c);
   if (rc == GGEM_OK) {
     if ((e = c->err.ensure(1)) || (e = cudaMemset(c->err.p, 0, sizeof(int))) ||
-        (e = cudaMallocHost((void **)&c->h_red, 4096 * sizeof(double))))
+        (e = cudaMallocHost((void **)&c->h_red, 4096 * sizeof(double))) ||
+        (e = cudaStreamSynchronize(c->stream)))  // (the FP64 tensor's pieces)
       rc = cuda_fail(c, e, "context buffers");
   }
   if (rc != GGEM_OK) {

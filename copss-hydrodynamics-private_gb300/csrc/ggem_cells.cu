@@ -1022,7 +1022,7 @@ int cell_flag_error(ggem_ctx *c, int flags) {
 void launch_pair_list(ggem_ctx *c, int nst, int W, cudaStream_t st) {
   if (c->prm.nb_mode == GGEM_NB_REFERENCE) {
     launch_dependent(k_run_list, dim3((unsigned)((c->n + kRunWarps - 1) / kRunWarps)), 32 * kRunWarps, 0, st,
-                   c->n, c->grid, c->d_runs.p, c->n_runs, c->cell_start.p, c->pos32.p, W, c->nb_cnt.p,
+                   c->n, c->grid, c->d_runs, c->n_runs, c->cell_start.p, c->pos32.p, W, c->nb_cnt.p,
         c->nb_list.p, c->nb_stat.p, c->err.p);
     return;
   }

@@ -142,99 +142,6 @@ int fit_tensor_table(const ggem_constants &c, double s_max, int nt, std::vector<
   return (worst < 1e-5) ? 0 : -1;
 }
 
-// A(s) and B(s) for the FP64 fit: the alternating series where ksi^2 s is
-// small (the closed form cancels there), otherwise the closed form with the
-// difference of the two erf as a difference of erfc (both small at large r)
-static void tensor_ab64(const ggem_constants &c, double s, double *A, double *B) {
-  const double k = c.one_eight_pi_mu;
-  if (c.ksi2 * s < 0.25) {
-    double sp = 0.0, sm = 0.0, kp = c.ksi, ap = c.alpha, w = 1.0, wm = 1.0 / s;
-    for (int n = 0; n < 16; ++n) {  // 0.25^16 / 16! is far below 2^-53
-      const double d = (kp - ap) * w;
-      sp += d * (1.0 / (2.0 * n + 1.0) + 1.0);
-      if (n > 0) sm += (kp - ap) * wm * (1.0 / (2.0 * n + 1.0) - 1.0);
-      kp *= c.ksi2;
-      ap *= c.alpha2;
-      w *= -s / (n + 1.0);
-      wm = n == 0 ? -1.0 : wm * (-s / (n + 1.0));
-    }
-    const double two_sqrt_pi = 2.0 / std::sqrt(kPi);
-    *A = k * two_sqrt_pi * sp;
-    *B = k * two_sqrt_pi * sm;
-    return;
-  }
-  const double r = std::sqrt(s);
-  const double kr = c.ksi * r, ar = c.alpha * r;
-  const double c1 = (ar > 0.5 ? std::erfc(ar) - std::erfc(kr) : std::erf(kr) - std::erf(ar)) / r;
-  const double c2 = c.two_ksi_sqrt_pi * std::exp(-c.ksi2 * s) -
-                    c.two_alpha_sqrt_pi * std::exp(-c.alpha2 * s);
-  *A = k * (c1 + c2);
-  *B = k * (c1 - c2) / s;
-}
-
-// Chebyshev interpolants at 12 points of every piece, cut at degree 5 (the
-// oversampling averages the rounding of the samples).  The first piece ends
-// where ksi^2 s = 2^-6 at most; with 2^7 pieces per octave above it the
-// dropped terms stay below 2e-17 of A(0): the functions vary on the scale
-// 1 / alpha^2 and 1 / ksi^2 of s and, beyond it, algebraically.
-void fit_tensor_f64(const ggem_constants &c, double s_max, std::vector<double4_32a> &rec,
-                    Tensor64 *t) {
-  constexpr int M = 12, D = kTab64Deg;
-  static_assert(D == 5, "record layout");
-  const int e0 = (int)std::floor(std::log2(0.0168 / c.ksi2));
-  const double s0 = std::ldexp(1.0, e0);
-  const int sub = 1 << kTab64Sub;
-  int np = 1;  // up to the piece that holds s_max
-  if (s_max > s0) {
-    const int oct = (int)std::floor(std::log2(s_max / s0));
-    np += oct * sub + std::min(sub, 1 + (int)((std::ldexp(s_max / s0, -oct) - 1.0) * sub));
-  }
-  rec.assign((size_t)3 * np, double4_32a{0.0, 0.0, 0.0, 0.0});
-  double node[M], T[M][D + 1];
-  for (int j = 0; j < M; ++j) {
-    node[j] = std::cos(kPi * (j + 0.5) / M);
-    for (int q = 0; q <= D; ++q) T[j][q] = std::cos(q * kPi * (j + 0.5) / M);
-  }
-  for (int i = 0; i < np; ++i) {
-    double mid, half;
-    if (i == 0) {
-      mid = half = 0.5 * s0;
-    } else {
-      const double lo = std::ldexp(s0, (i - 1) / sub);
-      half = 0.5 * lo / sub;
-      mid = lo + (2 * ((i - 1) % sub) + 1) * half;
-    }
-    double ch[2][D + 1] = {};
-    for (int j = 0; j < M; ++j) {
-      double v[2];
-      tensor_ab64(c, mid + half * node[j], &v[0], &v[1]);
-      for (int w = 0; w < 2; ++w)
-        for (int q = 0; q <= D; ++q) ch[w][q] += v[w] * T[j][q] * (q ? 2.0 : 1.0) / M;
-    }
-    // T_0 .. T_5 as monomials, smallest contributions first
-    double m[2][D + 1];
-    for (int w = 0; w < 2; ++w) {
-      const double *a = ch[w];
-      m[w][0] = (a[4] - a[2]) + a[0];
-      m[w][1] = (5.0 * a[5] - 3.0 * a[3]) + a[1];
-      m[w][2] = -8.0 * a[4] + 2.0 * a[2];
-      m[w][3] = -20.0 * a[5] + 4.0 * a[3];
-      m[w][4] = 8.0 * a[4];
-      m[w][5] = 16.0 * a[5];
-      double sc = 1.0;
-      for (int q = 0; q <= D; ++q, sc /= half) m[w][q] *= sc;
-    }
-    for (int q = 0; q < 3; ++q)
-      rec[3 * (size_t)i + q] = double4_32a{m[0][2 * q], m[1][2 * q], m[0][2 * q + 1],
-                                           m[1][2 * q + 1]};
-  }
-  uint64_t bits;
-  std::memcpy(&bits, &s0, sizeof bits);
-  t->base = (int)(bits >> (52 - kTab64Sub)) - 1;
-  t->last = np - 1;
-  t->mid0 = 0.5 * s0;
-}
-
 // Analytic form of the FP32 tensor: A(s) = e^{-alpha^2 s} a(s) and
 // B(s) = e^{-alpha^2 s} b(s).  a and b are entire in s (the 1/r singularities
 // of the two erf terms cancel), so one Chebyshev interpolant of degree

@@ -150,7 +150,7 @@ struct ggem_ctx {
   bool f64_list_exact = true;  // the list's FP32 filter is sound in this box (ggem_api.cu)
   // the list is the FP64 path's own (default mode), not one the caller asked for
   bool f64_list_is_own() const { return prm.precision == GGEM_FP64 && f64_list != 1; }
-  ggem::DevBuf<int4> d_runs;  // reference mode: the stencil's runs along x
+  const int4 *d_runs = nullptr;  // reference mode: the stencil's runs along x (in d_stencil)
   int n_runs = 0;
   ggem::DevBuf<double4_32a> tab64;
   ggem::Tensor64 t64{};
@@ -372,10 +372,8 @@ int fit_tensor_table(const ggem_constants &c, double s_max, int nt, std::vector<
                      double *max_err);
 int fit_tensor_poly(const ggem_constants &c, double s_max, float *a, float *b, float *x0,
                     float *x1, float *e_coef, double *max_err);
-// the FP64 piecewise tensor for s in [0, s_max] (records of three double4_32a
-// per piece); base, last and mid0 of *t are set, rec is the caller's
-void fit_tensor_f64(const ggem_constants &c, double s_max, std::vector<double4_32a> &rec,
-                    Tensor64 *t);
+// the FP64 piecewise tensor of c for s in [0, s_max] (ggem_pair.cu)
+int fit_tensor64(ggem_ctx *c, double s_max);
 bool tensor_b_nonnegative(const ggem_constants &c, double s_max);
 void tridiag_extremes(int k, const double *a, const double *b, double *lmin, double *lmax);
 void cheb_coeffs_host(int N, double da, double db, int method, double *coef);
