@@ -2899,11 +2899,13 @@ extern "C" int ggem_autotune_pair_storage(ggem_ctx *ctx, int reps, double matvec
   cudaEventCreate(&b);
   const bool timing = ctx->timing;
   ctx->timing = false;
-  auto time_matvecs = [&](double *ms) -> int {
+  auto time_matvecs = [&](double *ms, bool first = false) -> int {
     if (int rc = matvec_slots(ctx, 1, ctx->w_in.p, ctx->w_out.p, GGEM_SELF_BEAD)) return rc;
     cudaEventRecord(a, ctx->stream);
-    for (int r = 0; r < reps; ++r)
+    for (int r = 0; r < reps; ++r) {
+      if (first) ctx->pretensor_pending = n > 0;
       if (int rc = matvec_slots(ctx, 1, ctx->w_in.p, ctx->w_out.p, GGEM_SELF_BEAD)) return rc;
+    }
     cudaEventRecord(b, ctx->stream);
     cudaEventSynchronize(b);
     float t = 0.f;
@@ -2932,28 +2934,24 @@ extern "C" int ggem_autotune_pair_storage(ggem_ctx *ctx, int reps, double matvec
   }
   if (!rc && ctx->use_pretensor) {
     ctx->allow_pretensor = true;
-    cudaEventRecord(a, ctx->stream);
     rc = build_pair_tensors(ctx);
-    if (!rc) rc = form_pair_tensors(ctx);
-    cudaEventRecord(b, ctx->stream);
-    cudaEventSynchronize(b);
-    float t_pass = 0.f;
-    cudaEventElapsedTime(&t_pass, a, b);
     if (!rc && ctx->pretensor_ok) {
-      // every stored-tensor kernel shape; the fastest stays selected
+      // every stored-tensor kernel shape, its first product over a list (which
+      // forms the tensors, in its own kernel or before it) spread over the
+      // products per build; the fastest stays selected
       int best_v = 0;
-      double best_mv = 1e30;
       for (int v = 0; v < kNumStoredVariants && !rc; ++v) {
         ctx->stored_variant = v;
-        double t_mv = 0.0;
+        double t_mv = 0.0, t_first = 0.0;
         rc = time_matvecs(&t_mv);
-        if (!rc && t_mv < best_mv) {
-          best_mv = t_mv;
+        if (!rc) rc = time_matvecs(&t_first, true);
+        const double t = t_mv + std::max(0.0, t_first - t_mv) / matvecs_per_build;
+        if (!rc && t < t_store) {
+          t_store = t;
           best_v = v;
         }
       }
       ctx->stored_variant = best_v;
-      t_store = best_mv + t_pass / matvecs_per_build;
     }
   }
   cudaEventDestroy(a);

@@ -58,13 +58,13 @@ int ggem_set_fp64_pair_list(ggem_ctx *ctx, int enable);
 int ggem_set_symmetric_pairs(ggem_ctx *ctx, int enable);
 /* autotune the pair storage on the current configuration (cells and list
  * built, FP32): times `reps` single-RHS matvecs with tensors evaluated per
- * pair and with stored tensors (plus the one tensor pass per build,
- * amortised over matvecs_per_build matvecs) by CUDA events on the context's
- * stream; each form is timed for each of its kernel shapes (per-matvec
+ * pair and with stored tensors (the first product over a list, which forms
+ * them, amortised over matvecs_per_build matvecs) by CUDA events on the
+ * context's stream; each form is timed for each of its kernel shapes (per-matvec
  * tensors: registers capped for 6 or for 5 blocks of 256 per SM; stored
  * tensors: lanes per target, entries in flight, pipelined stream).  The
  * fastest stays selected for this context; both costs are reported in ms
- * per matvec (the stored one with its amortised pass) and variants[0],
+ * per matvec (the stored one with its amortised first product) and variants[0],
  * variants[1] receive the chosen computed and stored shapes */
 int ggem_autotune_pair_storage(ggem_ctx *ctx, int reps, double matvecs_per_build,
                                int *use_stored, double *ms_computed, double *ms_stored,
