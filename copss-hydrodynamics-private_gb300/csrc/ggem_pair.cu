@@ -91,8 +91,20 @@ __device__ __forceinline__ void min_image3(const MinImage &mi, double &x, double
   }
 }
 
-// one 256-bit read-only load
+// one 256-bit read-only load of what an earlier kernel wrote: volatile and
+// with a memory clobber, so that it stays behind wait_prior_grid
 __device__ __forceinline__ double4_32a ld_f64x4(const double4_32a *p) {
+  double4_32a v;
+  asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
+// the same of the tensor's pieces, written once before any product: the
+// compiler may move it anywhere
+__device__ __forceinline__ double4_32a ld_piece(const double4_32a *p) {
   double4_32a v;
   asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
       : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
@@ -109,7 +121,7 @@ __device__ __forceinline__ void tensor64(const Tensor64 &T, double s, long long 
   const int hi = __double2hiint(s);
   const int idx = min(max((hi >> (20 - kTab64Sub)) - T.base, 0), T.last);
   const double4_32a *r = T.rec + 3 * idx;
-  const double4_32a r2 = ld_f64x4(r + 2), r1 = ld_f64x4(r + 1), r0 = ld_f64x4(r);
+  const double4_32a r2 = ld_piece(r + 2), r1 = ld_piece(r + 1), r0 = ld_piece(r);
   constexpr int low = (1 << (20 - kTab64Sub)) - 1;
   const double mid = __hiloint2double((hi & ~low) | ((low + 1) >> 1), 0);
   const double t = s - (idx == 0 ? T.mid0 : mid);
@@ -915,10 +927,11 @@ __device__ __forceinline__ float ex2_sfu(float x) {
 // warp touches each sector once instead of twice
 __device__ __forceinline__ Rec32 ld_rec32(const Rec32 *p) {
   Rec32 r;
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y),
-        "=f"(r.b.z), "=f"(r.b.w)
-      : "l"(p));
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y),
+                 "=f"(r.b.z), "=f"(r.b.w)
+               : "l"(p)
+               : "memory");
   return r;
 }
 
