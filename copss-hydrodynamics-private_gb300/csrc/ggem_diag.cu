@@ -163,6 +163,12 @@ extern "C" int ggem_get_pair_storage(const ggem_ctx *ctx, int *row_width, int *t
   return GGEM_OK;
 }
 
+extern "C" int ggem_set_series_polls(ggem_ctx *ctx, uint32_t polls) {
+  if (!ctx) return GGEM_ERR_BAD_ARG;
+  ctx->series_polls = polls ? polls : 1u << 26;
+  return GGEM_OK;
+}
+
 extern "C" int ggem_set_fp64_pair_list(ggem_ctx *ctx, int enable) {
   if (!ctx) return GGEM_ERR_BAD_ARG;
   if (ctx->prm.precision != GGEM_FP64 || ctx->prm.nb_mode != GGEM_NB_CUTOFF)

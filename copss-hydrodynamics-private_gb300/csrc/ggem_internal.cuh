@@ -236,6 +236,7 @@ struct ggem_ctx {
   ggem::DevBuf<float> w_fb2;    // the next term's staging in a fused batched series
   ggem::DevBuf<double> w_red;   // reduction partials
   // the one-launch FP64 series: control block and coefficients; its vectors
+  uint32_t series_polls = 1u << 26;  // of each of its waits (ggem_set_series_polls)
   ggem::DevBuf<double> s64_tab;
   ggem::DevBuf<double4_32a> s64_vec;
   ggem::DevBuf<double> lz_Q;    // Lanczos basis

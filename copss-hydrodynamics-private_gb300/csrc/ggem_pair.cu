@@ -2714,7 +2714,7 @@ int series_f64(ggem_ctx *c, int N, const double *coef, double da, double db, dou
   a.check_every = check_every;
   a.k_first = k_first;
   a.out_y = out_y ? 1 : 0;
-  a.polls = 1u << 26;
+  a.polls = c->series_polls;
   a.da = da;
   a.db = db;
   a.tol = tol;

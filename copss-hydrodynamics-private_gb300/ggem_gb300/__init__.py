@@ -124,6 +124,7 @@ def lib():
         "ggem_get_pair_storage": (i, [vp, P(i), P(i)]),
         "ggem_set_pair_tensors": (i, [vp, i]),
         "ggem_set_fp64_pair_list": (i, [vp, i]),
+        "ggem_set_series_polls": (i, [vp, C.c_uint32]),
         "ggem_set_symmetric_pairs": (i, [vp, i]),
         "ggem_autotune_pair_storage": (i, [vp, i, d, P(i), P(d), P(d), P(i)]),
         "ggem_set_pair_variant": (i, [vp, i, i]),
@@ -628,6 +629,11 @@ class Context:
     def set_fp64_pair_list(self, enable: bool):
         """FP64 cutoff contexts: walk the exact pair list instead of the cells"""
         self._check(lib().ggem_set_fp64_pair_list(self.h, 1 if enable else 0))
+
+    def set_series_polls(self, polls):
+        """test hook: polls of each wait of the one-launch FP64 series (0 =
+        the default)"""
+        self._check(lib().ggem_set_series_polls(self.h, int(polls)))
 
     def set_symmetric_pairs(self, enable: bool):
         """FP32 cutoff contexts: evaluate each unordered pair once (half list)"""

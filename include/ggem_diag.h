@@ -49,6 +49,9 @@ int ggem_set_pair_tensors(ggem_ctx *ctx, int enable);
  * configurations that the operator is applied to, where it takes at most a
  * quarter of the free device memory. */
 int ggem_set_fp64_pair_list(ggem_ctx *ctx, int enable);
+/* test hook: polls of each wait of the one-launch FP64 series (0 = the
+ * default); a wait that runs out ends the series with GGEM_ERR_TIMEOUT */
+int ggem_set_series_polls(ggem_ctx *ctx, uint32_t polls);
 /* GGEM_FP32 cutoff contexts: 1 = single-RHS matvecs with tensors evaluated
  * per pair use the symmetry G_ij = G_ji: the list build also writes the
  * half list, each unordered pair is evaluated once and its source side added

@@ -194,3 +194,20 @@ def test_tensor_core_wait_timeout_is_reported_and_recovers():
     loss_o, _ = M.loss_and_grad(sur.params, sur.norm, X, Y)
     assert loss == pytest.approx(loss_o, rel=1e-4)
     sur.close()
+
+
+@pytest.mark.parametrize("n", [1, 300, 4000])
+def test_training_wait_timeout(n):
+    """the training pass and the gradients under a zero poll budget: the waits
+    give up, the products in flight complete, TMEM is freed, the call reports
+    GGEM_ERR_TIMEOUT, and the next gradient is the same as before"""
+    sur, X, Y = _random_net(7, n)
+    want = sur.gradient(X, Y)
+    sur.set_poll_budget(0)
+    with pytest.raises(G.GGEMError) as e:
+        sur.gradient(X, Y)
+    assert e.value.code == G.ERR_TIMEOUT
+    sur.set_poll_budget(1 << 22)
+    got = sur.gradient(X, Y)
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
+    sur.close()
