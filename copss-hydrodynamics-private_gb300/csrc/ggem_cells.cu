@@ -347,11 +347,9 @@ __device__ __forceinline__ void gather_one(int64_t s, const Grid &g,
                                            const int32_t *__restrict__ order,
                                            const int32_t *__restrict__ cell_of,
                                            const double4_32a *__restrict__ wrapped,
-                                           int32_t *__restrict__ rank,
                                            double4_32a *__restrict__ pos64,
                                            float4 *__restrict__ pos32) {
   const int32_t i = order[s];
-  rank[i] = (int32_t)s;
   const double4_32a p = wrapped[i];
   pos64[s] = p;
   const int32_t cid = cell_of[i];
@@ -371,7 +369,9 @@ __global__ void k_gather_sorted(int64_t n, Grid g, const int32_t *__restrict__ o
                                 float4 *__restrict__ pos32) {
   wait_prior_grid();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s < n) gather_one(s, g, order, cell_of, wrapped, rank, pos64, pos32);
+  if (s >= n) return;
+  rank[order[s]] = (int32_t)s;
+  gather_one(s, g, order, cell_of, wrapped, pos64, pos32);
 }
 
 // neighbour cell of cell coordinate (cx,cy,cz) shifted by o; -1 if outside a
@@ -799,11 +799,10 @@ __global__ void k_batch_gather(int64_t ntot, const BatchGeo *__restrict__ geo,
                                const int32_t *__restrict__ order,
                                const int32_t *__restrict__ cell_of,
                                const double4_32a *__restrict__ wrapped,
-                               int32_t *__restrict__ rank, double4_32a *__restrict__ pos64,
-                               float4 *__restrict__ pos32) {
+                               double4_32a *__restrict__ pos64, float4 *__restrict__ pos32) {
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= ntot) return;
-  gather_one(s, geo[susp[s]].g, order, cell_of, wrapped, rank, pos64, pos32);
+  gather_one(s, geo[susp[s]].g, order, cell_of, wrapped, pos64, pos32);
 }
 
 __global__ void __launch_bounds__(32, 32) k_batch_list(
@@ -1191,7 +1190,7 @@ void batch_cells(const BatchBuild &b, const double *xyz, const int64_t *off, cud
                                       b.order);
   k_sort_cells<<<(unsigned)((b.ncell + 255) / 256), 256, 0, st>>>(b.ncell, b.cell_start, b.order,
                                                                    b.cell_fill);
-  k_batch_gather<<<bn, 256, 0, st>>>(b.ntot, b.geo, b.susp, b.order, b.cell_of, b.wrapped, b.rank,
+  k_batch_gather<<<bn, 256, 0, st>>>(b.ntot, b.geo, b.susp, b.order, b.cell_of, b.wrapped,
                                      b.pos64, b.pos32);
 }
 

@@ -34,7 +34,6 @@ namespace ens {
 
 constexpr int kR = GGEM_ENSEMBLE_MAX_RHS;  // right-hand-side lanes per slot
 constexpr int kE = 3 * kR;                 // doubles per slot in a vector
-constexpr int kEnsUnroll = 4;              // entries in flight per lane (ens_row)
 
 // [bead][nrhs][3] (ensemble order) <-> [slot][8][3] (zero padded)
 __global__ void k_ens_to_slots(int64_t ntot, int nrhs, const int32_t *__restrict__ order_g,
@@ -79,20 +78,21 @@ __device__ __forceinline__ double f2d(float x) {
 }
 
 // the pair sum of one target and right-hand side over its stored rows
-// [e0, e1) (e0 a multiple of 8): U entries, their tensors and their sources'
-// forces are requested before the first is used, then added one by one
-// (every eighth into the compensated sums), so that a lane waits out one
+// [e0, e1) (e0 a multiple of 8): U = 4 entries, their tensors and their
+// sources' forces are requested before the first is used, then added one by
+// one (every eighth into the compensated sums), so that a lane waits out one
 // L2 round trip per U entries.  64 suspensions, 14 passes: 4.9 -> 4.4 ms per
-// step with rebuild at U = 4 (4.55 at U = 2; at 40 registers and 6 blocks per
-// SM, which beats 64 registers and 4 blocks).  NC: the forces are constant
-// during the kernel.
+// step with rebuild (4.55 at U = 2; at 40 registers and 6 blocks per SM, which
+// beats 64 registers and 4 blocks).  NC: the forces are constant during the
+// kernel.
 struct EnsSum {
   float h[3], l[3];
 };
 
-template <int U, bool NC>
+template <bool NC>
 __device__ __forceinline__ EnsSum ens_row(int64_t e0, int cnt, const uint32_t *__restrict__ list,
                                           const float4 *__restrict__ ten, const float4 *F, int r) {
+  constexpr int U = 4;
   float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
   float bx = 0.f, by = 0.f, bz = 0.f;
   auto add = [&](const float4 &t, const float4 &fj) {
@@ -113,17 +113,11 @@ __device__ __forceinline__ EnsSum ens_row(int64_t e0, int cnt, const uint32_t *_
   for (; m + U <= cnt; m += U) {
     uint32_t en[U];
     float4 t[U], fj[U];
-    if (U == 4) {
-      const uint4 q = __ldg(reinterpret_cast<const uint4 *>(lp + m));
-      en[0] = q.x;
-      en[1 % U] = q.y;
-      en[2 % U] = q.z;
-      en[3 % U] = q.w;
-    } else {
-      const uint2 q = __ldg(reinterpret_cast<const uint2 *>(lp + m));
-      en[0] = q.x;
-      en[1] = q.y;
-    }
+    const uint4 q4 = __ldg(reinterpret_cast<const uint4 *>(lp + m));
+    en[0] = q4.x;
+    en[1] = q4.y;
+    en[2] = q4.z;
+    en[3] = q4.w;
 #pragma unroll
     for (int q = 0; q < U; ++q) t[q] = __ldg(tp + m + q);
 #pragma unroll
@@ -168,7 +162,7 @@ __global__ void k_ens_pair(int64_t ntot, const int32_t *__restrict__ cnt, int W,
   const int64_t s = gid / kR;
   const int r = (int)(gid % kR);
   if (s >= ntot) return;  // 8 consecutive lanes share s: whole groups leave
-  const EnsSum v8 = ens_row<kEnsUnroll, true>(s * (int64_t)W, cnt[s], list, ten, f4, r);
+  const EnsSum v8 = ens_row<true>(s * (int64_t)W, cnt[s], list, ten, f4, r);
   const float *hs = v8.h, *ls = v8.l;
   const int64_t k0 = (s * kR + r) * 3;
   if (!TERM) {
@@ -414,7 +408,7 @@ __global__ void __launch_bounds__(NT, MINB) k_ens_series(SeriesArgs a) {
       // reads after every write another block released for the previous pass
       // (PTX memory model, message passing); L1 keeps the sources that
       // neighbouring targets share)
-      const EnsSum v8 = ens_row<kEnsUnroll, false>(s * (int64_t)a.W, __ldg(a.cnt + s), a.list,
+      const EnsSum v8 = ens_row<false>(s * (int64_t)a.W, __ldg(a.cnt + s), a.list,
                                                    a.ten, Fsrc, r);
       const float *hs = v8.h, *ls = v8.l;
       const int64_t k0 = (s * kR + r) * 3;
@@ -555,7 +549,7 @@ struct ggem_ensemble {
   double self_c = 0.0;
   bool built = false;
   int block = 256;  // threads per block of the pair kernels (autotuned)
-  DevBuf<int32_t> cnt, susp, order_g, rank_g;
+  DevBuf<int32_t> cnt, susp, order_g;
   DevBuf<uint32_t> list;
   DevBuf<float4> ten;
   DevBuf<int64_t> d_off;
@@ -867,7 +861,7 @@ extern "C" int ggem_ensemble_set_particles_dev(ggem_ensemble *e, const int64_t *
   const size_t nt = (size_t)e->ntot;
   const int32_t *counters = e->cell_count.p;
   if ((c = e->cnt.ensure(nt)) || (c = e->susp.ensure(nt)) || (c = e->order_g.ensure(nt)) ||
-      (c = e->rank_g.ensure(nt)) || (c = e->cell_of.ensure(nt)) || (c = e->wrapped.ensure(nt)) ||
+      (c = e->cell_of.ensure(nt)) || (c = e->wrapped.ensure(nt)) ||
       (c = e->pos64.ensure(nt)) || (c = e->pos32.ensure(nt)) || (c = e->xyz.ensure(3 * nt)) ||
       (c = e->cell_count.ensure(e->ncell)) || (c = e->cell_fill.ensure(e->ncell)) ||
       (c = e->cell_start.ensure(e->ncell + 1)))
@@ -884,7 +878,6 @@ extern "C" int ggem_ensemble_set_particles_dev(ggem_ensemble *e, const int64_t *
   B.cell_fill = e->cell_fill.p;
   B.cell_start = e->cell_start.p;
   B.order = e->order_g.p;
-  B.rank = e->rank_g.p;
   B.cnt = e->cnt.p;
   B.wrapped = e->wrapped.p;
   B.pos64 = e->pos64.p;

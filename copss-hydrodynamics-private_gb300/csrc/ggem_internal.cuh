@@ -422,7 +422,7 @@ struct BatchBuild {
   const int32_t *susp = nullptr;     // [ntot] suspension of every slot and of every bead
   const int32_t *cell_susp = nullptr;  // [ncell]
   int32_t *cell_of = nullptr, *cell_count = nullptr, *cell_fill = nullptr, *cell_start = nullptr;
-  int32_t *order = nullptr, *rank = nullptr, *cnt = nullptr;
+  int32_t *order = nullptr, *cnt = nullptr;
   double4_32a *wrapped = nullptr, *pos64 = nullptr;
   float4 *pos32 = nullptr;
   uint32_t *list = nullptr;

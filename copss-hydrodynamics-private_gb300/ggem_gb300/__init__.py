@@ -644,7 +644,7 @@ class Context:
 
     def autotune_pair_storage(self, reps=10, matvecs_per_build=12.0):
         """(use_stored, ms per matvec computed, ms per matvec stored incl. the
-        amortised tensor pass); the faster form and the fastest kernel shape
+        amortised first product); the faster form and the fastest kernel shape
         of each stay selected (``pair_variants``: computed, stored)"""
         u, a, b, v = C.c_int(), C.c_double(), C.c_double(), (C.c_int * 2)()
         self._check(lib().ggem_autotune_pair_storage(self.h, int(reps), float(matvecs_per_build),
