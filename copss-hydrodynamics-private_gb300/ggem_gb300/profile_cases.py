@@ -217,7 +217,14 @@ def all_kernels() -> None:
         run("ev forces", lambda: c.ev_gaussian_forces(0.37, 0.21))
         c.set_pair_tensors(True)
         c.build_cells()
-        run("stored", lambda: c.local_matvec(f))
+        run("stored", lambda: c.local_matvec(f))  # forms the tensors
+        run("stored again", lambda: c.local_matvec(f))
+        run("stored series", lambda: c.brownian_displacement(xi, 50, lo / 1.05, hi * 1.05, 1e-3,
+                                                             check_every=0))
+        c.set_pair_tensors(False)
+        c.set_symmetric_pairs(True)
+        c.build_cells()
+        run("symmetric", lambda: c.local_matvec(f))
         c.synchronize()
     # chains: spring forces
     cxyz, cL = G.make_chains(5, 500, 20)
@@ -227,15 +234,17 @@ def all_kernels() -> None:
         bonds = np.array([(20 * k + j, 20 * k + j + 1) for k in range(500) for j in range(19)])
         c.set_bonds(bonds)
         run("springs", lambda: c.spring_forces(G.SPRING_FENE, 1.0, 3.0))
-    # FP64 cut-off context: the cell sweep, the exact-list kernel, the field
-    # points, the per-point spread and element right-hand sides
+    # FP64 cut-off context: the cell sweep, the list and the series over it,
+    # the field points, the per-point spread and element right-hand sides
     with G.Context(box_hi=(L,) * 3, rc=7.0, precision=G.FP64) as c:
+        c.set_fp64_pair_list(False)
         c.set_particles(xyz)
         c.build_cells()
         run("fp64 sweep", lambda: c.local_matvec(f))
         c.set_fp64_pair_list(True)
         c.build_cells()
         run("fp64 list", lambda: c.local_matvec(f))
+        run("fp64 series", lambda: c.cheb_inv_sqrt(xi, 50, lo / 1.05, hi * 1.05, 1e-3))
         t = rng.uniform(0, L, (20000, 3))
         run("field", lambda: c.local_field(t, f))
         run("spread qp", lambda: c.spread_qp(t, f, spread_rc=8.0))
@@ -272,8 +281,8 @@ def all_kernels() -> None:
     X = rng.standard_normal((512, G.SUR_FEATURES)).astype(np.float32)
     Y = rng.standard_normal((512, G.SUR_OUTPUTS)).astype(np.float32)
     run("predict", lambda: sur.predict(X))
+    run("predict by layers", lambda: sur.predict_layers(X))
     run("train", lambda: sur.train(X, Y, 1, batch=256))
-    sur.close()
     # a small ensemble, both step forms
     K = 8
     sus = [G.make_suspension(100 + b, 2000 + 500 * b, 0.1) for b in range(K)]
@@ -281,6 +290,8 @@ def all_kernels() -> None:
     d_xyz = torch.from_numpy(np.concatenate([x for x, _ in sus]).reshape(-1)).cuda()
     e.set_particles_dev([len(x) for x, _ in sus], d_xyz.data_ptr())
     beads, _ = e.sizes()
+    run("intervals", lambda: e.intervals(sur))
+    sur.close()
     lz = [e.lanczos(b, 24, 7) for b in range(K)]
     elo = np.array([x[0] for x in lz]) / 1.05
     ehi = np.array([x[1] for x in lz]) * 1.05
