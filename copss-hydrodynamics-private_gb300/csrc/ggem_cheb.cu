@@ -647,7 +647,7 @@ int ensure_cheb_buffers(ggem_ctx *c, size_t len) {
 constexpr int kRestartCheb = 1;
 
 // Chebyshev on xi (caller order, device; left unchanged); leaves y in c->w_y
-// (slot order).
+// (slot order), unless the series ran as one launch (*out_done, see out).
 //
 // check_every = 1: the reference's loop (brownian_system.C:1089-1155): the
 //   error-check matvec dw_mid = M dw and both estimators every term.

@@ -5,9 +5,10 @@
 // by another allocator (a framework's caching pool or a solver's own
 // arena), they run where an allocation would block or is not allowed (a
 // solver callback, a real-time loop), or their build budgets device memory
-// statically.  ggem_local_matvec_noalloc serves them: it runs the FP64
-// cut-off cell-list pair sweep (the same arithmetic as the context path of
-// ggem_local_matvec_dev with GGEM_FP64) with all of its scratch -- cell
+// statically.  ggem_local_matvec_noalloc serves them: it runs an FP64
+// cut-off cell-list pair sweep (the operator of ggem_local_matvec_dev with
+// GGEM_FP64, which keeps a pair list and the tensor's pieces in memory; here
+// erf and exp per pair, equal to rounding) with all of its scratch -- cell
 // counts, the sorted cell list and slot-ordered copies of positions and
 // forces -- in one fixed device array declared in this file.  Nothing is
 // allocated, on the device or the host.

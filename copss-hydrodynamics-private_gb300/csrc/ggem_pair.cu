@@ -409,9 +409,9 @@ __device__ __forceinline__ int64_t block_target_by_length(int64_t n, const int32
 // Measured there: 0.42 ms; 0.45 ms with the box-face additions for every
 // pair, 0.50 ms also with the targets in slot order (lanes idle at the ends
 // of uneven rows), 2.85 ms also with erf and exp per pair; the cell
-// sweep takes 4.8 ms, 15.0 ms with erf and exp.  The tensors themselves are closer to the exact ones than
-// the formula's: 1.2e-16 of u from their rounding against 3.8e-16 (N = 400,
-// 30-digit reference), since the closed form cancels.
+// sweep takes 4.8 ms, 15.0 ms with erf and exp.  u is closer to 34 digits
+// than with the formula, which cancels (N = 500, norm-wise): 3.0e-16 against
+// 5.5e-16 at alpha = 0.5, 1.1e-16 against 2.2e-16 at 0.1.
 template <int NR, int G>
 __global__ void __launch_bounds__(256) k_pair_list_f64(int64_t n, MinImage mi, DevConsts K,
                                                        Tensor64 T, long long eps2,
@@ -2139,9 +2139,11 @@ int launch_f64(ggem_ctx *c, const double *f, double *u, int self_mode, int r0) {
     // lanes per target: four fill the FP64 pipe from ~80k targets on (fewer
     // lanes would idle in rows of ~35 entries of uneven length); smaller
     // counts need more lanes to cover the latency of a row walk.  us per
-    // application with 4 / 8 / 16 / 32 lanes, phi = 0.1: N = 1000 (phi 0.05)
-    // 21 / 15 / 13 / 11, 4000 33 / 21 / 23 / 29, 12000 58 / 48 / 46 / 63,
-    // 60000 173 / 171 / 199 / 269, 200000 499 / 528 / 637 / 866
+    // kernel with 4 / 8 / 16 / 32 lanes, phi = 0.1: N = 1000 (phi 0.05) 20 / 14
+    // / 12 / 10, 2000 31 / 19 / 14 / 18, 4000 31 / 20 / 22 / 29, 12000 50 / 42 /
+    // 46 / 60, 40000 110 / 108 / 125 / 174, 80000 189 / 197 / 236 / 334, 200000
+    // 426 / 464 / 570 / 813; element lists of 1000 47 / 28 / 19 / 14, of 20000
+    // 129 / 111 / 110 / 131
     if (c->n >= 80000) launch_list_f64<NR, 4>(c, f, u, self_mode, r0, eps2);
     else if (c->n >= 2500) launch_list_f64<NR, 8>(c, f, u, self_mode, r0, eps2);
     else launch_list_f64<NR, 32>(c, f, u, self_mode, r0, eps2);
@@ -2676,9 +2678,10 @@ double self_coefficient(const ggem_ctx *c, int self_mode) {
 }
 
 // The whole FP64 series of one right-hand side (k_series_f64): xi and out in
-// caller order, y left in w_y.  *done = false: not taken (no pair list, the
-// kernel timer or the launch trace wants the single launches, a deferred
-// list build to be checked first, or no cooperative launch).
+// caller order (y stays in the series' own records).  *done = false: not taken
+// (no pair list, the kernel timer or the launch trace wants the single
+// launches, a deferred list build to be checked first, or no cooperative
+// launch).
 int series_f64(ggem_ctx *c, int N, const double *coef, double da, double db, double tol,
                int check_every, int k_first, int self_mode, const double *xi, double *out,
                bool out_y, ggem_cheb_report *rep, int *first_check, bool *done) {
@@ -2735,6 +2738,15 @@ int series_f64(ggem_ctx *c, int N, const double *coef, double da, double db, dou
   a.dm = c->w_out.p;
   a.out = out;
   a.ctl = reinterpret_cast<SeriesCtl *>(c->s64_tab.p);
+  // the cached tensors wherever every target is resident, then lanes per
+  // target as for single products.  us per step, with its host copies, of <16,
+  // 4> / <8, 4> / <32, 4> / <16, 2> / <16, 6> / <16, 0> / <8, 0>: N = 1000, phi =
+  // 0.05 117 / 124 / 134 / 117 / 119 / 143 / 179, N = 1500, phi = 0.1 180 / 192
+  // / 203 / 196 / 180 / 258 / 270, N = 3600, phi = 0.1 221 / 253 / 577 / 253 /
+  // 228 / 329 / 352.  Of <4, 0> / <8, 0> / <16, 0> / <16, 4> at phi = 0.1: N =
+  // 4000 417 / 351 / 399 / 513, 17000 935 / 897 / 1021 / 1209, 40000 2007 / 1941
+  // / 2212 / 2390, 80000 3516 / 3531 / 4147 / 4467, 200000 7799 / 8067 / 9511 /
+  // 11107
   int rc = launch_series_f64<16, 4>(c, a, 1, done);
   if (!rc && !*done) {
     if (c->n >= 80000) rc = launch_series_f64<4, 0>(c, a, 1 << 30, done);

@@ -80,7 +80,9 @@ int ggem_set_pair_variant(ggem_ctx *ctx, int computed, int stored);
 int ggem_probe_fp32_peak(ggem_ctx *ctx, double *tflops);
 /* kernel timing: when enabled, CUDA events on the context's stream bracket
  * every launch of the kernels below; totals are read back (with a stream
- * synchronisation) by ggem_get_kernel_timing.  Enabling resets the totals. */
+ * synchronisation) by ggem_get_kernel_timing.  Enabling resets the totals.
+ * A timed (or traced) context runs an FP64 series, otherwise one launch, as
+ * its single launches, which take longer. */
 #define GGEM_KERNEL_PAIR_FP32 0  /* FP32 pair-list sum                        */
 #define GGEM_KERNEL_PAIR_FP64 1  /* FP64 pair sum (cell sweep or pair list)   */
 #define GGEM_KERNEL_CHEB_TERM 2  /* fused Chebyshev term                       */

@@ -5,12 +5,13 @@
  * The reference runs one suspension per COPSS job (Copss::fixman_integrate,
  * copss.C:1560-1686, with its own GGEMStokes, PointMesh and BrownianSystem).
  * An ensemble holds K periodic suspensions with their own boxes and bead
- * counts: each is built as an ordinary context (cell list, pair list,
- * stored pair tensors), and their lists are concatenated into one
- * block-diagonal operator, so that a matvec or a Chebyshev term of all K
- * suspensions and up to 8 right-hand sides each is a single kernel launch.
- * The unchecked stretch of Chebyshev terms is captured once as a CUDA graph
- * and replayed.  Every series keeps its own eigen interval, coefficients,
+ * counts.  Their cells and slots are concatenated and one build, a launch
+ * per phase, makes the cell lists, pair lists and pair tensors of all of
+ * them as one block-diagonal operator, so that a matvec or a Chebyshev term
+ * of all K suspensions and up to 8 right-hand sides each is a single kernel
+ * launch.  A whole step of all series runs as one persistent launch, or as
+ * one launch per term with the unchecked stretch captured once as a CUDA
+ * graph (ggem_ensemble_set_series_mode).  Every series keeps its own eigen interval, coefficients,
  * error estimators and stopping decision (brownian_system.C:967-1178).
  *
  * Vector layout: [bead][rhs][3] float64, beads in ensemble order (the K
@@ -42,7 +43,7 @@ const char *ggem_ensemble_last_error(const ggem_ensemble *e);
 
 /* positions of all suspensions (device, [sum n][3], ensemble order) with
  * n[b] beads in suspension b: cell lists, pair lists and pair tensors of
- * every suspension, then the concatenated operator */
+ * all suspensions in one build */
 int ggem_ensemble_set_particles_dev(ggem_ensemble *e, const int64_t *n, const double *d_xyz);
 /* total beads and ordered in-cutoff pairs of the current configuration */
 int ggem_ensemble_sizes(const ggem_ensemble *e, int64_t *beads, int64_t *pairs);

@@ -9,9 +9,10 @@
  * that budget device memory statically.  Those callers cannot create a
  * ggem_ctx, which allocates its cell lists and workspaces.
  *
- * ggem_local_matvec_noalloc computes the same u = M_loc f as
- * ggem_local_matvec_dev on a GGEM_FP64 / GGEM_NB_CUTOFF context (the FP64
- * cut-off cell-list pair sweep plus the chosen self term), but keeps every
+ * ggem_local_matvec_noalloc computes the u = M_loc f of
+ * ggem_local_matvec_dev on a GGEM_FP64 / GGEM_NB_CUTOFF context, equal to
+ * rounding (a cut-off cell-list pair sweep with erf and exp per pair instead
+ * of a pair list and fitted tensors), plus the chosen self term, but keeps every
  * intermediate array in one fixed device array of GGEM_NOALLOC_SCRATCH_BYTES
  * (2.5 MiB) compiled into the library.  Every GPU that loads the library
  * holds that array until the process exits.
