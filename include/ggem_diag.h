@@ -47,7 +47,9 @@ int ggem_set_pair_tensors(ggem_ctx *ctx, int enable);
  * cells around every bead.  Takes effect at the next ggem_build_cells.
  * Without this call the context builds the list itself for the
  * configurations that the operator is applied to, where it takes at most a
- * quarter of the free device memory. */
+ * quarter of the free device memory, cells are no longer than 64 cut-offs
+ * and at most 2^21 or 8 per particle; products under stream capture sweep
+ * the cells. */
 int ggem_set_fp64_pair_list(ggem_ctx *ctx, int enable);
 /* test hook: polls of each wait of the one-launch FP64 series (0 = the
  * default); a wait that runs out ends the series with GGEM_ERR_TIMEOUT */
