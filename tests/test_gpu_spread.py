@@ -243,3 +243,40 @@ def test_fp32_spread_lanes_per_point(p, members, nm):
         want, got = ctx.spread_elements(f, G.FP64), ctx.spread_elements(f, G.FP32)
         assert np.array_equal(got, ctx.spread_elements(f, G.FP32))
     assert rel(got, want) <= 1e-6
+
+
+@pytest.mark.parametrize("prec", [G.FP64, G.FP32])
+def test_captured_spread_follows_rebuilds(prec):
+    """a caller's graph of the spread reads the context's stencil bitmap,
+    which was sent up before, and the cells of the configuration at replay"""
+    import torch
+    nm, h, n = 20, 1.4, 700
+    L = nm * h
+    rng = np.random.default_rng(8)
+    q, nq = _grid_points((0, 0, 0), (L,) * 3, (nm,) * 3, (2, 2, 2), (0, 1, 2))
+    f = torch.from_numpy(rng.standard_normal((n, 3))).cuda()
+    rho = torch.zeros((len(q), 3), dtype=torch.float64, device="cuda")
+    st = torch.cuda.Stream()
+    with G.Context(alpha=ALPHA, box_hi=(L,) * 3, nb_mode=G.NB_REFERENCE, n_mesh=(nm,) * 3,
+                   search_radius_e=0.5 * h + 8.0 + 1e-3, precision=G.FP64) as ctx:
+        ctx.set_stream(st.cuda_stream)
+        torch.cuda.synchronize()
+        ctx.set_particles(rng.uniform(0, L, (n, 3)))
+        ctx.build_cells()
+        ctx.set_quadrature(q, nq)
+        ctx.spread_elements_dev(f.data_ptr(), rho.data_ptr(), prec)
+        ctx.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            ctx.spread_elements_dev(f.data_ptr(), rho.data_ptr(), prec)
+        for _ in range(2):
+            ctx.set_particles(rng.uniform(0, L, (n, 3)))
+            ctx.build_cells()
+            ctx.spread_elements_dev(f.data_ptr(), rho.data_ptr(), prec)
+            ctx.synchronize()
+            live = rho.clone()
+            rho.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(rho, live) and float(live.abs().max()) > 0.0
+        ctx.set_stream(0)
